@@ -40,8 +40,8 @@ constexpr uint32_t kNaMaxBig = 1u << 13;        // large triangles (more than 32
 constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
 // layout of the arena (byte offsets)
-constexpr size_t kOffScene = 0;
-constexpr size_t kOffCtr = align256(kOffScene + sizeof(RasterSceneDev));
+constexpr size_t kOffWork = 0;
+constexpr size_t kOffCtr = align256(kOffWork + sizeof(BinWork));
 constexpr size_t kOffSetup = align256(kOffCtr + sizeof(FrameCounters));
 constexpr size_t kOffLargeSeg = align256(kOffSetup + sizeof(TriSetup) * kNaMaxTris);
 constexpr size_t kOffLargeWalk = align256(kOffLargeSeg + sizeof(uint2) * kNaMaxSegs);
@@ -106,22 +106,18 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
   if (arena_for_device(dev, &base, &ctas) != cudaSuccess) return PIKO_ERR_CUDA;
   cudaStream_t st = (cudaStream_t)stream;
 
-  RasterSceneDev sd;
-  scene_dev_geometry(sd, width, height, count, (int)kNaTile);
-  sd.input_kind = kInputWtri;
-  sd.wtri_xyz = d_xyz; sd.wtri_icol = d_icol;
-  sd.fb = d_rgba; sd.depth = d_depth;
-
   // the arena keeps the previous call's contents: zero what must start at zero
-  if (cudaMemcpyAsync(base + kOffScene, &sd, sizeof(sd), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemsetAsync(base + kOffCtr, 0, sizeof(FrameCounters), st) != cudaSuccess ||
+  if (cudaMemsetAsync(base + kOffWork, 0, sizeof(BinWork), st) != cudaSuccess ||
       cudaMemsetAsync(base + kOffCnt, 0, sizeof(uint32_t) * n_tiles, st) != cudaSuccess ||
       cudaMemsetAsync(base + kOffFlags, 0, sizeof(unsigned long long) * kNaScanBlocks, st) != cudaSuccess)
     return PIKO_ERR_CUDA;
 
   RasterFrameArgs a;
   memset(&a, 0, sizeof(a));
-  a.scenes = reinterpret_cast<const RasterSceneDev*>(base + kOffScene);
+  scene_dev_geometry(a.one, width, height, count, (int)kNaTile);
+  a.one.input_kind = kInputWtri;
+  a.one.wtri_xyz = d_xyz; a.one.wtri_icol = d_icol;
+  a.one.fb = d_rgba; a.one.depth = d_depth;
   a.n_scenes = 1;
   a.tile = (int)kNaTile;
   a.n_tris_total = (uint32_t)count;
@@ -141,6 +137,7 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
   a.large_walk = reinterpret_cast<WalkTri*>(base + kOffLargeWalk);
   a.big_cap = kNaMaxBig;
   a.scan_flags = reinterpret_cast<unsigned long long*>(base + kOffFlags);
+  a.work = reinterpret_cast<BinWork*>(base + kOffWork);
   a.ctr = reinterpret_cast<FrameCounters*>(base + kOffCtr);
   if (launch_raster_frame(a, ctas, st, nullptr) != cudaSuccess) return PIKO_ERR_CUDA;
 
@@ -150,7 +147,7 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
   if (cudaMemcpyAsync(&c, base + kOffCtr, sizeof(c), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return PIKO_ERR_CUDA;
-  if (c.status & kStatusScanTimeout) return PIKO_ERR_TIMEOUT;
-  if (c.status & kStatusListOverflow) return PIKO_ERR_QUEUE_OVERFLOW;
+  if (c.bin.status & kStatusScanTimeout) return PIKO_ERR_TIMEOUT;
+  if (c.bin.status & kStatusListOverflow) return PIKO_ERR_QUEUE_OVERFLOW;
   return PIKO_OK;
 }

@@ -172,28 +172,45 @@ static_assert(sizeof(TriSetup) == 80, "TriSetup layout");
 
 constexpr uint32_t kTriRisk = 1u;
 
-// Per-frame counters (zeroed before each frame).  The heavy-tile queue and the
-// large-triangle queue each reserve slots and work-item ranges with one 64-bit
-// atomic, so that slot order and item order agree and an item's slot can be
-// found by a search over the slots' first items.
+// What the binning passes (setup, large count, scan) count.  The heavy-tile
+// queue and the large-triangle queue each reserve slots and work-item ranges
+// with one 64-bit atomic, so that slot order and item order agree and an item's
+// slot can be found by a search over the slots' first items.
 constexpr uint32_t kPairParts = 128;
-struct FrameCounters {
+struct BinCounts {
   uint32_t status;
-  uint32_t scan_ticket;
-  uint32_t work_next;
   uint32_t list_total;
   uint32_t kept;
-  uint32_t cov_count;
-  unsigned long long covered;
+  uint32_t pair_part_max;        // largest partition fill asked for (past its capacity: overflow)
   unsigned long long risk;
   unsigned long long heavy_acc;  // heavy tiles << 32 | 8x8 list chunks
   unsigned long long large_acc;  // large triangles << 32 | their box-tile segments
+};
+
+// A frame's result: the binning counts as the scatter pass found them, and what
+// the fragment kernel counts (started at 0 by the scatter pass).
+struct FrameCounters {
+  BinCounts bin;
+  unsigned long long covered;
+  uint32_t work_next;
+  uint32_t cov_count;
+};
+
+// Per-frame working counters.  No launch clears them before a frame (the
+// scene-record copy and three memsets that used to precede the setup kernel
+// took 15 us of a frame, a fifth of the 1080p forest's): they are zero between
+// frames because a later kernel of the frame sets back what an earlier one
+// used -- raster_scatter the counts and the scan's flags, the fragment kernels
+// the pair partitions, scan_tiles the tile counters it has read.  The host
+// clears them when they are allocated and after a launch that failed.
+struct BinWork {
+  BinCounts bin;
+  uint32_t scan_ticket;
+  uint32_t pad[3];
   // The count passes record their (triangle, tile) pairs in kPairParts
   // partitions of list_cap / kPairParts slots each (a warp takes partition
   // (its global warp index) mod kPairParts), so that slot reservations spread
   // over kPairParts counters instead of queueing on one address.
-  uint32_t pair_part_max;        // largest partition fill asked for (past its capacity: overflow)
-  uint32_t pad[3];
   uint32_t pair_part[kPairParts];
 };
 
@@ -217,7 +234,8 @@ struct __align__(16) WalkTri {
 static_assert(sizeof(WalkTri) == 112, "WalkTri layout");
 
 struct RasterFrameArgs {
-  const RasterSceneDev* scenes;
+  RasterSceneDev one;       // the scene of a one-scene frame: it travels with the launch, no copy precedes the frame
+  const RasterSceneDev* scenes;  // [n_scenes] when there are several
   int n_scenes;
   int tile;                 // tile edge in pixels: 8, 16 or 32
   uint32_t n_tris_total;    // sum of N
@@ -253,9 +271,11 @@ struct RasterFrameArgs {
   uint32_t* hdone;          // [heavy_cap] chunks finished
   unsigned long long* chunk_keys;  // [chunk_cap][tile * tile]
   uint32_t chunk_cap;
-  unsigned long long* scan_flags;  // per scan block, epoch-tagged
-  uint32_t epoch;
+  unsigned long long* scan_flags;  // per scan block
+  BinWork* work;
   FrameCounters* ctr;
+  BinCounts* host_bin;      // pinned host memory (or null): the fragment kernel leaves ctr->bin there, so that
+                            // checking a frame takes no copy
   // coverage dump (parity tests): one (triangle id, pixel index) record per
   // covered sample, appended in any order; counted in ctr->cov_count
   uint32_t* cov_tri;

@@ -48,6 +48,17 @@ constexpr uint32_t kLargeTiles = 32;  // box tiles above which a triangle's walk
 constexpr uint32_t kLargeSeg = 128;   // box tiles per work item of the large-triangle walk
 
 // ------------------------------------------------------------------ helpers
+// Scene s of the frame.  The kernels that read scene records exist for one
+// scene (ONE: its record is a kernel argument, read as constants; reading it
+// through a pointer that could be either cost raster_setup 6 us of 21 on the
+// 1080p forest) and for several (a table in global memory).
+template <bool ONE>
+__device__ __forceinline__ const RasterSceneDev& scene_at(const RasterFrameArgs& a, int s)
+{
+  if constexpr (ONE) return a.one;
+  else return a.scenes[s];
+}
+
 template <class S>
 __device__ __forceinline__ int find_base(const S* sc, int n, uint32_t g, bool by_tile)
 {
@@ -64,15 +75,16 @@ __device__ __forceinline__ int find_base(const S* sc, int n, uint32_t g, bool by
 // CAP scenes; larger ones search the scene records), so that finding a
 // triangle's or a tile's scene is a shared-memory search.
 constexpr int kSceneTable = 1024;
-template <int CAP>
+template <bool ONE, int CAP>
 __device__ __forceinline__ void load_scene_table(const RasterFrameArgs& a, uint32_t* tb, bool by_tile)
 {
-  if (a.n_scenes > CAP) return;
+  if (ONE || a.n_scenes > CAP) return;
   for (int i = threadIdx.x; i < a.n_scenes; i += blockDim.x) tb[i] = by_tile ? a.scenes[i].tile_base : a.scenes[i].tri_base;
 }
-template <int CAP>
+template <bool ONE, int CAP>
 __device__ __forceinline__ int scene_of(const RasterFrameArgs& a, const uint32_t* tb, uint32_t x, bool by_tile)
 {
+  if (ONE) return 0;
   if (a.n_scenes > CAP) return find_base(a.scenes, a.n_scenes, x, by_tile);
   int lo = 0, hi = a.n_scenes - 1;
   while (lo < hi) {
@@ -81,9 +93,10 @@ __device__ __forceinline__ int scene_of(const RasterFrameArgs& a, const uint32_t
   }
   return lo;
 }
+template <bool ONE>
 __device__ __forceinline__ int scene_of_tile(const RasterFrameArgs& a, const uint32_t* tb, uint32_t tile)
 {
-  return scene_of<kSceneTable>(a, tb, tile, true);
+  return scene_of<ONE, kSceneTable>(a, tb, tile, true);
 }
 
 // The last index i in [0, n) with base[i] <= x, for an ascending base with
@@ -233,11 +246,11 @@ __device__ __forceinline__ void count_pairs(const RasterFrameArgs& a, const uint
   const uint32_t part_cap = a.list_cap / kPairParts;
   uint32_t base = 0;
   if (lane == 0) {
-    base = atomicAdd(&a.ctr->pair_part[part], n);
+    base = atomicAdd(&a.work->pair_part[part], n);
     if (base + n > part_cap) {
       // the host grows the lists so that every partition fits, and draws again
-      atomicMax(&a.ctr->pair_part_max, base + n);
-      atomicOr(&a.ctr->status, kStatusListOverflow);
+      atomicMax(&a.work->bin.pair_part_max, base + n);
+      atomicOr(&a.work->bin.status, kStatusListOverflow);
     }
   }
   base = __shfl_sync(kFull, base, 0);
@@ -259,10 +272,20 @@ __device__ __forceinline__ void count_pairs(const RasterFrameArgs& a, const uint
 // A frame whose pairs overran the list buffers is drawn again with larger
 // ones; its tile lists have entries that no pair filled (a pair counted in
 // tile_cnt but past list_cap has no record), so the fragment kernels must not
-// read them.  The status is final once the scan has run.
+// read them.  The status is final once the scan has run; the scatter pass
+// copies it to the frame's result.
 __device__ __forceinline__ bool list_overflowed(const RasterFrameArgs& a)
 {
-  return (*(volatile uint32_t*)&a.ctr->status & kStatusListOverflow) != 0;
+  return (a.ctr->bin.status & kStatusListOverflow) != 0;
+}
+
+// First thing a fragment kernel does: the pair partitions, which the scatter
+// pass has read, go back to 0, and the binning counts go to the host.
+__device__ __forceinline__ void frame_begin(const RasterFrameArgs& a)
+{
+  if (blockIdx.x != 0) return;
+  if (threadIdx.x < kPairParts) a.work->pair_part[threadIdx.x] = 0u;
+  if (threadIdx.x == 0 && a.host_bin) *a.host_bin = a.ctr->bin;
 }
 
 // Walks every (triangle, tile) pair of a warp's 32 triangles with all 32 lanes
@@ -357,13 +380,14 @@ __device__ __forceinline__ float4 load_attr3(const float4* a4, const float* a3, 
 // 128-thread CTAs: one wave holds the scene's triangle blocks spread nearly
 // evenly over the SMs.
 constexpr int kSetupThreads = 128;
-__global__ void __launch_bounds__(kSetupThreads) raster_setup(RasterFrameArgs a)
+template <bool ONE>
+__global__ void __launch_bounds__(kSetupThreads) raster_setup(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_trigger();
   __shared__ WalkTri s_walk[kSetupThreads];
   __shared__ unsigned s_kept[kSetupThreads / 32], s_risk[kSetupThreads / 32];
   __shared__ uint32_t s_tb[kSceneTable];
-  load_scene_table<kSceneTable>(a, s_tb, false);
+  load_scene_table<ONE, kSceneTable>(a, s_tb, false);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   unsigned nk = 0, nr = 0;
@@ -374,8 +398,8 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(RasterFrameArgs a)
   uint32_t ntiles = 0;
   bool kept_flag = false, risk_flag = false;
   if (g < a.n_tris_total) {
-    const int s = scene_of<kSceneTable>(a, s_tb, g, false);
-    const RasterSceneDev& S = a.scenes[s];
+    const int s = scene_of<ONE, kSceneTable>(a, s_tb, g, false);
+    const RasterSceneDev& S = scene_at<ONE>(a, s);
     const uint32_t id = g - S.tri_base;
     float sx[3], sy[3], sz[3];
     uint32_t ic[3] = {0u, 0u, 0u};
@@ -527,7 +551,7 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(RasterFrameArgs a)
       if (lane >= o) incl += t;
     }
     unsigned long long old = 0;
-    if (lane == 31) old = atomicAdd(&a.ctr->large_acc, ((unsigned long long)__popc(big) << 32) | incl);
+    if (lane == 31) old = atomicAdd(&a.work->bin.large_acc, ((unsigned long long)__popc(big) << 32) | incl);
     old = __shfl_sync(kFull, old, 31);
     if (is_big) {
       // the triangle's walk record, then one (large triangle, segment) item
@@ -539,10 +563,10 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(RasterFrameArgs a)
         a.large_walk[bi] = s_walk[threadIdx.x];
         for (uint32_t k = 0; k < nseg; ++k) {
           if (first + k < a.seg_cap) a.large_seg[first + k] = make_uint2(bi, k);
-          else { atomicOr(&a.ctr->status, kStatusListOverflow); break; }
+          else { atomicOr(&a.work->bin.status, kStatusListOverflow); break; }
         }
       } else {
-        atomicOr(&a.ctr->status, kStatusListOverflow);
+        atomicOr(&a.work->bin.status, kStatusListOverflow);
       }
       ntiles = 0;
     }
@@ -563,16 +587,17 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(RasterFrameArgs a)
     unsigned k = 0, rr = 0;
 #pragma unroll
     for (int w = 0; w < kSetupThreads / 32; ++w) { k += s_kept[w]; rr += s_risk[w]; }
-    if (k) atomicAdd(&a.ctr->kept, k);
-    if (rr) atomicAdd(&a.ctr->risk, (unsigned long long)rr);
+    if (k) atomicAdd(&a.work->bin.kept, k);
+    if (rr) atomicAdd(&a.work->bin.risk, (unsigned long long)rr);
   }
 }
 
 // ------------------------------------------------------------------ kernel 2
-// Exclusive scan of tile_cnt (decoupled look-back).  Flags per block hold
-// (epoch << 34) | (state << 32) | value, state 1 = aggregate, 2 = inclusive.
+// Exclusive scan of tile_cnt (decoupled look-back); the counters are set back
+// to 0 as they are read.  Flags per block hold (state << 32) | value, state
+// 1 = aggregate, 2 = inclusive.
 
-__global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
+__global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_wait();
   pdl_trigger();
@@ -580,7 +605,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
   __shared__ uint32_t s_warp[kScanThreads / 32];
   __shared__ uint32_t s_prefix;
   __shared__ unsigned long long s_heavy[kScanThreads / 32];   // per warp: (heavy tiles << 32) | chunks
-  if (threadIdx.x == 0) s_bid = atomicAdd(&a.ctr->scan_ticket, 1u);
+  if (threadIdx.x == 0) s_bid = atomicAdd(&a.work->scan_ticket, 1u);
   __syncthreads();
   const uint32_t bid = s_bid;
   const uint32_t n = a.n_tiles_total;
@@ -590,6 +615,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     v[i] = (base + i < n) ? a.tile_cnt[base + i] : 0u;
+    if (v[i]) a.tile_cnt[base + i] = 0u;
     sum += v[i];
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -628,7 +654,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
     unsigned long long tot = 0;
 #pragma unroll
     for (int w = 0; w < kScanThreads / 32; ++w) tot += s_heavy[w];
-    unsigned long long run_h = tot ? atomicAdd(&a.ctr->heavy_acc, tot) : 0ull;
+    unsigned long long run_h = tot ? atomicAdd(&a.work->bin.heavy_acc, tot) : 0ull;
 #pragma unroll
     for (int w = 0; w < kScanThreads / 32; ++w) {
       const unsigned long long cnt = s_heavy[w];
@@ -642,16 +668,15 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
     if (w < warp) warp_excl += s_warp[w];
     agg += s_warp[w];
   }
-  const unsigned long long ep = (unsigned long long)a.epoch << 34;
   if (warp == 0) {
     // Look-back by the whole warp: lane j reads the flag of block
     // (end - j), so 32 predecessors are examined per step.  The window is
     // summed once every lane up to the nearest inclusive prefix is published.
     uint32_t prefix = 0;
     if (bid == 0) {
-      if (lane == 0) atomicExch(&a.scan_flags[0], ep | (2ull << 32) | agg);
+      if (lane == 0) atomicExch(&a.scan_flags[0], (2ull << 32) | agg);
     } else {
-      if (lane == 0) atomicExch(&a.scan_flags[bid], ep | (1ull << 32) | agg);
+      if (lane == 0) atomicExch(&a.scan_flags[bid], (1ull << 32) | agg);
       int end = (int)bid - 1;
       uint32_t spins = 0;
       for (;;) {
@@ -659,7 +684,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
         uint32_t state = 2, val = 0;  // lanes before block 0 read as an inclusive 0
         if (idx >= 0) {
           const unsigned long long f = __ldcv(&a.scan_flags[idx]);
-          state = (f >> 34) == a.epoch ? (uint32_t)(f >> 32) & 3u : 0u;
+          state = (uint32_t)(f >> 32) & 3u;
           val = (uint32_t)f;
         }
         const unsigned pending = __ballot_sync(kFull, state == 0);
@@ -668,7 +693,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
         const unsigned need = first == 31 ? kFull : ((2u << first) - 1u);
         if (pending & need) {
           if (++spins > (1u << 22)) {
-            if (lane == 0) atomicOr(&a.ctr->status, kStatusScanTimeout);
+            if (lane == 0) atomicOr(&a.work->bin.status, kStatusScanTimeout);
             break;
           }
           __nanosleep(32);
@@ -678,7 +703,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
         if (inclusive) break;
         end -= 32;
       }
-      if (lane == 0) atomicExch(&a.scan_flags[bid], ep | (2ull << 32) | (uint32_t)(prefix + agg));
+      if (lane == 0) atomicExch(&a.scan_flags[bid], (2ull << 32) | (uint32_t)(prefix + agg));
     }
     if (lane == 0) s_prefix = prefix;
   }
@@ -704,10 +729,10 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
             for (uint32_t j = 0; j < nch && c + j < a.chunk_cap; ++j) a.chunk_heavy[c + j] = h;
             c += nch;
             // chunks past the key buffers are not rasterized: report it
-            if (c > a.chunk_cap) atomicOr(&a.ctr->status, kStatusListOverflow);
+            if (c > a.chunk_cap) atomicOr(&a.work->bin.status, kStatusListOverflow);
           }
         } else {
-          atomicOr(&a.ctr->status, kStatusListOverflow);
+          atomicOr(&a.work->bin.status, kStatusListOverflow);
         }
         ++h;
       }
@@ -717,8 +742,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(RasterFrameArgs a)
   if (base < n && base + kScanItems >= n) {
     // the thread holding the last element publishes the total
     a.tile_off[n] = run;
-    a.ctr->list_total = run;
-    if (run > a.list_cap) atomicOr(&a.ctr->status, kStatusListOverflow);
+    a.work->bin.list_total = run;
+    if (run > a.list_cap) atomicOr(&a.work->bin.status, kStatusListOverflow);
   }
 }
 
@@ -756,11 +781,11 @@ __device__ __forceinline__ void large_segment(const RasterFrameArgs& a, uint32_t
 }
 
 // The count pass of the large triangles' segments.
-__global__ void __launch_bounds__(256, 4) raster_large_count(RasterFrameArgs a)
+__global__ void __launch_bounds__(256, 4) raster_large_count(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_wait();
   pdl_trigger();
-  const uint32_t items = min((uint32_t)a.ctr->large_acc, a.seg_cap);
+  const uint32_t items = min((uint32_t)a.work->bin.large_acc, a.seg_cap);
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items; it += warps)
     large_segment(a, it, threadIdx.x & 31);
@@ -769,15 +794,28 @@ __global__ void __launch_bounds__(256, 4) raster_large_count(RasterFrameArgs a)
 // The scatter pass (the compaction): every recorded pair becomes its list
 // entry at tile_off[tile] + its index in the tile, a streaming pass with no
 // atomics; four pairs per thread per trip, loads first.
-__global__ void __launch_bounds__(256) raster_scatter(RasterFrameArgs a)
+__global__ void __launch_bounds__(256) raster_scatter(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_wait();
   pdl_trigger();
+  // the counts are final: they become the frame's result, and the next frame
+  // finds the working counters and the scan's flags at 0
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.ctr->bin = a.work->bin;
+    a.ctr->covered = 0ull;
+    a.ctr->work_next = 0u;
+    a.ctr->cov_count = 0u;
+    a.work->bin = BinCounts{};
+    a.work->scan_ticket = 0u;
+  }
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (a.n_tiles_total + kScanTile - 1) / kScanTile;
+       i += gridDim.x * blockDim.x)
+    a.scan_flags[i] = 0ull;
   // gridDim.x is a multiple of kPairParts: every partition gets
   // gridDim.x / kPairParts CTAs
   const uint32_t p = blockIdx.x % kPairParts, sub = blockIdx.x / kPairParts;
   const uint32_t part_cap = a.list_cap / kPairParts;
-  const uint32_t n = min(a.ctr->pair_part[p], part_cap);
+  const uint32_t n = min(a.work->pair_part[p], part_cap);
   const unsigned long long* ptl = a.pair_tl + (size_t)p * part_cap;
   const uint32_t* pg = a.pair_g + (size_t)p * part_cap;
   const uint32_t stride = (gridDim.x / kPairParts) * blockDim.x;
@@ -1056,10 +1094,11 @@ __device__ __forceinline__ void tiles_resolve(const RasterFrameArgs& a, const Ra
 // from one counter -- the chunks of the heavy tiles' lists (each chunk leaves
 // its keys in chunk_keys; the warp finishing a tile's last chunk merges them
 // and resolves the tile), or, without chunk buffers, the heavy tiles whole.
-template <int T>
-__global__ void __launch_bounds__(T == 32 ? 128 : 256) raster_tiles(RasterFrameArgs a)
+template <int T, bool ONE>
+__global__ void __launch_bounds__(T == 32 ? 128 : 256) raster_tiles(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_wait();
+  frame_begin(a);
   if (list_overflowed(a)) return;
   constexpr int CTA = T == 32 ? 128 : 256;
   constexpr int NW = CTA / 32;    // warps per CTA, one work item each
@@ -1071,7 +1110,7 @@ __global__ void __launch_bounds__(T == 32 ? 128 : 256) raster_tiles(RasterFrameA
   constexpr int kTb = T == 32 ? 128 : 512;   // scene table (static shared memory stays under 48 KB)
   __shared__ uint32_t s_tb[kTb];
   for (int i = threadIdx.x; i < 256; i += CTA) s_inv255[i] = (float)i / 255.0f;
-  load_scene_table<kTb>(a, s_tb, true);
+  load_scene_table<ONE, kTb>(a, s_tb, true);
   __syncthreads();
   const int wid = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -1079,7 +1118,7 @@ __global__ void __launch_bounds__(T == 32 ? 128 : 256) raster_tiles(RasterFrameA
   TileTri* st = s_tri[wid];
   unsigned covered = 0;
   const bool chunked = a.chunk_base != nullptr;
-  const unsigned long long hacc = a.ctr->heavy_acc;
+  const unsigned long long hacc = a.ctr->bin.heavy_acc;
   const uint32_t n_heavy = min((uint32_t)(hacc >> 32), a.heavy_cap);
   const uint32_t n_chunks = chunked ? min((uint32_t)hacc, a.chunk_cap) : 0u;
   const uint32_t n_first = chunked ? n_chunks : n_heavy;   // items before the plain tiles
@@ -1123,11 +1162,11 @@ __global__ void __launch_bounds__(T == 32 ? 128 : 256) raster_tiles(RasterFrameA
       }
     } else {
       tile = w - n_first;
-      e = a.tile_cnt[tile];
+      e = a.tile_off[tile + 1] - a.tile_off[tile];
       if (e > a.heavy_threshold) continue;  // served from the heavy queue
     }
-    const int s = scene_of<kTb>(a, s_tb, tile, true);
-    const RasterSceneDev& S = a.scenes[s];
+    const int s = scene_of<ONE, kTb>(a, s_tb, tile, true);
+    const RasterSceneDev& S = scene_at<ONE>(a, s);
     uint32_t ltx;
     const uint32_t lty = fast_divmod(tile - S.tile_base, (uint32_t)S.tiles_x, S.tiles_x_m, ltx);
     const int X0 = (int)ltx * T, Y0 = (int)lty * T;
@@ -1189,11 +1228,12 @@ struct Tile8 {
 };
 
 // Scene and pixel origin of an 8x8 tile (list range left empty).
+template <bool ONE>
 __device__ __forceinline__ Tile8 tile8_geom(const RasterFrameArgs& a, const uint32_t* tb, uint32_t tile)
 {
   Tile8 t;
-  const int s = scene_of_tile(a, tb, tile);
-  t.S = &a.scenes[s];
+  const int s = scene_of_tile<ONE>(a, tb, tile);
+  t.S = &scene_at<ONE>(a, s);
   uint32_t tx;
   const uint32_t ty = fast_divmod(tile - t.S->tile_base, (uint32_t)t.S->tiles_x, t.S->tiles_x_m, tx);
   t.X0 = (int)tx * kRefBin;
@@ -1203,11 +1243,12 @@ __device__ __forceinline__ Tile8 tile8_geom(const RasterFrameArgs& a, const uint
   return t;
 }
 
+template <bool ONE>
 __device__ __forceinline__ Tile8 tile8_at(const RasterFrameArgs& a, const uint32_t* tb, uint32_t tile)
 {
   Tile8 t;
-  const int s = scene_of_tile(a, tb, tile);
-  t.S = &a.scenes[s];
+  const int s = scene_of_tile<ONE>(a, tb, tile);
+  t.S = &scene_at<ONE>(a, s);
   uint32_t tx;
   const uint32_t ty = fast_divmod(tile - t.S->tile_base, (uint32_t)t.S->tiles_x, t.S->tiles_x_m, tx);
   t.X0 = (int)tx * kRefBin;
@@ -1425,6 +1466,7 @@ __device__ __forceinline__ void resolve8_staged(const Tile8& tl, int lane, unsig
 // queue_min (<= 32 / kLightGroup) entries each: their offsets, list entries
 // and setup records are fetched together (one round of loads for the group,
 // at most 32 entries, one per lane), then each tile is tested and resolved.
+template <bool ONE>
 __device__ __forceinline__ void light_group(const RasterFrameArgs& a, const uint32_t* tb, uint32_t t0, uint32_t t1,
                                             uint32_t lim, BinTri* st, BinShade* sh, int lane, unsigned& covered,
                                             const float* inv255)
@@ -1461,7 +1503,7 @@ __device__ __forceinline__ void light_group(const RasterFrameArgs& a, const uint
     if ((uint32_t)lane >= inc[q]) j = q + 1;
   const uint32_t off = __shfl_sync(kFull, offj, j);
   if ((uint32_t)lane < total) {
-    const Tile8 g = tile8_geom(a, tb, t0 + (uint32_t)j);
+    const Tile8 g = tile8_geom<ONE>(a, tb, t0 + (uint32_t)j);
     uint32_t first = 0;
 #pragma unroll
     for (int q = 0; q < kLightGroup - 1; ++q)
@@ -1517,7 +1559,7 @@ __device__ __forceinline__ void light_group(const RasterFrameArgs& a, const uint
   for (int q = 0; q < nt; ++q) {
     const uint32_t iq = __shfl_sync(kFull, incl, q);
     if ((served_m >> q) & 1u) {  // (longer lists are drawn as chunks)
-      const Tile8 tl = tile8_geom(a, tb, t0 + (uint32_t)q);
+      const Tile8 tl = tile8_geom<ONE>(a, tb, t0 + (uint32_t)q);
       unsigned long long k0 = kInitKey, k1 = kInitKey;
       int w0 = 0, w1 = 0;
       frag8_test<true>(a, tl, st + first, (int)(iq - first), lane, covered, k0, k1, w0, w1);
@@ -1534,9 +1576,11 @@ __device__ __forceinline__ void light_group(const RasterFrameArgs& a, const uint
 // completes a tile's last chunk takes the per-pixel minimum over the tile's
 // chunks and resolves the tile.  The key order makes the result independent of
 // which warp merges when.
-__global__ void __launch_bounds__(256, 4) raster_frag8(RasterFrameArgs a)
+template <bool ONE>
+__global__ void __launch_bounds__(256, 4) raster_frag8(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_wait();
+  frame_begin(a);
   if (list_overflowed(a)) return;
   __shared__ BinTri s_tri[8][32];
   __shared__ BinShade s_shade[8][32];
@@ -1544,14 +1588,14 @@ __global__ void __launch_bounds__(256, 4) raster_frag8(RasterFrameArgs a)
   __shared__ unsigned s_cov[8];
   __shared__ uint32_t s_tb[kSceneTable];
   s_inv255[threadIdx.x] = (float)threadIdx.x / 255.0f;
-  load_scene_table<kSceneTable>(a, s_tb, true);
+  load_scene_table<ONE, kSceneTable>(a, s_tb, true);
   __syncthreads();
   const int wid = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   BinTri* st = s_tri[wid];
   unsigned covered = 0;
   const uint32_t C = a.chunk;
-  const unsigned long long hacc = a.ctr->heavy_acc;
+  const unsigned long long hacc = a.ctr->bin.heavy_acc;
   const uint32_t n_heavy = min((uint32_t)(hacc >> 32), a.heavy_cap);
   const uint32_t n_chunks = min((uint32_t)hacc, a.chunk_cap);
 
@@ -1566,7 +1610,7 @@ __global__ void __launch_bounds__(256, 4) raster_frag8(RasterFrameArgs a)
   const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t g = blockIdx.x * (blockDim.x >> 5) + (uint32_t)wid; g < n_groups; g += nwarps) {
     const uint32_t t0 = g * kLightGroup;
-    light_group(a, s_tb, t0, min(t0 + kLightGroup, a.n_tiles_total), a.queue_min, st, s_shade[wid], lane, covered,
+    light_group<ONE>(a, s_tb, t0, min(t0 + kLightGroup, a.n_tiles_total), a.queue_min, st, s_shade[wid], lane, covered,
                 s_inv255);
   }
   for (;;) {
@@ -1577,7 +1621,7 @@ __global__ void __launch_bounds__(256, 4) raster_frag8(RasterFrameArgs a)
     const uint32_t h = a.chunk_heavy[ci];
     if (h >= n_heavy) continue;  // only after a heavy-queue overflow (reported; the frame is redrawn)
     const uint32_t c0 = a.chunk_base[h];
-    const Tile8 tl = tile8_at(a, s_tb, a.heavy[h]);
+    const Tile8 tl = tile8_at<ONE>(a, s_tb, a.heavy[h]);
     const uint32_t nch = (tl.cnt + C - 1) / C;
     if (ci - c0 >= nch) continue;  // only after a heavy-queue overflow (reported; the frame is redrawn)
     unsigned long long k0 = kInitKey, k1 = kInitKey;
@@ -1621,10 +1665,6 @@ __global__ void __launch_bounds__(256, 4) raster_frag8(RasterFrameArgs a)
 }
 
 // ------------------------------------------------------------------ launch
-struct RasterLaunchInfo {
-  int persistent_ctas;
-};
-
 int raster_scan_blocks(uint32_t n_tiles) { return (int)((n_tiles + kScanTile - 1) / kScanTile); }
 
 // CTAs of one full wave of a kernel on the current device (cached; every
@@ -1666,10 +1706,12 @@ static cudaError_t launch_pdl(K kernel, int grid, int block, cudaStream_t st, co
 
 cudaError_t launch_raster_frame(const RasterFrameArgs& a, int raster_ctas, cudaStream_t st, cudaEvent_t* ev)
 {
-  static std::atomic<int> setup_wave{0}, scatter_wave{0}, large_wave{0};
+  static std::atomic<int> setup_wave[2] = {{0}, {0}}, scatter_wave{0}, large_wave{0};
+  const bool one = a.n_scenes == 1;
   const int tri_blocks = (int)((a.n_tris_total + 255) / 256);
+  const auto setup = one ? raster_setup<true> : raster_setup<false>;
   const int setup_blocks = min((int)((a.n_tris_total + kSetupThreads - 1) / kSetupThreads),
-                               wave_ctas(raster_setup, &setup_wave, kSetupThreads));
+                               wave_ctas(setup, &setup_wave[one], kSetupThreads));
   // the scatter grid covers the list groups of every triangle plus the large
   // triangles' segments (a grid-stride loop takes any excess)
   const int scatter_blocks = std::max(1, wave_ctas(raster_scatter, &scatter_wave) / (int)kPairParts) * (int)kPairParts;
@@ -1678,18 +1720,18 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& a, int raster_ctas, cudaS
   // every launch after the first may start while its predecessor drains
   // (programmatic dependent launch); each waits for it before touching memory
   cudaError_t e = cudaSuccess;
-  if (tri_blocks) raster_setup<<<setup_blocks, kSetupThreads, 0, st>>>(a);
+  if (tri_blocks) setup<<<setup_blocks, kSetupThreads, 0, st>>>(a);
   if (tri_blocks && !e) e = launch_pdl(raster_large_count, large_blocks, 256, st, a);
   if (ev) cudaEventRecord(ev[1], st);
   if (!e) e = launch_pdl(scan_tiles, raster_scan_blocks(a.n_tiles_total), kScanThreads, st, a);
   if (ev) cudaEventRecord(ev[2], st);
-  if (tri_blocks && !e) e = launch_pdl(raster_scatter, scatter_blocks, 256, st, a);
+  if (!e) e = launch_pdl(raster_scatter, scatter_blocks, 256, st, a);
   if (ev) cudaEventRecord(ev[3], st);
   if (!e) {
     switch (a.tile) {
-      case 8: e = launch_pdl(raster_frag8, raster_ctas, 256, st, a); break;
-      case 32: e = launch_pdl(raster_tiles<32>, raster_ctas, 128, st, a); break;
-      default: e = launch_pdl(raster_tiles<16>, raster_ctas, 256, st, a); break;
+      case 8: e = launch_pdl(one ? raster_frag8<true> : raster_frag8<false>, raster_ctas, 256, st, a); break;
+      case 32: e = launch_pdl(one ? raster_tiles<32, true> : raster_tiles<32, false>, raster_ctas, 128, st, a); break;
+      default: e = launch_pdl(one ? raster_tiles<16, true> : raster_tiles<16, false>, raster_ctas, 256, st, a); break;
     }
   }
   if (ev) cudaEventRecord(ev[4], st);
@@ -1697,18 +1739,12 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& a, int raster_ctas, cudaS
   return cudaGetLastError();
 }
 
-cudaError_t launch_scan_tiles(const RasterFrameArgs& a, cudaStream_t st)
-{
-  scan_tiles<<<raster_scan_blocks(a.n_tiles_total), kScanThreads, 0, st>>>(a);
-  return cudaGetLastError();
-}
-
 cudaError_t raster_tiles_occupancy(int tile, int* blocks_per_sm)
 {
   switch (tile) {
-    case 8: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_frag8, 256, 0);
-    case 32: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_tiles<32>, 128, 0);
-    default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_tiles<16>, 256, 0);
+    case 8: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_frag8<false>, 256, 0);
+    case 32: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_tiles<32, false>, 128, 0);
+    default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_tiles<16, false>, 256, 0);
   }
 }
 

@@ -63,7 +63,7 @@ uint32_t heavy_threshold(int tile)
 
 // Enqueues one frame of draws [0, n) sharing one scratch.
 piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, RasterScratch& scr, int T, int ctas,
-                                 cudaStream_t st, bool timed, bool coverage, uint32_t chunk)
+                                 cudaStream_t st, bool timed, bool coverage, uint32_t chunk, bool table_ready)
 {
   if (chunk == 0) chunk = kDefaultChunk;
   uint32_t tris = 0, tiles = 0;
@@ -77,19 +77,37 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   static_assert(kQueueMin <= kQueueMax, "a group of short lists must fit one warp");
   const uint32_t queue_min = std::min(kQueueMin, chunk);
   CU(ctx, scr.ensure_heavy(tiles, T, chunk, queue_min));
-  uint32_t tb = 0, rb = 0;
-  for (int i = 0; i < n; ++i) {
-    int tx, ty;
-    fill_scene_dev(draws[i], T, tb, rb, scr.h_scenes[i]);
-    tb += (uint32_t)tiles_for(draws[i].mesh->W, draws[i].mesh->H, T, &tx, &ty);
-    rb += (uint32_t)draws[i].mesh->N;
-  }
-  CU(ctx, cudaMemcpyAsync(scr.d_scenes, scr.h_scenes, sizeof(RasterSceneDev) * n, cudaMemcpyHostToDevice, st));
-  CU(ctx, cudaMemsetAsync(scr.ctr, 0, sizeof(FrameCounters), st));
-  CU(ctx, cudaMemsetAsync(scr.tile_cnt, 0, sizeof(uint32_t) * tiles, st));
-  CU(ctx, cudaMemsetAsync(scr.scan_flags, 0, sizeof(unsigned long long) * raster_scan_blocks(tiles), st));
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CU(ctx, cudaStreamIsCapturing(st, &capture));
+  const bool capturing = capture != cudaStreamCaptureStatusNone;
   RasterFrameArgs a;
   memset(&a, 0, sizeof(a));
+  if (n == 1) {
+    fill_scene_dev(draws[0], T, 0u, 0u, a.one);
+  } else if (!table_ready) {
+    // Frames may be queued faster than the device takes them: the source of a
+    // copy is pageable memory, which the call has read when it returns, and
+    // not a pinned buffer that the next frame would overwrite under the copy.
+    // (A captured copy reads its source at every replay: memory of its own.)
+    scr.h_scenes.resize((size_t)n);
+    RasterSceneDev* src = capturing ? scr.cap_scenes : scr.h_scenes.data();
+    uint32_t tb = 0, rb = 0;
+    for (int i = 0; i < n; ++i) {
+      int tx, ty;
+      fill_scene_dev(draws[i], T, tb, rb, src[i]);
+      tb += (uint32_t)tiles_for(draws[i].mesh->W, draws[i].mesh->H, T, &tx, &ty);
+      rb += (uint32_t)draws[i].mesh->N;
+    }
+    CU(ctx, cudaMemcpyAsync(scr.d_scenes, src, sizeof(RasterSceneDev) * n, cudaMemcpyHostToDevice, st));
+  }
+  if (!scr.clean) {
+    // fresh counters, or a frame whose launches failed part way (memsets that a
+    // capture records have not run yet)
+    CU(ctx, cudaMemsetAsync(scr.work, 0, sizeof(BinWork), st));
+    CU(ctx, cudaMemsetAsync(scr.tile_cnt, 0, sizeof(uint32_t) * scr.tiles_cap, st));
+    CU(ctx, cudaMemsetAsync(scr.scan_flags, 0, sizeof(unsigned long long) * scr.scan_cap, st));
+    scr.clean = !capturing;
+  }
   a.scenes = scr.d_scenes;
   a.n_scenes = n;
   a.tile = T;
@@ -117,34 +135,38 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   a.chunk_keys = scr.chunk_keys;
   a.chunk_cap = scr.chunk_cap;
   a.scan_flags = scr.scan_flags;
-  a.epoch = 0;
+  a.work = scr.work;
   a.ctr = scr.ctr;
+  a.host_bin = &scr.h_ctr->bin;
   if (coverage) {
     a.cov_tri = scr.cov_tri;
     a.cov_pix = scr.cov_pix;
     a.cov_cap = scr.cov_cap;
   }
-  CU(ctx, launch_raster_frame(a, ctas, st, timed ? scr.ev : nullptr));
+  const cudaError_t le = launch_raster_frame(a, ctas, st, timed ? scr.ev : nullptr);
+  if (le != cudaSuccess) scr.clean = false;
+  CU(ctx, le);
   return PIKO_OK;
 }
 
 piko_status enqueue_raster(piko_ctx* ctx, piko_scene* const* scenes, int n, RasterScratch& scr, const TuneCfg& cfg,
-                           cudaStream_t st, bool timed, bool coverage)
+                           cudaStream_t st, bool timed, bool coverage, bool table_ready)
 {
   std::vector<RasterDraw> draws((size_t)n);
   for (int i = 0; i < n; ++i) draws[i] = RasterDraw{scenes[i], &scenes[i]->state, scenes[i]->fb, scenes[i]->depth};
   return enqueue_raster_draws(ctx, draws.data(), n, scr, cfg.tile, raster_ctas(ctx, cfg.tile, cfg.ctas_per_sm), st, timed,
-                              coverage, cfg.chunk);
+                              coverage, cfg.chunk, table_ready);
 }
 
 namespace {
 
-// The status of a frame whose counters are already in scr.h_ctr; grows the
-// bin-queue capacity when the device reported an overflow.  Returns
+// The status of a completed frame (its binning counts are in scr.h_ctr: the
+// fragment kernel leaves them in that pinned memory); grows the bin-queue
+// capacity when the device reported an overflow.  Returns
 // PIKO_ERR_QUEUE_OVERFLOW when a re-run is needed.
 piko_status check_counters(piko_ctx* ctx, RasterScratch& scr)
 {
-  const FrameCounters& c = *scr.h_ctr;
+  const BinCounts& c = scr.h_ctr->bin;
   if (c.status & kStatusScanTimeout) return set_err(ctx, PIKO_ERR_TIMEOUT, "%s", "tile scan look-back timed out");
   if (c.status & kStatusListOverflow) {
     CU(ctx, scr.regrow(c));
@@ -153,10 +175,11 @@ piko_status check_counters(piko_ctx* ctx, RasterScratch& scr)
   return PIKO_OK;
 }
 
-// Reads the counters of the last frame and checks them (check_counters).
-piko_status check_frame(piko_ctx* ctx, RasterScratch& scr, cudaStream_t st)
+// Waits for the last frame and checks it (check_counters); counters: h_ctr also
+// gets what the fragment kernel counted.
+piko_status check_frame(piko_ctx* ctx, RasterScratch& scr, cudaStream_t st, bool counters)
 {
-  CU(ctx, cudaMemcpyAsync(scr.h_ctr, scr.ctr, sizeof(FrameCounters), cudaMemcpyDeviceToHost, st));
+  if (counters) CU(ctx, cudaMemcpyAsync(scr.h_ctr, scr.ctr, sizeof(FrameCounters), cudaMemcpyDeviceToHost, st));
   CU(ctx, cudaStreamSynchronize(st));
   return check_counters(ctx, scr);
 }
@@ -470,7 +493,7 @@ piko_status piko_frame_finish(piko_scene* s)
   if (s->pipe->kind == kPipeReyes) return piko_reyes_finish(s);
   piko_ctx* ctx = s->pipe->ctx;
   for (int attempt = 0; attempt < 4; ++attempt) {
-    piko_status r = check_frame(ctx, s->scr, s->last_stream);
+    piko_status r = check_frame(ctx, s->scr, s->last_stream, false);
     if (r == PIKO_OK) { s->pending = false; return PIKO_OK; }
     if (r != PIKO_ERR_QUEUE_OVERFLOW) return r;
     piko_scene* one[1] = {s};
@@ -492,10 +515,9 @@ piko_status piko_frame_read(piko_scene* s, uint32_t* rgba, float* depth)
     return e;
   };
   if (s->pending && s->pipe->kind == kPipeRaster) {
-    // one wait for the frame's counters and image together; a frame that
+    // one wait for the frame's counts and image together; a frame that
     // overflowed its queues is drawn again (finish) and copied again
     cudaStream_t st = s->last_stream;
-    CU(ctx, cudaMemcpyAsync(s->scr.h_ctr, s->scr.ctr, sizeof(FrameCounters), cudaMemcpyDeviceToHost, st));
     CU(ctx, copy_image(st));
     CU(ctx, cudaStreamSynchronize(st));
     const piko_status r = check_counters(ctx, s->scr);
@@ -528,11 +550,11 @@ piko_status piko_frame_device_buffers(piko_scene* s, uint32_t** rgba, float** de
 static void fill_stats(const RasterScratch& scr, bool timed, piko_frame_stats* o)
 {
   const FrameCounters& c = *scr.h_ctr;
-  o->prims_kept += c.kept;
-  o->bin_entries += c.list_total;
+  o->prims_kept += c.bin.kept;
+  o->bin_entries += c.bin.list_total;
   o->covered += c.covered;
-  o->wrap_risk += c.risk;
-  o->status |= c.status;
+  o->wrap_risk += c.bin.risk;
+  o->status |= c.bin.status;
   if (timed && scr.ev_made) {
     o->n_kernels = 4;
     for (int i = 0; i < 4; ++i) {
@@ -577,7 +599,7 @@ piko_status piko_frame_coverage(piko_scene* s, uint32_t* tri, uint32_t* pix, uin
     piko_scene* one[1] = {s};
     r = enqueue_raster(ctx, one, 1, s->scr, pipe_cfg(s->pipe), st, false, true);
     if (r != PIKO_OK) return r;
-    r = check_frame(ctx, s->scr, st);
+    r = check_frame(ctx, s->scr, st, true);
     if (r == PIKO_OK) break;
     if (r != PIKO_ERR_QUEUE_OVERFLOW) return r;
   }
@@ -626,7 +648,8 @@ piko_status batch_make(piko_ctx* ctx, piko_scene* const* scenes, int n, const Tu
 
 // Enqueues every group: group 0 on st, the others on their own streams forked
 // from st and joined back into it (parallel branches when captured).
-static piko_status batch_enqueue(piko_batch* b, cudaStream_t st, bool timed)
+// table_ready: the groups' scene tables already hold the scenes as they are now.
+static piko_status batch_enqueue(piko_batch* b, cudaStream_t st, bool timed, bool table_ready = false)
 {
   piko_ctx* ctx = b->ctx;
   const bool fork = b->groups.size() > 1;
@@ -635,7 +658,8 @@ static piko_status batch_enqueue(piko_batch* b, cudaStream_t st, bool timed)
     BatchGroup* g = b->groups[k];
     cudaStream_t gs = k == 0 ? st : g->stream;
     if (k > 0) CU(ctx, cudaStreamWaitEvent(gs, b->fork, 0));
-    piko_status r = enqueue_raster(ctx, g->scenes.data(), (int)g->scenes.size(), g->scr, g->cfg, gs, timed, false);
+    piko_status r = enqueue_raster(ctx, g->scenes.data(), (int)g->scenes.size(), g->scr, g->cfg, gs, timed, false,
+                                   table_ready);
     if (r != PIKO_OK) return r;
     if (k > 0) CU(ctx, cudaEventRecord(g->done, gs));
   }
@@ -681,8 +705,9 @@ piko_status piko_batch_run(piko_batch* b, void* stream, int use_graph)
       piko_status r = batch_enqueue(b, st, false);
       if (r != PIKO_OK) return r;
       CU(ctx, cudaStreamSynchronize(st));
+      // the frame just drawn filled the scene tables: the graph is its kernels alone
       CU(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      r = batch_enqueue(b, st, false);
+      r = batch_enqueue(b, st, false, true);
       cudaGraph_t g = nullptr;
       cudaError_t e = cudaStreamEndCapture(st, &g);
       if (r != PIKO_OK) { if (g) cudaGraphDestroy(g); return r; }
@@ -708,7 +733,7 @@ piko_status piko_batch_finish(piko_batch* b, piko_frame_stats* out)
   if (b->pending) {
     for (auto* g : b->groups) {
       for (int attempt = 0;; ++attempt) {
-        piko_status r = check_frame(ctx, g->scr, b->last_stream);
+        piko_status r = check_frame(ctx, g->scr, b->last_stream, out != nullptr);
         if (r == PIKO_OK) break;
         if (r != PIKO_ERR_QUEUE_OVERFLOW || attempt >= 3) return r;
         drop_graph(b);  // the queue buffers moved

@@ -114,10 +114,13 @@ struct RasterScratch {
   uint32_t heavy_cap = 0, chunk_cap = 0;
   uint32_t chunk_stride = 0;                // keys per chunk (tile * tile)
   unsigned long long* scan_flags = nullptr;
+  BinWork* work = nullptr;
   FrameCounters* ctr = nullptr;
-  FrameCounters* h_ctr = nullptr;  // pinned
-  RasterSceneDev* d_scenes = nullptr;
-  RasterSceneDev* h_scenes = nullptr;  // pinned
+  FrameCounters* h_ctr = nullptr;  // pinned; the fragment kernel writes its bin part
+  bool clean = false;              // tile_cnt, scan_flags and work are all zero (every frame leaves them so)
+  RasterSceneDev* d_scenes = nullptr;      // scene table of launch sequences over several scenes
+  std::vector<RasterSceneDev> h_scenes;    // pageable: a copy from it has read it when the call returns
+  RasterSceneDev* cap_scenes = nullptr;    // pinned: the source of a copy that a stream capture records
   uint32_t tris_cap = 0, tiles_cap = 0, list_cap = 0, scan_cap = 0;
   int scenes_cap = 0;
   uint32_t cov_cap = 0;
@@ -131,10 +134,11 @@ struct RasterScratch {
     dfree(setup); dfree(tile_cnt); dfree(tile_off); dfree(tile_list); dfree(pair_tl); dfree(pair_g);
     dfree(heavy); dfree(large_seg); dfree(large_walk); dfree(chunk_base); dfree(hdone); dfree(chunk_keys);
     dfree(chunk_heavy);
-    dfree(scan_flags); dfree(ctr); dfree(d_scenes); dfree(cov_tri); dfree(cov_pix);
+    dfree(scan_flags); dfree(work); dfree(ctr); dfree(d_scenes); dfree(cov_tri); dfree(cov_pix);
     if (h_ctr) cudaFreeHost(h_ctr);
-    if (h_scenes) cudaFreeHost(h_scenes);
-    h_ctr = nullptr; h_scenes = nullptr;
+    if (cap_scenes) cudaFreeHost(cap_scenes);
+    h_ctr = nullptr; cap_scenes = nullptr;
+    clean = false;
     if (ev_made) for (auto& e : ev) cudaEventDestroy(e);
     ev_made = false;
     tris_cap = tiles_cap = list_cap = scan_cap = heavy_cap = chunk_cap = seg_cap = chunk_stride = 0;
@@ -207,7 +211,7 @@ struct RasterScratch {
   // After a frame whose counters report a queue overflow: grows what
   // overflowed (the tile lists and / or the chunk key buffers) so that the
   // frame can be drawn again.
-  cudaError_t regrow(const FrameCounters& c)
+  cudaError_t regrow(const BinCounts& c)
   {
     cudaError_t e = cudaSuccess;
     // the lists hold every pair, and each pair partition its share
@@ -240,6 +244,7 @@ struct RasterScratch {
       tris_cap = n_tris;
     }
     if (n_tiles > tiles_cap) {
+      clean = false;
       dfree(tile_cnt); dfree(tile_off);
       if ((e = dalloc(&tile_cnt, n_tiles))) return e;
       if ((e = dalloc(&tile_off, (size_t)n_tiles + 1))) return e;
@@ -247,6 +252,7 @@ struct RasterScratch {
     }
     uint32_t sb = (uint32_t)raster_scan_blocks(n_tiles);
     if (sb > scan_cap) {
+      clean = false;
       dfree(scan_flags);
       if ((e = dalloc(&scan_flags, sb))) return e;
       scan_cap = sb;
@@ -255,16 +261,18 @@ struct RasterScratch {
       if ((e = grow_list(list_need))) return e;
     }
     if (!ctr) {
+      clean = false;
+      if ((e = dalloc(&work, 1))) return e;
       if ((e = dalloc(&ctr, 1))) return e;
       if ((e = cudaMallocHost((void**)&h_ctr, sizeof(FrameCounters)))) return e;
       memset(h_ctr, 0, sizeof(FrameCounters));
     }
-    if (n_scenes > scenes_cap) {
+    if (n_scenes > 1 && n_scenes > scenes_cap) {
       dfree(d_scenes);
-      if (h_scenes) cudaFreeHost(h_scenes);
-      h_scenes = nullptr;
+      if (cap_scenes) cudaFreeHost(cap_scenes);
+      cap_scenes = nullptr;
       if ((e = dalloc(&d_scenes, n_scenes))) return e;
-      if ((e = cudaMallocHost((void**)&h_scenes, sizeof(RasterSceneDev) * n_scenes))) return e;
+      if ((e = cudaMallocHost((void**)&cap_scenes, sizeof(RasterSceneDev) * n_scenes))) return e;
       scenes_cap = n_scenes;
     }
     if (!ev_made) {
@@ -369,10 +377,12 @@ struct RasterDraw {
 // lists longer than kQueueMin entries are queued as chunks
 constexpr uint32_t kDefaultChunk = 32;
 constexpr uint32_t kQueueMin = 8;
+// table_ready: the scene table in scr already holds these draws
 piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, RasterScratch& scr, int T, int ctas,
-                                 cudaStream_t st, bool timed, bool coverage, uint32_t chunk = 0);
+                                 cudaStream_t st, bool timed, bool coverage, uint32_t chunk = 0,
+                                 bool table_ready = false);
 // One launch sequence over resident scenes drawn with their own camera states.
 piko_status enqueue_raster(piko_ctx* ctx, piko_scene* const* scenes, int n, RasterScratch& scr, const TuneCfg& cfg,
-                           cudaStream_t st, bool timed, bool coverage);
+                           cudaStream_t st, bool timed, bool coverage, bool table_ready = false);
 int raster_ctas(piko_ctx* ctx, int tile, int ctas_per_sm);
 uint32_t heavy_threshold(int tile);

@@ -231,14 +231,13 @@ piko_status finish_lane(piko_server* sv, SrvLane& lane)
     RasterScratch& scr = lane.scr[kv.first];
     piko_status st = PIKO_ERR_QUEUE_OVERFLOW;
     for (int attempt = 0; attempt < 5; ++attempt) {
-      cudaError_t e = cudaMemcpyAsync(scr.h_ctr, scr.ctr, sizeof(FrameCounters), cudaMemcpyDeviceToHost, lane.st);
-      if (!e) e = cudaStreamSynchronize(lane.st);
+      const cudaError_t e = cudaStreamSynchronize(lane.st);
       if (e) { st = PIKO_ERR_CUDA; break; }
-      const uint32_t status = scr.h_ctr->status;
+      const uint32_t status = scr.h_ctr->bin.status;
       if (status & kStatusScanTimeout) { st = PIKO_ERR_TIMEOUT; break; }
       if (!(status & kStatusListOverflow)) { st = PIKO_OK; break; }
       if (attempt == 4) break;   // still overflowing: reported
-      if (scr.regrow(*scr.h_ctr) != cudaSuccess) { st = PIKO_ERR_OOM; break; }
+      if (scr.regrow(scr.h_ctr->bin) != cudaSuccess) { st = PIKO_ERR_OOM; break; }
       const int cps = kv.second.front().mesh->pipe->ctas_per_sm;
       const piko_status r = enqueue_raster_draws(sv->ctx, kv.second.data(), (int)kv.second.size(), scr, kv.first,
                                                  raster_ctas(sv->ctx, kv.first, cps), lane.st, false, false,
