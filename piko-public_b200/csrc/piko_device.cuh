@@ -30,10 +30,10 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 2;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-// 8x8 raster queue: short lists (at most kQueueMax entries, so a group's
-// entries fit one warp) are handed out kLightGroup tiles per pop
-constexpr int kLightGroup = 4;
-constexpr uint32_t kQueueMax = 32 / kLightGroup;
+// 8x8 raster queue: short lists (at most kQueueMax entries, one per lane) are
+// drawn in groups of up to kLightGroup consecutive tiles
+constexpr int kLightGroup = 8;
+constexpr uint32_t kQueueMax = 32;
 
 // 16/32-px tiles: a heavy tile's list is cut into at most kMaxTileChunks
 // chunks of at least `chunk` entries (different warps rasterize them; the last
@@ -165,12 +165,13 @@ struct __align__(16) TriSetup {
   uint32_t bxr, byr;    // clamped reference-bin range: lo | hi << 16
   int32_t hix, hiy;     // pixel bounding box high corner (28.4, rounded up to 16 px)
   uint32_t rank1;       // submission rank + 1 (0 = culled)
-  uint32_t flags;       // bit 0: wrapping possible inside the bin range (no tile-level reject)
+  uint32_t flags;       // kTriRisk (no tile-level reject), kTriAreaRisk
   uint32_t id;          // triangle index within its scene
 };
 static_assert(sizeof(TriSetup) == 80, "TriSetup layout");
 
-constexpr uint32_t kTriRisk = 1u;
+constexpr uint32_t kTriRisk = 1u;      // an edge value may wrap inside the bin range
+constexpr uint32_t kTriAreaRisk = 2u;  // the area may wrap: its reciprocal says nothing of the depth's range
 
 // What the binning passes (setup, large count, scan) count.  The heavy-tile
 // queue and the large-triangle queue each reserve slots and work-item ranges
@@ -233,6 +234,17 @@ struct __align__(16) WalkTri {
 };
 static_assert(sizeof(WalkTri) == 112, "WalkTri layout");
 
+// A chunk of a heavy tile's list, written by the scan: all that the warp that
+// takes it needs, in one 32-byte read.
+struct __align__(16) ChunkDesc {
+  uint32_t tile;
+  uint32_t off, n;     // list entries [off, off + n)
+  uint32_t h;          // the heavy tile (its counter of finished chunks is hdone[h])
+  uint32_t j, nch;     // chunk j of the tile's nch
+  uint32_t pad[2];
+};
+static_assert(sizeof(ChunkDesc) == 32, "ChunkDesc layout");
+
 struct RasterFrameArgs {
   RasterSceneDev one;       // the scene of a one-scene frame: it travels with the launch, no copy precedes the frame
   const RasterSceneDev* scenes;  // [n_scenes] when there are several
@@ -245,7 +257,7 @@ struct RasterFrameArgs {
   uint32_t* tile_off;       // [n_tiles_total + 1]
   uint32_t* tile_list;      // [list_cap]
   uint32_t list_cap;
-  uint32_t* heavy;          // [heavy_cap] tiles served first (8x8: tiles split into chunks)
+  uint32_t* heavy;          // [heavy_cap] heavy tiles, when there are no chunk buffers
   uint32_t heavy_threshold; // 16/32-px tiles: list entries above which a tile is heavy
   uint32_t heavy_cap;
   // one record per (triangle, tile) pair, written by the count passes: the
@@ -263,11 +275,11 @@ struct RasterFrameArgs {
   // warps rasterize.  Each chunk leaves its per-pixel keys (tile * tile of
   // them) in chunk_keys; the warp that completes a tile's last chunk takes the
   // per-pixel minimum over the tile's chunks and resolves the tile.  Without
-  // chunk buffers (chunk_base null) heavy tiles are rasterized whole, first.
+  // chunk buffers (chunk_desc null) heavy tiles are rasterized whole, first.
   uint32_t chunk;
   uint32_t queue_min;       // 8x8 tiles with more entries than this are queued as chunks
-  uint32_t* chunk_base;     // [heavy_cap] first chunk of heavy tile h (ascending in h)
-  uint32_t* chunk_heavy;    // [chunk_cap] the heavy tile (index h) of each chunk
+  uint32_t group;           // 8x8 tiles per short-list group (at most kLightGroup)
+  ChunkDesc* chunk_desc;    // [chunk_cap]; the chunks of a tile are consecutive
   uint32_t* hdone;          // [heavy_cap] chunks finished
   unsigned long long* chunk_keys;  // [chunk_cap][tile * tile]
   uint32_t chunk_cap;

@@ -78,20 +78,26 @@ constexpr int kSceneTable = 1024;
 template <bool ONE, int CAP>
 __device__ __forceinline__ void load_scene_table(const RasterFrameArgs& a, uint32_t* tb, bool by_tile)
 {
-  if (ONE || a.n_scenes > CAP) return;
-  for (int i = threadIdx.x; i < a.n_scenes; i += blockDim.x) tb[i] = by_tile ? a.scenes[i].tile_base : a.scenes[i].tri_base;
+  if constexpr (!ONE) {
+    if (a.n_scenes > CAP) return;
+    for (int i = threadIdx.x; i < a.n_scenes; i += blockDim.x)
+      tb[i] = by_tile ? a.scenes[i].tile_base : a.scenes[i].tri_base;
+  }
 }
 template <bool ONE, int CAP>
 __device__ __forceinline__ int scene_of(const RasterFrameArgs& a, const uint32_t* tb, uint32_t x, bool by_tile)
 {
-  if (ONE) return 0;
-  if (a.n_scenes > CAP) return find_base(a.scenes, a.n_scenes, x, by_tile);
-  int lo = 0, hi = a.n_scenes - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tb[mid] <= x) lo = mid; else hi = mid - 1;
+  if constexpr (ONE) {
+    return 0;
+  } else {
+    if (a.n_scenes > CAP) return find_base(a.scenes, a.n_scenes, x, by_tile);
+    int lo = 0, hi = a.n_scenes - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (tb[mid] <= x) lo = mid; else hi = mid - 1;
+    }
+    return lo;
   }
-  return lo;
 }
 template <bool ONE>
 __device__ __forceinline__ int scene_of_tile(const RasterFrameArgs& a, const uint32_t* tb, uint32_t tile)
@@ -149,6 +155,18 @@ struct F3 { float x, y, z; };
 
 __device__ __forceinline__ float sat1(float v) { return v > 1.0f ? 1.0f : (v < 0.0f ? 0.0f : v); }
 
+// toABGR by truncation (piko/math.h:279-289).  One range test for the three
+// channels: only a triangle whose edge values wrapped can leave it (and a NaN
+// channel converts to 0 either way).
+__device__ __forceinline__ uint32_t pack_abgr(float r, float g, float b)
+{
+  const float fr = r * 255.0f, fg = g * 255.0f, fb = b * 255.0f;
+  if (fmaxf(fmaxf(fabsf(fr), fabsf(fg)), fabsf(fb)) < 2147483648.0f)
+    return 0xff000000u | ((uint32_t)__float2int_rz(fb) << 16) | ((uint32_t)__float2int_rz(fg) << 8) |
+           (uint32_t)__float2int_rz(fr);
+  return 0xff000000u | (cvt_u32_x86(fb) << 16) | (cvt_u32_x86(fg) << 8) | cvt_u32_x86(fr);
+}
+
 // computeLightingHost + toABGRHost (main.cpp:317-334)
 __device__ __forceinline__ uint32_t light_abgr(F3 n, F3 l, F3 m)
 {
@@ -157,7 +175,7 @@ __device__ __forceinline__ uint32_t light_abgr(F3 n, F3 l, F3 m)
   float r = sat1(d * m.x + 0.15f);
   float g = sat1(d * m.y + 0.15f);
   float b = sat1(d * m.z + 0.30f);
-  return 0xff000000u | (cvt_u32_x86(b * 255.0f) << 16) | (cvt_u32_x86(g * 255.0f) << 8) | cvt_u32_x86(r * 255.0f);
+  return pack_abgr(r, g, b);
 }
 
 // E_i(X, Y) = (Y - y_i) * dx_i - (X - x_i) * dy_i  (wrapping int32)
@@ -524,6 +542,9 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(const __grid_const
           worst = max(worst, ay * dx + ax * dy + 512 * (dx + dy));
         }
         if (worst >= 2147483647LL) r.flags |= kTriRisk;
+        const long long area = (long long)(r.y[2] - r.y[0]) * (r.x[1] - r.x[0]) -
+                               (long long)(r.x[2] - r.x[0]) * (r.y[1] - r.y[0]);
+        if (area >= 2147483647LL) r.flags |= kTriAreaRisk;
         risk_flag = (r.flags & kTriRisk) != 0;
       }
     }
@@ -628,7 +649,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
   // Heavy tiles (lists longer than the threshold) and their chunks: counted
   // now, reserved below with one atomic per block while warp 0 looks back
   const bool t8 = a.tile == kRefBin;
-  const bool chunked = a.chunk_base != nullptr;
+  const bool chunked = a.chunk_desc != nullptr;
   const uint32_t thr = t8 ? a.queue_min : a.heavy_threshold;
   uint32_t nh = 0, nc = 0;
 #pragma unroll
@@ -709,9 +730,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
   }
   __syncthreads();
   uint32_t run = s_prefix + warp_excl + (incl - sum);
-  // With chunk buffers a heavy list becomes tile_chunks(len) chunks; the
-  // tile's first chunk and its finished-chunk counter are all the queue stores
-  // per tile.
+  // With chunk buffers a heavy list becomes tile_chunks(len) chunks
   const unsigned long long old = s_heavy[warp];
   uint32_t h = (uint32_t)(old >> 32) + hi - nh;
   uint32_t c = (uint32_t)old + ci - nc;
@@ -721,15 +740,19 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
       a.tile_off[base + i] = run;
       if (v[i] > thr) {
         if (h < a.heavy_cap) {
-          a.heavy[h] = base + i;
           if (chunked) {
-            a.chunk_base[h] = c;
             a.hdone[h] = 0;
-            const uint32_t nch = tile_chunks(v[i], a.chunk, t8);
-            for (uint32_t j = 0; j < nch && c + j < a.chunk_cap; ++j) a.chunk_heavy[c + j] = h;
+            const uint32_t ce = tile_chunk_entries(v[i], a.chunk, t8), nch = (v[i] + ce - 1) / ce;
+            for (uint32_t j = 0; j < nch && c + j < a.chunk_cap; ++j) {
+              uint4* d = reinterpret_cast<uint4*>(&a.chunk_desc[c + j]);
+              d[0] = make_uint4(base + i, run + j * ce, min(ce, v[i] - j * ce), h);
+              d[1] = make_uint4(j, nch, 0u, 0u);
+            }
             c += nch;
             // chunks past the key buffers are not rasterized: report it
             if (c > a.chunk_cap) atomicOr(&a.work->bin.status, kStatusListOverflow);
+          } else {
+            a.heavy[h] = base + i;
           }
         } else {
           atomicOr(&a.work->bin.status, kStatusListOverflow);
@@ -1009,8 +1032,7 @@ __device__ __forceinline__ uint32_t shade_winner(const RasterSceneDev& S, const 
     col[1] = col[1] * inv255[t.y];
     col[2] = col[2] * inv255[t.z];
   }
-  return 0xff000000u | (cvt_u32_x86(col[2] * 255.0f) << 16) | (cvt_u32_x86(col[1] * 255.0f) << 8) |
-         cvt_u32_x86(col[0] * 255.0f);
+  return pack_abgr(col[0], col[1], col[2]);
 }
 
 // Rasterizes list entries [b, e) of the tile at (X0, Y0) of scene S into the
@@ -1117,7 +1139,7 @@ __global__ void __launch_bounds__(T == 32 ? 128 : 256) raster_tiles(const __grid
   unsigned long long* keys = s_keys[wid];
   TileTri* st = s_tri[wid];
   unsigned covered = 0;
-  const bool chunked = a.chunk_base != nullptr;
+  const bool chunked = a.chunk_desc != nullptr;
   const unsigned long long hacc = a.ctr->bin.heavy_acc;
   const uint32_t n_heavy = min((uint32_t)(hacc >> 32), a.heavy_cap);
   const uint32_t n_chunks = chunked ? min((uint32_t)hacc, a.chunk_cap) : 0u;
@@ -1145,16 +1167,14 @@ __global__ void __launch_bounds__(T == 32 ? 128 : 256) raster_tiles(const __grid
     bool chunk_item = false;
     if (w < n_first) {
       if (chunked) {
-        h = a.chunk_heavy[w];
-        if (h >= n_heavy) continue;  // only after a heavy-queue overflow (reported; the frame is redrawn)
-        c0 = a.chunk_base[h];
-        tile = a.heavy[h];
-        const uint32_t cnt = a.tile_off[tile + 1] - a.tile_off[tile];
-        const uint32_t ce = tile_chunk_entries(cnt, a.chunk, false);
-        nch = (cnt + ce - 1) / ce;
-        if (w - c0 >= nch) continue;  // only after a heavy-queue overflow (reported; the frame is redrawn)
-        b = (w - c0) * ce;
-        e = min(b + ce, cnt);
+        const uint4* dp = reinterpret_cast<const uint4*>(&a.chunk_desc[w]);
+        const uint4 d0 = dp[0], d1 = dp[1];
+        tile = d0.x;
+        h = d0.w;
+        c0 = w - d1.x;
+        nch = d1.y;
+        b = d0.y - a.tile_off[tile];
+        e = b + d0.z;
         chunk_item = true;
       } else {
         tile = a.heavy[w];
@@ -1201,33 +1221,37 @@ __global__ void __launch_bounds__(T == 32 ? 128 : 256) raster_tiles(const __grid
   if (lane == 0 && covered) atomicAdd(&a.ctr->covered, (unsigned long long)covered);
 }
 
-// 8x8 tiles (one reference bin each): a warp takes a tile, or a chunk of a
-// long tile list, and each lane two of the tile's pixels, (lane & 7, lane >> 3)
-// and the pixel 4 rows above.  Entries are taken 32 at a time: first every
-// lane tests its two pixels against all 32 entries (integer edge functions
-// only, independent across entries) and collects one coverage bit per entry
-// and pixel; then each lane runs the barycentric depth and the key update for
-// its set bits alone, so the float work is not repeated across a warp for
-// pixels an entry does not cover.  Each lane keeps its pixels' smallest
-// fragment key in registers.  Lists hold exactly the reference's (triangle,
-// bin) pairs.
+// 8x8 tiles (one reference bin each): a warp takes up to 32 list entries at a
+// time, one per lane, of one tile or of several with short lists.  Lists hold
+// exactly the reference's (triangle, bin) pairs.
+//
+//   1. Each lane builds its entry's coverage of the tile as a 64-bit mask:
+//      the edge functions are stepped over the pixels, and the sign of their
+//      OR is shifted into the mask (5 instructions a pixel for 32 entries at
+//      once; testing every entry by the whole warp, two pixels a lane, took
+//      about 34 warp instructions an entry, this takes about 14).
+//   2. The entries are put in the order of a lower bound of their depth in the
+//      tile, and the masks transposed (five shuffle stages), so that lane p
+//      holds one bit per entry for pixels p and p + 32.
+//   3. Each lane evaluates the depth of its covered entries, nearest bound
+//      first, and stops at the first whose bound lies behind its pixel's
+//      current depth: with the mix's overdraw most entries are never evaluated.
 struct __align__(16) BinTri {
-  int32_t e0, e1, e2, sx0;      // edge values at the centre of the tile's pixel (0, 0); per-pixel x steps
-  int32_t sx1, sx2, sy0, sy1;   // per-pixel y steps
-  int32_t sy2, lxe, lye, flags; // bbox limit (pixel < limit), tile-local; kBinDraw | kBinAccept
-  float inv, z2, z0mz2, z1mz2;
-  uint32_t rank1, gidx, pad0, pad1;
+  int32_t e1, e2, sx1, sx2;     // edge values at the centre of the tile's pixel (0, 0); per-pixel x steps
+  int32_t sy1, sy2;             // per-pixel y steps
+  float inv, z2;
+  float z0mz2, z1mz2;
+  uint32_t rank1;
+  uint32_t bound;               // the high 24 bits of the depth key no fragment of the entry in this tile is below
 };
-constexpr int32_t kBinDraw = 1;    // the entry has pixels to test in this tile
-constexpr int32_t kBinAccept = 2;  // trivially accepted bin: all 64 pixels covered
+static_assert(sizeof(BinTri) == 48, "BinTri layout");
 
+// Scene and pixel origin of an 8x8 tile.
 struct Tile8 {
   const RasterSceneDev* S;
   int X0, Y0;
-  uint32_t off, cnt;     // list range; cnt as counted (not clamped)
 };
 
-// Scene and pixel origin of an 8x8 tile (list range left empty).
 template <bool ONE>
 __device__ __forceinline__ Tile8 tile8_geom(const RasterFrameArgs& a, const uint32_t* tb, uint32_t tile)
 {
@@ -1238,131 +1262,245 @@ __device__ __forceinline__ Tile8 tile8_geom(const RasterFrameArgs& a, const uint
   const uint32_t ty = fast_divmod(tile - t.S->tile_base, (uint32_t)t.S->tiles_x, t.S->tiles_x_m, tx);
   t.X0 = (int)tx * kRefBin;
   t.Y0 = (int)ty * kRefBin;
-  t.off = 0;
-  t.cnt = 0;
   return t;
 }
 
-template <bool ONE>
-__device__ __forceinline__ Tile8 tile8_at(const RasterFrameArgs& a, const uint32_t* tb, uint32_t tile)
+// One stage of a 32x32 bit transpose over the warp's lanes.
+__device__ __forceinline__ uint32_t transpose_stage(uint32_t x, int s, uint32_t m, int lane)
 {
-  Tile8 t;
-  const int s = scene_of_tile<ONE>(a, tb, tile);
-  t.S = &scene_at<ONE>(a, s);
-  uint32_t tx;
-  const uint32_t ty = fast_divmod(tile - t.S->tile_base, (uint32_t)t.S->tiles_x, t.S->tiles_x_m, tx);
-  t.X0 = (int)tx * kRefBin;
-  t.Y0 = (int)ty * kRefBin;
-  t.off = a.tile_off[tile];
-  t.cnt = a.tile_off[tile + 1] - t.off;
-  return t;
+  const uint32_t y = __shfl_xor_sync(kFull, x, s);
+  return (lane & s) ? ((x & ~m) | ((y >> s) & m)) : ((x & m) | ((y << s) & ~m));
+}
+// Word `lane` becomes the bits `lane` of the 32 lanes' words.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane)
+{
+  x = transpose_stage(x, 16, 0x0000ffffu, lane);
+  x = transpose_stage(x, 8, 0x00ff00ffu, lane);
+  x = transpose_stage(x, 4, 0x0f0f0f0fu, lane);
+  x = transpose_stage(x, 2, 0x33333333u, lane);
+  return transpose_stage(x, 1, 0x55555555u, lane);
 }
 
-// The tile-local form of list entry gi for the 8x8 tile at (X0, Y0).
-__device__ __forceinline__ void frag8_build(const RasterFrameArgs& a, uint32_t gi, int X0, int Y0, BinTri& out)
+// A lower bound of the depth that the fragments of entry t (least vertex depth
+// zmin, greatest magnitude zmax) can have in its tile: the larger of the least
+// vertex depth and the least corner value of the depth plane over the
+// tile's pixel centres, less the rounding that the reference's float sequence
+// (and this one) can add.  With u = 2^-24 every factor below is exact to 4u and
+// every sum to a few u of the magnitudes added, so a margin of 2^-18 of those
+// magnitudes (64 u) covers both.  Returned as the high 24 bits of a fragment
+// key's depth half (frag_key), rounded down; 0 (no bound) where the bound is
+// not positive -- negative depths order the other way round -- or not a
+// number.  Not for triangles whose edge values or area may wrap.
+__device__ __forceinline__ uint32_t depth_bound(const BinTri& t, float zmin, float zmax)
 {
-  TileTri t;
-  build_tile_tri(load_setup(&a.setup[gi]), X0, Y0, kRefBin, t);
-  BinTri q;
-  q.e0 = t.e[0]; q.e1 = t.e[1]; q.e2 = t.e[2];
-  q.sx0 = t.sx[0]; q.sx1 = t.sx[1]; q.sx2 = t.sx[2];
-  q.sy0 = t.sy[0]; q.sy1 = t.sy[1]; q.sy2 = t.sy[2];
-  q.lxe = t.lxe; q.lye = t.lye;
-  const bool draw = (t.trm & 1u) && t.ex1 >= t.ex0 && t.ey1 >= t.ey0 && t.rank1 != 0u;
-  q.flags = (draw ? kBinDraw : 0) | ((t.tam & 1u) ? kBinAccept : 0);
-  q.inv = t.inv; q.z2 = t.z2; q.z0mz2 = t.z0mz2; q.z1mz2 = t.z1mz2;
-  q.rank1 = t.rank1; q.gidx = gi; q.pad0 = 0; q.pad1 = 0;
-  out = q;
+  constexpr float kMargin = 3.814697265625e-6f;   // 2^-18
+  const float vertex = zmin - kMargin * zmax;
+  const float d0 = t.inv * t.z0mz2, d1 = t.inv * t.z1mz2;
+  const float t0 = (float)t.e1 * d0, t1 = (float)t.e2 * d1;
+  const float x0 = 7.0f * ((float)t.sx1 * d0), x1 = 7.0f * ((float)t.sx2 * d1);
+  const float y0 = 7.0f * ((float)t.sy1 * d0), y1 = 7.0f * ((float)t.sy2 * d1);
+  const float mag = fabsf(t.z2) + fabsf(t0) + fabsf(t1) + fabsf(x0) + fabsf(x1) + fabsf(y0) + fabsf(y1) + zmax;
+  const float plane = t.z2 + t0 + t1 + fminf(x0 + x1, 0.0f) + fminf(y0 + y1, 0.0f) - kMargin * mag;
+  const float lb = plane > vertex ? plane : vertex;
+  return lb > 0.0f ? (__float_as_uint(lb) | 0x80000000u) >> 8 : 0u;
 }
 
-// Entry t's fragment at tile pixel (ox, ly): barycentrics from the edge
-// values, z in the reference's operation order, and the order-independent key
-// update of that pixel (k, and the winning entry's index w when TRACK).
-template <bool TRACK>
-__device__ __forceinline__ void frag8_depth(const RasterFrameArgs& a, const Tile8& tl, const BinTri& t, int i, int ox,
-                                            int ly, unsigned long long& k, int& w)
+// What the resolve of a tile needs of an entry besides its BinTri, staged in
+// shared memory when the entry is built, so a pixel's winner is shaded from
+// shared memory: the vertex colours as floats (byte / 255) and the texture
+// coordinates, each as vertex 2's value and vertex 0's and 1's minus it -- the
+// differences shade_winner forms for every pixel, formed once.
+struct __align__(16) BinShade {
+  float c2[3], dc0[3], dc1[3];   // per channel
+  float u2, du0, du1;
+  float v2, dv0, dv1, pad;
+};
+static_assert(sizeof(BinShade) == 64, "BinShade layout");
+
+// A warp's entries.
+struct WarpEntries {
+  BinTri tri[32];
+  BinShade shade[32];
+  uint32_t mlo[32], mhi[32];   // coverage of pixel rows 0-3 and 4-7
+};
+
+// Depth bounds and their order are worth their cost (some 130 warp
+// instructions for 32 entries) only where the entries cover the tile's pixels
+// several times over: with at most this many covered samples (2.5 a pixel of
+// one tile) the entries stay in list order and every one is evaluated.
+constexpr unsigned kSparseSamples = 160;
+
+// Builds n <= 32 entries, entry l by lane l -- and lane l + 16 when n <= 16:
+// the two lanes then take four pixel rows each.  The lane's entry is list entry
+// gi (nothing drawn when ok is false) in the tile of scene S at (X0, Y0); seq
+// numbers the tiles of the entries, ascending with l.  Entries land in w
+// ordered by (seq, depth bound); m0 / m1 get bit i set where entry i covers the
+// lane's pixel (lane & 7, lane >> 3) / the pixel 4 rows above.  stage: w.shade
+// too.
+__device__ __forceinline__ void frag8_build(const RasterFrameArgs& a, const RasterSceneDev& S, int n, bool ok,
+                                            uint32_t gi, uint32_t seq, int X0, int Y0, bool stage, WarpEntries& w,
+                                            int lane, const float* inv255, unsigned& covered, uint32_t& m0,
+                                            uint32_t& m1)
+{
+  const bool pair = n <= 16;
+  const int ent = pair ? lane & 15 : lane;
+  BinTri t;
+  uint32_t lo = 0u, hi = 0u, vc[3] = {0u, 0u, 0u};
+  float2 q0 = make_float2(0.0f, 0.0f), q1 = q0, q2 = q0;
+  bool bounded = false;
+  float zmin = 0.0f, zmax = 0.0f;
+  if (ok) {
+    // the uv arrays are indexed by triangle id = setup slot - the scene's base
+    if (stage && S.uv) {
+      const uint32_t id = gi - S.tri_base;
+      q0 = __ldg(&S.uv[id]);
+      q1 = __ldg(&S.uv[(size_t)S.N + id]);
+      q2 = __ldg(&S.uv[2 * (size_t)S.N + id]);
+    }
+    const TriSetup r = load_setup(&a.setup[gi]);
+    const int32_t Xc = X0 * 16 + 8, Yc = Y0 * 16 + 8;
+    int32_t e[3], sx[3], sy[3], ta = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int j = i == 2 ? 0 : i + 1;
+      const int32_t dx = wsub(r.x[j], r.x[i]), dy = wsub(r.y[j], r.y[i]);
+      e[i] = edge_at(Xc, Yc, r.x[i], r.y[i], dx, dy);
+      sx[i] = -wshl(dy, 4);
+      sy[i] = wshl(dx, 4);
+      // trivial accept at the first pixel centre (raster.pikostage:201-211)
+      int32_t off = dy >= 0 ? sx[i] : 0;
+      off = wadd(off, dx < 0 ? sy[i] : 0);
+      ta |= wadd(e[i], wshl(off, kRefBinLg2));
+    }
+    // the bin is the triangle's: only its pixels remain to be tested
+    if (ta >= 0) {
+      lo = hi = 0xffffffffu;
+    } else if (r.hix > X0 * 16 && r.hiy > Y0 * 16) {
+      // (the box's high corner is rounded up to 16 px: it cuts no tile)
+      int ya = 0, yb = kRefBin - 1;
+      if (!(r.flags & kTriRisk)) {   // covered centres lie inside the triangle when no edge value can wrap
+        ya = max((min(min(r.y[0], r.y[1]), r.y[2]) >> 4) - 1 - Y0, 0);
+        yb = min((max(max(r.y[0], r.y[1]), r.y[2]) >> 4) - Y0, kRefBin - 1);
+      }
+      if (pair) {   // (the other lane of the pair takes the other rows)
+        if (lane < 16) yb = min(yb, 3); else ya = max(ya, 4);
+      }
+      int32_t r0 = wadd(e[0], wmul(ya, sy[0])), r1 = wadd(e[1], wmul(ya, sy[1])), r2 = wadd(e[2], wmul(ya, sy[2]));
+      unsigned long long m = 0ull;
+#pragma unroll 1
+      for (int y = ya; y <= yb; ++y) {
+        // pixel 7 first, so that pixel 0 ends in bit 0: bits of outside pixels
+        int32_t f0 = wadd(r0, wmul(7, sx[0])), f1 = wadd(r1, wmul(7, sx[1])), f2 = wadd(r2, wmul(7, sx[2]));
+        uint32_t out = 0u;
+#pragma unroll
+        for (int x = 0; x < kRefBin; ++x) {
+          out = __funnelshift_l((uint32_t)(f0 | f1 | f2), out, 1);
+          f0 = wsub(f0, sx[0]); f1 = wsub(f1, sx[1]); f2 = wsub(f2, sx[2]);
+        }
+        m |= (unsigned long long)(~out & 0xffu) << (8 * y);
+        r0 = wadd(r0, sy[0]); r1 = wadd(r1, sy[1]); r2 = wadd(r2, sy[2]);
+      }
+      lo = (uint32_t)m;
+      hi = (uint32_t)(m >> 32);
+    }
+    if (pair) {
+      if (lane < 16) hi = 0u; else lo = 0u;
+    }
+    t.e1 = e[1]; t.e2 = e[2];
+    t.sx1 = sx[1]; t.sx2 = sx[2];
+    t.sy1 = sy[1]; t.sy2 = sy[2];
+    t.inv = r.inv; t.z2 = r.z[2];
+    t.z0mz2 = r.z[0] - r.z[2];
+    t.z1mz2 = r.z[1] - r.z[2];
+    t.rank1 = r.rank1;
+    vc[0] = r.c[0]; vc[1] = r.c[1]; vc[2] = r.c[2];
+    bounded = !(r.flags & (kTriRisk | kTriAreaRisk));
+    zmin = fminf(fminf(r.z[0], r.z[1]), r.z[2]);
+    zmax = fmaxf(fmaxf(fabsf(r.z[0]), fabsf(r.z[1])), fabsf(r.z[2]));
+    if (a.cov_cap) {   // coverage dump
+      for (unsigned long long m = ((unsigned long long)hi << 32) | lo; m; m &= m - 1) {
+        const int p = __ffsll(m) - 1;
+        const uint32_t slot = atomicAdd(&a.ctr->cov_count, 1u);
+        if (slot < a.cov_cap) {
+          a.cov_tri[slot] = gi - S.tri_base;
+          a.cov_pix[slot] = (uint32_t)((Y0 + (p >> 3)) * S.W + X0 + (p & 7));
+        }
+      }
+    }
+  }
+  const unsigned mine = __popc(lo) + __popc(hi);
+  covered += mine;
+  // place by (tile, depth bound, lane)
+  int at = ent;
+  t.bound = 0u;
+  if (__reduce_add_sync(kFull, mine) > kSparseSamples) {
+    if (bounded) t.bound = depth_bound(t, zmin, zmax);
+    const uint32_t key = (seq << 29) | (t.bound << 5) | (uint32_t)ent;
+    at = 0;
+    for (int i = 0; i < n; ++i) at += __shfl_sync(kFull, key, i) < key ? 1 : 0;
+  }
+  __syncwarp();   // every lane is done with the entries that w held
+  if (lane < n) {
+    w.tri[at] = t;
+    if (stage) {
+      BinShade h;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float v0 = inv255[(vc[0] >> (8 * c)) & 255u], v1 = inv255[(vc[1] >> (8 * c)) & 255u];
+        const float v2 = inv255[(vc[2] >> (8 * c)) & 255u];
+        h.c2[c] = v2;
+        h.dc0[c] = v0 - v2;
+        h.dc1[c] = v1 - v2;
+      }
+      h.u2 = q2.x; h.du0 = q0.x - q2.x; h.du1 = q1.x - q2.x;
+      h.v2 = q2.y; h.dv0 = q0.y - q2.y; h.dv1 = q1.y - q2.y;
+      h.pad = 0.0f;
+      w.shade[at] = h;
+    }
+  }
+  if (ent >= n) at = ent;   // no entry: an empty mask
+  if (!pair || lane < 16) w.mlo[at] = lo;
+  if (!pair) w.mhi[at] = hi;
+  else if (lane >= 16) w.mhi[at] = hi;
+  if (pair && lane >= 16) { w.mlo[lane] = 0u; }
+  if (pair && lane < 16) { w.mhi[lane + 16] = 0u; }
+  __syncwarp();
+  m0 = transpose32(w.mlo[lane], lane);
+  m1 = transpose32(w.mhi[lane], lane);
+}
+
+// Entry t's fragment at tile pixel (ox, ly): barycentrics from the edge values,
+// z in the reference's operation order, as a key of the order-independent depth
+// test.
+__device__ __forceinline__ unsigned long long frag8_key(const BinTri& t, int ox, int ly)
 {
   const int32_t g1 = wadd(wadd(t.e1, wmul(ox, t.sx1)), wmul(ly, t.sy1));
   const int32_t g2 = wadd(wadd(t.e2, wmul(ox, t.sx2)), wmul(ly, t.sy2));
   const float alpha = (float)g1 * t.inv;
   const float beta = (float)g2 * t.inv;
   const float z = t.z2 + alpha * t.z0mz2 + beta * t.z1mz2;
-  const unsigned long long key = frag_key(z, t.rank1);
-  if (key < k) { k = key; if (TRACK) w = i; }
-  if (a.cov_cap) {
-    const uint32_t slot = atomicAdd(&a.ctr->cov_count, 1u);
-    if (slot < a.cov_cap) {
-      a.cov_tri[slot] = t.gidx - tl.S->tri_base;
-      a.cov_pix[slot] = (uint32_t)((tl.Y0 + ly) * tl.S->W + tl.X0 + ox);
-    }
-  }
+  return frag_key(z, t.rank1);
 }
 
-// Tests the lane's two pixels of tile tl against entries st[0, n) (n <= 32)
-// and folds the covered fragments into the lane's keys.  TRACK: w0 / w1 also
-// follow the entry index (into st) of each pixel's current winner.
-template <bool TRACK>
-__device__ __forceinline__ void frag8_test(const RasterFrameArgs& a, const Tile8& tl, const BinTri* st, int n, int lane,
-                                           unsigned& covered, unsigned long long& k0, unsigned long long& k1,
-                                           int& w0, int& w1)
+// Folds the fragments of entries m0 / m1 (bits: the lane's two pixels) into the
+// lane's keys; w0 / w1 follow the entry of each pixel's current winner.  A trip
+// takes the next covered entry of each pixel: two independent evaluations
+// without a branch (a pixel that is done evaluates entry 31 or 0 and drops the
+// result).  A pixel is done when its bits are, or at the first entry whose
+// bound lies behind its depth: later ones of the tile lie behind it too.
+__device__ __forceinline__ void frag8_test(const BinTri* st, uint32_t m0, uint32_t m1, int lane,
+                                           unsigned long long& k0, unsigned long long& k1, int& w0, int& w1)
 {
   const int ox = lane & 7, oy = lane >> 3;   // first pixel; the second is (ox, oy + 4)
-  // coverage: bit i of m0 / m1 = entry i covers the lane's first / second pixel
-  uint32_t m0 = 0, m1 = 0;
-#pragma unroll 4
-  for (int i = 0; i < n; ++i) {
-    const int4 q2 = *reinterpret_cast<const int4*>(&st[i].sy2);
-    const bool draw = (q2.w & kBinDraw) != 0, accept = (q2.w & kBinAccept) != 0;
-    bool c0 = draw, c1 = draw;
-    if (draw && !accept) {   // (one entry for the whole warp: a uniform branch)
-      const int4 q0 = *reinterpret_cast<const int4*>(&st[i].e0);
-      const int4 q1 = *reinterpret_cast<const int4*>(&st[i].sx1);
-      const int32_t f0 = wadd(wadd(q0.x, wmul(ox, q0.w)), wmul(oy, q1.z));
-      const int32_t f1 = wadd(wadd(q0.y, wmul(ox, q1.x)), wmul(oy, q1.w));
-      const int32_t f2 = wadd(wadd(q0.z, wmul(ox, q1.y)), wmul(oy, q2.x));
-      const int32_t g0 = wadd(f0, wshl(q1.z, 2)), g1 = wadd(f1, wshl(q1.w, 2)), g2 = wadd(f2, wshl(q2.x, 2));
-      const bool inx = ox < q2.y;
-      c0 = inx && oy < q2.z && (f0 | f1 | f2) >= 0;
-      c1 = inx && oy + 4 < q2.z && (g0 | g1 | g2) >= 0;
-    }
-    m0 |= (uint32_t)c0 << i;
-    m1 |= (uint32_t)c1 << i;
-  }
-  covered += __popc(m0) + __popc(m1);
-  // depth: barycentrics from the same edge values, z in the reference's
-  // operation order, and the order-independent key update
-  // one covered entry of each of the lane's two pixels per trip (two
-  // independent depth evaluations); each pixel still takes its entries in
-  // ascending order
   while (m0 | m1) {
-    if (m0) {
-      const int i = __ffs(m0) - 1;
-      m0 &= m0 - 1u;
-      frag8_depth<TRACK>(a, tl, st[i], i, ox, oy, k0, w0);
-    }
-    if (m1) {
-      const int i = __ffs(m1) - 1;
-      m1 &= m1 - 1u;
-      frag8_depth<TRACK>(a, tl, st[i], i, ox, oy + 4, k1, w1);
-    }
-  }
-}
-
-// Rasterizes list entries [b, e) of tile tl into the lane's two keys, 32
-// entries at a time.
-__device__ __forceinline__ void frag8_entries(const RasterFrameArgs& a, const Tile8& tl, uint32_t b, uint32_t e,
-                                              BinTri* st, int lane, unsigned& covered, unsigned long long& k0,
-                                              unsigned long long& k1)
-{
-  // entries past the list capacity are never read (the frame reports the overflow)
-  const uint32_t lim = a.list_cap - min(tl.off, a.list_cap);
-  e = min(e, lim);
-  for (uint32_t b0 = b; b0 < e; b0 += 32) {
-    if (b0 + lane < e) frag8_build(a, a.tile_list[tl.off + b0 + lane], tl.X0, tl.Y0, st[lane]);
-    __syncwarp();
-    int w0 = 0, w1 = 0;
-    frag8_test<false>(a, tl, st, (int)min(32u, e - b0), lane, covered, k0, k1, w0, w1);
-    __syncwarp();  // every lane is done with st[] before it is rebuilt
+    const int i0 = (__ffs(m0) - 1) & 31, i1 = (__ffs(m1) - 1) & 31;
+    const BinTri a = st[i0], b = st[i1];
+    const unsigned long long ka = frag8_key(a, ox, oy), kb = frag8_key(b, ox, oy + 4);
+    const bool pa = m0 != 0u && a.bound <= (uint32_t)(k0 >> 40), pb = m1 != 0u && b.bound <= (uint32_t)(k1 >> 40);
+    if (pa && ka < k0) { k0 = ka; w0 = i0; }
+    if (pb && kb < k1) { k1 = kb; w1 = i1; }
+    m0 = pa ? m0 & (m0 - 1u) : 0u;
+    m1 = pb ? m1 & (m1 - 1u) : 0u;
   }
 }
 
@@ -1393,18 +1531,6 @@ __device__ __forceinline__ void resolve8(const RasterFrameArgs& a, const Tile8& 
   }
 }
 
-// What the resolve of a light tile needs of an entry besides its BinTri,
-// staged in shared memory when the entry is built, so a pixel's winner is
-// shaded from shared memory: the vertex colours as floats (byte / 255) and the
-// texture coordinates, each as vertex 2's value and vertex 0's and 1's minus
-// it -- the differences shade_winner forms for every pixel, formed once.
-struct __align__(16) BinShade {
-  float c2[3], dc0[3], dc1[3];   // per channel
-  float u2, du0, du1;
-  float v2, dv0, dv1, pad;
-};
-static_assert(sizeof(BinShade) == 64, "BinShade layout");
-
 // The colour of entry t / sh at tile pixel (ox, ly): shade_winner's arithmetic
 // (raster.pikostage:244-309) from the tile-local edge values, which equal the
 // pixel-centre edge values bit for bit (both are the same wrapping int32
@@ -1429,8 +1555,7 @@ __device__ __forceinline__ uint32_t shade_entry(const RasterSceneDev& S, const B
     col[1] = col[1] * inv255[tt.y];
     col[2] = col[2] * inv255[tt.z];
   }
-  return 0xff000000u | (cvt_u32_x86(col[2] * 255.0f) << 16) | (cvt_u32_x86(col[1] * 255.0f) << 8) |
-         cvt_u32_x86(col[0] * 255.0f);
+  return pack_abgr(col[0], col[1], col[2]);
 }
 
 // Writes the lane's two pixels of a light tile from its winners' staged data
@@ -1462,128 +1587,27 @@ __device__ __forceinline__ void resolve8_staged(const Tile8& tl, int lane, unsig
   }
 }
 
-// A group of up to kLightGroup consecutive tiles whose lists hold at most
-// queue_min (<= 32 / kLightGroup) entries each: their offsets, list entries
-// and setup records are fetched together (one round of loads for the group,
-// at most 32 entries, one per lane), then each tile is tested and resolved.
-template <bool ONE>
-__device__ __forceinline__ void light_group(const RasterFrameArgs& a, const uint32_t* tb, uint32_t t0, uint32_t t1,
-                                            uint32_t lim, BinTri* st, BinShade* sh, int lane, unsigned& covered,
-                                            const float* inv255)
-{
-  const int nt = (int)(t1 - t0);
-  // lane j <= nt holds tile_off[t0 + j]
-  const uint32_t offj = lane <= nt ? a.tile_off[t0 + lane] : 0u;
-  uint32_t cnt = 0;     // lane j < nt: entries of tile t0 + j (0 when it is served as chunks)
-  bool served = false;  // lane j < nt: tile t0 + j is drawn by this group (its list fits)
-  {
-    const uint32_t next = __shfl_down_sync(kFull, offj, 1);
-    if (lane < nt) {
-      cnt = next - offj;
-      served = cnt <= lim;
-      if (!served) cnt = 0;
-    }
-  }
-  const unsigned served_m = __ballot_sync(kFull, served);
-  // inclusive prefix of the counts over the group's tiles
-  uint32_t incl = cnt;
-#pragma unroll
-  for (int o = 1; o < kLightGroup; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += v;
-  }
-  uint32_t inc[kLightGroup];
-#pragma unroll
-  for (int q = 0; q < kLightGroup; ++q) inc[q] = __shfl_sync(kFull, incl, q);
-  const uint32_t total = inc[kLightGroup - 1];
-  // lane l < total builds entry l, of tile j = the first with inc[j] > l
-  int j = 0;
-#pragma unroll
-  for (int q = 0; q < kLightGroup - 1; ++q)
-    if ((uint32_t)lane >= inc[q]) j = q + 1;
-  const uint32_t off = __shfl_sync(kFull, offj, j);
-  if ((uint32_t)lane < total) {
-    const Tile8 g = tile8_geom<ONE>(a, tb, t0 + (uint32_t)j);
-    uint32_t first = 0;
-#pragma unroll
-    for (int q = 0; q < kLightGroup - 1; ++q)
-      if (q < j) first = inc[q];
-    const uint32_t idx = off + ((uint32_t)lane - first);
-    if (idx < a.list_cap) {
-      const uint32_t gi = a.tile_list[idx];
-      // the entry's colours and texture coordinates, for the resolve (the
-      // uv arrays are indexed by triangle id = setup slot - the scene's base)
-      const RasterSceneDev& S = *g.S;
-      float2 q0 = make_float2(0.0f, 0.0f), q1 = q0, q2 = q0;
-      if (S.uv) {
-        const uint32_t id = gi - S.tri_base;
-        q0 = __ldg(&S.uv[id]);
-        q1 = __ldg(&S.uv[(size_t)S.N + id]);
-        q2 = __ldg(&S.uv[2 * (size_t)S.N + id]);
-      }
-      const TriSetup r = load_setup(&a.setup[gi]);
-      TileTri t;
-      build_tile_tri(r, g.X0, g.Y0, kRefBin, t);
-      BinTri bq;
-      bq.e0 = t.e[0]; bq.e1 = t.e[1]; bq.e2 = t.e[2];
-      bq.sx0 = t.sx[0]; bq.sx1 = t.sx[1]; bq.sx2 = t.sx[2];
-      bq.sy0 = t.sy[0]; bq.sy1 = t.sy[1]; bq.sy2 = t.sy[2];
-      bq.lxe = t.lxe; bq.lye = t.lye;
-      const bool draw = (t.trm & 1u) && t.ex1 >= t.ex0 && t.ey1 >= t.ey0 && t.rank1 != 0u;
-      bq.flags = (draw ? kBinDraw : 0) | ((t.tam & 1u) ? kBinAccept : 0);
-      bq.inv = t.inv; bq.z2 = t.z2; bq.z0mz2 = t.z0mz2; bq.z1mz2 = t.z1mz2;
-      bq.rank1 = t.rank1; bq.gidx = gi; bq.pad0 = 0; bq.pad1 = 0;
-      st[lane] = bq;
-      BinShade hq;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float v0 = inv255[(r.c[0] >> (8 * c)) & 255u], v1 = inv255[(r.c[1] >> (8 * c)) & 255u];
-        const float v2 = inv255[(r.c[2] >> (8 * c)) & 255u];
-        hq.c2[c] = v2;
-        hq.dc0[c] = v0 - v2;
-        hq.dc1[c] = v1 - v2;
-      }
-      hq.u2 = q2.x; hq.du0 = q0.x - q2.x; hq.du1 = q1.x - q2.x;
-      hq.v2 = q2.y; hq.dv0 = q0.y - q2.y; hq.dv1 = q1.y - q2.y;
-      hq.pad = 0.0f;
-      sh[lane] = hq;
-    } else {
-      st[lane].flags = 0;  // past the list capacity: the frame reports the overflow
-    }
-  }
-  __syncwarp();
-  // one copy of the test and resolve code (the loop stays rolled: the kernel's
-  // instruction footprint matters more than the loop overhead)
-  uint32_t first = 0;
-#pragma unroll 1
-  for (int q = 0; q < nt; ++q) {
-    const uint32_t iq = __shfl_sync(kFull, incl, q);
-    if ((served_m >> q) & 1u) {  // (longer lists are drawn as chunks)
-      const Tile8 tl = tile8_geom<ONE>(a, tb, t0 + (uint32_t)q);
-      unsigned long long k0 = kInitKey, k1 = kInitKey;
-      int w0 = 0, w1 = 0;
-      frag8_test<true>(a, tl, st + first, (int)(iq - first), lane, covered, k0, k1, w0, w1);
-      resolve8_staged(tl, lane, k0, k1, w0, w1, st + first, sh + first, inv255);
-    }
-    first = iq;
-  }
-  __syncwarp();  // every lane is done with st[] before the next group rebuilds it
-}
-
-// Persistent: warp w of the grid first draws the short-list groups w,
-// w + warps, ... (light_group), then takes chunks of the long lists (scan_tiles
-// queued them) from a counter; each chunk stores its keys, and the warp that
-// completes a tile's last chunk takes the per-pixel minimum over the tile's
-// chunks and resolves the tile.  The key order makes the result independent of
-// which warp merges when.
+// Persistent.  A warp works in passes of up to 32 list entries (one copy of the
+// code for every kind of pass: the kernel's instruction footprint matters more
+// than the branches between them).  Warp w of the grid first draws the
+// short-list groups w, w + warps, ... (a.group consecutive tiles; of these
+// the ones with at most a.queue_min entries, as many tiles at a time as have 32
+// entries together); then it takes chunks of the longer lists (scan_tiles
+// queued them) from a counter, which also evens out the warps' finishing times.
+// A tile whose list fits one pass is resolved from shared memory.  Of a list
+// in several chunks each leaves its keys, and the warp that completes the last
+// one takes the per-pixel minimum over the tile's chunks and resolves the tile.
+// The key order makes the result independent of which warp merges when.
+// (Taking most chunks by warp index instead, with the next one's list read
+// ahead, measured 5-20% slower: the short-list phase leaves the warps too
+// uneven.  So did asking for the next chunk before the current one is done.)
 template <bool ONE>
 __global__ void __launch_bounds__(256, 4) raster_frag8(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_wait();
   frame_begin(a);
   if (list_overflowed(a)) return;
-  __shared__ BinTri s_tri[8][32];
-  __shared__ BinShade s_shade[8][32];
+  __shared__ WarpEntries s_ent[8];
   __shared__ float s_inv255[256];
   __shared__ unsigned s_cov[8];
   __shared__ uint32_t s_tb[kSceneTable];
@@ -1592,64 +1616,128 @@ __global__ void __launch_bounds__(256, 4) raster_frag8(const __grid_constant__ R
   __syncthreads();
   const int wid = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  BinTri* st = s_tri[wid];
+  WarpEntries& w = s_ent[wid];
   unsigned covered = 0;
-  const uint32_t C = a.chunk;
-  const unsigned long long hacc = a.ctr->bin.heavy_acc;
-  const uint32_t n_heavy = min((uint32_t)(hacc >> 32), a.heavy_cap);
-  const uint32_t n_chunks = min((uint32_t)hacc, a.chunk_cap);
-
-  // The short lists first, kLightGroup consecutive tiles per group, warp w
-  // of the grid taking groups w, w + warps, ... (no counter: the groups cost
-  // about the same); then one counter hands out the heavy tiles' chunks (every
-  // list longer than a.queue_min entries, cut into chunks of a.chunk), which
-  // also evens out the warps' finishing times.  (Asking for the next item
-  // while working on the current one measured slower: a warp busy with a long
-  // item holds work that idle warps could take.)
-  const uint32_t n_groups = (a.n_tiles_total + kLightGroup - 1) / kLightGroup;
+  const uint32_t n_chunks = min((uint32_t)a.ctr->bin.heavy_acc, a.chunk_cap);
+  const uint32_t n_groups = (a.n_tiles_total + a.group - 1) / a.group;
   const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t g = blockIdx.x * (blockDim.x >> 5) + (uint32_t)wid; g < n_groups; g += nwarps) {
-    const uint32_t t0 = g * kLightGroup;
-    light_group<ONE>(a, s_tb, t0, min(t0 + kLightGroup, a.n_tiles_total), a.queue_min, st, s_shade[wid], lane, covered,
-                s_inv255);
-  }
+  uint32_t g = blockIdx.x * (blockDim.x >> 5) + (uint32_t)wid;   // the next group
+  // The group being drawn: tiles t0 + ja .. t0 + nt remain; lane j <= nt holds
+  // the offset, the entries (0 when it is served as chunks) and the inclusive
+  // prefix of tile t0 + j.
+  uint32_t t0 = 0, off_j = 0, cnt_j = 0, incl_j = 0;
+  unsigned served = 0;
+  int ja = 0, nt = 0;
+  // The chunk being drawn: entries [b0, len) at off remain; lane l < 8 holds
+  // word l of its descriptor.
+  uint32_t ci = 0, desc = 0, b0 = 0, len = 0;
+  unsigned long long k0 = kInitKey, k1 = kInitKey;
+  int w0 = 0, w1 = 0;
   for (;;) {
-    uint32_t ci = 0;
-    if (lane == 0) ci = atomicAdd(&a.ctr->work_next, 1u);
-    ci = __shfl_sync(kFull, ci, 0);
-    if (ci >= n_chunks) break;
-    const uint32_t h = a.chunk_heavy[ci];
-    if (h >= n_heavy) continue;  // only after a heavy-queue overflow (reported; the frame is redrawn)
-    const uint32_t c0 = a.chunk_base[h];
-    const Tile8 tl = tile8_at<ONE>(a, s_tb, a.heavy[h]);
-    const uint32_t nch = (tl.cnt + C - 1) / C;
-    if (ci - c0 >= nch) continue;  // only after a heavy-queue overflow (reported; the frame is redrawn)
-    unsigned long long k0 = kInitKey, k1 = kInitKey;
-    frag8_entries(a, tl, (ci - c0) * C, min((ci - c0) * C + C, tl.cnt), st, lane, covered, k0, k1);
-    if (nch == 1) {   // the whole list in one chunk: no keys to merge
-      resolve8(a, tl, lane, k0, k1, s_inv255);
-      continue;
-    }
-    // pixel p of the tile is key p of the chunk: the lane's pixels are lane and lane + 32
-    unsigned long long* ck = a.chunk_keys + (size_t)ci * 64;
-    ck[lane] = k0;
-    ck[lane + 32] = k1;
-    __threadfence();
-    __syncwarp();
-    uint32_t done = 0;
-    if (lane == 0) done = atomicAdd(&a.hdone[h], 1u);
-    done = __shfl_sync(kFull, done, 0);
-    if (done + 1 == nch) {
-      // the tile's last chunk: every other chunk's keys are in chunk_keys
-      __threadfence();
-      for (uint32_t j = 0; j < nch; ++j) {
-        if (c0 + j == ci) continue;
-        const unsigned long long* cj = a.chunk_keys + (size_t)(c0 + j) * 64;
-        k0 = min(k0, __ldcg(&cj[lane]));
-        k1 = min(k1, __ldcg(&cj[lane + 32]));
+    const bool light = ja < nt || g < n_groups;
+    bool ok, stage = true;
+    int n, jb;
+    uint32_t base = 0, tile, idx, seq = 0;
+    if (light) {
+      if (ja >= nt) {
+        t0 = g * a.group;
+        nt = (int)min(a.group, a.n_tiles_total - t0);
+        g += nwarps;
+        ja = 0;
+        off_j = lane <= nt ? a.tile_off[t0 + lane] : 0u;
+        cnt_j = __shfl_down_sync(kFull, off_j, 1) - off_j;
+        const bool fits = lane < nt && cnt_j <= a.queue_min;
+        if (!fits) cnt_j = 0;
+        served = __ballot_sync(kFull, fits);
+        incl_j = cnt_j;
+#pragma unroll
+        for (int o = 1; o < kLightGroup; o <<= 1) {
+          const uint32_t v = __shfl_up_sync(kFull, incl_j, o);
+          if (lane >= o) incl_j += v;
+        }
       }
-      resolve8(a, tl, lane, k0, k1, s_inv255);
+      // tiles [ja, jb): as many as have at most 32 entries together
+      if (ja) base = __shfl_sync(kFull, incl_j, ja - 1);
+      jb = ja + __popc(__ballot_sync(kFull, lane >= ja && lane < nt && incl_j - base <= 32u));
+      n = (int)(__shfl_sync(kFull, incl_j, jb - 1) - base);
+      // entry l is of tile j = the first with an inclusive prefix above l
+      const uint32_t l = (uint32_t)(n <= 16 ? lane & 15 : lane);
+      int j = ja;
+      for (int q = ja; q < jb - 1; ++q) j += __shfl_sync(kFull, incl_j, q) - base <= l ? 1 : 0;
+      idx = __shfl_sync(kFull, off_j, j) + (l + base - __shfl_sync(kFull, incl_j - cnt_j, j));
+      ok = l < (uint32_t)n;
+      tile = t0 + (uint32_t)j;
+      seq = (uint32_t)(j - ja);
+    } else {
+      if (b0 >= len) {
+        if (lane == 0) ci = atomicAdd(&a.ctr->work_next, 1u);
+        ci = __shfl_sync(kFull, ci, 0);
+        if (ci >= n_chunks) break;
+        if (lane < 8) desc = reinterpret_cast<const uint32_t*>(&a.chunk_desc[ci])[lane];
+        len = __shfl_sync(kFull, desc, 2);
+        b0 = 0;
+        k0 = k1 = kInitKey;
+      }
+      ja = nt = 0;
+      jb = 1;
+      n = (int)min(32u, len - b0);
+      const uint32_t l = (uint32_t)(n <= 16 ? lane & 15 : lane);
+      tile = __shfl_sync(kFull, desc, 0);
+      idx = __shfl_sync(kFull, desc, 1) + b0 + l;
+      ok = l < (uint32_t)n;
+      stage = len <= 32u && __shfl_sync(kFull, desc, 5) == 1u;
+      b0 += 32;
     }
+    uint32_t m0 = 0u, m1 = 0u;
+    if (n) {
+      const Tile8 tl = tile8_geom<ONE>(a, s_tb, tile);
+      ok = ok && idx < a.list_cap;   // (past the list capacity: the frame reports the overflow)
+      frag8_build(a, *tl.S, n, ok, ok ? a.tile_list[idx] : 0u, seq, tl.X0, tl.Y0, stage, w, lane, s_inv255, covered, m0,
+                  m1);
+    }
+#pragma unroll 1
+    for (int q = ja; q < jb; ++q) {
+      uint32_t bits = 0xffffffffu;
+      Tile8 tl;
+      if (light) {
+        if (!((served >> q) & 1u)) continue;   // (longer lists are drawn as chunks)
+        const uint32_t last = __shfl_sync(kFull, incl_j, q) - base, cnt = __shfl_sync(kFull, cnt_j, q);
+        if (cnt < 32u) bits = ((1u << cnt) - 1u) << ((last - cnt) & 31u);
+        tl = tile8_geom<ONE>(a, s_tb, t0 + (uint32_t)q);
+        k0 = k1 = kInitKey;
+      } else {
+        tl = tile8_geom<ONE>(a, s_tb, tile);
+      }
+      frag8_test(w.tri, m0 & bits, m1 & bits, lane, k0, k1, w0, w1);
+      if (stage) {
+        resolve8_staged(tl, lane, k0, k1, w0, w1, w.tri, w.shade, s_inv255);
+      } else if (b0 >= len) {
+        const uint32_t nch = __shfl_sync(kFull, desc, 5);
+        if (nch > 1) {
+          // pixel p of the tile is key p of the chunk: the lane's pixels are lane and lane + 32
+          unsigned long long* ck = a.chunk_keys + (size_t)ci * 64;
+          ck[lane] = k0;
+          ck[lane + 32] = k1;
+          __threadfence();
+          __syncwarp();
+          const uint32_t h = __shfl_sync(kFull, desc, 3), c0 = ci - __shfl_sync(kFull, desc, 4);
+          uint32_t done = 0;
+          if (lane == 0) done = atomicAdd(&a.hdone[h], 1u);
+          done = __shfl_sync(kFull, done, 0);
+          if (done + 1 != nch) continue;
+          // the tile's last chunk: every other chunk's keys are in chunk_keys
+          __threadfence();
+          for (uint32_t c = c0; c < c0 + nch; ++c) {
+            if (c == ci) continue;
+            const unsigned long long* cj = a.chunk_keys + (size_t)c * 64;
+            k0 = min(k0, __ldcg(&cj[lane]));
+            k1 = min(k1, __ldcg(&cj[lane + 32]));
+          }
+        }
+        resolve8(a, tl, lane, k0, k1, s_inv255);
+      }
+    }
+    ja = light ? jb : 0;
   }
 
   // fragment count: one atomic per CTA

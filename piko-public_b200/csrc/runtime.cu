@@ -65,7 +65,7 @@ uint32_t heavy_threshold(int tile)
 piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, RasterScratch& scr, int T, int ctas,
                                  cudaStream_t st, bool timed, bool coverage, uint32_t chunk, bool table_ready)
 {
-  if (chunk == 0) chunk = kDefaultChunk;
+  if (chunk == 0) chunk = T == kRefBin ? kDefaultChunk8 : kDefaultChunk;
   uint32_t tris = 0, tiles = 0;
   for (int i = 0; i < n; ++i) {
     int tx, ty;
@@ -74,8 +74,17 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   }
   uint32_t list_need = std::max<uint32_t>(scr.list_cap, 4u * tris + tiles + 1024u);
   CU(ctx, scr.ensure(tris, tiles, list_need, n));
-  static_assert(kQueueMin <= kQueueMax, "a group of short lists must fit one warp");
-  const uint32_t queue_min = std::min(kQueueMin, chunk);
+  static_assert(2 * kQueueMin <= kQueueMax, "a short list must fit one warp");
+  // 8x8 tiles: the short-list groups are sized so that every warp of the grid
+  // has one (giants at 1021x767, 12,288 tiles: fragment pass 29 -> 26 us with 4
+  // tiles a group instead of 8); with several groups of 8 per warp the lists
+  // they draw may be twice as long, which saves the counter's chain of reads
+  // for those tiles (24-scene batch: 293 -> 278 us; at one group per warp the
+  // forest's takes 39 us instead of 35)
+  const uint32_t warps = (uint32_t)ctas * 8u;
+  uint32_t group = (uint32_t)kLightGroup;
+  while (group > 1 && tiles / group < warps) group /= 2;
+  const uint32_t queue_min = std::min(tiles / warps >= 4u * kLightGroup ? 2u * kQueueMin : kQueueMin, chunk);
   CU(ctx, scr.ensure_heavy(tiles, T, chunk, queue_min));
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   CU(ctx, cudaStreamIsCapturing(st, &capture));
@@ -120,7 +129,6 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   a.pair_tl = scr.pair_tl;
   a.pair_g = scr.pair_g;
   a.list_cap = scr.list_cap;
-  a.heavy = scr.heavy;
   a.heavy_threshold = heavy_threshold(T);
   a.heavy_cap = scr.heavy_cap;
   a.large_seg = scr.large_seg;
@@ -129,8 +137,8 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   a.big_cap = scr.seg_cap;
   a.chunk = chunk;
   a.queue_min = queue_min;
-  a.chunk_base = scr.chunk_base;
-  a.chunk_heavy = scr.chunk_heavy;
+  a.group = group;
+  a.chunk_desc = scr.chunk_desc;
   a.hdone = scr.hdone;
   a.chunk_keys = scr.chunk_keys;
   a.chunk_cap = scr.chunk_cap;

@@ -103,14 +103,12 @@ struct RasterScratch {
   uint32_t* tile_list = nullptr;
   unsigned long long* pair_tl = nullptr;  // count-pass pair records, [list_cap] each
   uint32_t* pair_g = nullptr;
-  uint32_t* heavy = nullptr;
   uint2* large_seg = nullptr;   // large-triangle segment items
   uint32_t seg_cap = 0;
   WalkTri* large_walk = nullptr;  // walk records of the large triangles, [seg_cap]: each has a segment
-  uint32_t* chunk_base = nullptr;           // first chunk per heavy tile
   uint32_t* hdone = nullptr;                // finished chunks per heavy tile
   unsigned long long* chunk_keys = nullptr; // tile * tile keys per chunk
-  uint32_t* chunk_heavy = nullptr;          // heavy tile of each chunk
+  ChunkDesc* chunk_desc = nullptr;
   uint32_t heavy_cap = 0, chunk_cap = 0;
   uint32_t chunk_stride = 0;                // keys per chunk (tile * tile)
   unsigned long long* scan_flags = nullptr;
@@ -132,8 +130,8 @@ struct RasterScratch {
   void release()
   {
     dfree(setup); dfree(tile_cnt); dfree(tile_off); dfree(tile_list); dfree(pair_tl); dfree(pair_g);
-    dfree(heavy); dfree(large_seg); dfree(large_walk); dfree(chunk_base); dfree(hdone); dfree(chunk_keys);
-    dfree(chunk_heavy);
+    dfree(large_seg); dfree(large_walk); dfree(hdone); dfree(chunk_keys);
+    dfree(chunk_desc);
     dfree(scan_flags); dfree(work); dfree(ctr); dfree(d_scenes); dfree(cov_tri); dfree(cov_pix);
     if (h_ctr) cudaFreeHost(h_ctr);
     if (cap_scenes) cudaFreeHost(cap_scenes);
@@ -156,11 +154,9 @@ struct RasterScratch {
     const bool t8 = T == kRefBin;
     const uint32_t need_h = t8 ? std::min<uint32_t>(n_tiles, list_cap / (queue_min + 1) + 1) : n_tiles;
     cudaError_t e = cudaSuccess;
-    if (need_h > heavy_cap || !chunk_base) {
-      dfree(heavy); dfree(chunk_base); dfree(hdone);
+    if (need_h > heavy_cap || !hdone) {
+      dfree(hdone);
       heavy_cap = 0;
-      if ((e = dalloc(&heavy, need_h))) return e;
-      if ((e = dalloc(&chunk_base, need_h))) return e;
       if ((e = dalloc(&hdone, need_h))) return e;
       heavy_cap = need_h;
     }
@@ -200,10 +196,10 @@ struct RasterScratch {
   cudaError_t grow_chunks(uint32_t n, uint32_t stride)
   {
     dfree(chunk_keys);
-    dfree(chunk_heavy);
+    dfree(chunk_desc);
     chunk_cap = 0;
     cudaError_t e = dalloc(&chunk_keys, (size_t)n * stride);
-    if (!e) e = dalloc(&chunk_heavy, n);
+    if (!e) e = dalloc(&chunk_desc, n);
     if (!e) { chunk_cap = n; chunk_stride = stride; }
     return e;
   }
@@ -222,7 +218,7 @@ struct RasterScratch {
       if ((e = grow_list(need + need / 4 + 1024))) return e;
     }
     const uint32_t chunks = (uint32_t)c.heavy_acc;
-    if (chunk_base && chunks > chunk_cap) {
+    if (chunk_desc && chunks > chunk_cap) {
       if ((e = grow_chunks(chunks + chunks / 4 + 64, chunk_stride))) return e;
     }
     // every large triangle has at least one segment: seg_cap bounds both
@@ -375,7 +371,7 @@ struct RasterDraw {
 };
 // chunk: list entries per chunk of the 8x8 tile queue (kDefaultChunk when 0);
 // lists longer than kQueueMin entries are queued as chunks
-constexpr uint32_t kDefaultChunk = 32;
+constexpr uint32_t kDefaultChunk = 32, kDefaultChunk8 = 64;
 constexpr uint32_t kQueueMin = 8;
 // table_ready: the scene table in scr already holds these draws
 piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, RasterScratch& scr, int T, int ctas,
