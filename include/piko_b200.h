@@ -99,7 +99,8 @@ typedef struct piko_pipe_desc {
   int max_splits;
   int dice_grid;
   /* device tuning: list entries per work item of the 8x8 raster tile queue; a
-   * tile with a longer list is split over several warps (0 = 32) */
+   * tile with a longer list is split over several warps (0 = 64, 128 for 32-px
+   * tiles) */
   int chunk_entries;
   /* Reyes sampling and shading variants, no reference counterpart (0 = the
    * reference: one sample at the pixel centre, corners lit and averaged).
@@ -248,7 +249,7 @@ piko_status piko_batch_destroy(piko_batch* batch);
  * <= 1280x720, larger) x triangle class (< 4K, < 16K, < 64K, more);
  * bucket = resolution_class * 4 + triangle_class.  Each bucket holds a tile
  * edge (8/16/32 px), persistent CTAs per SM (0 = occupancy) and 8x8-queue
- * chunk size (0 = 32).  Every configuration renders the identical image. */
+ * chunk size (0 = 64, 128 at 32-px tiles).  Every configuration renders the identical image. */
 #define PIKO_TUNE_BUCKETS 16
 typedef struct piko_tuner piko_tuner;
 typedef struct piko_tune_cfg {

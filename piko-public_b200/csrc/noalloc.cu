@@ -131,7 +131,8 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
   a.list_cap = kNaMaxList;
   a.heavy = reinterpret_cast<uint32_t*>(base + kOffHeavy);
   a.heavy_cap = kNaMaxTiles;
-  a.heavy_threshold = heavy_threshold((int)kNaTile);
+  a.queue_min = kQueueMin;
+  a.group = 1;
   a.large_seg = reinterpret_cast<uint2*>(base + kOffLargeSeg);
   a.seg_cap = kNaMaxSegs;
   a.large_walk = reinterpret_cast<WalkTri*>(base + kOffLargeWalk);

@@ -174,9 +174,8 @@ constexpr uint32_t kTriRisk = 1u;      // an edge value may wrap inside the bin 
 constexpr uint32_t kTriAreaRisk = 2u;  // the area may wrap: its reciprocal says nothing of the depth's range
 
 // What the binning passes (setup, large count, scan) count.  The heavy-tile
-// queue and the large-triangle queue each reserve slots and work-item ranges
-// with one 64-bit atomic, so that slot order and item order agree and an item's
-// slot can be found by a search over the slots' first items.
+// queue and the large-triangle queue each reserve two ranges with one 64-bit
+// atomic.
 constexpr uint32_t kPairParts = 128;
 struct BinCounts {
   uint32_t status;
@@ -184,7 +183,7 @@ struct BinCounts {
   uint32_t kept;
   uint32_t pair_part_max;        // largest partition fill asked for (past its capacity: overflow)
   unsigned long long risk;
-  unsigned long long heavy_acc;  // heavy tiles << 32 | 8x8 list chunks
+  unsigned long long heavy_acc;  // key slots << 32 | items (chunks, or without chunk buffers heavy tiles)
   unsigned long long large_acc;  // large triangles << 32 | their box-tile segments
 };
 
@@ -239,7 +238,7 @@ static_assert(sizeof(WalkTri) == 112, "WalkTri layout");
 struct __align__(16) ChunkDesc {
   uint32_t tile;
   uint32_t off, n;     // list entries [off, off + n)
-  uint32_t h;          // the heavy tile (its counter of finished chunks is hdone[h])
+  uint32_t ks;         // the tile's first key slot (lists in several chunks)
   uint32_t j, nch;     // chunk j of the tile's nch
   uint32_t pad[2];
 };
@@ -258,7 +257,6 @@ struct RasterFrameArgs {
   uint32_t* tile_list;      // [list_cap]
   uint32_t list_cap;
   uint32_t* heavy;          // [heavy_cap] heavy tiles, when there are no chunk buffers
-  uint32_t heavy_threshold; // 16/32-px tiles: list entries above which a tile is heavy
   uint32_t heavy_cap;
   // one record per (triangle, tile) pair, written by the count passes: the
   // tile | the pair's index in the tile's list << 32 (the old value of the
@@ -270,19 +268,21 @@ struct RasterFrameArgs {
   uint32_t seg_cap;
   WalkTri* large_walk;      // [big_cap] walk record of each large triangle, written by raster_setup
   uint32_t big_cap;
-  // Heavy tiles (8x8: lists longer than queue_min; 16/32 px: longer than
-  // heavy_threshold) are split into chunks (tile_chunk_entries) that different
-  // warps rasterize.  Each chunk leaves its per-pixel keys (tile * tile of
-  // them) in chunk_keys; the warp that completes a tile's last chunk takes the
-  // per-pixel minimum over the tile's chunks and resolves the tile.  Without
-  // chunk buffers (chunk_desc null) heavy tiles are rasterized whole, first.
+  // Heavy tiles (lists longer than queue_min) are split into chunks
+  // (tile_chunk_entries) that different warps rasterize.  Of a tile in several
+  // chunks each leaves its per-pixel keys (tile * tile of them) in its key slot;
+  // the warp that completes the last chunk takes the per-pixel minimum over the
+  // tile's chunks and resolves the tile.  Without chunk buffers (chunk_desc
+  // null) heavy tiles are rasterized whole.
   uint32_t chunk;
   uint32_t queue_min;       // 8x8 tiles with more entries than this are queued as chunks
-  uint32_t group;           // 8x8 tiles per short-list group (at most kLightGroup)
+  uint32_t group;           // 8x8 tiles per short-list group (at most kLightGroup); 16/32-px tiles: 8x8 bins
+                            // of a quad that a work item draws (1 or 4)
   ChunkDesc* chunk_desc;    // [chunk_cap]; the chunks of a tile are consecutive
-  uint32_t* hdone;          // [heavy_cap] chunks finished
-  unsigned long long* chunk_keys;  // [chunk_cap][tile * tile]
   uint32_t chunk_cap;
+  uint32_t* hdone;          // [key_cap][bins per tile] finished chunks, at a tile's first key slot
+  unsigned long long* chunk_keys;  // [key_cap][tile * tile]
+  uint32_t key_cap;
   unsigned long long* scan_flags;  // per scan block
   BinWork* work;
   FrameCounters* ctr;

@@ -14,17 +14,15 @@
 //   raster_large_count, which walks them the same way over the whole grid.
 //   scan_tiles      exclusive prefix sum of the tile counts (single pass,
 //                   decoupled look-back) -> per-tile list offsets.  Tiles with
-//                   long lists are queued: 16/32-px tiles whole or as chunks,
-//                   8x8 tiles as chunks of a fixed number of list entries.
+//                   long lists are queued as chunks of list entries.
 //   raster_scatter  a streaming pass over the pair records: each becomes its
 //                   list entry at its tile's offset plus its index (no walk, no
 //                   atomics): the compaction.
-//   raster_tiles /  persistent CTAs (Schedule).  The 8x8 kernel (one reference
-//   raster_frag8    bin per tile) gives each warp a tile or a chunk of one: the
-//                   warp tests every list entry against the tile's 64 pixels,
-//                   two per lane, and keeps each pixel's winning fragment key in
-//                   registers.  The 16/32-px kernel walks each entry's candidate
-//                   pixels triangle-parallel with shared-memory key atomics.
+//   raster_frag8 /  persistent CTAs.  A warp takes up to 32 list entries of an
+//   raster_bins     8x8 reference bin, or of several with short lists: each lane
+//                   builds one entry's coverage as a 64-bit mask, the masks are
+//                   transposed over the warp, and each lane resolves the depth
+//                   of two pixels from registers, nearest entries first.
 //                   Coverage is the reference's 28.4 edge test with its 8x8-bin
 //                   trivial reject/accept (R6, raster.pikostage:124-242); the z
 //                   test, the shading of each pixel's winner and the composite
@@ -625,7 +623,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
   __shared__ uint32_t s_bid;
   __shared__ uint32_t s_warp[kScanThreads / 32];
   __shared__ uint32_t s_prefix;
-  __shared__ unsigned long long s_heavy[kScanThreads / 32];   // per warp: (heavy tiles << 32) | chunks
+  __shared__ unsigned long long s_heavy[kScanThreads / 32];   // per warp: (key slots << 32) | items
   if (threadIdx.x == 0) s_bid = atomicAdd(&a.work->scan_ticket, 1u);
   __syncthreads();
   const uint32_t bid = s_bid;
@@ -646,28 +644,31 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
     uint32_t t = __shfl_up_sync(kFull, incl, o);
     if (lane >= o) incl += t;
   }
-  // Heavy tiles (lists longer than the threshold) and their chunks: counted
-  // now, reserved below with one atomic per block while warp 0 looks back
+  // Heavy tiles (lists longer than queue_min) become items of the fragment
+  // kernel's queue -- their chunks, or without chunk buffers the tiles -- and
+  // the chunks of lists in several chunks need key slots: counted now, reserved
+  // below with one atomic per block while warp 0 looks back
   const bool t8 = a.tile == kRefBin;
   const bool chunked = a.chunk_desc != nullptr;
-  const uint32_t thr = t8 ? a.queue_min : a.heavy_threshold;
-  uint32_t nh = 0, nc = 0;
+  const uint32_t thr = a.queue_min, bins = (uint32_t)(a.tile / kRefBin) * (uint32_t)(a.tile / kRefBin);
+  uint32_t nk = 0, nc = 0;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     if (base + i < n && v[i] > thr) {
-      ++nh;
-      if (chunked) nc += tile_chunks(v[i], a.chunk, t8);
+      const uint32_t nch = chunked ? tile_chunks(v[i], a.chunk, t8) : 1u;
+      nc += nch;
+      if (nch > 1) nk += nch;
     }
   }
-  uint32_t hi = nh, ci = nc;
+  uint32_t ki = nk, ci = nc;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t th = __shfl_up_sync(kFull, hi, o), tc = __shfl_up_sync(kFull, ci, o);
-    if (lane >= o) { hi += th; ci += tc; }
+    const uint32_t tk = __shfl_up_sync(kFull, ki, o), tc = __shfl_up_sync(kFull, ci, o);
+    if (lane >= o) { ki += tk; ci += tc; }
   }
   if (lane == 31) {
     s_warp[warp] = incl;
-    s_heavy[warp] = ((unsigned long long)hi << 32) | ci;
+    s_heavy[warp] = ((unsigned long long)ki << 32) | ci;
   }
   __syncthreads();
   if (warp == 1 && lane == 0) {
@@ -730,34 +731,32 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
   }
   __syncthreads();
   uint32_t run = s_prefix + warp_excl + (incl - sum);
-  // With chunk buffers a heavy list becomes tile_chunks(len) chunks
   const unsigned long long old = s_heavy[warp];
-  uint32_t h = (uint32_t)(old >> 32) + hi - nh;
+  uint32_t ks = (uint32_t)(old >> 32) + ki - nk;
   uint32_t c = (uint32_t)old + ci - nc;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     if (base + i < n) {
       a.tile_off[base + i] = run;
       if (v[i] > thr) {
-        if (h < a.heavy_cap) {
-          if (chunked) {
-            a.hdone[h] = 0;
-            const uint32_t ce = tile_chunk_entries(v[i], a.chunk, t8), nch = (v[i] + ce - 1) / ce;
-            for (uint32_t j = 0; j < nch && c + j < a.chunk_cap; ++j) {
-              uint4* d = reinterpret_cast<uint4*>(&a.chunk_desc[c + j]);
-              d[0] = make_uint4(base + i, run + j * ce, min(ce, v[i] - j * ce), h);
-              d[1] = make_uint4(j, nch, 0u, 0u);
-            }
-            c += nch;
-            // chunks past the key buffers are not rasterized: report it
-            if (c > a.chunk_cap) atomicOr(&a.work->bin.status, kStatusListOverflow);
-          } else {
-            a.heavy[h] = base + i;
+        if (chunked) {
+          const uint32_t ce = tile_chunk_entries(v[i], a.chunk, t8), nch = (v[i] + ce - 1) / ce;
+          for (uint32_t j = 0; j < nch && c + j < a.chunk_cap; ++j) {
+            uint4* d = reinterpret_cast<uint4*>(&a.chunk_desc[c + j]);
+            d[0] = make_uint4(base + i, run + j * ce, min(ce, v[i] - j * ce), ks);
+            d[1] = make_uint4(j, nch, 0u, 0u);
           }
+          if (nch > 1 && ks + nch <= a.key_cap)
+            for (uint32_t k = 0; k < bins; ++k) a.hdone[(size_t)ks * bins + k] = 0;
+          c += nch;
+          if (nch > 1) ks += nch;
+          // chunks past the buffers are not rasterized: report it
+          if (c > a.chunk_cap || ks > a.key_cap) atomicOr(&a.work->bin.status, kStatusListOverflow);
         } else {
-          atomicOr(&a.work->bin.status, kStatusListOverflow);
+          if (c < a.heavy_cap) a.heavy[c] = base + i;
+          else atomicOr(&a.work->bin.status, kStatusListOverflow);
+          ++c;
         }
-        ++h;
       }
     }
     run += v[i];
@@ -864,87 +863,6 @@ __global__ void __launch_bounds__(256) raster_scatter(const __grid_constant__ Ra
 }
 
 // ------------------------------------------------------------------ kernel 4
-// A triangle as one tile sees it (tile-local), built by the thread that takes
-// the list entry.
-struct TileTri {
-  int32_t e[3];          // edge values at the centre of the tile's pixel (0, 0)
-  int32_t sx[3], sy[3];  // per-pixel steps in x and y
-  uint32_t trm, tam;     // per reference bin of the tile: assigned, trivially accepted
-  int32_t lxe, lye;      // tile-local pixel limit of the bbox (pixel < limit)
-  int32_t ex0, ex1, ey0, ey1;  // candidate pixels, clipped to the tile (inclusive)
-  float inv, z2, z0mz2, z1mz2;
-  uint32_t rank1;
-  uint32_t gidx;         // setup index (coverage dump)
-};
-
-__device__ __forceinline__ void build_tile_tri(const TriSetup& r, int X0, int Y0, int T, TileTri& t)
-{
-  const int32_t Xc = X0 * 16 + 8, Yc = Y0 * 16 + 8;
-  int32_t dx[3], dy[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    int j = i == 2 ? 0 : i + 1;
-    dx[i] = wsub(r.x[j], r.x[i]);
-    dy[i] = wsub(r.y[j], r.y[i]);
-    t.e[i] = edge_at(Xc, Yc, r.x[i], r.y[i], dx[i], dy[i]);
-    t.sx[i] = -wshl(dy[i], 4);
-    t.sy[i] = wshl(dx[i], 4);
-  }
-  const int bx1 = (int)(r.bxr & 0xffff), bx2 = (int)(r.bxr >> 16);
-  const int by1 = (int)(r.byr & 0xffff), by2 = (int)(r.byr >> 16);
-  const int BPT = T / kRefBin;
-  uint32_t trm = 0, tam = 0;
-  for (int bj = 0; bj < BPT; ++bj) {
-    const int by = Y0 / kRefBin + bj;
-    if (by < by1 || by > by2) continue;
-    for (int bi = 0; bi < BPT; ++bi) {
-      const int bx = X0 / kRefBin + bi;
-      if (bx < bx1 || bx > bx2) continue;
-      // trivial reject at the bin corner (raster.pikostage:77-105, 128 = 8 px in 28.4)
-      const int32_t BX = bx * 128, BY = by * 128;
-      int32_t tr = 0, ta = 0;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        int32_t off = dy[i] < 0 ? -wshl(dy[i], 7) : 0;
-        off = wadd(off, dx[i] >= 0 ? wshl(dx[i], 7) : 0);
-        tr |= wadd(off, edge_at(BX, BY, r.x[i], r.y[i], dx[i], dy[i]));
-        // trivial accept at the first pixel centre (raster.pikostage:201-211)
-        int32_t offa = dy[i] >= 0 ? -wshl(dy[i], 4) : 0;
-        offa = wadd(offa, dx[i] < 0 ? wshl(dx[i], 4) : 0);
-        ta |= wadd(edge_at(BX + 8, BY + 8, r.x[i], r.y[i], dx[i], dy[i]), wshl(offa, kRefBinLg2));
-      }
-      if (tr >= 0) {
-        const uint32_t bit = 1u << (bj * BPT + bi);
-        trm |= bit;
-        if ((ta & (int32_t)0x80000000) == 0) tam |= bit;
-      }
-    }
-  }
-  t.trm = trm;
-  t.tam = tam;
-  t.lxe = (r.hix >> 4) - X0;
-  t.lye = (r.hiy >> 4) - Y0;
-  int ex0, ex1, ey0, ey1;
-  if (r.flags & kTriRisk) {
-    ex0 = bx1 * kRefBin - X0; ex1 = bx2 * kRefBin + kRefBin - 1 - X0;
-    ey0 = by1 * kRefBin - Y0; ey1 = by2 * kRefBin + kRefBin - 1 - Y0;
-  } else {
-    // covered centres lie inside the triangle when no edge value can wrap
-    ex0 = (min(min(r.x[0], r.x[1]), r.x[2]) >> 4) - 1 - X0;
-    ex1 = (max(max(r.x[0], r.x[1]), r.x[2]) >> 4) - X0;
-    ey0 = (min(min(r.y[0], r.y[1]), r.y[2]) >> 4) - 1 - Y0;
-    ey1 = (max(max(r.y[0], r.y[1]), r.y[2]) >> 4) - Y0;
-  }
-  t.ex0 = max(ex0, 0); t.ex1 = min(ex1, T - 1);
-  t.ey0 = max(ey0, 0); t.ey1 = min(ey1, T - 1);
-  if (!trm) t.ex1 = -1;  // nothing assigned in this tile
-  t.inv = r.inv;
-  t.z2 = r.z[2];
-  t.z0mz2 = r.z[0] - r.z[2];
-  t.z1mz2 = r.z[1] - r.z[2];
-  t.rank1 = r.rank1;
-}
-
 // Inverse of submission_rank: the triangle id with the given rank.
 __device__ __forceinline__ uint32_t rank_to_id(uint32_t r, const RasterSceneDev& S)
 {
@@ -959,32 +877,6 @@ __device__ __forceinline__ uint32_t rank_to_id(uint32_t r, const RasterSceneDev&
   const uint32_t start = kVsChunk * (lo * S.vs_q + min(lo, S.vs_rem)) - (S.vs_last < lo ? S.vs_deficit : 0u);
   const uint32_t pos = r - start;
   return (lo + (pos / kVsChunk) * nVS) * kVsChunk + pos % kVsChunk;
-}
-
-
-// Depth test of one candidate pixel (raster.pikostage:201-285): assigned bin,
-// trivial accept or the bbox-limited edge test, barycentric depth, then the
-// order-independent keep-the-smaller-key update.  Within one step of a warp no
-// two lanes hold the same pixel, and the warp owns its tile, so the update
-// needs no atomic.
-template <int T>
-__device__ __forceinline__ bool frag(const TileTri& t, int lx, int ly, unsigned long long* keys)
-{
-  constexpr int BPT = T / kRefBin;
-  const uint32_t bit = 1u << ((ly >> kRefBinLg2) * BPT + (lx >> kRefBinLg2));
-  if (!(t.trm & bit)) return false;
-  const int32_t f0 = wadd(wadd(t.e[0], wmul(lx, t.sx[0])), wmul(ly, t.sy[0]));
-  const int32_t f1 = wadd(wadd(t.e[1], wmul(lx, t.sx[1])), wmul(ly, t.sy[1]));
-  const int32_t f2 = wadd(wadd(t.e[2], wmul(lx, t.sx[2])), wmul(ly, t.sy[2]));
-  const bool cov = (t.tam & bit) || ((lx < t.lxe) && (ly < t.lye) && ((f0 | f1 | f2) >= 0));
-  if (!cov) return false;
-  const float alpha = (float)f1 * t.inv;
-  const float beta = (float)f2 * t.inv;
-  const float z = t.z2 + alpha * t.z0mz2 + beta * t.z1mz2;
-  const unsigned long long key = frag_key(z, t.rank1);
-  unsigned long long* k = &keys[ly * T + lx];
-  if (key < *k) *k = key;
-  return true;
 }
 
 
@@ -1033,192 +925,6 @@ __device__ __forceinline__ uint32_t shade_winner(const RasterSceneDev& S, const 
     col[2] = col[2] * inv255[t.z];
   }
   return pack_abgr(col[0], col[1], col[2]);
-}
-
-// Rasterizes list entries [b, e) of the tile at (X0, Y0) of scene S into the
-// warp's tile keys (16/32-px tiles): 32 entries at a time each lane builds one
-// entry's tile-local form, then the warp takes them one at a time, lanes
-// spread over the entry's candidate box in 8x4 blocks.
-template <int T>
-__device__ __forceinline__ void tiles_entries(const RasterFrameArgs& a, const RasterSceneDev& S, int X0, int Y0,
-                                              uint32_t off, uint32_t b, uint32_t e, unsigned long long* keys,
-                                              TileTri* st, int lane, unsigned& covered)
-{
-  // entries past the list capacity are never read (the frame reports the overflow)
-  const uint32_t lim = a.list_cap - min(off, a.list_cap);
-  e = min(e, lim);
-  for (uint32_t b0 = b; b0 < e; b0 += 32) {
-    if (b0 + lane < e) {
-      const uint32_t gi = a.tile_list[off + b0 + lane];
-      build_tile_tri(load_setup(&a.setup[gi]), X0, Y0, T, st[lane]);
-      st[lane].gidx = gi;
-      if (st[lane].ex1 < st[lane].ex0 || st[lane].ey1 < st[lane].ey0) st[lane].rank1 = 0u;
-    }
-    __syncwarp();
-    const int n = (int)min(32u, e - b0);
-    for (int i = 0; i < n; ++i) {
-      const TileTri& t = st[i];
-      if (t.rank1) {
-        const int ex1 = min(t.ex1, T - 1), ey1 = min(t.ey1, T - 1);
-        const int lx0 = max(t.ex0, 0) + (lane & 7), ly0 = max(t.ey0, 0) + (lane >> 3);
-        for (int ly = ly0; ly <= ey1; ly += 4) {
-          for (int lx = lx0; lx <= ex1; lx += 8) {
-            if (frag<T>(t, lx, ly, keys)) {
-              ++covered;
-              if (a.cov_cap) {
-                const uint32_t slot = atomicAdd(&a.ctr->cov_count, 1u);
-                if (slot < a.cov_cap) {
-                  a.cov_tri[slot] = t.gidx - S.tri_base;
-                  a.cov_pix[slot] = (uint32_t)((Y0 + ly) * S.W + X0 + lx);
-                }
-              }
-            }
-          }
-        }
-      }
-      __syncwarp();  // the next triangle may touch the same pixels
-    }
-    __syncwarp();    // every lane is done with st[] before it is rebuilt
-  }
-}
-
-// Resolve of a 16/32-px tile from the warp's keys: each pixel's winner is
-// shaded once, the tile written once.
-template <int T>
-__device__ __forceinline__ void tiles_resolve(const RasterFrameArgs& a, const RasterSceneDev& S, int X0, int Y0,
-                                              const unsigned long long* keys, int lane, const float* inv255)
-{
-  constexpr int PPT = T * T / 32;
-#pragma unroll 4
-  for (int j = 0; j < PPT; ++j) {
-    const int p = j * 32 + lane;
-    const int lx = p % T, ly = p / T;
-    const int px = X0 + lx, py = Y0 + ly;
-    const unsigned long long key = keys[p];
-    if (px < S.W && py < S.H) {
-      uint32_t c = kClearColor;
-      float z = 1.0f;
-      if (key != kInitKey) {
-        const uint32_t rank = ~(uint32_t)key - 1u;
-        z = __uint_as_float((uint32_t)(key >> 32) ^ 0x80000000u);
-        const uint32_t id = rank_to_id(rank, S);
-        c = shade_winner(S, a.setup + S.tri_base, id, px, py, inv255);
-      }
-      const size_t idx = (size_t)py * S.W + px;
-      S.fb[idx] = c;
-      S.depth[idx] = z;
-    }
-  }
-}
-
-// 16/32-px tiles, persistent: warp w of the grid first draws the plain tiles
-// w, w + warps, ... (a heavy tile among them is skipped), then takes work items
-// from one counter -- the chunks of the heavy tiles' lists (each chunk leaves
-// its keys in chunk_keys; the warp finishing a tile's last chunk merges them
-// and resolves the tile), or, without chunk buffers, the heavy tiles whole.
-template <int T, bool ONE>
-__global__ void __launch_bounds__(T == 32 ? 128 : 256) raster_tiles(const __grid_constant__ RasterFrameArgs a)
-{
-  pdl_wait();
-  frame_begin(a);
-  if (list_overflowed(a)) return;
-  constexpr int CTA = T == 32 ? 128 : 256;
-  constexpr int NW = CTA / 32;    // warps per CTA, one work item each
-  constexpr int NPX = T * T;
-  constexpr int PPT = NPX / 32;   // pixels per lane
-  __shared__ unsigned long long s_keys[NW][NPX];
-  __shared__ TileTri s_tri[NW][32];
-  __shared__ float s_inv255[256];
-  constexpr int kTb = T == 32 ? 128 : 512;   // scene table (static shared memory stays under 48 KB)
-  __shared__ uint32_t s_tb[kTb];
-  for (int i = threadIdx.x; i < 256; i += CTA) s_inv255[i] = (float)i / 255.0f;
-  load_scene_table<ONE, kTb>(a, s_tb, true);
-  __syncthreads();
-  const int wid = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  unsigned long long* keys = s_keys[wid];
-  TileTri* st = s_tri[wid];
-  unsigned covered = 0;
-  const bool chunked = a.chunk_desc != nullptr;
-  const unsigned long long hacc = a.ctr->bin.heavy_acc;
-  const uint32_t n_heavy = min((uint32_t)(hacc >> 32), a.heavy_cap);
-  const uint32_t n_chunks = chunked ? min((uint32_t)hacc, a.chunk_cap) : 0u;
-  const uint32_t n_first = chunked ? n_chunks : n_heavy;   // items before the plain tiles
-
-  // The plain tiles first, warp w of the grid taking tiles w, w + warps, ...;
-  // then the heavy items (chunks, or whole heavy tiles) from a counter, which
-  // also evens out the warps' finishing times.
-  uint32_t plain = blockIdx.x * (uint32_t)NW + (uint32_t)wid;
-  const uint32_t nwarps = gridDim.x * (uint32_t)NW;
-  for (;;) {
-    uint32_t w = 0;
-    if (plain < a.n_tiles_total) {
-      w = n_first + plain;
-      plain += nwarps;
-    } else {
-      if (lane == 0) w = atomicAdd(&a.ctr->work_next, 1u);
-      w = __shfl_sync(kFull, w, 0);
-      if (w >= n_first) break;
-    }
-#pragma unroll
-    for (int j = 0; j < PPT; ++j) keys[j * 32 + lane] = kInitKey;
-    __syncwarp();
-    uint32_t tile, b = 0, e = 0, h = 0, c0 = 0, nch = 1;
-    bool chunk_item = false;
-    if (w < n_first) {
-      if (chunked) {
-        const uint4* dp = reinterpret_cast<const uint4*>(&a.chunk_desc[w]);
-        const uint4 d0 = dp[0], d1 = dp[1];
-        tile = d0.x;
-        h = d0.w;
-        c0 = w - d1.x;
-        nch = d1.y;
-        b = d0.y - a.tile_off[tile];
-        e = b + d0.z;
-        chunk_item = true;
-      } else {
-        tile = a.heavy[w];
-        e = a.tile_off[tile + 1] - a.tile_off[tile];
-      }
-    } else {
-      tile = w - n_first;
-      e = a.tile_off[tile + 1] - a.tile_off[tile];
-      if (e > a.heavy_threshold) continue;  // served from the heavy queue
-    }
-    const int s = scene_of<ONE, kTb>(a, s_tb, tile, true);
-    const RasterSceneDev& S = scene_at<ONE>(a, s);
-    uint32_t ltx;
-    const uint32_t lty = fast_divmod(tile - S.tile_base, (uint32_t)S.tiles_x, S.tiles_x_m, ltx);
-    const int X0 = (int)ltx * T, Y0 = (int)lty * T;
-    tiles_entries<T>(a, S, X0, Y0, a.tile_off[tile], b, e, keys, st, lane, covered);
-    __syncwarp();
-    if (chunk_item) {
-      // this chunk's keys, then the finished-chunk count of its tile
-      unsigned long long* ck = a.chunk_keys + (size_t)w * NPX;
-#pragma unroll
-      for (int j = 0; j < PPT; ++j) ck[j * 32 + lane] = keys[j * 32 + lane];
-      __threadfence();
-      __syncwarp();
-      uint32_t done = 0;
-      if (lane == 0) done = atomicAdd(&a.hdone[h], 1u);
-      done = __shfl_sync(kFull, done, 0);
-      if (done + 1 != nch) continue;
-      // the tile's last chunk: every other chunk's keys are in chunk_keys
-      __threadfence();
-      for (uint32_t j = 0; j < nch; ++j) {
-        if (c0 + j == w) continue;
-        const unsigned long long* cj = a.chunk_keys + (size_t)(c0 + j) * NPX;
-#pragma unroll
-        for (int q = 0; q < PPT; ++q) keys[q * 32 + lane] = min(keys[q * 32 + lane], __ldcg(&cj[q * 32 + lane]));
-      }
-      __syncwarp();
-    }
-    tiles_resolve<T>(a, S, X0, Y0, keys, lane, s_inv255);
-    __syncwarp();
-  }
-  // fragment count: one atomic per warp
-  covered = __reduce_add_sync(kFull, covered);
-  if (lane == 0 && covered) atomicAdd(&a.ctr->covered, (unsigned long long)covered);
 }
 
 // 8x8 tiles (one reference bin each): a warp takes up to 32 list entries at a
@@ -1587,6 +1293,34 @@ __device__ __forceinline__ void resolve8_staged(const Tile8& tl, int lane, unsig
   }
 }
 
+// Chunk j of nch of a tile (key slots from ks on) is done with bin `bin` of the
+// tile's `bins`: leaves its keys; true for the last chunk to arrive, whose
+// k0 / k1 are then the least keys over the tile's chunks.
+__device__ __forceinline__ bool merge_chunks(const RasterFrameArgs& a, uint32_t bins, uint32_t bin, uint32_t ks,
+                                             uint32_t j, uint32_t nch, int lane, unsigned long long& k0,
+                                             unsigned long long& k1)
+{
+  // pixel p of the bin is key p: the lane's pixels are lane and lane + 32
+  unsigned long long* ck = a.chunk_keys + ((size_t)(ks + j) * bins + bin) * 64;
+  ck[lane] = k0;
+  ck[lane + 32] = k1;
+  __threadfence();
+  __syncwarp();
+  uint32_t done = 0;
+  if (lane == 0) done = atomicAdd(&a.hdone[(size_t)ks * bins + bin], 1u);
+  done = __shfl_sync(kFull, done, 0);
+  if (done + 1 != nch) return false;
+  // the last chunk: every other chunk's keys are in chunk_keys
+  __threadfence();
+  for (uint32_t o = 0; o < nch; ++o) {
+    if (o == j) continue;
+    const unsigned long long* cj = a.chunk_keys + ((size_t)(ks + o) * bins + bin) * 64;
+    k0 = min(k0, __ldcg(&cj[lane]));
+    k1 = min(k1, __ldcg(&cj[lane + 32]));
+  }
+  return true;
+}
+
 // Persistent.  A warp works in passes of up to 32 list entries (one copy of the
 // code for every kind of pass: the kernel's instruction footprint matters more
 // than the branches between them).  Warp w of the grid first draws the
@@ -1713,27 +1447,8 @@ __global__ void __launch_bounds__(256, 4) raster_frag8(const __grid_constant__ R
         resolve8_staged(tl, lane, k0, k1, w0, w1, w.tri, w.shade, s_inv255);
       } else if (b0 >= len) {
         const uint32_t nch = __shfl_sync(kFull, desc, 5);
-        if (nch > 1) {
-          // pixel p of the tile is key p of the chunk: the lane's pixels are lane and lane + 32
-          unsigned long long* ck = a.chunk_keys + (size_t)ci * 64;
-          ck[lane] = k0;
-          ck[lane + 32] = k1;
-          __threadfence();
-          __syncwarp();
-          const uint32_t h = __shfl_sync(kFull, desc, 3), c0 = ci - __shfl_sync(kFull, desc, 4);
-          uint32_t done = 0;
-          if (lane == 0) done = atomicAdd(&a.hdone[h], 1u);
-          done = __shfl_sync(kFull, done, 0);
-          if (done + 1 != nch) continue;
-          // the tile's last chunk: every other chunk's keys are in chunk_keys
-          __threadfence();
-          for (uint32_t c = c0; c < c0 + nch; ++c) {
-            if (c == ci) continue;
-            const unsigned long long* cj = a.chunk_keys + (size_t)c * 64;
-            k0 = min(k0, __ldcg(&cj[lane]));
-            k1 = min(k1, __ldcg(&cj[lane + 32]));
-          }
-        }
+        if (nch > 1 && !merge_chunks(a, 1, 0, __shfl_sync(kFull, desc, 3), __shfl_sync(kFull, desc, 4), nch, lane, k0, k1))
+          continue;
         resolve8(a, tl, lane, k0, k1, s_inv255);
       }
     }
@@ -1748,6 +1463,221 @@ __global__ void __launch_bounds__(256, 4) raster_frag8(const __grid_constant__ R
     unsigned long long t = 0;
 #pragma unroll
     for (int w = 0; w < 8; ++w) t += s_cov[w];
+    if (t) atomicAdd(&a.ctr->covered, t);
+  }
+}
+
+// The bins of the 2 x 2 quad at pixel (X0, Y0) that triangle gi is assigned to
+// (bit 2 * dy + dx): its bin range and the trivial reject at each bin's corner
+// (raster.pikostage:77-105, 128 = 8 px in 28.4).
+__device__ __forceinline__ uint32_t quad_assigned(const RasterFrameArgs& a, uint32_t gi, int X0, int Y0)
+{
+  const TriSetup r = load_setup(&a.setup[gi]);
+  int32_t t00 = 0, t10 = 0, t01 = 0, t11 = 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int j = i == 2 ? 0 : i + 1;
+    const int32_t dx = wsub(r.x[j], r.x[i]), dy = wsub(r.y[j], r.y[i]);
+    const int32_t sx = -wshl(dy, 7), sy = wshl(dx, 7);
+    int32_t t = wadd(dy < 0 ? sx : 0, dx >= 0 ? sy : 0);
+    t = wadd(t, edge_at(X0 * 16, Y0 * 16, r.x[i], r.y[i], dx, dy));
+    t00 |= t;
+    t10 |= wadd(t, sx);
+    t01 |= wadd(t, sy);
+    t11 |= wadd(wadd(t, sx), sy);
+  }
+  const int bx = X0 / kRefBin, by = Y0 / kRefBin;
+  const int bx1 = (int)(r.bxr & 0xffff), bx2 = (int)(r.bxr >> 16), by1 = (int)(r.byr & 0xffff), by2 = (int)(r.byr >> 16);
+  const uint32_t cols = (bx >= bx1 && bx <= bx2 ? 5u : 0u) | (bx + 1 >= bx1 && bx + 1 <= bx2 ? 10u : 0u);
+  const uint32_t rows = (by >= by1 && by <= by2 ? 3u : 0u) | (by + 1 >= by1 && by + 1 <= by2 ? 12u : 0u);
+  return cols & rows & ((t00 >= 0 ? 1u : 0u) | (t10 >= 0 ? 2u : 0u) | (t01 >= 0 ? 4u : 0u) | (t11 >= 0 ? 8u : 0u));
+}
+
+// 16/32-px tiles: raster_frag8's passes over the reference bins of a tile.  An
+// item is a list (a short one by warp index, a chunk of a longer one from the
+// counter, or without chunk buffers a heavy tile's whole list) and a quad of
+// the tile's bins, or one bin of it (a.group).  The list's entries are tested against the quad's four bins
+// at once, 32 at a time, and queued per bin; a bin with 32 queued entries gets a
+// pass of its own, and the remainders share passes at the end.  A bin drawn by
+// one pass is resolved from shared memory, one drawn by several keeps its keys
+// there in between.  (Spreading the warp's lanes over one entry's pixels after
+// the other, with the tile's keys in shared memory, left most lanes idle on
+// small triangles: a 61,200-triangle forest at 800x600 in 16-px tiles, lists of
+// up to 400 entries, took 83 us.)
+struct BinsSmem {
+  WarpEntries ent[8];
+  unsigned long long keys[8][4][64];
+  uint16_t queue[8][4][64];
+  float inv255[256];
+  unsigned cov[8];
+  uint32_t tb[512];
+};
+
+template <int T, bool ONE>
+__global__ void __launch_bounds__(256, 4) raster_bins(const __grid_constant__ RasterFrameArgs a)
+{
+  pdl_wait();
+  frame_begin(a);
+  if (list_overflowed(a)) return;
+  constexpr uint32_t QPT = T / (2 * kRefBin), QUADS = QPT * QPT, NB = 4 * QUADS;
+  extern __shared__ __align__(16) unsigned char bins_smem[];
+  BinsSmem& B = *reinterpret_cast<BinsSmem*>(bins_smem);
+  B.inv255[threadIdx.x] = (float)threadIdx.x / 255.0f;
+  load_scene_table<ONE, 512>(a, B.tb, true);
+  __syncthreads();
+  const int wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  WarpEntries& w = B.ent[wid];
+  unsigned covered = 0;
+  const bool chunked = a.chunk_desc != nullptr;
+  // parts of a tile: its quads, or the single bins of its quads
+  const uint32_t split = 4u / a.group, parts = QUADS * split;
+  const uint32_t n_items = min((uint32_t)a.ctr->bin.heavy_acc, chunked ? a.chunk_cap : a.heavy_cap) * parts;
+  const uint32_t n_light = a.n_tiles_total * parts;
+  const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+  uint32_t g = blockIdx.x * (blockDim.x >> 5) + (uint32_t)wid;
+  for (;;) {
+    uint32_t tile, quad, off, len, ks = 0, j = 0, nch = 1;   // (quad: the part, then its quad)
+    if (g < n_light) {
+      tile = g / parts;
+      quad = g % parts;
+      g += nwarps;
+      off = a.tile_off[tile];
+      len = a.tile_off[tile + 1] - off;
+      if (len > a.queue_min) continue;   // drawn from the queue
+    } else {
+      uint32_t it = 0;
+      if (lane == 0) it = atomicAdd(&a.ctr->work_next, 1u);
+      it = __shfl_sync(kFull, it, 0);
+      if (it >= n_items) break;
+      quad = it % parts;
+      if (chunked) {
+        const uint4* d = reinterpret_cast<const uint4*>(&a.chunk_desc[it / parts]);
+        const uint4 d0 = d[0], d1 = d[1];
+        tile = d0.x; off = d0.y; len = d0.z; ks = d0.w;
+        j = d1.x; nch = d1.y;
+      } else {
+        tile = a.heavy[it / parts];
+        off = a.tile_off[tile];
+        len = a.tile_off[tile + 1] - off;
+      }
+    }
+    // entries past the list capacity are never read (the frame reports the overflow)
+    len = min(len, a.list_cap - min(off, a.list_cap));
+    int done = 0, bins_end = 4;    // bins [done, bins_end) of the quad are to be resolved
+    if (split > 1) {
+      done = (int)(quad & 3u);
+      bins_end = done + 1;
+      quad >>= 2;
+    }
+    const uint32_t mine = ((1u << bins_end) - 1u) & ~((1u << done) - 1u);
+    Tile8 tl;   // the quad's scene and first pixel
+    {
+      const int s = scene_of<ONE, 512>(a, B.tb, tile, true);
+      tl.S = &scene_at<ONE>(a, s);
+      uint32_t tx;
+      const uint32_t ty = fast_divmod(tile - tl.S->tile_base, (uint32_t)tl.S->tiles_x, tl.S->tiles_x_m, tx);
+      tl.X0 = (int)(tx * T + 2 * (quad % QPT) * kRefBin);
+      tl.Y0 = (int)(ty * T + 2 * (quad / QPT) * kRefBin);
+    }
+    uint32_t b0 = 0, q_base = 0;   // entries [b0, len) remain; queued entries are numbered from q_base
+    uint32_t queued = 0;           // lane q < 4: entries queued for bin q
+    unsigned touched = 0;          // bins with keys in shared memory
+    while (done < bins_end) {
+      unsigned full = __ballot_sync(kFull, queued >= 32u);
+      while (!full && b0 < len) {
+        if (!__any_sync(kFull, queued != 0u)) q_base = b0;
+        if (b0 - q_base >= 65504u) break;   // (queue entries are 16-bit: drain first)
+        uint32_t in = 0;
+        if (b0 + lane < len) in = quad_assigned(a, a.tile_list[off + b0 + lane], tl.X0, tl.Y0) & mine;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const unsigned m = __ballot_sync(kFull, (in >> q) & 1u);
+          const uint32_t at = __shfl_sync(kFull, queued, q);
+          if ((in >> q) & 1u) B.queue[wid][q][at + __popc(m & lt)] = (uint16_t)(b0 - q_base + lane);
+          if (lane == q) queued += __popc(m);
+        }
+        b0 += 32;
+        full = __ballot_sync(kFull, queued >= 32u);
+      }
+      __syncwarp();
+      // the pass: 32 entries of a bin that has as many, or what remains of bins [ja, jb)
+      const bool last = !full && b0 >= len;
+      int ja, jb;
+      uint32_t cnt;   // lane q: entries of bin q in this pass
+      if (last) {
+        ja = done;
+        uint32_t incl = lane >= ja && lane < 4 ? queued : 0u;
+        const uint32_t up1 = __shfl_up_sync(kFull, incl, 1);
+        if (lane >= 1) incl += up1;
+        const uint32_t up2 = __shfl_up_sync(kFull, incl, 2);
+        if (lane >= 2) incl += up2;
+        jb = ja + __popc(__ballot_sync(kFull, lane >= ja && lane < bins_end && incl <= 32u));
+        cnt = lane >= ja && lane < jb ? queued : 0u;
+      } else {
+        if (!full) full = __ballot_sync(kFull, queued != 0u);
+        ja = __ffs(full) - 1;
+        jb = ja + 1;
+        cnt = lane == ja ? min(queued, 32u) : 0u;
+      }
+      uint32_t incl = cnt;
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int n = (int)__shfl_sync(kFull, incl, 3);
+      const bool stage = last && nch == 1;   // (for the bins that have no keys yet)
+      uint32_t m0 = 0u, m1 = 0u;
+      if (n) {
+        const uint32_t l = (uint32_t)(n <= 16 ? lane & 15 : lane);
+        uint32_t bin = 0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) bin += __shfl_sync(kFull, incl, q) <= l ? 1u : 0u;
+        const uint32_t top = __shfl_sync(kFull, queued, bin), end = __shfl_sync(kFull, incl, bin);
+        const bool ok = l < (uint32_t)n;
+        const uint32_t gi = ok ? a.tile_list[off + q_base + B.queue[wid][bin][top - (end - l)]] : 0u;
+        frag8_build(a, *tl.S, n, ok, gi, bin, tl.X0 + (int)(bin & 1u) * kRefBin, tl.Y0 + (int)(bin >> 1) * kRefBin, stage, w,
+                    lane, B.inv255, covered, m0, m1);
+        queued -= cnt;
+      }
+#pragma unroll 1
+      for (int q = ja; q < jb; ++q) {
+        const uint32_t cq = __shfl_sync(kFull, cnt, q), eq = __shfl_sync(kFull, incl, q);
+        const uint32_t bits = cq >= 32u ? 0xffffffffu : ((1u << cq) - 1u) << ((eq - cq) & 31u);
+        unsigned long long* keys = B.keys[wid][q];
+        const bool had = (touched >> q) & 1u;
+        unsigned long long k0 = kInitKey, k1 = kInitKey;
+        int w0 = 0, w1 = 0;
+        if (had) { k0 = keys[lane]; k1 = keys[lane + 32]; }
+        frag8_test(w.tri, m0 & bits, m1 & bits, lane, k0, k1, w0, w1);
+        if (!last) {
+          keys[lane] = k0;
+          keys[lane + 32] = k1;
+          touched |= 1u << q;
+          continue;
+        }
+        const Tile8 bt = {tl.S, tl.X0 + (q & 1) * kRefBin, tl.Y0 + (q >> 1) * kRefBin};
+        if (stage && !had) {
+          resolve8_staged(bt, lane, k0, k1, w0, w1, w.tri, w.shade, B.inv255);
+          continue;
+        }
+        if (nch > 1 && !merge_chunks(a, NB, quad * 4 + q, ks, j, nch, lane, k0, k1)) continue;
+        resolve8(a, bt, lane, k0, k1, B.inv255);
+      }
+      if (last) done = jb;
+    }
+  }
+
+  // fragment count: one atomic per CTA
+  covered = __reduce_add_sync(kFull, covered);
+  if (lane == 0) B.cov[wid] = covered;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long t = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += B.cov[k];
     if (t) atomicAdd(&a.ctr->covered, t);
   }
 }
@@ -1777,12 +1707,12 @@ static int wave_ctas(K kernel, std::atomic<int>* cache, int threads = 256)
 // A launch that may begin while the previous kernel of the stream finishes
 // (the kernel's pdl_wait() holds it until that kernel's writes are visible).
 template <typename K>
-static cudaError_t launch_pdl(K kernel, int grid, int block, cudaStream_t st, const RasterFrameArgs& a)
+static cudaError_t launch_pdl(K kernel, int grid, int block, cudaStream_t st, const RasterFrameArgs& a, size_t smem = 0)
 {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1790,6 +1720,26 @@ static cudaError_t launch_pdl(K kernel, int grid, int block, cudaStream_t st, co
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+// raster_bins needs more shared memory than a static allocation may have; set
+// once per device the library runs on.
+static cudaError_t bins_setup()
+{
+  static std::atomic<unsigned long long> done{0};   // a bit per device ordinal
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (e || (done.load(std::memory_order_acquire) & bit)) return e;
+  const auto set = [](const void* f) {
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinsSmem));
+  };
+  e = set((const void*)raster_bins<16, true>);
+  if (!e) e = set((const void*)raster_bins<16, false>);
+  if (!e) e = set((const void*)raster_bins<32, true>);
+  if (!e) e = set((const void*)raster_bins<32, false>);
+  if (!e) done.fetch_or(bit, std::memory_order_release);
+  return e;
 }
 
 cudaError_t launch_raster_frame(const RasterFrameArgs& a, int raster_ctas, cudaStream_t st, cudaEvent_t* ev)
@@ -1815,11 +1765,12 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& a, int raster_ctas, cudaS
   if (ev) cudaEventRecord(ev[2], st);
   if (!e) e = launch_pdl(raster_scatter, scatter_blocks, 256, st, a);
   if (ev) cudaEventRecord(ev[3], st);
+  if (!e && a.tile != kRefBin) e = bins_setup();
   if (!e) {
     switch (a.tile) {
       case 8: e = launch_pdl(one ? raster_frag8<true> : raster_frag8<false>, raster_ctas, 256, st, a); break;
-      case 32: e = launch_pdl(one ? raster_tiles<32, true> : raster_tiles<32, false>, raster_ctas, 128, st, a); break;
-      default: e = launch_pdl(one ? raster_tiles<16, true> : raster_tiles<16, false>, raster_ctas, 256, st, a); break;
+      case 32: e = launch_pdl(one ? raster_bins<32, true> : raster_bins<32, false>, raster_ctas, 256, st, a, sizeof(BinsSmem)); break;
+      default: e = launch_pdl(one ? raster_bins<16, true> : raster_bins<16, false>, raster_ctas, 256, st, a, sizeof(BinsSmem)); break;
     }
   }
   if (ev) cudaEventRecord(ev[4], st);
@@ -1829,11 +1780,12 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& a, int raster_ctas, cudaS
 
 cudaError_t raster_tiles_occupancy(int tile, int* blocks_per_sm)
 {
-  switch (tile) {
-    case 8: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_frag8<false>, 256, 0);
-    case 32: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_tiles<32, false>, 128, 0);
-    default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_tiles<16, false>, 256, 0);
-  }
+  if (tile == kRefBin) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_frag8<false>, 256, 0);
+  const cudaError_t e = bins_setup();
+  if (e) return e;
+  if (tile == 32)
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_bins<32, false>, 256, sizeof(BinsSmem));
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, raster_bins<16, false>, 256, sizeof(BinsSmem));
 }
 
 }  // namespace piko

@@ -55,17 +55,11 @@ int raster_ctas(piko_ctx* ctx, int tile, int ctas_per_sm)
   return ctx->sms * per_sm;
 }
 
-uint32_t heavy_threshold(int tile)
-{
-  // list entries above which a tile is served from the heavy queue first
-  return tile == 8 ? 32u : 64u;
-}
-
 // Enqueues one frame of draws [0, n) sharing one scratch.
 piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, RasterScratch& scr, int T, int ctas,
                                  cudaStream_t st, bool timed, bool coverage, uint32_t chunk, bool table_ready)
 {
-  if (chunk == 0) chunk = T == kRefBin ? kDefaultChunk8 : kDefaultChunk;
+  if (chunk == 0) chunk = default_chunk(T);
   uint32_t tris = 0, tiles = 0;
   for (int i = 0; i < n; ++i) {
     int tx, ty;
@@ -84,7 +78,11 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   const uint32_t warps = (uint32_t)ctas * 8u;
   uint32_t group = (uint32_t)kLightGroup;
   while (group > 1 && tiles / group < warps) group /= 2;
-  const uint32_t queue_min = std::min(tiles / warps >= 4u * kLightGroup ? 2u * kQueueMin : kQueueMin, chunk);
+  // 16/32-px tiles: a work item tests its list against a quad of bins at once,
+  // but a frame with few bins for the grid's warps spreads better bin by bin
+  // (800x600, 7,500 bins for 4,736 warps: frame 59 -> 42 us)
+  if (T != kRefBin) group = tiles * (uint32_t)(T / kRefBin) * (uint32_t)(T / kRefBin) < 4u * warps ? 1u : 4u;
+  const uint32_t queue_min = std::min(T == kRefBin && tiles / warps >= 4u * kLightGroup ? 2u * kQueueMin : kQueueMin, chunk);
   CU(ctx, scr.ensure_heavy(tiles, T, chunk, queue_min));
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   CU(ctx, cudaStreamIsCapturing(st, &capture));
@@ -129,8 +127,6 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   a.pair_tl = scr.pair_tl;
   a.pair_g = scr.pair_g;
   a.list_cap = scr.list_cap;
-  a.heavy_threshold = heavy_threshold(T);
-  a.heavy_cap = scr.heavy_cap;
   a.large_seg = scr.large_seg;
   a.seg_cap = scr.seg_cap;
   a.large_walk = scr.large_walk;
@@ -142,6 +138,7 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   a.hdone = scr.hdone;
   a.chunk_keys = scr.chunk_keys;
   a.chunk_cap = scr.chunk_cap;
+  a.key_cap = scr.key_cap;
   a.scan_flags = scr.scan_flags;
   a.work = scr.work;
   a.ctr = scr.ctr;

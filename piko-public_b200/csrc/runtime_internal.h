@@ -106,11 +106,11 @@ struct RasterScratch {
   uint2* large_seg = nullptr;   // large-triangle segment items
   uint32_t seg_cap = 0;
   WalkTri* large_walk = nullptr;  // walk records of the large triangles, [seg_cap]: each has a segment
-  uint32_t* hdone = nullptr;                // finished chunks per heavy tile
-  unsigned long long* chunk_keys = nullptr; // tile * tile keys per chunk
+  uint32_t* hdone = nullptr;                // finished chunks, per key slot and bin of the tile
+  unsigned long long* chunk_keys = nullptr; // tile * tile keys per key slot
   ChunkDesc* chunk_desc = nullptr;
-  uint32_t heavy_cap = 0, chunk_cap = 0;
-  uint32_t chunk_stride = 0;                // keys per chunk (tile * tile)
+  uint32_t chunk_cap = 0, key_cap = 0;
+  uint32_t key_stride = 0;                  // keys per key slot (tile * tile)
   unsigned long long* scan_flags = nullptr;
   BinWork* work = nullptr;
   FrameCounters* ctr = nullptr;
@@ -139,32 +139,28 @@ struct RasterScratch {
     clean = false;
     if (ev_made) for (auto& e : ev) cudaEventDestroy(e);
     ev_made = false;
-    tris_cap = tiles_cap = list_cap = scan_cap = heavy_cap = chunk_cap = seg_cap = chunk_stride = 0;
+    tris_cap = tiles_cap = list_cap = scan_cap = chunk_cap = key_cap = seg_cap = key_stride = 0;
     scenes_cap = 0;
     cov_cap = 0;
   }
 
-  // Heavy-tile queue.  16/32-px tiles: any tile may be heavy.  8x8 tiles: a
-  // heavy tile has more than `queue_min` list entries, so at most
-  // list_cap / (queue_min + 1) of them exist.  Heavy lists are cut into
-  // chunks, each with T * T keys in chunk_keys; the key buffers start at an
-  // estimate and grow after a frame reports that it needed more (regrow).
+  // Heavy-tile queue.  A heavy tile has more than `queue_min` list entries, so
+  // at most list_cap / (queue_min + 1) of them exist, and their lists make at
+  // most list_cap / chunk further chunks: descriptors for all of these.  Key
+  // slots, T * T keys each, are for lists in several chunks only; they start at
+  // an estimate and grow after a frame reports that it needed more (regrow).
   cudaError_t ensure_heavy(uint32_t n_tiles, int T, uint32_t chunk, uint32_t queue_min)
   {
-    const bool t8 = T == kRefBin;
-    const uint32_t need_h = t8 ? std::min<uint32_t>(n_tiles, list_cap / (queue_min + 1) + 1) : n_tiles;
     cudaError_t e = cudaSuccess;
-    if (need_h > heavy_cap || !hdone) {
-      dfree(hdone);
-      heavy_cap = 0;
-      if ((e = dalloc(&hdone, need_h))) return e;
-      heavy_cap = need_h;
+    const uint32_t need = std::min<uint32_t>(n_tiles, list_cap / (queue_min + 1)) + list_cap / chunk + 1;
+    if (need > chunk_cap) {
+      dfree(chunk_desc);
+      chunk_cap = 0;
+      if ((e = dalloc(&chunk_desc, need))) return e;
+      chunk_cap = need;
     }
-    const uint32_t stride = (uint32_t)(T * T);
-    const uint32_t want = t8 ? need_h / 2 + list_cap / (4 * chunk) + 64 : list_cap / (8 * chunk) + 64;
-    if (want > chunk_cap || stride != chunk_stride) {
-      if ((e = grow_chunks(std::max(want, stride == chunk_stride ? chunk_cap : 0u), stride))) return e;
-    }
+    const uint32_t stride = (uint32_t)(T * T), want = list_cap / (8 * chunk) + 64;
+    if (want > key_cap || stride != key_stride) return grow_keys(std::max(want, stride == key_stride ? key_cap : 0u), stride);
     return cudaSuccess;
   }
 
@@ -192,20 +188,20 @@ struct RasterScratch {
     return e;
   }
 
-  // key buffers of n chunks of `stride` keys each
-  cudaError_t grow_chunks(uint32_t n, uint32_t stride)
+  // n key slots of `stride` keys each, with a counter for each 8x8 bin
+  cudaError_t grow_keys(uint32_t n, uint32_t stride)
   {
     dfree(chunk_keys);
-    dfree(chunk_desc);
-    chunk_cap = 0;
+    dfree(hdone);
+    key_cap = 0;
     cudaError_t e = dalloc(&chunk_keys, (size_t)n * stride);
-    if (!e) e = dalloc(&chunk_desc, n);
-    if (!e) { chunk_cap = n; chunk_stride = stride; }
+    if (!e) e = dalloc(&hdone, (size_t)n * (stride / (kRefBin * kRefBin)));
+    if (!e) { key_cap = n; key_stride = stride; }
     return e;
   }
 
   // After a frame whose counters report a queue overflow: grows what
-  // overflowed (the tile lists and / or the chunk key buffers) so that the
+  // overflowed (the tile lists and / or the key slots) so that the
   // frame can be drawn again.
   cudaError_t regrow(const BinCounts& c)
   {
@@ -217,9 +213,9 @@ struct RasterScratch {
     if (need > list_cap || c.pair_part_max > list_cap / kPairParts) {
       if ((e = grow_list(need + need / 4 + 1024))) return e;
     }
-    const uint32_t chunks = (uint32_t)c.heavy_acc;
-    if (chunk_desc && chunks > chunk_cap) {
-      if ((e = grow_chunks(chunks + chunks / 4 + 64, chunk_stride))) return e;
+    const uint32_t keys = (uint32_t)(c.heavy_acc >> 32);
+    if (key_stride && keys > key_cap) {
+      if ((e = grow_keys(keys + keys / 4 + 64, key_stride))) return e;
     }
     // every large triangle has at least one segment: seg_cap bounds both
     const uint32_t segs = std::max((uint32_t)c.large_acc, (uint32_t)(c.large_acc >> 32));
@@ -309,7 +305,7 @@ struct piko_scene {
 
 // Launch configuration of a raster launch sequence: tile edge, persistent
 // CTAs per SM (0 = the kernel's occupancy) and list entries per chunk of the
-// 8x8 tile queue (0 = kDefaultChunk).
+// tile queue (0 = default_chunk).
 struct TuneCfg {
   int tile = 8;
   int ctas_per_sm = 0;
@@ -369,9 +365,11 @@ struct RasterDraw {
   uint32_t* fb;
   float* depth;
 };
-// chunk: list entries per chunk of the 8x8 tile queue (kDefaultChunk when 0);
-// lists longer than kQueueMin entries are queued as chunks
-constexpr uint32_t kDefaultChunk = 32, kDefaultChunk8 = 64;
+// chunk: list entries per chunk of the tile queue (default_chunk when 0); lists
+// longer than kQueueMin entries are queued as chunks
+// (the parts of a 32-px list that one bin takes fill a pass better from longer
+// chunks: 200K triangles at 1080p 206 -> 186 us, 24-scene batch 494 -> 457)
+inline uint32_t default_chunk(int tile) { return tile == 32 ? 128u : 64u; }
 constexpr uint32_t kQueueMin = 8;
 // table_ready: the scene table in scr already holds these draws
 piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, RasterScratch& scr, int T, int ctas,
@@ -381,4 +379,3 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
 piko_status enqueue_raster(piko_ctx* ctx, piko_scene* const* scenes, int n, RasterScratch& scr, const TuneCfg& cfg,
                            cudaStream_t st, bool timed, bool coverage, bool table_ready = false);
 int raster_ctas(piko_ctx* ctx, int tile, int ctas_per_sm);
-uint32_t heavy_threshold(int tile);

@@ -83,3 +83,38 @@ def test_wrapping_area(pk, ctx, oracle_mod):
     sc["xyz"] = np.concatenate([big, sc["xyz"]])
     sc["icol"] = np.concatenate([np.full((2, 3), 0xFF3060C0, np.uint32), sc["icol"]])
     check(pk, ctx, oracle_mod, sc)
+
+
+def spread(kind, n, W, H, seed, size):
+    """payload() with the triangles spread over the frame, some of them large."""
+    sc = payload(kind, n, W, H, seed, size)
+    g = np.random.Generator(np.random.Philox(seed + 1))
+    dx, dy = g.uniform(-W / 2, W / 2, n), g.uniform(-H / 2, H / 2, n)
+    sc["xyz"][:, 0::3] += dx[:, None].astype(np.float32)
+    sc["xyz"][:, 1::3] += dy[:, None].astype(np.float32)
+    return sc
+
+
+@pytest.mark.parametrize("tile", [16, 32])
+@pytest.mark.parametrize("chunk", [0, 1, 40, 4096])
+def test_bins_of_larger_tiles(pk, ctx, oracle_mod, tile, chunk):
+    """16/32-px tiles: a bin's entries gathered from a tile list that other bins
+    share, in frames drawn bin by bin and (the large one) quad by quad."""
+    cases = [payload("planes", n, 64, 72, n, s) for n in (1, 8, 9, 33, 300) for s in (3.0, 40.0)]
+    cases += [payload("signed", 200, 40, 33, 3, 20.0), spread("near", 5000, 333, 257, 4, 6.0)]
+    if chunk in (0, 40):
+        cases.append(spread("planes", 30000, 1920, 1080, 5, 12.0))
+    for sc in cases:
+        pipe = pk.Pipe(ctx, "raster", tile_px=tile, chunk_entries=chunk)
+        s = pk.Scene(pipe, sc)
+        try:
+            s.run()
+            fb, depth = s.read()
+            st = s.stats()
+        finally:
+            s.close()
+            pipe.close()
+        ofb, odepth, ost = oracle_mod.raster_frame(sc["W"], sc["H"], sc["xyz"], sc["icol"])
+        assert np.array_equal(depth.view(np.uint32), odepth.view(np.uint32))
+        assert np.array_equal(fb, ofb)
+        assert st["covered"] == ost["covered"]
