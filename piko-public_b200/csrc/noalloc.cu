@@ -149,6 +149,7 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
       cudaStreamSynchronize(st) != cudaSuccess)
     return PIKO_ERR_CUDA;
   if (c.bin.status & kStatusScanTimeout) return PIKO_ERR_TIMEOUT;
-  if (c.bin.status & kStatusListOverflow) return PIKO_ERR_QUEUE_OVERFLOW;
+  // (the documented limit counts every queue entry, listed here or not)
+  if ((c.bin.status & kStatusListOverflow) || c.bin.list_total + c.bin.skipped > kNaMaxList) return PIKO_ERR_QUEUE_OVERFLOW;
   return PIKO_OK;
 }

@@ -179,9 +179,12 @@ constexpr uint32_t kTriAreaRisk = 2u;  // the area may wrap: its reciprocal says
 constexpr uint32_t kPairParts = 128;
 struct BinCounts {
   uint32_t status;
-  uint32_t list_total;
+  uint32_t list_total;           // list entries
   uint32_t kept;
   uint32_t pair_part_max;        // largest partition fill asked for (past its capacity: overflow)
+  // (triangle, tile) pairs that pass the tile-level reject but cannot hold a
+  // covered pixel: part of the bin queues of the reference, not listed here
+  unsigned long long skipped;
   unsigned long long risk;
   unsigned long long heavy_acc;  // key slots << 32 | items (chunks, or without chunk buffers heavy tiles)
   unsigned long long large_acc;  // large triangles << 32 | their box-tile segments
@@ -208,20 +211,20 @@ struct BinWork {
   uint32_t scan_ticket;
   uint32_t pad[3];
   // The count passes record their (triangle, tile) pairs in kPairParts
-  // partitions of list_cap / kPairParts slots each (a warp takes partition
-  // (its global warp index) mod kPairParts), so that slot reservations spread
-  // over kPairParts counters instead of queueing on one address.
+  // partitions of list_cap / kPairParts slots each (chosen by block and warp),
+  // so that slot reservations spread over kPairParts counters instead of
+  // queueing on one address.
   uint32_t pair_part[kPairParts];
 };
 
-// A triangle's box-tile walk: its 28.4 vertices, reference bin range, first
-// tile and tiles per row (with the divide-by-tw magic), global setup slot and
-// scene tile base, and for 8x8 tiles the reference's trivial-reject value of
-// each edge at the first bin with its change per bin in x and y (wrapping
-// int32, so equal to evaluating each bin directly).  Large triangles keep
-// theirs in memory for the segment walk (112 bytes, 16-byte aligned).
+// A triangle's box-tile walk: its reference bin range, first tile and tiles per
+// row (with the divide-by-tw magic), global setup slot and scene tile base, the
+// part of the box that is listed, and for 8x8 tiles the reference's
+// trivial-reject value of each edge at the first bin with its change per bin in
+// x and y (wrapping int32, so equal to evaluating each bin directly), for larger
+// tiles the 28.4 vertices.  Large triangles keep theirs in memory for the
+// segment walk (96 bytes, 16-byte aligned).
 struct __align__(16) WalkTri {
-  int32_t x[3], y[3];
   int32_t bx1, bx2, by1, by2;
   int32_t tx1, ty1, tw;
   uint32_t tw_m;          // divmod_magic(tw)
@@ -229,9 +232,13 @@ struct __align__(16) WalkTri {
   uint32_t tile_base;
   int32_t tiles_x;
   uint32_t flags;
-  int32_t tr0[3], trx[3], try_[3];
+  uint32_t ltx, lty;      // columns and rows of the box that are listed: lo | hi << 16 (lty 1: none)
+  union {
+    struct { int32_t tr0[3], trx[3], try_[3]; };
+    struct { int32_t x[3], y[3]; };
+  };
 };
-static_assert(sizeof(WalkTri) == 112, "WalkTri layout");
+static_assert(sizeof(WalkTri) == 96, "WalkTri layout");
 
 // A chunk of a heavy tile's list, written by the scan: all that the warp that
 // takes it needs, in one 32-byte read.
@@ -251,6 +258,7 @@ struct RasterFrameArgs {
   int tile;                 // tile edge in pixels: 8, 16 or 32
   uint32_t n_tris_total;    // sum of N
   uint32_t n_tiles_total;
+  uint32_t batch;           // triangles a raster_setup CTA takes at a time (set by the launch)
   TriSetup* setup;          // [n_tris_total]; written only for triangles that reach a bin (rank1 != 0)
   uint32_t* tile_cnt;       // [n_tiles_total]
   uint32_t* tile_off;       // [n_tiles_total + 1]

@@ -5,11 +5,11 @@
 //   raster_setup    one thread per triangle.  Vertex shading + triangle setup
 //                   (R1: main.cpp:299-400 moved on device; R3: vertexShader.pikostage:36-109)
 //                   from coalesced SoA loads, then AssignBin (R4,
-//                   raster.pikostage:40-117) as a warp-cooperative tile walk: one
+//                   raster.pikostage:40-117) as a block-cooperative tile walk: one
 //                   counter atomic per (triangle, tile) pair (shared by the
 //                   warp's lanes with the same tile at 16/32-px tiles), whose old
 //                   value is the pair's index in the tile's list, and a pair
-//                   record.  Triangles with more than 32 box tiles are queued
+//                   record.  Triangles with more than 256 box tiles are queued
 //                   as 128-tile segments for
 //   raster_large_count, which walks them the same way over the whole grid.
 //   scan_tiles      exclusive prefix sum of the tile counts (single pass,
@@ -42,7 +42,11 @@
 namespace piko {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr uint32_t kLargeTiles = 32;  // box tiles above which a triangle's walk is spread over the grid
+constexpr int kSetupThreads = 256;
+constexpr uint32_t kLargeTiles = 256; // box tiles above which a triangle's walk is spread over the grid
+constexpr uint32_t kWalkQueue = 256;  // tiles a warp of the walk can have queued
+constexpr uint32_t kItemMap = 4096;   // row items of a block's walk whose triangle is looked up
+static_assert(kLargeTiles <= 256 && kSetupThreads <= 256, "the walk's queue holds 8-bit tiles and triangles");
 constexpr uint32_t kLargeSeg = 128;   // box tiles per work item of the large-triangle walk
 
 // ------------------------------------------------------------------ helpers
@@ -182,23 +186,12 @@ __device__ __forceinline__ int32_t edge_at(int32_t X, int32_t Y, int32_t xi, int
   return wsub(wmul(wsub(Y, yi), dx), wmul(wsub(X, xi), dy));
 }
 
-// Per-lane staging for the warp-cooperative tile walk.
-
-// Conservative tile-level trivial reject (exact int64 arithmetic): the tile,
-// clipped to the triangle's bin range, can hold an assigned reference bin only
-// if every edge function is >= 0 at the tile corner that maximises it.  Only
-// used for triangles whose edge values cannot wrap inside the bin range.
+// Conservative trivial reject of a 16/32-px tile (exact int64 arithmetic): the
+// tile, clipped to the triangle's bin range, can hold an assigned reference bin
+// only if every edge function is >= 0 at the tile corner that maximises it.
+// Only used for triangles whose edge values cannot wrap inside the bin range.
 __device__ __forceinline__ bool tile_may_cover(const WalkTri& w, int tx, int ty, int T)
 {
-  if (T == kRefBin) {
-    // the tile is one reference bin: the reference's own trivial reject at the
-    // bin corner (raster.pikostage:77-105), stepped from bin (tx1, ty1)
-    const int32_t k = tx - w.tx1, m = ty - w.ty1;
-    int32_t tr = 0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) tr |= wadd(wadd(w.tr0[i], wmul(k, w.trx[i])), wmul(m, w.try_[i]));
-    return tr >= 0;
-  }
   if (w.flags & kTriRisk) return true;
   long long X0 = (long long)max(tx * T, w.bx1 * kRefBin) * 16;
   long long X1 = (long long)min((tx + 1) * T, (w.bx2 + 1) * kRefBin) * 16;
@@ -258,7 +251,8 @@ __device__ __forceinline__ void count_pairs(const RasterFrameArgs& a, const uint
     n += (uint32_t)__popc(m[q]);
   }
   if (n == 0) return;
-  const uint32_t part = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) & (kPairParts - 1u);
+  // (by block first: a block's first warps record the most)
+  const uint32_t part = (blockIdx.x + (threadIdx.x >> 5) * (kPairParts / 8)) & (kPairParts - 1u);
   const uint32_t part_cap = a.list_cap / kPairParts;
   uint32_t base = 0;
   if (lane == 0) {
@@ -304,59 +298,155 @@ __device__ __forceinline__ void frame_begin(const RasterFrameArgs& a)
   if (threadIdx.x == 0 && a.host_bin) *a.host_bin = a.ctr->bin;
 }
 
-// Walks every (triangle, tile) pair of a warp's 32 triangles with all 32 lanes
-// busy: pair j belongs to the lane whose inclusive tile-count prefix first
-// exceeds j; the pairs that pass the tile-level reject are counted and
-// recorded, four rounds of 32 at a time so that four counter atomics per lane
-// are in flight together.
-__device__ __forceinline__ void walk_tiles(const RasterFrameArgs& a, const WalkTri* wt, uint32_t ntiles)
+// Which of columns [c0, c0 + n) (n <= 32) of row `row` of triangle w's box tiles
+// pass the tile-level reject, as bits.  At 8x8 tiles that is the reference's
+// own trivial reject at the bin corner (raster.pikostage:77-105), stepped from
+// bin (tx1, ty1).
+__device__ __forceinline__ uint32_t row_mask(const WalkTri& w, uint32_t row, uint32_t c0, uint32_t n, int T)
 {
-  const int lane = threadIdx.x & 31;
-  uint32_t incl = ntiles;
+  uint32_t m = 0;
+  if (T == kRefBin) {
+    // last column first, so that column c0 ends in bit 0: bits of rejected tiles
+    int32_t t[3], dx[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      dx[i] = w.trx[i];
+      t[i] = wadd(wadd(w.tr0[i], wmul((int32_t)row, w.try_[i])), wmul((int32_t)(c0 + n - 1), dx[i]));
+    }
+#pragma unroll 4
+    for (uint32_t k = 0; k < n; ++k) {
+      m = __funnelshift_l((uint32_t)(t[0] | t[1] | t[2]), m, 1);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) t[i] = wsub(t[i], dx[i]);
+    }
+    return ~m & (n < 32u ? (1u << n) - 1u : 0xffffffffu);
+  }
+  for (uint32_t k = 0; k < n; ++k)
+    m |= (uint32_t)tile_may_cover(w, w.tx1 + (int)(c0 + k), w.ty1 + (int)row, T) << k;
+  return m;
+}
+
+// The tiles of row_mask's range that can hold a covered pixel centre (the box
+// that holds the triangle's tiles is rounded up to 16 px and one bin beyond).
+__device__ __forceinline__ uint32_t listed_mask(const WalkTri& w, uint32_t row, uint32_t c0, uint32_t n)
+{
+  const uint32_t x0 = w.ltx & 0xffffu, x1 = w.ltx >> 16, y0 = w.lty & 0xffffu, y1 = w.lty >> 16;
+  if (row < y0 || row > y1 || x0 >= c0 + n || x1 < c0) return 0u;   // (no tile: y0 > y1)
+  const uint32_t lo = x0 > c0 ? x0 - c0 : 0u, hi = min(x1 - c0, n - 1);
+  return (0xffffffffu >> (31u - hi)) & (0xffffffffu << lo);
+}
+
+// Counts and records queue entries [first, first + n), n <= 128, one per lane at
+// a time; key_of(entry, gidx) turns an entry into its global tile.
+template <class F>
+__device__ __forceinline__ void record_queue(const RasterFrameArgs& a, const uint16_t* queue, uint32_t first, uint32_t n,
+                                             int lane, F key_of)
+{
+  uint32_t key[4], gidx[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t p = (uint32_t)(q * 32 + lane);
+    key[q] = 0xffffffffu;
+    gidx[q] = 0;
+    if (p < n) key[q] = key_of(queue[first + p], gidx[q]);
+  }
+  count_pairs<4>(a, key, gidx, lane);
+}
+
+// Appends the tiles of the warp's masks to its queue of qn entries (a mask per
+// lane: bit k of m is tile at + k of the lane's triangle, tagged tag) and
+// records them 128 at a time, so that all of count_pairs' rounds are full; fewer
+// than 128 stay queued.
+template <class F>
+__device__ __forceinline__ void queue_masks(const RasterFrameArgs& a, uint16_t* queue, uint32_t& qn, uint32_t m,
+                                            uint32_t tag, uint32_t at, int lane, F key_of)
+{
+  uint32_t incl = (uint32_t)__popc(m);
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    uint32_t v = __shfl_up_sync(kFull, incl, o);
+    const uint32_t v = __shfl_up_sync(kFull, incl, o);
     if (lane >= o) incl += v;
   }
-  const uint32_t excl = incl - ntiles;
-  const uint32_t total = __shfl_sync(kFull, incl, 31);
-  constexpr int kRounds = 4;
-  for (uint32_t base = 0; base < total; base += 32 * kRounds) {
-    uint32_t key[kRounds], gidx[kRounds];
-#pragma unroll
-    for (int q = 0; q < kRounds; ++q) {
-      const uint32_t j = base + (uint32_t)q * 32u + (uint32_t)lane;
-      int lo = 0, hi = 31;
-#pragma unroll
-      for (int st = 0; st < 5; ++st) {
-        const int mid = (lo + hi) >> 1;
-        const uint32_t v = __shfl_sync(kFull, incl, mid);
-        if (v > j) hi = mid; else lo = mid + 1;
-      }
-      const int owner = lo;
-      const uint32_t oexcl = __shfl_sync(kFull, excl, owner);
-      key[q] = 0xffffffffu;
-      gidx[q] = 0;
-      if (j < total) {
-        const WalkTri& w = wt[owner];
-        uint32_t lx;
-        const uint32_t ly = fast_divmod(j - oexcl, (uint32_t)w.tw, w.tw_m, lx);
-        const int tx = w.tx1 + (int)lx, ty = w.ty1 + (int)ly;
-        if (tile_may_cover(w, tx, ty, a.tile)) {
-          key[q] = w.tile_base + (uint32_t)(ty * w.tiles_x + tx);
-          gidx[q] = w.gidx;
-        }
-      }
-    }
-    count_pairs<kRounds>(a, key, gidx, lane);
+  uint32_t pos = qn + incl - (uint32_t)__popc(m), end = qn + __shfl_sync(kFull, incl, 31);
+  for (;;) {
+    for (; m && pos < kWalkQueue; m &= m - 1u, ++pos)
+      queue[pos] = (uint16_t)((tag << 8) | (at + (uint32_t)__ffs(m) - 1u));
+    __syncwarp();
+    const uint32_t had = min(end, kWalkQueue);
+    for (qn = had; qn >= 128u; qn -= 128u) record_queue(a, queue, qn - 128u, 128u, lane, key_of);
+    if (end <= kWalkQueue) return;
+    __syncwarp();   // the queue is refilled behind its first qn entries
+    pos -= had - qn;
+    end -= had - qn;
   }
 }
 
+__device__ __forceinline__ uint32_t tile_key(const WalkTri& w, uint32_t j)
+{
+  uint32_t lx;
+  const uint32_t ly = fast_divmod(j, (uint32_t)w.tw, w.tw_m, lx);
+  return w.tile_base + (uint32_t)((w.ty1 + (int)ly) * w.tiles_x + w.tx1 + (int)lx);
+}
+
+// Walks the box tiles of the block's triangles wt[0, n) (at most kLargeTiles
+// each) with all of its threads: a thread tests a row of a triangle's box (up to
+// 32 columns of it), stepping the edge values (row item i belongs to triangle
+// item_tri[i], the first whose inclusive item-count prefix pre[] exceeds i; past
+// kItemMap items it is searched).  The tiles that
+// can hold a covered pixel are counted and recorded, one per lane; the others
+// that pass the reject are returned as a number, the warp's in each lane.  (A
+// thread per tile, each with its own search and divide, took about 110
+// instructions a box tile where this takes some 25.)
+__device__ __forceinline__ uint32_t walk_tiles(const RasterFrameArgs& a, const WalkTri* wt, const uint32_t* pre,
+                                               const uint8_t* item_tri, int n, uint16_t* queue)
+{
+  const int lane = threadIdx.x & 31;
+  const uint32_t total = n ? pre[n - 1] : 0u;
+  const auto key_of = [&](uint32_t e, uint32_t& gidx) {
+    const WalkTri& w = wt[e >> 8];
+    gidx = w.gidx;
+    return tile_key(w, e & 255u);
+  };
+  uint32_t skipped = 0, qn = 0;
+  for (uint32_t base = threadIdx.x & ~31u; base < total; base += kSetupThreads) {
+    const uint32_t i = base + (uint32_t)lane;
+    uint32_t m = 0, tri = 0, at = 0;
+    if (i < total) {
+      if (i < kItemMap) {
+        tri = item_tri[i];
+      } else {
+        int lo = 0, hi = n - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (pre[mid] > i) hi = mid; else lo = mid + 1;
+        }
+        tri = (uint32_t)lo;
+      }
+      const WalkTri& w = wt[tri];
+      const uint32_t tw = (uint32_t)w.tw, parts = (tw + 31u) >> 5;
+      uint32_t row = i - (tri ? pre[tri - 1] : 0u), c0 = 0;
+      if (parts > 1) {
+        c0 = (row % parts) * 32u;
+        row /= parts;
+      }
+      const uint32_t cols = min(tw - c0, 32u);
+      m = row_mask(w, row, c0, cols, a.tile);
+      skipped += (uint32_t)__popc(m);
+      m &= listed_mask(w, row, c0, cols);
+      skipped -= (uint32_t)__popc(m);
+      at = row * tw + c0;
+    }
+    queue_masks(a, queue, qn, m, tri, at, lane, key_of);
+  }
+  if (qn) record_queue(a, queue, 0u, qn, lane, key_of);
+  return __reduce_add_sync(kFull, skipped);
+}
+
+// The walk record of triangle g, and the number of tiles in its box.
 __device__ __forceinline__ void fill_walk(const RasterFrameArgs& a, const RasterSceneDev& S, const TriSetup& r,
                                           uint32_t g, WalkTri& w, uint32_t& ntiles)
 {
   const int tsh = __ffs(a.tile) - 1 - kRefBinLg2;   // tile edge = 8 << tsh
-  for (int k = 0; k < 3; ++k) { w.x[k] = r.x[k]; w.y[k] = r.y[k]; }
   w.bx1 = (int)(r.bxr & 0xffff); w.bx2 = (int)(r.bxr >> 16);
   w.by1 = (int)(r.byr & 0xffff); w.by2 = (int)(r.byr >> 16);
   w.tx1 = w.bx1 >> tsh;
@@ -369,6 +459,19 @@ __device__ __forceinline__ void fill_walk(const RasterFrameArgs& a, const Raster
   w.tiles_x = S.tiles_x;
   w.flags = r.flags;
   ntiles = (uint32_t)w.tw * (uint32_t)(ty2 - w.ty1 + 1);
+  // The tiles to list: those that hold a pixel centre of the triangle's own
+  // bounds (a covered centre lies inside the triangle unless an edge value may
+  // wrap; then all).
+  int lx0 = w.tx1, lx1 = tx2, ly0 = w.ty1, ly1 = ty2;
+  if (!(r.flags & kTriRisk)) {
+    const int px0 = (min(min(r.x[0], r.x[1]), r.x[2]) + 7) >> 4, px1 = (max(max(r.x[0], r.x[1]), r.x[2]) - 8) >> 4;
+    const int py0 = (min(min(r.y[0], r.y[1]), r.y[2]) + 7) >> 4, py1 = (max(max(r.y[0], r.y[1]), r.y[2]) - 8) >> 4;
+    lx0 = max(lx0, px0 >> (kRefBinLg2 + tsh)); lx1 = min(lx1, px1 >> (kRefBinLg2 + tsh));
+    ly0 = max(ly0, py0 >> (kRefBinLg2 + tsh)); ly1 = min(ly1, py1 >> (kRefBinLg2 + tsh));
+    if (px0 > px1 || py0 > py1 || lx0 > lx1) ly1 = ly0 - 1;
+  }
+  w.ltx = (uint32_t)(lx0 - w.tx1) | ((uint32_t)(lx1 - w.tx1) << 16);
+  w.lty = ly0 <= ly1 ? (uint32_t)(ly0 - w.ty1) | ((uint32_t)(ly1 - w.ty1) << 16) : 1u;   // (rows [1, 0]: none)
   if (tsh == 0) {
     const int32_t BX = w.tx1 * 128, BY = w.ty1 * 128;   // bin corner, 28.4
 #pragma unroll
@@ -381,6 +484,8 @@ __device__ __forceinline__ void fill_walk(const RasterFrameArgs& a, const Raster
       w.trx[i] = -wshl(dy, 7);
       w.try_[i] = wshl(dx, 7);
     }
+  } else {
+    for (int k = 0; k < 3; ++k) { w.x[k] = r.x[k]; w.y[k] = r.y[k]; }
   }
 }
 
@@ -393,135 +498,219 @@ __device__ __forceinline__ float4 load_attr3(const float4* a4, const float* a3, 
 }
 
 // ------------------------------------------------------------------ kernel 1
-// 128-thread CTAs: one wave holds the scene's triangle blocks spread nearly
-// evenly over the SMs.
-constexpr int kSetupThreads = 128;
+// A block takes a.batch triangles at a time (at most its threads), in steps
+// that each spread what is left of them over all threads:
+//   1. a thread per triangle: transform, 28.4 quantisation and the culls;
+//   2. the kept triangles' vertices, one per thread, are lit (a culled
+//      triangle's colours are never read: only kept ones load normals);
+//   3. a thread per kept triangle: bin range, setup record, walk record;
+//   4. a thread per row of a kept triangle's box tiles: the tile walk.
+// (One thread taking its triangle through all of it had half of its lanes culled
+// on the batched mix, three quarters on the forest.  Setup and large count of
+// one frame together, before and now: 1,000 triangles 13 -> 8 us, 1080p forest
+// 33 -> 24, 200K triangles 47 -> 34, 24-scene batch 111 -> 98.)  The walk counts every
+// pair that passes the reject, as the reference's queues do, but lists only
+// tiles that can hold a covered pixel centre: a third fewer list entries, which
+// the later kernels do not touch (200K triangles: fragment pass 100 -> 92 us).
+constexpr int kSetupWarps = kSetupThreads / 32;
+
+struct SetupSmem {
+  WalkTri walk[kSetupThreads];
+  union {
+    struct {   // the kept triangles, in order (steps 1 to 3)
+      int32_t x[3][kSetupThreads], y[3][kSetupThreads];
+      float z[3][kSetupThreads];
+      uint32_t c[3][kSetupThreads];
+      uint32_t g[kSetupThreads];
+    };
+    struct {   // step 4
+      uint32_t pre[kSetupThreads];
+      uint8_t item_tri[kItemMap];
+      uint16_t queue[kSetupWarps][kWalkQueue];
+    };
+  };
+  uint32_t warp[kSetupWarps];
+  unsigned nk, nr;
+  unsigned skipped;   // pairs that pass the reject and are not listed (of one CTA: below 2^32)
+};
+
+// Inclusive scan of v over the block.
+__device__ __forceinline__ uint32_t block_scan_incl(uint32_t v, uint32_t* s_warp)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(kFull, v, o);
+    if (lane >= o) v += t;
+  }
+  if (lane == 31) s_warp[warp] = v;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kSetupWarps; ++w)
+    if (w < warp) v += s_warp[w];
+  return v;
+}
+
 template <bool ONE>
 __global__ void __launch_bounds__(kSetupThreads) raster_setup(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_trigger();
-  __shared__ WalkTri s_walk[kSetupThreads];
-  __shared__ unsigned s_kept[kSetupThreads / 32], s_risk[kSetupThreads / 32];
-  __shared__ uint32_t s_tb[kSceneTable];
+  extern __shared__ __align__(16) unsigned char setup_smem[];
+  SetupSmem& B = *reinterpret_cast<SetupSmem*>(setup_smem);
+  uint32_t* s_tb = reinterpret_cast<uint32_t*>(&B + 1);   // the scene table, several scenes only
   load_scene_table<ONE, kSceneTable>(a, s_tb, false);
+  if (threadIdx.x == 0) B.nk = B.nr = B.skipped = 0u;
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  unsigned nk = 0, nr = 0;
-  // one wave of CTAs strides over blocks of kSetupThreads triangles
-  for (uint32_t base = blockIdx.x * (uint32_t)kSetupThreads; base < a.n_tris_total;
-       base += gridDim.x * (uint32_t)kSetupThreads) {
-  const uint32_t g = base + threadIdx.x;
-  uint32_t ntiles = 0;
-  bool kept_flag = false, risk_flag = false;
-  if (g < a.n_tris_total) {
-    const int s = scene_of<ONE, kSceneTable>(a, s_tb, g, false);
-    const RasterSceneDev& S = scene_at<ONE>(a, s);
-    const uint32_t id = g - S.tri_base;
-    float sx[3], sy[3], sz[3];
-    uint32_t ic[3] = {0u, 0u, 0u};
-    const bool soa = S.input_kind == kInputSoA;
-    if (soa || S.input_kind == kInputWtriWorld) {
-      // R1, main.cpp:299-308: vtransform, perspective divide, viewport.  The
-      // per-vertex lighting follows the culls: a culled triangle's colours are
-      // never read, so only kept triangles load normals and are lit.  World
-      // raster_wtri input: the vertex stage's vtxTransform (rasterMacros.h:14-21,
-      // matmultfloat4 and rcp_approx = 1.0f / w on the CPU) is the same float
-      // sequence; that mode has no colours (left 0).
+  for (uint32_t base = blockIdx.x * a.batch; base < a.n_tris_total; base += gridDim.x * a.batch) {
+    // 1
+    const uint32_t g = base + threadIdx.x;
+    int32_t x[3], y[3];
+    float z[3];
+    bool keep = false;
+    if (threadIdx.x < a.batch && g < a.n_tris_total) {
+      const int s = scene_of<ONE, kSceneTable>(a, s_tb, g, false);
+      const RasterSceneDev& S = scene_at<ONE>(a, s);
+      const uint32_t id = g - S.tri_base;
+      float sx[3], sy[3];
+      const bool soa = S.input_kind == kInputSoA;
+      if (soa || S.input_kind == kInputWtriWorld) {
+        // R1, main.cpp:299-308: vtransform, perspective divide, viewport.  World
+        // raster_wtri input: the vertex stage's vtxTransform (rasterMacros.h:14-21,
+        // matmultfloat4 and rcp_approx = 1.0f / w on the CPU) is the same float
+        // sequence; that mode has no colours (left 0).
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        float4 p;
-        if (soa) {
-          p = load_attr3(S.pos, S.pos3, (size_t)k * S.N + id);
-        } else {
-          p.x = __ldg(&S.wtri_xyz[(size_t)id * 9 + 3 * k + 0]);
-          p.y = __ldg(&S.wtri_xyz[(size_t)id * 9 + 3 * k + 1]);
-          p.z = __ldg(&S.wtri_xyz[(size_t)id * 9 + 3 * k + 2]);
-          p.w = 1.0f;
+        for (int k = 0; k < 3; ++k) {
+          float4 p;
+          if (soa) {
+            p = load_attr3(S.pos, S.pos3, (size_t)k * S.N + id);
+          } else {
+            p.x = __ldg(&S.wtri_xyz[(size_t)id * 9 + 3 * k + 0]);
+            p.y = __ldg(&S.wtri_xyz[(size_t)id * 9 + 3 * k + 1]);
+            p.z = __ldg(&S.wtri_xyz[(size_t)id * 9 + 3 * k + 2]);
+            p.w = 1.0f;
+          }
+          const float* m = S.vp;
+          float tx = p.x * m[0] + p.y * m[4] + p.z * m[8] + m[12];
+          float ty = p.x * m[1] + p.y * m[5] + p.z * m[9] + m[13];
+          float tz = p.x * m[2] + p.y * m[6] + p.z * m[10] + m[14];
+          float tw = p.x * m[3] + p.y * m[7] + p.z * m[11] + m[15];
+          float onebyw = 1.0f / tw;
+          sx[k] = (tx * onebyw + 1.0f) * S.halfW;
+          sy[k] = (ty * onebyw + 1.0f) * S.halfH;
+          z[k] = (tz * onebyw);
         }
-        const float* m = S.vp;
-        float tx = p.x * m[0] + p.y * m[4] + p.z * m[8] + m[12];
-        float ty = p.x * m[1] + p.y * m[5] + p.z * m[9] + m[13];
-        float tz = p.x * m[2] + p.y * m[6] + p.z * m[10] + m[14];
-        float tw = p.x * m[3] + p.y * m[7] + p.z * m[11] + m[15];
-        float onebyw = 1.0f / tw;
-        sx[k] = (tx * onebyw + 1.0f) * S.halfW;
-        sy[k] = (ty * onebyw + 1.0f) * S.halfH;
-        sz[k] = (tz * onebyw);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          sx[k] = S.wtri_xyz[(size_t)id * 9 + 3 * k + 0];
+          sy[k] = S.wtri_xyz[(size_t)id * 9 + 3 * k + 1];
+          z[k] = S.wtri_xyz[(size_t)id * 9 + 3 * k + 2];
+        }
       }
-    } else {
+      // R3: 28.4 quantisation by truncation and the three culls
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        sx[k] = S.wtri_xyz[(size_t)id * 9 + 3 * k + 0];
-        sy[k] = S.wtri_xyz[(size_t)id * 9 + 3 * k + 1];
-        sz[k] = S.wtri_xyz[(size_t)id * 9 + 3 * k + 2];
-        ic[k] = S.wtri_icol[(size_t)id * 3 + k];
+        x[k] = cvt_i32_x86(sx[k] * 16.0f);
+        y[k] = cvt_i32_x86(sy[k] * 16.0f);
       }
-    }
-    // R3: 28.4 quantisation by truncation and the three culls
-    TriSetup r;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      r.x[k] = cvt_i32_x86(sx[k] * 16.0f);
-      r.y[k] = cvt_i32_x86(sy[k] * 16.0f);
-      r.z[k] = sz[k];
-      r.c[k] = ic[k];
-    }
-    r.id = id;
-    r.flags = 0;
-    r.rank1 = 0;
-    r.inv = 0.0f;
-    r.bxr = r.byr = 0;
-    r.hix = r.hiy = 0;
-    bool keep = wsub(wmul(wsub(r.y[2], r.y[0]), wsub(r.x[1], r.x[0])),
-                     wmul(wsub(r.x[2], r.x[0]), wsub(r.y[1], r.y[0]))) > 0;
-    const int32_t Wf = cvt_i32_x86((float)S.W * 16.0f), Hf = cvt_i32_x86((float)S.H * 16.0f);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      keep = keep && !(r.x[k] < -kGuard || r.x[k] >= wadd(Wf, kGuard));
-      keep = keep && !(r.y[k] < -kGuard || r.y[k] >= wadd(Hf, kGuard));
-    }
-    const int32_t loy0 = min(min(r.y[0], r.y[1]), r.y[2]);
-    const int32_t hiy0 = max(max(r.y[0], r.y[1]), r.y[2]);
-    keep = keep && !((wsub(loy0, 8) >> 4) == (wsub(hiy0, 8) >> 4));
-    kept_flag = keep;
-    if (keep && soa) {
-      // R1, main.cpp:310-400: per-vertex Gouraud lighting with the normal
-      // normalised by HOST::normalize; no colour array: the reference's fixed
-      // material colour (main.cpp:380)
+      keep = wsub(wmul(wsub(y[2], y[0]), wsub(x[1], x[0])), wmul(wsub(x[2], x[0]), wsub(y[1], y[0]))) > 0;
+      const int32_t Wf = cvt_i32_x86((float)S.W * 16.0f), Hf = cvt_i32_x86((float)S.H * 16.0f);
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        const float4 n4 = load_attr3(S.nrm, S.nrm3, (size_t)k * S.N + id);
-        const float4 c4 = S.col ? __ldg(&S.col[(size_t)k * S.N + id]) : make_float4(0.9f, 0.9f, 0.6f, 1.0f);
+        keep = keep && !(x[k] < -kGuard || x[k] >= wadd(Wf, kGuard));
+        keep = keep && !(y[k] < -kGuard || y[k] >= wadd(Hf, kGuard));
+      }
+      const int32_t loy = min(min(y[0], y[1]), y[2]), hiy = max(max(y[0], y[1]), y[2]);
+      keep = keep && !((wsub(loy, 8) >> 4) == (wsub(hiy, 8) >> 4));
+    }
+    {
+      const unsigned m = __ballot_sync(kFull, keep);
+      if (lane == 0) B.warp[threadIdx.x >> 5] = (uint32_t)__popc(m);
+      __syncthreads();
+      uint32_t at = (uint32_t)__popc(m & ((1u << lane) - 1u));
+#pragma unroll
+      for (int w = 0; w < kSetupWarps; ++w)
+        if (w < (int)(threadIdx.x >> 5)) at += B.warp[w];
+      if (keep) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          B.x[k][at] = x[k];
+          B.y[k][at] = y[k];
+          B.z[k][at] = z[k];
+        }
+        B.g[at] = g;
+      }
+    }
+    uint32_t n = 0;
+#pragma unroll
+    for (int w = 0; w < kSetupWarps; ++w) n += B.warp[w];
+    __syncthreads();
+    // 2.  R1, main.cpp:310-400: per-vertex Gouraud lighting with the normal
+    // normalised by HOST::normalize; no colour array: the reference's fixed
+    // material colour (main.cpp:380)
+    for (uint32_t v = threadIdx.x; v < 3 * n; v += kSetupThreads) {
+      const uint32_t t = v / 3u, k = v - 3u * t, vg = B.g[t];
+      const int s = scene_of<ONE, kSceneTable>(a, s_tb, vg, false);
+      const RasterSceneDev& S = scene_at<ONE>(a, s);
+      const uint32_t id = vg - S.tri_base;
+      uint32_t col = 0u;
+      if (S.input_kind == kInputSoA) {
+        const size_t i = (size_t)k * S.N + id;
+        const float4 n4 = load_attr3(S.nrm, S.nrm3, i);
+        const float4 c4 = S.col ? __ldg(&S.col[i]) : make_float4(0.9f, 0.9f, 0.6f, 1.0f);
         float mag = sqrtf(n4.x * n4.x + n4.y * n4.y + n4.z * n4.z);
-        F3 n = {n4.x / mag, n4.y / mag, n4.z / mag};
+        F3 nn = {n4.x / mag, n4.y / mag, n4.z / mag};
         F3 l;
         if (S.light_mode == 1) {
-          const float4 p = load_attr3(S.pos, S.pos3, (size_t)k * S.N + id);
+          const float4 p = load_attr3(S.pos, S.pos3, i);
           l.x = S.eye[0] - p.x; l.y = S.eye[1] - p.y; l.z = S.eye[2] - p.z;
           float mm = sqrtf(l.x * l.x + l.y * l.y + l.z * l.z);
           if (mm != 0.0f) { float rr = 1.0f / mm; l.x = l.x * rr; l.y = l.y * rr; l.z = l.z * rr; }
         } else {
           l.x = S.light[0]; l.y = S.light[1]; l.z = S.light[2];
         }
-        r.c[k] = light_abgr(n, l, F3{c4.x, c4.y, c4.z});
+        col = light_abgr(nn, l, F3{c4.x, c4.y, c4.z});
+      } else if (S.input_kind == kInputWtri) {
+        col = S.wtri_icol[(size_t)id * 3 + k];
       }
+      B.c[k][t] = col;
     }
-    if (keep) {
+    __syncthreads();
+    // 3
+    uint32_t ntiles = 0;
+    bool risk_flag = false;
+    if (threadIdx.x < n) {
+      const uint32_t t = threadIdx.x, kg = B.g[t];
+      const int s = scene_of<ONE, kSceneTable>(a, s_tb, kg, false);
+      const RasterSceneDev& S = scene_at<ONE>(a, s);
+      TriSetup r;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        r.x[k] = B.x[k][t];
+        r.y[k] = B.y[k][t];
+        r.z[k] = B.z[k][t];
+        r.c[k] = B.c[k][t];
+      }
+      r.id = kg - S.tri_base;
+      r.flags = 0;
       // R4: pixel bounding box rounded to 16 px, reference bin range (8x8)
       const int32_t lox = min(min(r.x[0], r.x[1]), r.x[2]) & (int32_t)0xffffff00;
-      const int32_t loy = loy0 & (int32_t)0xffffff00;
+      const int32_t loy = min(min(r.y[0], r.y[1]), r.y[2]) & (int32_t)0xffffff00;
       const int32_t hix = wadd(max(max(r.x[0], r.x[1]), r.x[2]), 0xff) & (int32_t)0xffffff00;
-      const int32_t hiy = wadd(hiy0, 0xff) & (int32_t)0xffffff00;
+      const int32_t hiy = wadd(max(max(r.y[0], r.y[1]), r.y[2]), 0xff) & (int32_t)0xffffff00;
       const int bits = 4 + kRefBinLg2;
-      int bx1 = max(0, lox >> bits), bx2 = min(hix >> bits, S.nBx - 1);
-      int by1 = max(0, loy >> bits), by2 = min(hiy >> bits, S.nBy - 1);
+      const int bx1 = max(0, lox >> bits), bx2 = min(hix >> bits, S.nBx - 1);
+      const int by1 = max(0, loy >> bits), by2 = min(hiy >> bits, S.nBy - 1);
       r.hix = hix; r.hiy = hiy;
       const int32_t x1mx0 = wsub(r.x[1], r.x[0]), y1my0 = wsub(r.y[1], r.y[0]);
       const int32_t x0mx2 = wsub(r.x[0], r.x[2]), y0my2 = wsub(r.y[0], r.y[2]);
       const int32_t barydenom = wadd(wmul(-y0my2, x1mx0), wmul(x0mx2, y1my0));
       r.inv = 1.0f / (float)barydenom;
+      // 80-byte record as five 16-byte stores, for the triangles that reach a
+      // tile list: only lists (and the winners they give) lead to a record
       if (bx1 <= bx2 && by1 <= by2) {
-        r.rank1 = submission_rank(id, S) + 1u;
+        r.rank1 = submission_rank(r.id, S) + 1u;
         r.bxr = (uint32_t)bx1 | ((uint32_t)bx2 << 16);
         r.byr = (uint32_t)by1 | ((uint32_t)by2 << 16);
         // can any edge value the reference compares wrap inside the bin range?
@@ -544,70 +733,72 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(const __grid_const
                                (long long)(r.x[2] - r.x[0]) * (r.y[1] - r.y[0]);
         if (area >= 2147483647LL) r.flags |= kTriAreaRisk;
         risk_flag = (r.flags & kTriRisk) != 0;
-      }
-    }
-    // 80-byte record as five 16-byte stores, for the triangles that reach a
-    // bin: only tile lists (and the winners they give) lead to a record
-    if (r.rank1) {
-      const uint4* src = reinterpret_cast<const uint4*>(&r);
-      uint4* dst = reinterpret_cast<uint4*>(&a.setup[g]);
+        fill_walk(a, S, r, kg, B.walk[t], ntiles);
+        if (B.walk[t].lty != 1u) {
+          const uint4* src = reinterpret_cast<const uint4*>(&r);
+          uint4* dst = reinterpret_cast<uint4*>(&a.setup[kg]);
 #pragma unroll
-      for (int k = 0; k < 5; ++k) dst[k] = src[k];
-      fill_walk(a, S, r, g, s_walk[threadIdx.x], ntiles);
-    }
-  }
-  // Triangles with many tiles in their box go to raster_large, which walks
-  // their box tiles in segments of kLargeSeg: one atomic per warp reserves
-  // the warp's segment items.
-  const bool is_big = ntiles > kLargeTiles;
-  const unsigned big = __ballot_sync(kFull, is_big);
-  if (big) {
-    const uint32_t nseg = is_big ? (ntiles + kLargeSeg - 1) / kLargeSeg : 0u;
-    uint32_t incl = nseg;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(kFull, incl, o);
-      if (lane >= o) incl += t;
-    }
-    unsigned long long old = 0;
-    if (lane == 31) old = atomicAdd(&a.work->bin.large_acc, ((unsigned long long)__popc(big) << 32) | incl);
-    old = __shfl_sync(kFull, old, 31);
-    if (is_big) {
-      // the triangle's walk record, then one (large triangle, segment) item
-      // per segment; records or items past the capacities are reported (the
-      // host grows the buffers and draws the frame again)
-      const uint32_t bi = (uint32_t)(old >> 32) + (uint32_t)__popc(big & ((1u << lane) - 1u));
-      const uint32_t first = (uint32_t)old + incl - nseg;
-      if (bi < a.big_cap) {
-        a.large_walk[bi] = s_walk[threadIdx.x];
-        for (uint32_t k = 0; k < nseg; ++k) {
-          if (first + k < a.seg_cap) a.large_seg[first + k] = make_uint2(bi, k);
-          else { atomicOr(&a.work->bin.status, kStatusListOverflow); break; }
+          for (int k = 0; k < 5; ++k) dst[k] = src[k];
         }
-      } else {
-        atomicOr(&a.work->bin.status, kStatusListOverflow);
       }
-      ntiles = 0;
     }
-  }
-  nk += __popc(__ballot_sync(kFull, kept_flag));
-  nr += __popc(__ballot_sync(kFull, risk_flag));
-  __syncwarp();
-  walk_tiles(a, &s_walk[threadIdx.x & ~31], ntiles);
-  __syncwarp();  // the warp's s_walk entries are rewritten by the next block
+    // Triangles with many tiles in their box go to raster_large_count, which
+    // walks their box tiles in segments of kLargeSeg: one atomic per warp
+    // reserves the warp's segment items.
+    const bool is_big = ntiles > kLargeTiles;
+    const unsigned big = __ballot_sync(kFull, is_big);
+    if (big) {
+      const uint32_t nseg = is_big ? (ntiles + kLargeSeg - 1) / kLargeSeg : 0u;
+      uint32_t incl = nseg;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+      }
+      unsigned long long old = 0;
+      if (lane == 31) old = atomicAdd(&a.work->bin.large_acc, ((unsigned long long)__popc(big) << 32) | incl);
+      old = __shfl_sync(kFull, old, 31);
+      if (is_big) {
+        // the triangle's walk record, then one (large triangle, segment) item
+        // per segment; records or items past the capacities are reported (the
+        // host grows the buffers and draws the frame again)
+        const uint32_t bi = (uint32_t)(old >> 32) + (uint32_t)__popc(big & ((1u << lane) - 1u));
+        const uint32_t first = (uint32_t)old + incl - nseg;
+        if (bi < a.big_cap) {
+          a.large_walk[bi] = B.walk[threadIdx.x];
+          for (uint32_t k = 0; k < nseg; ++k) {
+            if (first + k < a.seg_cap) a.large_seg[first + k] = make_uint2(bi, k);
+            else { atomicOr(&a.work->bin.status, kStatusListOverflow); break; }
+          }
+        } else {
+          atomicOr(&a.work->bin.status, kStatusListOverflow);
+        }
+        ntiles = 0;
+      }
+    }
+    const unsigned risks = (unsigned)__popc(__ballot_sync(kFull, risk_flag));
+    if (lane == 0 && risks) atomicAdd(&B.nr, risks);
+    if (threadIdx.x == 0) B.nk += n;
+    uint32_t items = 0;
+    if (ntiles) {
+      const uint32_t tw = (uint32_t)B.walk[threadIdx.x].tw;
+      items = (ntiles / tw) * ((tw + 31u) >> 5);
+    }
+    // (the scan's barrier lies between the last read of x .. g and this write)
+    const uint32_t incl = block_scan_incl(items, B.warp);
+    B.pre[threadIdx.x] = incl;
+    for (uint32_t i = incl - items; i < min(incl, kItemMap); ++i) B.item_tri[i] = (uint8_t)threadIdx.x;
+    __syncthreads();
+    // 4
+    const uint32_t skipped = walk_tiles(a, B.walk, B.pre, B.item_tri, (int)n, B.queue[threadIdx.x >> 5]);
+    if (lane == 0 && skipped) atomicAdd(&B.skipped, skipped);
+    __syncthreads();  // the shared arrays are rewritten by the next batch
   }
   // frame counters: one atomic per CTA
-  if (lane == 0) {
-    s_kept[threadIdx.x >> 5] = nk;
-    s_risk[threadIdx.x >> 5] = nr;
-  }
-  __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned k = 0, rr = 0;
-#pragma unroll
-    for (int w = 0; w < kSetupThreads / 32; ++w) { k += s_kept[w]; rr += s_risk[w]; }
-    if (k) atomicAdd(&a.work->bin.kept, k);
-    if (rr) atomicAdd(&a.work->bin.risk, (unsigned long long)rr);
+    if (B.nk) atomicAdd(&a.work->bin.kept, B.nk);
+    if (B.nr) atomicAdd(&a.work->bin.risk, (unsigned long long)B.nr);
+    if (B.skipped) atomicAdd(&a.work->bin.skipped, (unsigned long long)B.skipped);
   }
 }
 
@@ -770,36 +961,40 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
 }
 
 // ------------------------------------------------------------------ kernel 3
-// Large triangles (more than kLargeTiles tiles in their box): their box tiles
-// are cut into segments of kLargeSeg, and a warp takes one segment at a time,
-// its lanes striding over the segment's tiles (four per lane in flight), so a
-// huge triangle spreads over many warps.  The pairs are counted and recorded
-// like the small triangles' (count_pairs).
-__device__ __forceinline__ void large_segment(const RasterFrameArgs& a, uint32_t it, int lane)
+// Large triangles (more than kLargeTiles tiles in their box): their box tiles,
+// numbered row by row, are cut into segments of kLargeSeg, and a warp takes one
+// segment at a time, a run of consecutive tiles per lane, so a huge triangle
+// spreads over many warps.  The tiles are counted and recorded like the small
+// triangles'; returns the lane's number of tiles that pass and are not listed.
+__device__ __forceinline__ uint32_t large_segment(const RasterFrameArgs& a, uint32_t it, uint16_t* queue, int lane)
 {
+  constexpr uint32_t kLaneRun = kLargeSeg / 32;
   const uint2 sg = a.large_seg[it];
-  const uint32_t j0 = sg.y * kLargeSeg;
-  const WalkTri w = a.large_walk[sg.x];
-  const uint32_t g = w.gidx;
+  const WalkTri& w = a.large_walk[sg.x];
+  const uint32_t j0 = sg.y * kLargeSeg, tw = (uint32_t)w.tw;
   const int tsh = __ffs(a.tile) - 1 - kRefBinLg2;   // tile edge = 8 << tsh
-  const uint32_t ntiles = (uint32_t)w.tw * (uint32_t)((w.by2 >> tsh) - w.ty1 + 1);
-  const uint32_t j1 = min(j0 + kLargeSeg, ntiles);
-  for (uint32_t jb0 = j0; jb0 < j1; jb0 += 4 * 32) {   // warp-uniform trips
-    uint32_t key[4], gidx[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t j = jb0 + (uint32_t)lane + (uint32_t)q * 32u;
-      key[q] = 0xffffffffu;
-      gidx[q] = g;
-      if (j < j1) {
-        uint32_t lx;
-        const uint32_t ly = fast_divmod(j, (uint32_t)w.tw, w.tw_m, lx);
-        const int tx = w.tx1 + (int)lx, ty = w.ty1 + (int)ly;
-        if (tile_may_cover(w, tx, ty, a.tile)) key[q] = w.tile_base + (uint32_t)(ty * w.tiles_x + tx);
-      }
-    }
-    count_pairs<4>(a, key, gidx, lane);
+  const uint32_t ntiles = tw * (uint32_t)((w.by2 >> tsh) - w.ty1 + 1);
+  uint32_t m = 0, skipped = 0;
+  for (uint32_t k = 0; k < kLaneRun;) {   // the parts of the run that lie in one row
+    const uint32_t j = j0 + (uint32_t)lane * kLaneRun + k;
+    if (j >= ntiles) break;
+    uint32_t col;
+    const uint32_t row = fast_divmod(j, tw, w.tw_m, col);
+    const uint32_t n = min(kLaneRun - k, tw - col);
+    const uint32_t pass = row_mask(w, row, col, n, a.tile), list = pass & listed_mask(w, row, col, n);
+    skipped += (uint32_t)(__popc(pass) - __popc(list));
+    m |= list << k;
+    k += n;
   }
+  const auto key_of = [&](uint32_t e, uint32_t& gidx) {
+    gidx = w.gidx;
+    return tile_key(w, j0 + e);
+  };
+  uint32_t qn = 0;
+  __syncwarp();
+  queue_masks(a, queue, qn, m, 0u, (uint32_t)lane * kLaneRun, lane, key_of);
+  if (qn) record_queue(a, queue, 0u, qn, lane, key_of);
+  return skipped;
 }
 
 // The count pass of the large triangles' segments.
@@ -807,10 +1002,14 @@ __global__ void __launch_bounds__(256, 4) raster_large_count(const __grid_consta
 {
   pdl_wait();
   pdl_trigger();
+  __shared__ uint16_t s_queue[8][kWalkQueue];
   const uint32_t items = min((uint32_t)a.work->bin.large_acc, a.seg_cap);
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const int lane = threadIdx.x & 31;
+  unsigned long long skipped = 0;
   for (uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items; it += warps)
-    large_segment(a, it, threadIdx.x & 31);
+    skipped += __reduce_add_sync(kFull, large_segment(a, it, s_queue[threadIdx.x >> 5], lane));
+  if (lane == 0 && skipped) atomicAdd(&a.work->bin.skipped, skipped);
 }
 
 // The scatter pass (the compaction): every recorded pair becomes its list
@@ -1690,14 +1889,14 @@ int raster_scan_blocks(uint32_t n_tiles) { return (int)((n_tiles + kScanTile - 1
 // frames concurrently: the cache is an atomic, and two threads that both miss
 // it compute and store the same value.
 template <class K>
-static int wave_ctas(K kernel, std::atomic<int>* cache, int threads = 256)
+static int wave_ctas(K kernel, std::atomic<int>* cache, int threads = 256, size_t smem = 0)
 {
   int v = cache->load(std::memory_order_relaxed);
   if (v <= 0) {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
     v = sms * (per_sm > 0 ? per_sm : 1);
     cache->store(v, std::memory_order_relaxed);
   }
@@ -1742,14 +1941,21 @@ static cudaError_t bins_setup()
   return e;
 }
 
-cudaError_t launch_raster_frame(const RasterFrameArgs& a, int raster_ctas, cudaStream_t st, cudaEvent_t* ev)
+cudaError_t launch_raster_frame(const RasterFrameArgs& args, int raster_ctas, cudaStream_t st, cudaEvent_t* ev)
 {
+  RasterFrameArgs a = args;
   static std::atomic<int> setup_wave[2] = {{0}, {0}}, scatter_wave{0}, large_wave{0};
   const bool one = a.n_scenes == 1;
-  const int tri_blocks = (int)((a.n_tris_total + 255) / 256);
+  const bool tri_blocks = a.n_tris_total > 0;
   const auto setup = one ? raster_setup<true> : raster_setup<false>;
-  const int setup_blocks = min((int)((a.n_tris_total + kSetupThreads - 1) / kSetupThreads),
-                               wave_ctas(setup, &setup_wave[one], kSetupThreads));
+  const size_t setup_smem = sizeof(SetupSmem) + (one ? 0 : kSceneTable * sizeof(uint32_t));
+  // One wave of CTAs; every CTA takes the same number of equal batches, and a
+  // small scene is spread over the whole device, at least 8 triangles a batch.
+  const uint32_t wave = (uint32_t)wave_ctas(setup, &setup_wave[one], kSetupThreads, setup_smem);
+  const uint32_t rounds = (a.n_tris_total + wave * kSetupThreads - 1) / (wave * kSetupThreads);
+  a.batch = (a.n_tris_total + wave * rounds - 1) / std::max(wave * rounds, 1u);
+  a.batch = a.batch > 32 ? (a.batch + 31) & ~31u : std::max(a.batch, 8u);
+  const int setup_blocks = (int)std::min(wave, (a.n_tris_total + a.batch - 1) / a.batch);
   // the scatter grid covers the list groups of every triangle plus the large
   // triangles' segments (a grid-stride loop takes any excess)
   const int scatter_blocks = std::max(1, wave_ctas(raster_scatter, &scatter_wave) / (int)kPairParts) * (int)kPairParts;
@@ -1758,7 +1964,7 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& a, int raster_ctas, cudaS
   // every launch after the first may start while its predecessor drains
   // (programmatic dependent launch); each waits for it before touching memory
   cudaError_t e = cudaSuccess;
-  if (tri_blocks) setup<<<setup_blocks, kSetupThreads, 0, st>>>(a);
+  if (tri_blocks) setup<<<setup_blocks, kSetupThreads, setup_smem, st>>>(a);
   if (tri_blocks && !e) e = launch_pdl(raster_large_count, large_blocks, 256, st, a);
   if (ev) cudaEventRecord(ev[1], st);
   if (!e) e = launch_pdl(scan_tiles, raster_scan_blocks(a.n_tiles_total), kScanThreads, st, a);

@@ -556,7 +556,7 @@ static void fill_stats(const RasterScratch& scr, bool timed, piko_frame_stats* o
 {
   const FrameCounters& c = *scr.h_ctr;
   o->prims_kept += c.bin.kept;
-  o->bin_entries += c.bin.list_total;
+  o->bin_entries += c.bin.list_total + c.bin.skipped;
   o->covered += c.covered;
   o->wrap_risk += c.bin.risk;
   o->status |= c.bin.status;

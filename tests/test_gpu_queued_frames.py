@@ -34,6 +34,10 @@ def test_queued_frames_keep_their_camera(pk, ctx, oracle_mod, tile):
     pipe = pk.Pipe(ctx, "raster", tile_px=tile)
     s = pk.Scene(pipe, sc)
     try:
+        for st in states:   # the queues settle: a frame that overflows is drawn again with the latest camera
+            s.prepare(pk.const_state(st))
+            s.run()
+            s.finish()
         for last in range(4):
             for k in list(range(4)) * 25 + [last]:   # nothing waits between these
                 s.prepare(pk.const_state(states[k]))
@@ -54,6 +58,11 @@ def test_queued_batches_keep_their_cameras(pk, ctx, oracle_mod):
     scenes = [pk.Scene(pipe, sc) for sc in scs]
     batch = pk.Batch(ctx, scenes)
     try:
+        for k in range(3):   # the queues settle
+            for s, st in zip(scenes, states):
+                s.prepare(pk.const_state(st[k]))
+            batch.run(graph=False)
+            batch.finish()
         for last in range(3):
             for k in list(range(3)) * 20 + [last]:
                 for s, st in zip(scenes, states):
