@@ -218,8 +218,8 @@ typedef struct piko_frame_stats {
   uint32_t split_levels;    /* Reyes split levels run */
   int n_kernels;            /* entries of kernel_ms in use (time_kernels only) */
   float kernel_ms[8];       /* per-phase time of the last frame: raster [setup, scan,
-                               scatter, tiles]; Reyes [split, dice + depth pass, key pass,
-                               resolve pass] */
+                               scatter, tiles]; Reyes [split, dice + fragments, tie pass,
+                               pixel pass] */
 } piko_frame_stats;
 
 /* Finishes the last frame and returns its counters. */

@@ -6,9 +6,9 @@
 //       patch: project the 16 control points, measure the u/v screen extents,
 //       split at the halves (de Casteljau) or emit a leaf with its dice grid
 //       (R11, split.pikostage:240-343).  Each CTA expands its patches level
-//       after level in shared memory; children past what a CTA keeps go to a
-//       global frontier that the next step spreads over all CTAs, after a grid
-//       barrier; leaves are staged and written out in batches.  No host round
+//       after level in shared memory, with a stack of its own behind it; a
+//       global frontier evens the CTAs out after a grid barrier; leaves are
+//       staged and written out in batches.  No host round
 //       trip between levels (the reference copies the Split stage back to the
 //       host every level).
 //   reyes_dice     every CTA an equal range of dice rows; per group of rows,
@@ -17,14 +17,16 @@
 //       "Phong" colour and the mean depth (R12, dice.pikostage:159-312; R13
 //       colour, shade.pikostage:64-109), the 64-pixel Shade-bin range of three
 //       corners (shade.pikostage:51-56) cut with the four-corner bounds to one
-//       pixel rectangle, then a sample-parallel coverage pass and the first
-//       fragment pass (depth minimum) over that rectangle.
-//   reyes_big      the first fragment pass for micropolygons with more than
-//       kSmallPx candidate pixels, a warp each.
-//   reyes_keys, reyes_resolve  the other two fragment passes over the fragment
-//       list; reyes_pixels writes the pixels no fragment reached (averages a
-//       pixel's samples with 4 samples per pixel) and sets the per-sample
-//       state of the reached samples back to empty for the next frame.
+//       pixel rectangle, then a sample-parallel coverage pass over that
+//       rectangle; every covered sample is a 64-bit atomic minimum on the
+//       sample's state (depth, micropolygon).
+//   reyes_big      the same for micropolygons with more than kSmallPx candidate
+//       pixels, a warp each.
+//   reyes_ties     the samples at which two fragments met at one depth: the
+//       reference's order decides between them.
+//   reyes_pixels   writes every pixel from its samples' states (averages them
+//       with 4 samples per pixel) and sets the reached ones back to empty for
+//       the next frame.
 //       Shade work is spread per micropolygon and per fragment, not per
 //       screen tile, so silhouette tiles where thousands of micropolygons pile
 //       up cost no more than anywhere else.  The per-sample test is the
@@ -82,12 +84,12 @@ struct ReyesCounters {
   uint32_t levels_run;
   uint32_t negative_depth;
   uint32_t big_count;             // micropolygons queued for reyes_big
-  uint32_t frag_count;            // fragments appended by pass 1
+  uint32_t id_count;              // micropolygons with a covered sample
+  uint32_t tie_count;
+  uint32_t pad[1];
   unsigned long long bar_arrive;  // grid barrier of reyes_split: (arrivals << 40) | children
   unsigned long long bar_release; // (barriers passed << 32) | next level's patch count
 };
-
-struct FragRec;
 
 struct ReyesArgs {
   int W, H, nBx, nBy, nDice;
@@ -98,28 +100,28 @@ struct ReyesArgs {
   const float4* in_patches;
   PatchRec* lvl[2];
   uint32_t lvl_cap;
+  PatchRec* stack;                // [CTAs of the split][kSplitStack]
   PatchRec* leaves;
   uint32_t leaf_cap;
   UpolyRec* up;                   // micropolygons with more than kSmallPx candidate pixels
   uint32_t up_cap;
-  FragRec* frags;                 // covered samples with depth <= 1 (pass 1 output)
-  uint32_t frag_cap;
+  uint32_t* id_color;             // per micropolygon with a covered sample: colour (alpha: id_colour())
+  unsigned long long* id_key;     // and processing-order key + 1
+  uint32_t id_cap;
+  uint4* ties;                    // (sample, depth code, micropolygon, the one it met)
+  uint32_t tie_cap;
   ReyesCounters* ctr;
   uint32_t* fb;
   float* depth;
-  uint32_t* zmin;                 // per sample: order-mapped minimum depth
-  unsigned long long* kfirst;     // per sample: least key among fragments at the minimum
-  unsigned long long* klast;      // per sample: greatest key among fragments at the minimum
+  unsigned long long* samp;       // per sample: depth code << 32 | micropolygon of the least fragment so far
+  uint32_t* first0;               // per sample: the first micropolygon at a depth of +-0 (kNoId: none)
   // Multi-sample / Phong variant (no reference counterpart).  spp samples per
   // pixel (1: the reference's pixel centre; 4: one jittered sample per pixel
   // quadrant, seeded); phong = 1 lights the micropolygon's interpolated normal.
-  // With spp > 1 the resolve writes samples (scol, sdep) and reyes_pixels
-  // averages them into the pixel.
+  // With spp > 1 reyes_pixels averages the samples into the pixel.
   int spp;
   uint32_t seed;
   int phong;
-  uint32_t* scol;                 // per sample colour (spp > 1)
-  float* sdep;                    // per sample depth (spp > 1)
 };
 
 // Micropolygons whose shaded rectangle holds more pixels than this are shaded
@@ -138,10 +140,11 @@ __device__ __forceinline__ float zorder_inv(uint32_t o)
 {
   return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
 }
-// The cleared per-sample minimum: above zorder(z) of every depth z <= 1 (the
-// only fragments kept), so a sample's minimum stays kZminEmpty exactly when no
-// fragment reached it.
-constexpr uint32_t kZminEmpty = 0xffffffffu;
+// The cleared sample state: above the state of every fragment of depth z <= 1
+// (the only ones kept), so a sample stays empty exactly when no fragment
+// reached it.
+constexpr unsigned long long kSampEmpty = ~0ull;
+constexpr uint32_t kNoId = 0xffffffffu;
 
 // Sample s of pixel (x, y): the centre for one sample per pixel; otherwise
 // quadrant (s & 1, s >> 1) of the pixel at a jitter from an integer hash of
@@ -280,10 +283,9 @@ __device__ __forceinline__ uint32_t barrier_wait(ReyesCounters* c, uint32_t k, u
   return *s_count;
 }
 
-// The per-sample state (depth minimum, key bounds) starts every frame empty:
-// the buffers are set so when allocated, and reyes_pixels, which visits every
-// sample after the fragment passes, sets a reached sample back.  The split
-// clears nothing.
+// The per-sample state starts every frame empty: the buffers are set so when
+// allocated, and reyes_pixels, which visits every sample last, sets a reached
+// sample back.  The split clears nothing.
 
 // One patch of one split level (R11, split.pikostage:240-343), sixteen lanes
 // per patch: lane c holds control point c; the u and v polyline lengths are
@@ -346,25 +348,31 @@ __device__ __forceinline__ SplitDecision split_measure(const ReyesArgs& a, int L
 }
 
 // The split runs as one cooperative launch of kSplitThreads-thread CTAs, one
-// per SM, sixteen lanes per patch (a 16-lane group takes two patches of a
-// level), so a CTA works on up to kSplitKeep patches per level.  A CTA expands
-// its patches level after level in shared memory: the children of a level
-// stay in the CTA (up to kSplitKeep of them; the rest go to a global frontier
-// for the next step, spread evenly over the CTAs), and leaves are staged and
-// written out in batches.  A step ends with a grid barrier; the split ends at
-// the first step whose frontier is empty.  Patches of a step's frontier are at
-// least at level `step`, so there are at most max_splits + 1 steps.  Nothing
+// per SM, sixteen lanes per patch.  A CTA expands its patches level after level:
+// up to kSplitKeep children of a level stay in shared memory, further ones go to
+// a stack of the CTA's own in global memory (and, once that holds kSplitStack, to
+// the frontier), and leaves are staged and written out in batches.  A step ends
+// with a grid barrier, after which the patches on the global frontier are dealt
+// out to the CTAs, one each in turn, so that neighbours -- subtrees of similar
+// size -- go to different CTAs; the split ends at the first step whose frontier
+// is empty.  In the first step a CTA puts all patches of a level that has at
+// least kSplitShare of them on the frontier: with few input patches the CTAs'
+// subtrees differ in size, and dealt out at that width they even out (a split
+// that put every patch past 64 per level on the frontier took 89 us of the
+// default-constants sphere's 14 levels, in four steps; this takes SPLIT us).  Nothing
 // depends on which CTA or pass handles a patch: every leaf carries its input
 // index, level and in-level position (children of s are 2s and 2s + 1), which
 // give the order key.
 constexpr int kSplitThreads = 512;
-constexpr int kSplitKeep = 2 * (kSplitThreads / 16);   // patches a CTA keeps per level (two per 16-lane group)
-constexpr int kSplitStage = 128;
+constexpr int kSplitKeep = 128;         // patches a CTA takes per level
+constexpr int kSplitStage = 192;
+constexpr uint32_t kSplitStack = 1024;  // patches of a CTA's own stack
+constexpr uint32_t kSplitShare = 96;
 struct SplitSmem {
   PatchRec buf[2][2 * kSplitKeep];    // current level, children of the current level
   PatchRec stage[kSplitStage];        // leaves not yet written out
   uint32_t nnext, nleaf, ncur, maxlevel;
-  uint32_t children;                  // patches this CTA pushed to the frontier in this step
+  uint32_t children;                  // patches this CTA put on the frontier in this step
   uint32_t word[4];
 };
 constexpr size_t kSplitSmem = sizeof(SplitSmem);
@@ -378,22 +386,28 @@ __device__ __forceinline__ void copy_patches(PatchRec* dst, const PatchRec* src,
   for (uint32_t i = threadIdx.x; i < n * kQ; i += blockDim.x) d4[i] = from_l2 ? __ldcg(&s4[i]) : s4[i];
 }
 
-// Input patch i of a step: an input patch at level 0 (i0 = s = i) or a record
-// of the global frontier.
-__device__ __forceinline__ void load_inputs(const ReyesArgs& a, int step, uint32_t first, uint32_t n, PatchRec* dst)
+// Input patches first, first + stride, ... (n of them) of a step: input patches
+// at level 0 (i0 = s = i) or records of the global frontier.
+__device__ __forceinline__ void load_inputs(const ReyesArgs& a, int step, uint32_t first, uint32_t stride, uint32_t n,
+                                            PatchRec* dst)
 {
   if (step == 0) {
     for (uint32_t q = threadIdx.x; q < n * 16u; q += blockDim.x) {
-      const uint32_t i = q >> 4, c = q & 15u;
-      dst[i].cp[c] = __ldcg(&a.in_patches[(size_t)(first + i) * 16 + c]);
+      const uint32_t i = q >> 4, c = q & 15u, in = first + i * stride;
+      dst[i].cp[c] = __ldcg(&a.in_patches[(size_t)in * 16 + c]);
       if (c == 0) {
-        dst[i].i0 = first + i;
+        dst[i].i0 = in;
         dst[i].level = 0;
-        dst[i].s = first + i;
+        dst[i].s = in;
       }
     }
   } else {
-    copy_patches(dst, a.lvl[step & 1] + first, n, true);
+    constexpr uint32_t kQ = sizeof(PatchRec) / 16;
+    float4* d4 = reinterpret_cast<float4*>(dst);
+    for (uint32_t q = threadIdx.x; q < n * kQ; q += blockDim.x) {
+      const uint32_t i = q / kQ, c = q - i * kQ;
+      d4[q] = __ldcg(reinterpret_cast<const float4*>(a.lvl[step & 1] + (first + i * stride)) + c);
+    }
   }
 }
 
@@ -508,40 +522,42 @@ __global__ void __launch_bounds__(kSplitThreads, 1) reyes_split(ReyesArgs a)
   }
   uint32_t n_in = (uint32_t)a.P;
   for (int step = 0; n_in > 0; ++step) {   // n_in is uniform
-    // This CTA's share of the step's frontier.  With fewer patches than
-    // CTAs, 2^d CTAs share a patch: each takes the patch's descendants along
-    // its own d-bit path (the first d levels of the patch are computed by
-    // all of them), so every CTA has a subtree; a leaf met on the way is
-    // emitted by the group's CTA whose remaining path bits are all 0.
+    // This CTA's share of the step's frontier: patches blockIdx.x, blockIdx.x +
+    // gridDim.x, ...  With fewer patches than CTAs, 2^d CTAs share a patch:
+    // each takes the patch's descendants along its own d-bit path (the first d
+    // levels of the patch are computed by all of them), so every CTA has a
+    // subtree; a leaf met on the way is emitted by the group's CTA whose
+    // remaining path bits are all 0.
     uint32_t d = 0;
     while (d < 16 && ((unsigned long long)n_in << (d + 1)) <= gridDim.x) ++d;
-    uint32_t r0, r1, path = 0, dr = 0;
-    if (d > 0) {
-      const uint32_t owner = blockIdx.x >> d;
-      r0 = min(owner, n_in);
-      r1 = min(owner + 1, n_in);
-      path = blockIdx.x & ((1u << d) - 1u);
-      dr = d;
-    } else {
-      r0 = (uint32_t)((unsigned long long)n_in * blockIdx.x / gridDim.x);
-      r1 = (uint32_t)((unsigned long long)n_in * (blockIdx.x + 1) / gridDim.x);
-    }
+    const uint32_t path = blockIdx.x & ((1u << d) - 1u), owner = blockIdx.x >> d;
+    const uint32_t share = d > 0 ? (owner < n_in ? 1u : 0u)
+                                 : (blockIdx.x < n_in ? (n_in - blockIdx.x - 1) / gridDim.x + 1 : 0u);
+    uint32_t dr = d;
+    const bool deal = step == 0 && n_in < 8u * gridDim.x;   // too few patches to even out
     PatchRec* frontier = a.lvl[(step + 1) & 1];
-    uint32_t pos = r0, ncur = 0;
+    PatchRec* stack = a.stack + (size_t)blockIdx.x * kSplitStack;
+    uint32_t taken = 0, ncur = 0, top = 0;
     int cb = 0;   // buf[cb] holds the current patches
     __syncthreads();
-    while (ncur > 0 || pos < r1) {   // uniform
-      // top up the current patches from the share
-      const uint32_t take = min((uint32_t)kSplitKeep - ncur, r1 - pos);
-      if (take) load_inputs(a, step, pos, take, &S.buf[cb][ncur]);
-      pos += take;
-      ncur += take;
+    while (ncur > 0 || top > 0 || taken < share) {   // uniform
+      // top up the current patches from the stack, then from the share
+      if (const uint32_t pop = min((uint32_t)kSplitKeep - ncur, top)) {
+        top -= pop;
+        copy_patches(&S.buf[cb][ncur], stack + top, pop, true);
+        ncur += pop;
+      }
+      if (const uint32_t take = min((uint32_t)kSplitKeep - ncur, share - taken)) {
+        load_inputs(a, step, d > 0 ? owner : blockIdx.x + taken * gridDim.x, gridDim.x, take, &S.buf[cb][ncur]);
+        taken += take;
+        ncur += take;
+      }
       if (S.nleaf + (uint32_t)kSplitKeep > (uint32_t)kSplitStage) flush_leaves(a, S);
       if (threadIdx.x == 0) S.nnext = 0;
       __syncthreads();
       split_pass(a, S, S.buf[cb], S.buf[cb ^ 1], ncur);
       __syncthreads();
-      uint32_t nn = S.nnext;
+      uint32_t nn = S.nnext, keep = min(nn, (uint32_t)kSplitKeep);
       if (dr > 0) {
         // one patch on the CTA's path (ncur == 1): keep the child the path
         // names, or drop a leaf that another CTA of the group emits
@@ -553,25 +569,33 @@ __global__ void __launch_bounds__(kSplitThreads, 1) reyes_split(ReyesArgs a)
             const float4* src = reinterpret_cast<const float4*>(&S.buf[cb ^ 1][1]);
             if (threadIdx.x < sizeof(PatchRec) / 16) dst[threadIdx.x] = src[threadIdx.x];
           }
-          nn = 1;
+          keep = 1;
         }
         --dr;
-      } else if (nn > (uint32_t)kSplitKeep) {
-        // children past kSplitKeep go to the frontier of the next step
-        const uint32_t extra = nn - (uint32_t)kSplitKeep;
-        if (threadIdx.x == 0) {
-          S.word[3] = atomicAdd(&a.ctr->level_count[min(step + 1, 39)], extra);
-          S.children += extra;
+      } else {
+        if (deal && nn >= kSplitShare) keep = 0;   // the whole level to the frontier
+        uint32_t own = nn - keep;                  // children for the CTA's stack
+        if (deal && nn >= kSplitShare) own = 0;
+        own = min(own, kSplitStack - top);
+        if (own) {
+          copy_patches(stack + top, &S.buf[cb ^ 1][keep], own, false);
+          top += own;
         }
-        __syncthreads();
-        const uint32_t at = S.word[3];
-        if (at + extra <= a.lvl_cap) {
-          copy_patches(frontier + at, &S.buf[cb ^ 1][kSplitKeep], extra, false);
-        } else if (threadIdx.x == 0) {
-          atomicOr(&a.ctr->fc.status, kStatusPatchOverflow);
+        if (const uint32_t extra = nn - keep - own) {
+          if (threadIdx.x == 0) {
+            S.word[3] = atomicAdd(&a.ctr->level_count[min(step + 1, 39)], extra);
+            S.children += extra;
+          }
+          __syncthreads();
+          const uint32_t at = S.word[3];
+          if (at + extra <= a.lvl_cap) {
+            copy_patches(frontier + at, &S.buf[cb ^ 1][keep + own], extra, false);
+          } else if (threadIdx.x == 0) {
+            atomicOr(&a.ctr->fc.status, kStatusPatchOverflow);
+          }
         }
       }
-      ncur = min(nn, (uint32_t)kSplitKeep);
+      ncur = keep;
       cb ^= 1;
       __syncthreads();
     }
@@ -705,27 +729,27 @@ __device__ __forceinline__ bool exact_box(float mnx, float mxx, float mny, float
 
 // The depth resolve.  The CPU shades micropolygons in its processing order with
 //   while (remote > z) remote = atomicMin(bits, z);  pass iff zbuf == z
-// so, per pixel, the surviving depth is the minimum m (the cleared 1.0
+// so, per sample, the surviving depth is the minimum m (the cleared 1.0
 // included), its bits come from the FIRST fragment with depth m and the colour
-// from the LAST one.  Every fragment carries its micropolygon's order key;
-//   pass 1 (dice, reyes_big)  zmin <- min zorder(z); fragments with z <= 1
-//                             are appended to a fragment list
-//   pass 2 (reyes_keys)       klast <- max key of the fragments at m; where
-//                             m is +-0, kfirst <- their min key (64-bit
-//                             atomics): only there can the bits differ
-//   pass 3 (reyes_resolve)    the fragment whose key is klast writes the
-//                             colour and, unless m is +-0, the depth; at +-0
-//                             the one whose key is kfirst writes the depth.
-// A pixel nothing reaches keeps the cleared colour and depth; a fragment at
-// exactly 1.0 takes the colour but leaves the (identical) cleared depth bits.
-struct __align__(16) FragRec {
-  unsigned long long key;
-  uint32_t pix;
-  float z;
-  uint32_t color;
-  uint32_t pad[3];
-};
-static_assert(sizeof(FragRec) == 32, "FragRec layout");
+// from the LAST one.  A micropolygon with a covered sample of depth z <= 1 gets
+// a number (id), under which its colour and order key are kept, and each such
+// sample is one atomicMin of zorder(z) << 32 | id on the sample's state: the
+// least depth wins.  Two fragments of one depth at a sample see each other --
+// the later atomic finds the earlier one's depth -- and leave a tie record;
+// reyes_ties then gives the sample to the micropolygon with the greatest key of
+// all that met there.  Only at depth +-0 can fragments of one depth differ in
+// their bits: there every fragment leaves a record, and the one with the least
+// key is kept in first0.
+// (A list of all fragments, 32 bytes each, read again by a pass that took the
+// greatest key at each sample's minimum and by one that wrote colour and depth,
+// cost 35 us of the 4-sample 1280x720 sphere's 157.)
+
+// A micropolygon's colour with the sign of a zero depth in the alpha's low bit
+// (set for everything but -0; a colour's alpha is 255).
+__device__ __forceinline__ uint32_t id_colour(const UpolyRec& u)
+{
+  return u.color ^ (__float_as_uint(u.z) == 0x80000000u ? 0x01000000u : 0u);
+}
 
 __device__ __forceinline__ void add_covered(const ReyesArgs& a, unsigned covered)
 {
@@ -733,29 +757,63 @@ __device__ __forceinline__ void add_covered(const ReyesArgs& a, unsigned covered
   if ((threadIdx.x & 31) == 0 && covered) atomicAdd(&a.ctr->fc.covered, (unsigned long long)covered);
 }
 
-__device__ __forceinline__ void emit_fragment(const ReyesArgs& a, uint32_t slot, const UpolyRec& u, int x, int y,
-                                              int smp)
+__device__ __forceinline__ void put_id(const ReyesArgs& a, uint32_t id, const UpolyRec& u)
 {
-  const uint32_t pix = ((uint32_t)y * (uint32_t)a.W + (uint32_t)x) * (uint32_t)a.spp + (uint32_t)smp;
-  atomicMin(&a.zmin[pix], zorder(u.z));
-  if (slot < a.frag_cap) {
-    FragRec f;
-    f.key = u.key;
-    f.pix = pix;
-    f.z = u.z;
-    f.color = u.color;
-    f.pad[0] = f.pad[1] = f.pad[2] = 0;
-    const uint4* src = reinterpret_cast<const uint4*>(&f);
-    uint4* dst = reinterpret_cast<uint4*>(&a.frags[slot]);
-    dst[0] = src[0];
-    dst[1] = src[1];
+  if (id < a.id_cap) {
+    a.id_color[id] = id_colour(u);
+    a.id_key[id] = u.key;
   } else {
-    atomicOr(&a.ctr->fc.status, kStatusListOverflow);
+    atomicOr(&a.ctr->fc.status, kStatusListOverflow);   // the host grows the tables and runs again
   }
 }
 
+__device__ __forceinline__ uint32_t sample_index(const ReyesArgs& a, int x, int y, int smp)
+{
+  return ((uint32_t)y * (uint32_t)a.W + (uint32_t)x) * (uint32_t)a.spp + (uint32_t)smp;
+}
+
+// Tie records of a CTA not yet in the list (a global append each, a tenth to a
+// quarter of the fragments, took 16 us of the default-constants sphere's dice).
+constexpr uint32_t kTieStage = 384;
+struct TieStage {
+  uint4 rec[kTieStage];
+  uint32_t n, base;
+};
+
+__device__ __forceinline__ void put_tie(const ReyesArgs& a, uint32_t slot, uint4 t)
+{
+  if (slot < a.tie_cap) a.ties[slot] = t;
+  else atomicOr(&a.ctr->fc.status, kStatusListOverflow);
+}
+
+// The fragment (zo, id) found `old` at sample p: leaves a record where the two
+// share their depth, and at +-0 always.
+__device__ __forceinline__ void check_tie(const ReyesArgs& a, TieStage* stage, uint32_t p, uint32_t zo, uint32_t id,
+                                          bool zero, unsigned long long old)
+{
+  const bool met = (uint32_t)(old >> 32) == zo;
+  if (!met && !zero) return;
+  const uint4 t = make_uint4(p, zo, id, met ? (uint32_t)old : id);
+  const uint32_t at = stage ? atomicAdd(&stage->n, 1u) : kTieStage;
+  if (at < kTieStage) stage->rec[at] = t;
+  else put_tie(a, atomicAdd(&a.ctr->tie_count, 1u), t);
+}
+
+// Writes the staged records out once there are more than `keep`; every thread
+// of the CTA calls it, after a barrier behind the last check_tie.
+__device__ __forceinline__ void flush_ties(const ReyesArgs& a, TieStage& stage, uint32_t keep)
+{
+  const uint32_t n = min(stage.n, kTieStage);
+  if (n <= keep) return;   // uniform
+  if (threadIdx.x == 0) stage.base = atomicAdd(&a.ctr->tie_count, n);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) put_tie(a, stage.base + i, stage.rec[i]);
+  __syncthreads();
+  if (threadIdx.x == 0) stage.n = 0;
+}
+
 // Block-wide exclusive scan of n (all 256 threads call it) and one atomic on
-// the fragment counter; returns this thread's first slot.
+// the id counter; returns this thread's first id.
 __device__ __forceinline__ uint32_t block_append(const ReyesArgs& a, uint32_t n, uint32_t* s_warp, uint32_t* s_base)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -770,7 +828,7 @@ __device__ __forceinline__ uint32_t block_append(const ReyesArgs& a, uint32_t n,
   if (threadIdx.x == 0) {
     uint32_t tot = 0;
     for (int w = 0; w < 8; ++w) { const uint32_t v = s_warp[w]; s_warp[w] = tot; tot += v; }
-    *s_base = tot ? atomicAdd(&a.ctr->frag_count, tot) : 0u;
+    *s_base = tot ? atomicAdd(&a.ctr->id_count, tot) : 0u;
   }
   __syncthreads();
   const uint32_t r = *s_base + s_warp[warp] + inc - n;
@@ -883,8 +941,8 @@ __device__ __forceinline__ void make_upoly(const ReyesArgs& a, unsigned long lon
   }
 }
 
-// Dice (R12, R13), then fragment pass 1 for micropolygons with at most
-// kSmallPx candidate pixels (larger ones are queued for a warp each).
+// Dice (R12, R13), then the fragments of micropolygons with at most kSmallPx
+// candidate pixels (larger ones are queued for a warp each).
 //
 // The dice rows of all leaves (row k of a leaf: its micropolygons (k, 0..nv))
 // are numbered in leaf-slot order and every CTA takes an equal range of them.
@@ -928,6 +986,7 @@ struct DiceSmem {
   uint32_t scan[8], append[8];
   uint32_t total, base;
   uint32_t nseg, next_leaf, next_row, found;
+  TieStage ties;
 };
 constexpr size_t kDiceSmem = sizeof(DiceSmem);
 
@@ -1035,6 +1094,7 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
     if (threadIdx.x == 0) {
       S.next_leaf = lo;
       S.next_row = r_begin;
+      S.ties.n = 0;
     }
   }
   for (;;) {
@@ -1179,7 +1239,9 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
           }
         }
       }
+      // (the scan's barriers lie between the last batch's records and the flush)
       const uint32_t pre = block_scan((uint32_t)cnt, S.scan, &S.total);
+      flush_ties(a, S.ties, kTieStage / 2);
       const uint32_t total = S.total;
       for (uint32_t w0 = 0; w0 < total; w0 += kCellCap) {
         const int lo = max(0, (int)w0 - (int)pre), hi = min(cnt, (int)(w0 + kCellCap) - (int)pre);
@@ -1192,21 +1254,39 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
       unsigned long long mask = cnt > 0 ? S.mask[threadIdx.x] : 0ull;
       covered += __popcll(mask);
       if (cnt > 0 && !(o.z <= 1.0f)) mask = 0;  // behind the cleared depth (or NaN): never survives
-      uint32_t slot = block_append(a, __popcll(mask), S.append, &S.base);
-      while (mask) {
-        const int c = __ffsll(mask) - 1;
-        mask &= mask - 1;
-        int cx, cy;
-        cell_xy(cwm, org, c, cx, cy);
-        if (r == 1) emit_fragment(a, slot++, o, cx, cy, 0);
-        else emit_fragment(a, slot++, o, cx >> 1, cy >> 1, (cx & 1) | ((cy & 1) << 1));
+      const uint32_t id = block_append(a, mask ? 1u : 0u, S.append, &S.base);
+      if (mask) {
+        put_id(a, id, o);
+        const uint32_t zo = zorder(o.z);
+        const bool zero = o.z == 0.0f;
+        const unsigned long long st = ((unsigned long long)zo << 32) | id;
+        // an atomic's answer is looked at after the next one is on its way
+        unsigned long long old = kSampEmpty;
+        uint32_t at = 0;
+        bool first = true;
+        while (mask) {
+          const int c = __ffsll(mask) - 1;
+          mask &= mask - 1;
+          int cx, cy;
+          cell_xy(cwm, org, c, cx, cy);
+          const uint32_t p = r == 1 ? sample_index(a, cx, cy, 0)
+                                    : sample_index(a, cx >> 1, cy >> 1, (cx & 1) | ((cy & 1) << 1));
+          const unsigned long long got = atomicMin(&a.samp[p], st);
+          if (!first) check_tie(a, &S.ties, at, zo, id, zero, old);
+          first = false;
+          old = got;
+          at = p;
+        }
+        check_tie(a, &S.ties, at, zo, id, zero, old);
       }
     }
   }
+  __syncthreads();
+  flush_ties(a, S.ties, 0u);
   add_covered(a, covered);
 }
 
-// Fragment pass 1 for the queued micropolygons: a warp each, a lane per pixel.
+// The fragments of the queued micropolygons: a warp each, a lane per sample.
 __global__ void __launch_bounds__(256) reyes_big(ReyesArgs a)
 {
   pdl_wait();
@@ -1223,6 +1303,8 @@ __global__ void __launch_bounds__(256) reyes_big(ReyesArgs a)
     for (int q = 0; q < 4; ++q) dst[q] = src[q];
     const int bw = u.x1 - u.x0;
     const int n = bw * (u.y1 - u.y0) * a.spp;   // candidate samples
+    const uint32_t zo = zorder(u.z);
+    uint32_t id = kNoId;
     for (int k0 = 0; k0 < n; k0 += 32) {
       const int k = k0 + lane;
       const int pk = k / a.spp, smp = k - pk * a.spp;
@@ -1231,205 +1313,121 @@ __global__ void __launch_bounds__(256) reyes_big(ReyesArgs a)
       if (k < n) sample_pos(a.spp, a.seed, x, y, smp, px, py);
       const bool cov = k < n && upoly_covers(make_float4(u.sx[0], u.sx[1], u.sx[2], u.sx[3]),
                                               make_float4(u.sy[0], u.sy[1], u.sy[2], u.sy[3]), px, py);
-      const unsigned m = __ballot_sync(kFullR, cov);
       covered += cov ? 1u : 0u;
-      const unsigned keep = (u.z <= 1.0f) ? m : 0u;
-      uint32_t base = 0;
-      if (lane == 0 && keep) base = atomicAdd(&a.ctr->frag_count, (uint32_t)__popc(keep));
-      base = __shfl_sync(kFullR, base, 0);
-      if (keep & (1u << lane)) emit_fragment(a, base + __popc(keep & ((1u << lane) - 1u)), u, x, y, smp);
+      const unsigned keep = __ballot_sync(kFullR, cov && u.z <= 1.0f);
+      if (!keep) continue;
+      if (id == kNoId) {
+        if (lane == 0) {
+          id = atomicAdd(&a.ctr->id_count, 1u);
+          put_id(a, id, u);
+        }
+        id = __shfl_sync(kFullR, id, 0);
+      }
+      if ((keep >> lane) & 1u) {
+        const uint32_t p = sample_index(a, x, y, smp);
+        check_tie(a, nullptr, p, zo, id, u.z == 0.0f, atomicMin(&a.samp[p], ((unsigned long long)zo << 32) | id));
+      }
     }
   }
   add_covered(a, covered);
 }
 
-// Passes 2 and 3 are bound by the latency of dependent loads (fragment, then
-// its sample's minimum, then its keys): a thread takes kFragBatch fragments of
-// its grid-stride range at a time and issues each level of loads for all of
-// them before the next.  The fragments are independent, so the order changes
-// nothing.
-constexpr int kFragBatch = 4;
-
-// Key, sample index and depth of a fragment: its first 16 bytes in one load.
-struct FragHead {
-  unsigned long long key;
-  uint32_t pix;
-  float z;
-};
-
-__device__ __forceinline__ FragHead frag_head(const FragRec* f, uint32_t i)
-{
-  const uint4 q = __ldg(reinterpret_cast<const uint4*>(&f[i]));
-  FragHead h;
-  h.key = (unsigned long long)q.x | ((unsigned long long)q.y << 32);
-  h.pix = q.z;
-  h.z = __uint_as_float(q.w);
-  return h;
-}
-
-// Fragment pass 2: greatest key among the fragments at the minimum (the
-// colour), and the least one where the minimum is +-0 (the only depth whose
-// fragments can differ in their bits: elsewhere every fragment at the minimum
-// carries the same bits, and the colour's fragment writes them).
-__global__ void __launch_bounds__(256) reyes_keys(ReyesArgs a)
+// Samples at which fragments met at one depth: of all that did (each but the
+// first has a record, which names one it met), the one with the greatest key
+// takes the sample, if that depth is still the sample's.  At +-0 the one with
+// the least key goes to first0.
+__global__ void __launch_bounds__(256) reyes_ties(ReyesArgs a)
 {
   pdl_wait();
   pdl_trigger();
-  const uint32_t n = min(a.ctr->frag_count, a.frag_cap);
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kFragBatch * stride) {
-    FragHead h[kFragBatch];
-    bool ok[kFragBatch];
-    uint32_t zm[kFragBatch];
+  const uint32_t n = min(a.ctr->tie_count, a.tie_cap);
+  // after an overflow of the tables the frame runs again: no key to look up
+  if (a.ctr->id_count > a.id_cap) return;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint4 t = a.ties[i];
+    if ((uint32_t)(__ldcg(&a.samp[t.x]) >> 32) != t.y) continue;   // (this pass changes no depth)
+    const uint32_t ids[2] = {t.z, t.w};
 #pragma unroll
-    for (int u = 0; u < kFragBatch; ++u) {
-      ok[u] = (uint32_t)u * stride < n - i0;
-      if (ok[u]) h[u] = frag_head(a.frags, i0 + (uint32_t)u * stride);
-    }
-#pragma unroll
-    for (int u = 0; u < kFragBatch; ++u) zm[u] = ok[u] ? a.zmin[h[u].pix] : 0u;
-#pragma unroll
-    for (int u = 0; u < kFragBatch; ++u) {
-      if (!ok[u] || !(h[u].z == zorder_inv(zm[u]))) continue;
-      atomicMax(&a.klast[h[u].pix], h[u].key);
-      if (h[u].z == 0.0f) atomicMin(&a.kfirst[h[u].pix], h[u].key);
-    }
-  }
-}
-
-// Fragment pass 3: the last fragment at the minimum writes the colour and the
-// depth; at a minimum of +-0 the first one writes the depth bits.
-__global__ void __launch_bounds__(256) reyes_resolve(ReyesArgs a)
-{
-  pdl_wait();
-  pdl_trigger();
-  const uint32_t n = min(a.ctr->frag_count, a.frag_cap);
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kFragBatch * stride) {
-    FragHead h[kFragBatch];
-    uint32_t col[kFragBatch], zm[kFragBatch];
-    bool at[kFragBatch];
-    unsigned long long kl[kFragBatch], kf[kFragBatch];
-#pragma unroll
-    for (int u = 0; u < kFragBatch; ++u) {
-      at[u] = (uint32_t)u * stride < n - i0;
-      if (at[u]) {
-        const uint32_t i = i0 + (uint32_t)u * stride;
-        h[u] = frag_head(a.frags, i);
-        col[u] = __ldg(&a.frags[i].color);
+    for (int k = 0; k < 2; ++k) {
+      const unsigned long long key = a.id_key[ids[k]], mine = ((unsigned long long)t.y << 32) | ids[k];
+      unsigned long long cur = __ldcg(&a.samp[t.x]);
+      while (key > a.id_key[(uint32_t)cur]) {   // (the key kept only grows)
+        const unsigned long long was = atomicCAS(&a.samp[t.x], cur, mine);
+        if (was == cur) break;
+        cur = was;
       }
-    }
-#pragma unroll
-    for (int u = 0; u < kFragBatch; ++u) zm[u] = at[u] ? a.zmin[h[u].pix] : 0u;
-#pragma unroll
-    for (int u = 0; u < kFragBatch; ++u) {
-      at[u] = at[u] && h[u].z == zorder_inv(zm[u]);
-      kl[u] = at[u] ? a.klast[h[u].pix] : 0ull;
-      kf[u] = (at[u] && h[u].z == 0.0f) ? a.kfirst[h[u].pix] : 0ull;
-    }
-#pragma unroll
-    for (int u = 0; u < kFragBatch; ++u) {
-      if (!at[u]) continue;
-      const bool last = kl[u] == h[u].key;
-      const bool dep = h[u].z == 0.0f ? kf[u] == h[u].key : last;
-      const uint32_t p = h[u].pix;
-      if (a.spp == 1) {
-        if (last) a.fb[p] = col[u];
-        if (dep) a.depth[p] = h[u].z;
-      } else {
-        if (last) a.scol[p] = col[u];
-        if (dep) a.sdep[p] = h[u].z;
+      if (zorder_inv(t.y) != 0.0f) continue;
+      uint32_t f = __ldcg(&a.first0[t.x]);
+      while (f == kNoId || key < a.id_key[f]) {   // (the key kept only falls)
+        const uint32_t was = atomicCAS(&a.first0[t.x], f, ids[k]);
+        if (was == f) break;
+        f = was;
       }
     }
   }
 }
 
-// The last pass, over every pixel.  One sample per pixel: a pixel no fragment
-// reached gets the clear colour and depth 1 (the resolve wrote the others).
-// More samples: a pixel takes the rounded mean of its samples' colours per
-// channel (the clear colour where no fragment reached a sample) and the depth
-// of its nearest sample (the first such sample on ties).  Either way every
-// reached sample's depth minimum and key bounds are set back to empty, so the
-// next frame finds the per-sample state cleared.
+// Sample si's colour and depth from its state st; a reached one is set back.
+__device__ __forceinline__ bool take_sample(const ReyesArgs& a, size_t si, unsigned long long st, uint32_t& c, float& z)
+{
+  c = kClearColor;
+  z = 1.0f;
+  if (st == kSampEmpty) return false;
+  const uint32_t id = (uint32_t)st;
+  if (id >= a.id_cap) return true;   // the tables overflowed: the frame runs again
+  c = a.id_color[id] | 0xff000000u;
+  z = zorder_inv((uint32_t)(st >> 32));
+  if (z == 0.0f) {
+    const uint32_t f = a.first0[si];
+    a.first0[si] = kNoId;
+    if (f < a.id_cap && !(a.id_color[f] & 0x01000000u)) z = -0.0f;
+  }
+  return true;
+}
+
+// The last pass, over every pixel.  One sample per pixel: the sample's colour
+// and depth, the clear colour and depth 1 where no fragment reached it.  More
+// samples: a pixel takes the rounded mean of its samples' colours per channel
+// and the depth of its nearest sample (the first such sample on ties).  Every
+// reached sample's state is set back to empty, so the next frame finds it so.
 __global__ void __launch_bounds__(256) reyes_pixels(ReyesArgs a, uint32_t npx)
 {
   pdl_wait();
-  const uint32_t spp = (uint32_t)a.spp;
-  if (spp == 4) {
-    // a pixel's four samples are 16 (u32) or 32 (u64) contiguous, aligned
-    // bytes: one vector access per array; a pixel with any reached sample has
-    // all four set back (a sample not reached already holds the empty state)
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < npx; i += gridDim.x * blockDim.x) {
-      const size_t s0 = 4 * (size_t)i;
-      const uint4 zm = *reinterpret_cast<const uint4*>(&a.zmin[s0]);
-      const bool r[4] = {zm.x != kZminEmpty, zm.y != kZminEmpty, zm.z != kZminEmpty, zm.w != kZminEmpty};
-      uint32_t c[4] = {kClearColor, kClearColor, kClearColor, kClearColor};
-      float z[4] = {1.0f, 1.0f, 1.0f, 1.0f};
-      if (r[0] || r[1] || r[2] || r[3]) {
-        const uint4 sc = *reinterpret_cast<const uint4*>(&a.scol[s0]);
-        const float4 sd = *reinterpret_cast<const float4*>(&a.sdep[s0]);
-        *reinterpret_cast<uint4*>(&a.zmin[s0]) = make_uint4(kZminEmpty, kZminEmpty, kZminEmpty, kZminEmpty);
-        ulonglong2* kl = reinterpret_cast<ulonglong2*>(&a.klast[s0]);
-        ulonglong2* kf = reinterpret_cast<ulonglong2*>(&a.kfirst[s0]);
-        kl[0] = make_ulonglong2(0ull, 0ull);
-        kl[1] = make_ulonglong2(0ull, 0ull);
-        kf[0] = make_ulonglong2(~0ull, ~0ull);
-        kf[1] = make_ulonglong2(~0ull, ~0ull);
-        const uint32_t scv[4] = {sc.x, sc.y, sc.z, sc.w};
-        const float sdv[4] = {sd.x, sd.y, sd.z, sd.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (r[k]) { c[k] = scv[k]; z[k] = sdv[k]; }
-        }
-      }
-      uint32_t sum[3] = {0u, 0u, 0u};
-      float best = 1.0f;
-      uint32_t best_o = 0xffffffffu;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        sum[0] += c[k] & 255u;
-        sum[1] += (c[k] >> 8) & 255u;
-        sum[2] += (c[k] >> 16) & 255u;
-        const uint32_t o = zorder(z[k]);
-        if (k == 0 || o < best_o) { best_o = o; best = z[k]; }
-      }
-      a.fb[i] = 0xff000000u | (((sum[2] + 2u) / 4u) << 16) | (((sum[1] + 2u) / 4u) << 8) | ((sum[0] + 2u) / 4u);
-      a.depth[i] = best;
-    }
-    return;
-  }
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < npx; i += gridDim.x * blockDim.x) {
+    if (a.spp == 1) {
+      const unsigned long long st = a.samp[i];
+      uint32_t c;
+      float z;
+      if (take_sample(a, i, st, c, z)) a.samp[i] = kSampEmpty;
+      a.fb[i] = c;
+      a.depth[i] = z;
+      continue;
+    }
+    // four samples: 32 contiguous, aligned bytes; a pixel with any reached
+    // sample has all four set back
+    ulonglong2* sp = reinterpret_cast<ulonglong2*>(&a.samp[4 * (size_t)i]);
+    const ulonglong2 lo = sp[0], hi = sp[1];
+    const unsigned long long st[4] = {lo.x, lo.y, hi.x, hi.y};
+    uint32_t c[4] = {kClearColor, kClearColor, kClearColor, kClearColor};
+    float z[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+    if ((st[0] & st[1] & st[2] & st[3]) != kSampEmpty) {
+      sp[0] = make_ulonglong2(kSampEmpty, kSampEmpty);
+      sp[1] = make_ulonglong2(kSampEmpty, kSampEmpty);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) take_sample(a, 4 * (size_t)i + k, st[k], c[k], z[k]);
+    }
     uint32_t sum[3] = {0u, 0u, 0u};
     float best = 1.0f;
     uint32_t best_o = 0xffffffffu;
-    bool any = false;
-    for (uint32_t k = 0; k < spp; ++k) {
-      const uint32_t si = i * spp + k;
-      const bool reached = a.zmin[si] != kZminEmpty;
-      if (reached) {
-        a.zmin[si] = kZminEmpty;
-        a.klast[si] = 0ull;
-        a.kfirst[si] = ~0ull;
-        any = true;
-      }
-      if (spp == 1) continue;
-      const uint32_t c = reached ? a.scol[si] : kClearColor;
-      const float z = reached ? a.sdep[si] : 1.0f;
-      sum[0] += c & 255u;
-      sum[1] += (c >> 8) & 255u;
-      sum[2] += (c >> 16) & 255u;
-      const uint32_t o = zorder(z);
-      if (k == 0 || o < best_o) { best_o = o; best = z; }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      sum[0] += c[k] & 255u;
+      sum[1] += (c[k] >> 8) & 255u;
+      sum[2] += (c[k] >> 16) & 255u;
+      const uint32_t o = zorder(z[k]);
+      if (k == 0 || o < best_o) { best_o = o; best = z[k]; }
     }
-    if (spp == 1) {
-      if (!any) {
-        a.fb[i] = kClearColor;
-        a.depth[i] = 1.0f;
-      }
-      continue;
-    }
-    a.fb[i] = 0xff000000u | (((sum[2] + spp / 2u) / spp) << 16) | (((sum[1] + spp / 2u) / spp) << 8) |
-              ((sum[0] + spp / 2u) / spp);
+    a.fb[i] = 0xff000000u | (((sum[2] + 2u) / 4u) << 16) | (((sum[1] + 2u) / 4u) << 8) | ((sum[0] + 2u) / 4u);
     a.depth[i] = best;
   }
 }
@@ -1485,9 +1483,8 @@ cudaError_t launch_reyes_frame(const ReyesArgs& a, uint32_t npx, int sms, cudaSt
   e = launch_chained(reyes_dice, sms * dice_per_sm, kDiceThreads, kDiceSmem, st, a);
   if (!e) e = launch_chained(reyes_big, grid, 256, 0, st, a);
   if (ev) cudaEventRecord(ev[2], st);
-  if (!e) e = launch_chained(reyes_keys, grid, 256, 0, st, a);
+  if (!e) e = launch_chained(reyes_ties, sms * 4, 256, 0, st, a);
   if (ev) cudaEventRecord(ev[3], st);
-  if (!e) e = launch_chained(reyes_resolve, grid, 256, 0, st, a);
   if (!e) e = launch_chained(reyes_pixels, grid, 256, 0, st, a, npx);
   if (ev) cudaEventRecord(ev[4], st);
   if (e) return e;
@@ -1506,15 +1503,15 @@ using namespace piko;
 struct ReyesState {
   ReyesState* buffers = nullptr;  // borrowed work buffers (not owned), or null
   PatchRec* lvl[2] = {nullptr, nullptr};
+  PatchRec* stack = nullptr;
   PatchRec* leaves = nullptr;
   UpolyRec* up = nullptr;
-  FragRec* frags = nullptr;
-  uint32_t lvl_cap = 0, leaf_cap = 0, up_cap = 0, frag_cap = 0;
-  uint32_t* zmin = nullptr;
-  unsigned long long* kfirst = nullptr;
-  unsigned long long* klast = nullptr;
-  uint32_t* scol = nullptr;
-  float* sdep = nullptr;
+  uint32_t* id_color = nullptr;
+  unsigned long long* id_key = nullptr;
+  uint4* ties = nullptr;
+  uint32_t lvl_cap = 0, leaf_cap = 0, up_cap = 0, id_cap = 0, tie_cap = 0;
+  unsigned long long* samp = nullptr;
+  uint32_t* first0 = nullptr;
   size_t npx_cap = 0;   // samples
   bool clean = false;   // per-sample state all empty (set when allocated; every frame leaves it so)
   ReyesCounters* ctr = nullptr;
@@ -1525,8 +1522,8 @@ struct ReyesState {
 
 static void reyes_state_free(ReyesState* r)
 {
-  dfree(r->lvl[0]); dfree(r->lvl[1]); dfree(r->leaves); dfree(r->up); dfree(r->frags);
-  dfree(r->zmin); dfree(r->kfirst); dfree(r->klast); dfree(r->scol); dfree(r->sdep); dfree(r->ctr);
+  dfree(r->lvl[0]); dfree(r->lvl[1]); dfree(r->stack); dfree(r->leaves); dfree(r->up);
+  dfree(r->id_color); dfree(r->id_key); dfree(r->ties); dfree(r->samp); dfree(r->first0); dfree(r->ctr);
   if (r->h_ctr) cudaFreeHost(r->h_ctr);
   if (r->ev_made) for (auto& e : r->ev) cudaEventDestroy(e);
   delete r;
@@ -1550,13 +1547,13 @@ void reyes_borrow_buffers(piko_scene* s, ReyesState* b)
   s->reyes->buffers = b;
 }
 
-static cudaError_t reyes_alloc(ReyesState* r, uint32_t lvl_cap, uint32_t leaf_cap, uint32_t up_cap, uint32_t frag_cap,
-                               size_t npx)
+static cudaError_t reyes_alloc(ReyesState* r, uint32_t lvl_cap, uint32_t leaf_cap, uint32_t up_cap, uint32_t id_cap,
+                               uint32_t tie_cap, size_t npx)
 {
   cudaError_t e = cudaSuccess;
   if (r->buffers) {
-    if ((e = reyes_alloc(r->buffers, lvl_cap, leaf_cap, up_cap, frag_cap, npx))) return e;
-    lvl_cap = leaf_cap = up_cap = frag_cap = 0;
+    if ((e = reyes_alloc(r->buffers, lvl_cap, leaf_cap, up_cap, id_cap, tie_cap, npx))) return e;
+    lvl_cap = leaf_cap = up_cap = id_cap = tie_cap = 0;
     npx = 0;
   }
   if (lvl_cap > r->lvl_cap) {
@@ -1574,18 +1571,23 @@ static cudaError_t reyes_alloc(ReyesState* r, uint32_t lvl_cap, uint32_t leaf_ca
     if ((e = dalloc(&r->up, up_cap))) return e;
     r->up_cap = up_cap;
   }
-  if (frag_cap > r->frag_cap) {
-    dfree(r->frags);
-    if ((e = dalloc(&r->frags, frag_cap))) return e;
-    r->frag_cap = frag_cap;
+  if (id_cap > r->id_cap) {
+    dfree(r->id_color); dfree(r->id_key);
+    r->id_cap = 0;
+    if ((e = dalloc(&r->id_color, id_cap)) || (e = dalloc(&r->id_key, id_cap))) return e;
+    r->id_cap = id_cap;
+  }
+  if (tie_cap > r->tie_cap) {
+    dfree(r->ties);
+    r->tie_cap = 0;
+    if ((e = dalloc(&r->ties, tie_cap))) return e;
+    r->tie_cap = tie_cap;
   }
   if (npx > r->npx_cap) {
-    dfree(r->zmin); dfree(r->kfirst); dfree(r->klast); dfree(r->scol); dfree(r->sdep);
+    dfree(r->samp); dfree(r->first0);
     r->npx_cap = 0;
     r->clean = false;
-    if ((e = dalloc(&r->zmin, npx)) || (e = dalloc(&r->kfirst, npx)) || (e = dalloc(&r->klast, npx)) ||
-        (e = dalloc(&r->scol, npx)) || (e = dalloc(&r->sdep, npx)))
-      return e;
+    if ((e = dalloc(&r->samp, npx)) || (e = dalloc(&r->first0, npx))) return e;
     r->npx_cap = npx;
   }
   if (!r->ctr) {
@@ -1613,7 +1615,9 @@ piko_status piko_reyes_run(piko_scene* s, cudaStream_t st, bool timed)
   const size_t nsamp = npx * (size_t)p->samples_per_pixel;
   CU(ctx, reyes_alloc(r, std::max<uint32_t>(1u << 16, 64u * P), std::max<uint32_t>(1u << 16, 64u * P),
                       b->up_cap ? b->up_cap : (1u << 16),
-                      b->frag_cap ? b->frag_cap : (uint32_t)std::max<size_t>(1u << 20, nsamp), nsamp));
+                      b->id_cap ? b->id_cap : (uint32_t)std::max<size_t>(1u << 18, npx / 2),
+                      b->tie_cap ? b->tie_cap : (uint32_t)std::max<size_t>(1u << 18, nsamp / 8), nsamp));
+  if (!b->stack) CU(ctx, dalloc(&b->stack, (size_t)ctx->sms * kSplitStack));
   CU(ctx, cudaMemsetAsync(r->ctr, 0, sizeof(ReyesCounters), st));
   ReyesArgs a;
   memset(&a, 0, sizeof(a));
@@ -1626,21 +1630,21 @@ piko_status piko_reyes_run(piko_scene* s, cudaStream_t st, bool timed)
   a.grid = p->dice_grid;
   a.in_patches = s->patches;
   a.lvl[0] = b->lvl[0]; a.lvl[1] = b->lvl[1]; a.lvl_cap = b->lvl_cap;
+  a.stack = b->stack;
   a.leaves = b->leaves; a.leaf_cap = b->leaf_cap;
   a.up = b->up; a.up_cap = b->up_cap;
-  a.frags = b->frags; a.frag_cap = b->frag_cap;
+  a.id_color = b->id_color; a.id_key = b->id_key; a.id_cap = b->id_cap;
+  a.ties = b->ties; a.tie_cap = b->tie_cap;
   a.ctr = r->ctr;
   a.fb = s->fb; a.depth = s->depth;
-  a.zmin = b->zmin; a.kfirst = b->kfirst; a.klast = b->klast;
+  a.samp = b->samp; a.first0 = b->first0;
   a.spp = p->samples_per_pixel;
   a.seed = p->sample_seed;
   a.phong = p->phong;
-  a.scol = b->scol; a.sdep = b->sdep;
   if (!b->clean) {
     // fresh sample buffers, or a frame whose launches failed part way
-    CU(ctx, cudaMemsetAsync(b->zmin, 0xff, sizeof(uint32_t) * b->npx_cap, st));
-    CU(ctx, cudaMemsetAsync(b->kfirst, 0xff, sizeof(unsigned long long) * b->npx_cap, st));
-    CU(ctx, cudaMemsetAsync(b->klast, 0, sizeof(unsigned long long) * b->npx_cap, st));
+    CU(ctx, cudaMemsetAsync(b->samp, 0xff, sizeof(unsigned long long) * b->npx_cap, st));
+    CU(ctx, cudaMemsetAsync(b->first0, 0xff, sizeof(uint32_t) * b->npx_cap, st));
     b->clean = true;
   }
   const cudaError_t le = launch_reyes_frame(a, (uint32_t)npx, ctx->sms, st, timed ? r->ev : nullptr);
@@ -1668,11 +1672,15 @@ piko_status piko_reyes_finish(piko_scene* s)
     for (int i = 0; i < 40; ++i) maxlvl = std::max(maxlvl, c.level_count[i]);
     const uint32_t leaves = (uint32_t)(c.leaf_meta >> 40);
     const ReyesState* b = r->buffers ? r->buffers : r;
-    uint32_t lvl = b->lvl_cap, lf = b->leaf_cap, up = b->up_cap, fr = b->frag_cap;
+    uint32_t lvl = b->lvl_cap, lf = b->leaf_cap, up = b->up_cap, ids = b->id_cap, ties = b->tie_cap;
     if (st & kStatusPatchOverflow) { lvl = std::max(lvl, maxlvl + maxlvl / 2 + 1024); lf = std::max(lf, 2 * leaves + 1024); }
     if (st & kStatusUpolyOverflow) up = (uint32_t)std::min<unsigned long long>(c.big_count + c.big_count / 4ull + 4096, 0xffffffffull);
-    if (st & kStatusListOverflow) fr = (uint32_t)std::min<unsigned long long>(c.frag_count + c.frag_count / 4ull + 4096, 0xffffffffull);
-    CU(ctx, reyes_alloc(r, lvl, lf, up, fr, b->npx_cap));
+    const auto more = [](uint32_t n) {   // (an id of kNoId means none)
+      return (uint32_t)std::min<unsigned long long>(n + n / 4ull + 4096, 0xfffffffeull);
+    };
+    if (c.id_count > ids) ids = more(c.id_count);
+    if (c.tie_count > ties) ties = more(c.tie_count);
+    CU(ctx, reyes_alloc(r, lvl, lf, up, ids, ties, b->npx_cap));
     piko_status rr = piko_reyes_run(s, s->last_stream, s->timed);
     if (rr != PIKO_OK) return rr;
   }
