@@ -110,7 +110,8 @@ struct ReyesArgs {
   uint32_t id_cap;
   uint4* ties;                    // (sample, depth code, micropolygon, the one it met)
   uint32_t tie_cap;
-  ReyesCounters* ctr;
+  ReyesCounters* ctr;             // zero between frames
+  ReyesCounters* host_ctr;        // pinned: the last frame's
   uint32_t* fb;
   float* depth;
   unsigned long long* samp;       // per sample: depth code << 32 | micropolygon of the least fragment so far
@@ -510,6 +511,59 @@ __device__ __forceinline__ void split_pass(const ReyesArgs& a, SplitSmem& S, con
     split_one(a, S, cur, nxt, p);
 }
 
+// The first levels of the step's patch `owner` (share 1; 0: none), by one warp:
+// down the CTA's path of dr bits, then level by level until one has more than
+// kNarrow patches.  Leaves S.ncur patches in S.buf[S.word[0]].
+constexpr uint32_t kNarrow = 4;
+__device__ __forceinline__ void narrow_levels(const ReyesArgs& a, SplitSmem& S, int step, uint32_t owner,
+                                              uint32_t share, uint32_t path, uint32_t dr)
+{
+  const uint32_t lane = threadIdx.x;
+  uint32_t ncur = share, cb = 0;
+  if (share) {
+    if (step == 0) {
+      if (lane < 16) S.buf[0][0].cp[lane] = __ldcg(&a.in_patches[(size_t)owner * 16 + lane]);
+      if (lane == 0) {
+        S.buf[0][0].i0 = owner;
+        S.buf[0][0].level = 0;
+        S.buf[0][0].s = owner;
+      }
+    } else if (lane < sizeof(PatchRec) / 16) {
+      reinterpret_cast<float4*>(&S.buf[0][0])[lane] = __ldcg(reinterpret_cast<const float4*>(a.lvl[step & 1] + owner) + lane);
+    }
+  }
+  while (ncur > 0 && ncur <= kNarrow) {
+    // (a level adds at most kNarrow leaves; the stage has room for far more levels)
+    if (lane == 0) S.nnext = 0;
+    __syncwarp();
+    for (uint32_t p = lane >> 4; p < ncur; p += 2) split_one(a, S, S.buf[cb], S.buf[cb ^ 1], p);
+    __syncwarp();
+    uint32_t nn = S.nnext;
+    if (dr > 0) {
+      // one patch on the CTA's path: keep the child the path names, or drop a
+      // leaf that another CTA of the group emits
+      if (nn == 0) {
+        if ((path & ((1u << dr) - 1u)) != 0u && lane == 0) S.nleaf -= 1;
+      } else {
+        if ((path >> (dr - 1)) & 1u) {
+          float4* dst = reinterpret_cast<float4*>(&S.buf[cb ^ 1][0]);
+          const float4* src = reinterpret_cast<const float4*>(&S.buf[cb ^ 1][1]);
+          if (lane < sizeof(PatchRec) / 16) dst[lane] = src[lane];
+        }
+        nn = 1;
+      }
+      --dr;
+    }
+    ncur = nn;
+    cb ^= 1;
+    __syncwarp();
+  }
+  if (lane == 0) {
+    S.ncur = ncur;
+    S.word[0] = cb;
+  }
+}
+
 __global__ void __launch_bounds__(kSplitThreads, 1) reyes_split(ReyesArgs a)
 {
   pdl_trigger();
@@ -533,12 +587,21 @@ __global__ void __launch_bounds__(kSplitThreads, 1) reyes_split(ReyesArgs a)
     const uint32_t path = blockIdx.x & ((1u << d) - 1u), owner = blockIdx.x >> d;
     const uint32_t share = d > 0 ? (owner < n_in ? 1u : 0u)
                                  : (blockIdx.x < n_in ? (n_in - blockIdx.x - 1) / gridDim.x + 1 : 0u);
-    uint32_t dr = d;
     const bool deal = step == 0 && n_in < 8u * gridDim.x;   // too few patches to even out
     PatchRec* frontier = a.lvl[(step + 1) & 1];
     PatchRec* stack = a.stack + (size_t)blockIdx.x * kSplitStack;
     uint32_t taken = 0, ncur = 0, top = 0;
     int cb = 0;   // buf[cb] holds the current patches
+    if (d > 0) {
+      // One patch: its path and the first levels below it hold a few patches
+      // each, which the first warp expands by itself (a pass of the CTA with its
+      // barriers takes 1.2 us, one of a warp half of that)
+      if (threadIdx.x < 32) narrow_levels(a, S, step, owner, share, path, d);
+      __syncthreads();
+      taken = share;
+      ncur = S.ncur;
+      cb = (int)S.word[0];
+    }
     __syncthreads();
     while (ncur > 0 || top > 0 || taken < share) {   // uniform
       // top up the current patches from the stack, then from the share
@@ -548,7 +611,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) reyes_split(ReyesArgs a)
         ncur += pop;
       }
       if (const uint32_t take = min((uint32_t)kSplitKeep - ncur, share - taken)) {
-        load_inputs(a, step, d > 0 ? owner : blockIdx.x + taken * gridDim.x, gridDim.x, take, &S.buf[cb][ncur]);
+        load_inputs(a, step, blockIdx.x + taken * gridDim.x, gridDim.x, take, &S.buf[cb][ncur]);
         taken += take;
         ncur += take;
       }
@@ -558,21 +621,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) reyes_split(ReyesArgs a)
       split_pass(a, S, S.buf[cb], S.buf[cb ^ 1], ncur);
       __syncthreads();
       uint32_t nn = S.nnext, keep = min(nn, (uint32_t)kSplitKeep);
-      if (dr > 0) {
-        // one patch on the CTA's path (ncur == 1): keep the child the path
-        // names, or drop a leaf that another CTA of the group emits
-        if (nn == 0) {
-          if ((path & ((1u << dr) - 1u)) != 0u && threadIdx.x == 0) S.nleaf -= 1;
-        } else {
-          if ((path >> (dr - 1)) & 1u) {
-            float4* dst = reinterpret_cast<float4*>(&S.buf[cb ^ 1][0]);
-            const float4* src = reinterpret_cast<const float4*>(&S.buf[cb ^ 1][1]);
-            if (threadIdx.x < sizeof(PatchRec) / 16) dst[threadIdx.x] = src[threadIdx.x];
-          }
-          keep = 1;
-        }
-        --dr;
-      } else {
+      {
         if (deal && nn >= kSplitShare) keep = 0;   // the whole level to the frontier
         uint32_t own = nn - keep;                  // children for the CTA's stack
         if (deal && nn >= kSplitShare) own = 0;
@@ -713,6 +762,20 @@ __device__ __forceinline__ bool upoly_covers(float4 X4, float4 Y4, float px, flo
   return r1 || r2;
 }
 
+// The first winding alone.  With the corners in reverse order (1 and 3 swapped)
+// it is the second one, bit for bit.
+__device__ __forceinline__ bool upoly_covers_one(float4 X4, float4 Y4, float px, float py)
+{
+  const float X[4] = {X4.x, X4.y, X4.z, X4.w}, Y[4] = {Y4.x, Y4.y, Y4.z, Y4.w};
+  bool in = true;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float dX = X[(i + 1) & 3] - X[i], dY = Y[(i + 1) & 3] - Y[i];
+    if (!((py - Y[i]) * dX - (px - X[i]) * dY > 0.0f)) in = false;
+  }
+  return in;
+}
+
 // Which samples can pass upoly_covers at all.  When every corner coordinate is
 // at least 32 and the corners span less than 16 px per axis, each difference
 // the test takes (sample minus corner, corner minus corner) is exact
@@ -721,6 +784,12 @@ __device__ __forceinline__ bool upoly_covers(float4 X4, float4 Y4, float px, flo
 // number and lies strictly inside the corners' bounding box.  There the
 // coverage pass tests only the cells (pixel quadrants, or pixel centres with
 // one sample) whose sample range meets the open box; elsewhere it tests all.
+// There, too, at most one winding can pass, known from the area: a product's
+// rounding is monotone, so where all four rounded edge values are positive the
+// exact ones are none of them negative, and the exact ones add up to twice the
+// area wherever the sample is; the second winding needs them none positive.  The
+// area's own sign is the comparison of two rounded products of exact differences
+// (the diagonals), which orders the exact products unless they round equal.
 __device__ __forceinline__ bool exact_box(float mnx, float mxx, float mny, float mxy)
 {
   return mnx >= 32.0f && mny >= 32.0f && mxx - mnx < 16.0f && mxy - mny < 16.0f && mxx < 4194304.0f &&
@@ -789,10 +858,10 @@ __device__ __forceinline__ void put_tie(const ReyesArgs& a, uint32_t slot, uint4
 // The fragment (zo, id) found `old` at sample p: leaves a record where the two
 // share their depth, and at +-0 always.
 __device__ __forceinline__ void check_tie(const ReyesArgs& a, TieStage* stage, uint32_t p, uint32_t zo, uint32_t id,
-                                          bool zero, unsigned long long old)
+                                          unsigned long long old)
 {
   const bool met = (uint32_t)(old >> 32) == zo;
-  if (!met && !zero) return;
+  if (!met && zo != 0x80000000u) return;   // zorder(+-0)
   const uint4 t = make_uint4(p, zo, id, met ? (uint32_t)old : id);
   const uint32_t at = stage ? atomicAdd(&stage->n, 1u) : kTieStage;
   if (at < kTieStage) stage->rec[at] = t;
@@ -965,27 +1034,35 @@ constexpr int kMaxGridPts = 34 * 34;
 constexpr int kLeafBatch = 32;     // leaf segments per group
 constexpr int kDiceThreads = 256;
 constexpr int kUpBudget = 1024;    // micropolygons per group
-constexpr int kMaxPtRows = 64;     // grid point rows per group
+constexpr int kMaxPtRows = 128;    // grid point rows per group
 constexpr int kCellCap = 4096;     // cells per pass of the shared list
+
+constexpr uint32_t kNoDepth = 0xffffffffu;
+constexpr uint32_t kBothWindings = 1u << 31;   // (else the corners' order makes the first winding the one to test)
 
 struct DiceSmem {
   float4 cp[kLeafBatch][16];
   GridPt gp[kMaxGridPts];
-  DiceRow rowdat[kMaxPtRows];                  // control rows at each point row's u
-  float4 ux[kDiceThreads], uy[kDiceThreads];   // corners of each thread's micropolygon
-  int2 org[kDiceThreads];                      // first cell of its cell rectangle
-  uint32_t cwm[kDiceThreads];                  // rectangle width | (2^16 / width + 1) << 7
-  unsigned long long mask[kDiceThreads];       // covered cells
-  uint16_t cell[kCellCap];                     // (thread << 6) | cell index
+  union {
+    DiceRow rowdat[kMaxPtRows];                  // control rows at each point row's u (until the grid points stand)
+    struct {
+      float4 ux[kDiceThreads], uy[kDiceThreads];   // corners of each thread's micropolygon
+      int2 org[kDiceThreads];                      // first cell of its cell rectangle
+      uint32_t cwm[kDiceThreads];                  // rectangle width | (2^16 / width + 1) << 7 | kBothWindings
+      unsigned long long mask[kDiceThreads];       // covered cells (!SPARSE)
+      uint32_t zo[kDiceThreads];                   // depth code, kNoDepth: behind the cleared depth (SPARSE)
+      uint16_t cell[kCellCap];                     // (thread << 6) | cell index
+    };
+  };
   // the group's segments: rows k0 .. of leaf[i]; gpre / upre / rpre = first
   // grid point / micropolygon / point row of each segment in the group
   uint32_t leaf[kLeafBatch], k0[kLeafBatch], nu[kLeafBatch], nv[kLeafBatch];
   unsigned long long keyhi[kLeafBatch];
   uint32_t gpre[kLeafBatch + 1], upre[kLeafBatch + 1], rpre[kLeafBatch + 1];
-  uint32_t wnu[32], wnv[32], wrb[32];         // grid and first row of the next 32 leaves
   uint32_t scan[8], append[8];
   uint32_t total, base;
   uint32_t nseg, next_leaf, next_row, found;
+  uint32_t gid;         // the group's first id
   TieStage ties;
 };
 constexpr size_t kDiceSmem = sizeof(DiceSmem);
@@ -1041,25 +1118,118 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t n, uint32_t* s_warp, uin
 __device__ __forceinline__ void cell_xy(uint32_t cwm, int2 org, int li, int& cx, int& cy)
 {
   const int cw = (int)(cwm & 127u);
-  const int dy = (int)(((uint32_t)li * (cwm >> 7)) >> 16);
+  const int dy = (int)(((uint32_t)li * ((cwm >> 7) & 0x1ffffu)) >> 16);
   cx = org.x + li - dy * cw;
   cy = org.y + dy;
 }
 
-__device__ __forceinline__ void dice_cell(const ReyesArgs& a, DiceSmem& S, uint32_t q)
+// Tests cell q of the shared list: u = the thread whose micropolygon it is, li =
+// its index in the rectangle, (x, y, smp) its sample.
+__device__ __forceinline__ bool dice_cell(const ReyesArgs& a, const DiceSmem& S, uint32_t q, int& u, int& li, int& x,
+                                          int& y, int& smp)
 {
   const uint32_t e = S.cell[q];
-  const int u = (int)(e >> 6), li = (int)(e & 63u);
-  int cx, cy;
-  cell_xy(S.cwm[u], S.org[u], li, cx, cy);
+  u = (int)(e >> 6);
+  li = (int)(e & 63u);
+  const uint32_t cwm = S.cwm[u];
+  cell_xy(cwm, S.org[u], li, x, y);
+  smp = 0;
+  if (a.spp != 1) {
+    smp = (x & 1) | ((y & 1) << 1);
+    x >>= 1;
+    y >>= 1;
+  }
   float px, py;
-  if (a.spp == 1) sample_pos(1, a.seed, cx, cy, 0, px, py);
-  else sample_pos(a.spp, a.seed, cx >> 1, cy >> 1, (cx & 1) | ((cy & 1) << 1), px, py);
-  if (upoly_covers(S.ux[u], S.uy[u], px, py)) atomicOr(&S.mask[u], 1ull << li);
+  sample_pos(a.spp, a.seed, x, y, smp, px, py);
+  return (cwm & kBothWindings) ? upoly_covers(S.ux[u], S.uy[u], px, py) : upoly_covers_one(S.ux[u], S.uy[u], px, py);
+}
+
+// Chooses the next group: rows from row0 (of leaf leaf0) on, whole leaves, a
+// lane each, as many as the micropolygon budget, the shared grid points and the
+// point rows allow (of a leaf too large for them, as many rows), and of those
+// counts of leaves the one with the most micropolygons per step of the CTA: a
+// batch of kDiceThreads micropolygons is a step, and so is what comes before
+// them.  (One thread adding up to 16 leaves one after the other, 64 point rows
+// per group, took half of the dice time of 2 x 2 grids.)
+__device__ __forceinline__ void dice_group(const ReyesArgs& a, DiceSmem& S, uint32_t leaf0, uint32_t row0,
+                                           uint32_t nleaf, uint32_t r_end)
+{
+  const uint32_t lane = threadIdx.x, L = leaf0 + lane;
+  uint32_t nu = 0, nv = 0, first = r_end, k0 = 0, n = 0;
+  if (L < nleaf) {
+    nu = a.leaves[L].nu;
+    nv = a.leaves[L].nv;
+    const uint32_t rb = a.leaves[L].rowbase;
+    first = lane == 0 ? row0 : rb;
+    k0 = first - rb;
+    if (first < r_end) n = min(nu + 1 - k0, r_end - first);
+  }
+  const bool pow2 = ((nu & (nu - 1)) == 0) && ((nv & (nv - 1)) == 0);
+  uint32_t u = n * (nv + 1), g = pow2 && n ? (n + 1) * (nv + 2) : 0u, p = pow2 && n ? n + 1 : 0u;
+  uint32_t iu = u, ig = g, ip = p;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t tu = __shfl_up_sync(kFullR, iu, o), tg = __shfl_up_sync(kFullR, ig, o);
+    const uint32_t tp = __shfl_up_sync(kFullR, ip, o);
+    if (lane >= (uint32_t)o) { iu += tu; ig += tg; ip += tp; }
+  }
+  const bool fits = n > 0 && iu <= (uint32_t)kUpBudget && ig <= (uint32_t)kMaxGridPts && ip <= (uint32_t)kMaxPtRows;
+  const unsigned ok = __ballot_sync(kFullR, fits);
+  uint32_t m = (uint32_t)__ffs(~ok) - 1u;   // leading leaves that fit together (0xffffffff: all 32)
+  if (m > 32u) m = 32u;
+  if (m > 0) {
+    const uint32_t steps = (iu + kDiceThreads - 1) / kDiceThreads + 1;
+    const uint32_t score = lane < m ? ((iu << 12) / steps) << 5 | lane : 0u;
+    m = (__reduce_max_sync(kFullR, score) & 31u) + 1u;
+  } else {
+    // rows of the first leaf that fit
+    if (lane == 0) {
+      n = min(n, (uint32_t)kUpBudget / (nv + 1));
+      if (pow2) {
+        const uint32_t fit = min((uint32_t)kMaxGridPts / (nv + 2), (uint32_t)kMaxPtRows);
+        n = min(n, fit > 0 ? fit - 1 : 0u);
+      }
+      iu = u = n * (nv + 1);
+      ig = g = pow2 && n ? (n + 1) * (nv + 2) : 0u;
+      ip = p = pow2 && n ? n + 1 : 0u;
+    }
+    m = __shfl_sync(kFullR, n, 0) ? 1u : 0u;
+  }
+  if (lane < m) {
+    S.leaf[lane] = L;
+    S.k0[lane] = k0;
+    S.nu[lane] = nu;
+    S.nv[lane] = nv;
+    S.gpre[lane] = ig - g;
+    S.upre[lane] = iu - u;
+    S.rpre[lane] = ip - p;
+    if (lane == m - 1) {
+      S.gpre[m] = ig;
+      S.upre[m] = iu;
+      S.rpre[m] = ip;
+      S.next_row = first + n;
+      S.next_leaf = k0 + n == nu + 1 ? L + 1 : L;
+    }
+  }
+  if (lane == 0) {
+    S.nseg = m;
+    if (m == 0) {   // rows and leaves disagree (cannot happen): stop, never spin
+      S.gpre[0] = S.upre[0] = S.rpre[0] = 0;
+      S.next_row = r_end;
+    }
+  }
 }
 
 // Three CTAs per SM (at most 80 registers): the extra warps hide more of the
 // fixed-latency stalls than the few spilled values cost.
+//
+// SPARSE: a group takes the ids of all of its micropolygons when it starts (the
+// tables hold every micropolygon of the frame), and a covered cell is an atomic
+// right where it was tested.  Otherwise only micropolygons with a covered sample
+// get an id, by a block-wide scan, and their owners go over their covered cells
+// afterwards: for frames of so many micropolygons that ids or tables for all of
+// them would not fit.
+template <bool SPARSE>
 __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
 {
   pdl_wait();
@@ -1103,49 +1273,9 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
     if (row0 >= r_end) break;   // uniform
     __syncthreads();
     if (threadIdx.x < 32) {
-      const uint32_t L = leaf0 + threadIdx.x;
-      if (L < nleaf) {
-        S.wnu[threadIdx.x] = a.leaves[L].nu;
-        S.wnv[threadIdx.x] = a.leaves[L].nv;
-        S.wrb[threadIdx.x] = a.leaves[L].rowbase;
-      }
+      dice_group(a, S, leaf0, row0, nleaf, r_end);
       __syncwarp();
-      if (threadIdx.x == 0) {
-        // rows while the micropolygon budget and the shared grid points allow
-        uint32_t g = 0, u = 0, pr = 0, nseg = 0, leaf = leaf0, row = row0;
-        while (row < r_end && nseg < (uint32_t)kLeafBatch && leaf < nleaf && leaf - leaf0 < 32u) {
-          const uint32_t w = leaf - leaf0, nu = S.wnu[w], nv = S.wnv[w];
-          const uint32_t k0 = row - S.wrb[w];
-          const bool pow2 = ((nu & (nu - 1)) == 0) && ((nv & (nv - 1)) == 0);
-          uint32_t n = min(nu + 1 - k0, r_end - row);
-          n = min(n, ((uint32_t)kUpBudget - u) / (nv + 1));
-          if (pow2) {   // point rows that still fit
-            const uint32_t fit = min(((uint32_t)kMaxGridPts - g) / (nv + 2), (uint32_t)kMaxPtRows - pr);
-            n = min(n, fit > 0 ? fit - 1 : 0u);
-          }
-          if (n == 0) break;
-          S.leaf[nseg] = leaf;
-          S.k0[nseg] = k0;
-          S.nu[nseg] = nu;
-          S.nv[nseg] = nv;
-          S.gpre[nseg] = g;
-          S.upre[nseg] = u;
-          S.rpre[nseg] = pr;
-          g += pow2 ? (n + 1) * (nv + 2) : 0u;
-          pr += pow2 ? n + 1 : 0u;
-          u += n * (nv + 1);
-          ++nseg;
-          row += n;
-          if (k0 + n == nu + 1) ++leaf; else break;
-        }
-        if (nseg == 0) row = r_end;   // rows and leaves disagree (cannot happen): stop, never spin
-        S.gpre[nseg] = g;
-        S.upre[nseg] = u;
-        S.rpre[nseg] = pr;
-        S.nseg = nseg;
-        S.next_row = row;
-        S.next_leaf = leaf;
-      }
+      if (SPARSE && threadIdx.x == 0) S.gid = atomicAdd(&a.ctr->id_count, S.upre[S.nseg]);
     }
     __syncthreads();
     const int m = (int)S.nseg;
@@ -1156,10 +1286,15 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
     }
     __syncthreads();
     const uint32_t gtot = S.gpre[m], utot = S.upre[m], rtot = S.rpre[m];
-    for (uint32_t t = threadIdx.x; t < rtot; t += blockDim.x) {
+    // (a thread per control row of a point row)
+    for (uint32_t q = threadIdx.x; q < 4 * rtot; q += blockDim.x) {
+      const uint32_t t = q >> 2, c = q & 3u;
       const int i = batch_find(S.rpre, m, t);
       const uint32_t k = S.k0[i] + (t - S.rpre[i]);
-      dice_row(S.cp[i], (float)k * (1.0f / ((float)S.nu[i])), S.rowdat[t]);
+      const float u = (float)k * (1.0f / ((float)S.nu[i]));
+      const float4* P = &S.cp[i][4 * c];
+      S.rowdat[t].r[c] = bez(u, P[0], P[1], P[2], P[3]);
+      S.rowdat[t].d[c] = dbez(u, P[0], P[1], P[2], P[3]);
     }
     __syncthreads();
     for (uint32_t f = threadIdx.x; f < gtot; f += blockDim.x) {
@@ -1175,6 +1310,7 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
       UpolyRec o;
       int cnt = 0;          // cells to test
       uint32_t cwm = 0;
+      bool swap = false;
       int2 org = make_int2(0, 0);
       if (f < utot) {
         const int i = batch_find(S.upre, m, f);
@@ -1217,7 +1353,11 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
           const float mxx = std_maxf(std_maxf(o.sx[0], o.sx[1]), std_maxf(o.sx[2], o.sx[3]));
           const float mny = std_minf(std_minf(o.sy[0], o.sy[1]), std_minf(o.sy[2], o.sy[3]));
           const float mxy = std_maxf(std_maxf(o.sy[0], o.sy[1]), std_maxf(o.sy[2], o.sy[3]));
+          cwm = kBothWindings;
           if (exact_box(mnx, mxx, mny, mxy)) {
+            const float p = (o.sx[2] - o.sx[0]) * (o.sy[3] - o.sy[1]), q = (o.sx[3] - o.sx[1]) * (o.sy[2] - o.sy[0]);
+            if (p != q) cwm = 0u;
+            swap = p < q;
             if (r == 1) {   // centre x + 0.5 strictly inside (mnx, mxx)
               cx0 = max(cx0, (int)floorf(mnx - 0.5f) + 1); cx1 = min(cx1, (int)ceilf(mxx - 0.5f) - 1);
               cy0 = max(cy0, (int)floorf(mny - 0.5f) + 1); cy1 = min(cy1, (int)ceilf(mxy - 0.5f) - 1);
@@ -1229,13 +1369,20 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
           const int cw = cx1 - cx0 + 1, ch = cy1 - cy0 + 1;
           if (cw > 0 && ch > 0) {
             cnt = cw * ch;
-            cwm = (uint32_t)cw | ((0x10000u / (uint32_t)cw + 1u) << 7);
+            cwm |= (uint32_t)cw | ((0x10000u / (uint32_t)cw + 1u) << 7);
             org = make_int2(cx0, cy0);
-            S.ux[threadIdx.x] = make_float4(o.sx[0], o.sx[1], o.sx[2], o.sx[3]);
-            S.uy[threadIdx.x] = make_float4(o.sy[0], o.sy[1], o.sy[2], o.sy[3]);
+            // (the test of both windings takes the corners as they are)
+            const bool rev = swap && !(cwm & kBothWindings);
+            S.ux[threadIdx.x] = make_float4(o.sx[0], rev ? o.sx[3] : o.sx[1], o.sx[2], rev ? o.sx[1] : o.sx[3]);
+            S.uy[threadIdx.x] = make_float4(o.sy[0], rev ? o.sy[3] : o.sy[1], o.sy[2], rev ? o.sy[1] : o.sy[3]);
             S.org[threadIdx.x] = org;
             S.cwm[threadIdx.x] = cwm;
-            S.mask[threadIdx.x] = 0ull;
+            if (SPARSE) {
+              S.zo[threadIdx.x] = o.z <= 1.0f ? zorder(o.z) : kNoDepth;   // (a NaN depth never survives)
+              if (o.z <= 1.0f) put_id(a, S.gid + f, o);
+            } else {
+              S.mask[threadIdx.x] = 0ull;
+            }
           }
         }
       }
@@ -1248,9 +1395,31 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
         for (int c = lo; c < hi; ++c) S.cell[pre + (uint32_t)c - w0] = (uint16_t)((threadIdx.x << 6) | (uint32_t)c);
         __syncthreads();
         const uint32_t nw = min((uint32_t)kCellCap, total - w0);
-        for (uint32_t q = threadIdx.x; q < nw; q += blockDim.x) dice_cell(a, S, q);
+        // an atomic's answer is looked at after the next one is on its way
+        unsigned long long old = kSampEmpty;
+        uint32_t o_at = 0, o_zo = 0, o_id = 0;   // (no depth code is 0)
+        for (uint32_t q = threadIdx.x; q < nw; q += blockDim.x) {
+          int u, li, x, y, smp;
+          if (!dice_cell(a, S, q, u, li, x, y, smp)) continue;
+          if (!SPARSE) {
+            atomicOr(&S.mask[u], 1ull << li);
+            continue;
+          }
+          ++covered;
+          const uint32_t zo = S.zo[u];
+          if (zo == kNoDepth) continue;
+          const uint32_t id = S.gid + f0 + (uint32_t)u, at = sample_index(a, x, y, smp);
+          const unsigned long long got = atomicMin(&a.samp[at], ((unsigned long long)zo << 32) | id);
+          if (o_zo) check_tie(a, &S.ties, o_at, o_zo, o_id, old);
+          old = got;
+          o_at = at;
+          o_zo = zo;
+          o_id = id;
+        }
+        if (SPARSE && o_zo) check_tie(a, &S.ties, o_at, o_zo, o_id, old);
         __syncthreads();
       }
+      if (SPARSE) continue;
       unsigned long long mask = cnt > 0 ? S.mask[threadIdx.x] : 0ull;
       covered += __popcll(mask);
       if (cnt > 0 && !(o.z <= 1.0f)) mask = 0;  // behind the cleared depth (or NaN): never survives
@@ -1258,26 +1427,15 @@ __global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
       if (mask) {
         put_id(a, id, o);
         const uint32_t zo = zorder(o.z);
-        const bool zero = o.z == 0.0f;
-        const unsigned long long st = ((unsigned long long)zo << 32) | id;
-        // an atomic's answer is looked at after the next one is on its way
-        unsigned long long old = kSampEmpty;
-        uint32_t at = 0;
-        bool first = true;
         while (mask) {
           const int c = __ffsll(mask) - 1;
           mask &= mask - 1;
           int cx, cy;
           cell_xy(cwm, org, c, cx, cy);
-          const uint32_t p = r == 1 ? sample_index(a, cx, cy, 0)
-                                    : sample_index(a, cx >> 1, cy >> 1, (cx & 1) | ((cy & 1) << 1));
-          const unsigned long long got = atomicMin(&a.samp[p], st);
-          if (!first) check_tie(a, &S.ties, at, zo, id, zero, old);
-          first = false;
-          old = got;
-          at = p;
+          const uint32_t at = r == 1 ? sample_index(a, cx, cy, 0)
+                                     : sample_index(a, cx >> 1, cy >> 1, (cx & 1) | ((cy & 1) << 1));
+          check_tie(a, &S.ties, at, zo, id, atomicMin(&a.samp[at], ((unsigned long long)zo << 32) | id));
         }
-        check_tie(a, &S.ties, at, zo, id, zero, old);
       }
     }
   }
@@ -1325,7 +1483,7 @@ __global__ void __launch_bounds__(256) reyes_big(ReyesArgs a)
       }
       if ((keep >> lane) & 1u) {
         const uint32_t p = sample_index(a, x, y, smp);
-        check_tie(a, nullptr, p, zo, id, u.z == 0.0f, atomicMin(&a.samp[p], ((unsigned long long)zo << 32) | id));
+        check_tie(a, nullptr, p, zo, id, atomicMin(&a.samp[p], ((unsigned long long)zo << 32) | id));
       }
     }
   }
@@ -1340,29 +1498,31 @@ __global__ void __launch_bounds__(256) reyes_ties(ReyesArgs a)
 {
   pdl_wait();
   pdl_trigger();
+  const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  // the first record is read along with the counters (tie_cap is at least the grid)
+  uint4 t = a.ties[min(first, a.tie_cap - 1)];
   const uint32_t n = min(a.ctr->tie_count, a.tie_cap);
   // after an overflow of the tables the frame runs again: no key to look up
-  if (a.ctr->id_count > a.id_cap) return;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint4 t = a.ties[i];
-    if ((uint32_t)(__ldcg(&a.samp[t.x]) >> 32) != t.y) continue;   // (this pass changes no depth)
-    const uint32_t ids[2] = {t.z, t.w};
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const unsigned long long key = a.id_key[ids[k]], mine = ((unsigned long long)t.y << 32) | ids[k];
-      unsigned long long cur = __ldcg(&a.samp[t.x]);
-      while (key > a.id_key[(uint32_t)cur]) {   // (the key kept only grows)
-        const unsigned long long was = atomicCAS(&a.samp[t.x], cur, mine);
-        if (was == cur) break;
-        cur = was;
-      }
-      if (zorder_inv(t.y) != 0.0f) continue;
-      uint32_t f = __ldcg(&a.first0[t.x]);
-      while (f == kNoId || key < a.id_key[f]) {   // (the key kept only falls)
-        const uint32_t was = atomicCAS(&a.first0[t.x], f, ids[k]);
-        if (was == f) break;
-        f = was;
-      }
+  if (a.ctr->fc.status & kStatusListOverflow) return;
+  for (uint32_t i = first; i < n; i += stride, t = a.ties[min(i, a.tie_cap - 1)]) {
+    unsigned long long cur = __ldcg(&a.samp[t.x]);
+    const unsigned long long key_z = a.id_key[t.z], key_w = a.id_key[t.w];
+    if ((uint32_t)(cur >> 32) != t.y) continue;   // (this pass changes no depth)
+    const unsigned long long key = key_z > key_w ? key_z : key_w;
+    const unsigned long long mine = ((unsigned long long)t.y << 32) | (key_z > key_w ? t.z : t.w);
+    while (cur != mine && key > a.id_key[(uint32_t)cur]) {   // (the key kept only grows)
+      const unsigned long long was = atomicCAS(&a.samp[t.x], cur, mine);
+      if (was == cur) break;
+      cur = was;
+    }
+    if (t.y != 0x80000000u) continue;   // zorder(+-0)
+    const uint32_t low = key_z < key_w ? t.z : t.w;
+    const unsigned long long low_key = key_z < key_w ? key_z : key_w;
+    uint32_t f = __ldcg(&a.first0[t.x]);
+    while (f == kNoId || low_key < a.id_key[f]) {   // (the key kept only falls)
+      const uint32_t was = atomicCAS(&a.first0[t.x], f, low);
+      if (was == f) break;
+      f = was;
     }
   }
 }
@@ -1390,24 +1550,50 @@ __device__ __forceinline__ bool take_sample(const ReyesArgs& a, size_t si, unsig
 // samples: a pixel takes the rounded mean of its samples' colours per channel
 // and the depth of its nearest sample (the first such sample on ties).  Every
 // reached sample's state is set back to empty, so the next frame finds it so.
+//
+// The counters are final: block 0 hands them to the host and leaves them zero
+// for the next frame, so that no memset precedes a frame and no copy follows it
+// (together 7 us of a 320x240 sphere's 52).
 __global__ void __launch_bounds__(256) reyes_pixels(ReyesArgs a, uint32_t npx)
 {
   pdl_wait();
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < npx; i += gridDim.x * blockDim.x) {
-    if (a.spp == 1) {
-      const unsigned long long st = a.samp[i];
+  static_assert(sizeof(ReyesCounters) % 4 == 0 && sizeof(ReyesCounters) / 4 <= 256, "a word per thread");
+  if (blockIdx.x == 0 && threadIdx.x < sizeof(ReyesCounters) / 4) {
+    uint32_t* c = reinterpret_cast<uint32_t*>(a.ctr) + threadIdx.x;
+    reinterpret_cast<uint32_t*>(a.host_ctr)[threadIdx.x] = *c;
+    *c = 0u;
+  }
+  const uint32_t stride = gridDim.x * blockDim.x;
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a.spp == 1) {
+    // (the next pixel's state is on its way while this one's colour is fetched)
+    unsigned long long next = i < npx ? a.samp[i] : kSampEmpty;
+    for (; i < npx; i += stride) {
+      const unsigned long long st = next;
+      if (i + stride < npx) next = a.samp[i + stride];
       uint32_t c;
       float z;
       if (take_sample(a, i, st, c, z)) a.samp[i] = kSampEmpty;
       a.fb[i] = c;
       a.depth[i] = z;
-      continue;
     }
-    // four samples: 32 contiguous, aligned bytes; a pixel with any reached
-    // sample has all four set back
+    return;
+  }
+  // four samples: 32 contiguous, aligned bytes; a pixel with any reached sample
+  // has all four set back
+  ulonglong2 nlo = make_ulonglong2(kSampEmpty, kSampEmpty), nhi = nlo;
+  if (i < npx) {
+    const ulonglong2* sp = reinterpret_cast<const ulonglong2*>(&a.samp[4 * (size_t)i]);
+    nlo = sp[0];
+    nhi = sp[1];
+  }
+  for (; i < npx; i += stride) {
     ulonglong2* sp = reinterpret_cast<ulonglong2*>(&a.samp[4 * (size_t)i]);
-    const ulonglong2 lo = sp[0], hi = sp[1];
-    const unsigned long long st[4] = {lo.x, lo.y, hi.x, hi.y};
+    const unsigned long long st[4] = {nlo.x, nlo.y, nhi.x, nhi.y};
+    if (i + stride < npx) {
+      nlo = sp[2 * (size_t)stride];
+      nhi = sp[2 * (size_t)stride + 1];
+    }
     uint32_t c[4] = {kClearColor, kClearColor, kClearColor, kClearColor};
     float z[4] = {1.0f, 1.0f, 1.0f, 1.0f};
     if ((st[0] & st[1] & st[2] & st[3]) != kSampEmpty) {
@@ -1451,7 +1637,7 @@ static cudaError_t launch_chained(void (*kernel)(KArgs...), int grid, int block,
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-cudaError_t launch_reyes_frame(const ReyesArgs& a, uint32_t npx, int sms, cudaStream_t st, cudaEvent_t* ev)
+cudaError_t launch_reyes_frame(const ReyesArgs& a, uint32_t npx, int sms, bool sparse, cudaStream_t st, cudaEvent_t* ev)
 {
   // occupancies, found once per process (host threads may launch frames
   // concurrently; call_once makes the others wait for the first)
@@ -1464,8 +1650,9 @@ cudaError_t launch_reyes_frame(const ReyesArgs& a, uint32_t npx, int sms, cudaSt
     if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sp, reyes_split, kSplitThreads, kSplitSmem);
     // the split's grid barriers need every CTA resident: one per SM
     if (!e && sp < 1) e = cudaErrorCooperativeLaunchTooLarge;
-    if (!e) e = cudaFuncSetAttribute(reyes_dice, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiceSmem);
-    if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dp, reyes_dice, kDiceThreads, kDiceSmem);
+    if (!e) e = cudaFuncSetAttribute(reyes_dice<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiceSmem);
+    if (!e) e = cudaFuncSetAttribute(reyes_dice<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiceSmem);
+    if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dp, reyes_dice<true>, kDiceThreads, kDiceSmem);
     setup_err = e;
     dice_per_sm = std::max(1, dp);
   });
@@ -1480,7 +1667,7 @@ cudaError_t launch_reyes_frame(const ReyesArgs& a, uint32_t npx, int sms, cudaSt
   // the launches after the split may start while their predecessor drains
   // (programmatic dependent launch); each waits for it before touching memory
   const int grid = sms * 8;
-  e = launch_chained(reyes_dice, sms * dice_per_sm, kDiceThreads, kDiceSmem, st, a);
+  e = launch_chained(sparse ? reyes_dice<true> : reyes_dice<false>, sms * dice_per_sm, kDiceThreads, kDiceSmem, st, a);
   if (!e) e = launch_chained(reyes_big, grid, 256, 0, st, a);
   if (ev) cudaEventRecord(ev[2], st);
   if (!e) e = launch_chained(reyes_ties, sms * 4, 256, 0, st, a);
@@ -1513,9 +1700,11 @@ struct ReyesState {
   unsigned long long* samp = nullptr;
   uint32_t* first0 = nullptr;
   size_t npx_cap = 0;   // samples
+  bool sparse = true;   // an id for every micropolygon (reyes_dice); of a scene, not of borrowed buffers
   bool clean = false;   // per-sample state all empty (set when allocated; every frame leaves it so)
   ReyesCounters* ctr = nullptr;
-  ReyesCounters* h_ctr = nullptr;
+  ReyesCounters* h_ctr = nullptr;   // pinned, written by reyes_pixels
+  bool ctr_clean = false;
   cudaEvent_t ev[5] = {};
   bool ev_made = false;
 };
@@ -1546,6 +1735,8 @@ void reyes_borrow_buffers(piko_scene* s, ReyesState* b)
   if (!s->reyes) s->reyes = new ReyesState();
   s->reyes->buffers = b;
 }
+
+constexpr uint32_t kMaxSparse = 1u << 28;
 
 static cudaError_t reyes_alloc(ReyesState* r, uint32_t lvl_cap, uint32_t leaf_cap, uint32_t up_cap, uint32_t id_cap,
                                uint32_t tie_cap, size_t npx)
@@ -1615,10 +1806,16 @@ piko_status piko_reyes_run(piko_scene* s, cudaStream_t st, bool timed)
   const size_t nsamp = npx * (size_t)p->samples_per_pixel;
   CU(ctx, reyes_alloc(r, std::max<uint32_t>(1u << 16, 64u * P), std::max<uint32_t>(1u << 16, 64u * P),
                       b->up_cap ? b->up_cap : (1u << 16),
-                      b->id_cap ? b->id_cap : (uint32_t)std::max<size_t>(1u << 18, npx / 2),
+                      b->id_cap ? b->id_cap : (uint32_t)std::max<size_t>(1u << 20, npx),
                       b->tie_cap ? b->tie_cap : (uint32_t)std::max<size_t>(1u << 18, nsamp / 8), nsamp));
   if (!b->stack) CU(ctx, dalloc(&b->stack, (size_t)ctx->sms * kSplitStack));
-  CU(ctx, cudaMemsetAsync(r->ctr, 0, sizeof(ReyesCounters), st));
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CU(ctx, cudaStreamIsCapturing(st, &capture));
+  const bool ran = capture == cudaStreamCaptureStatusNone;   // (what a capture records has not run yet)
+  if (!r->ctr_clean) {   // fresh, or a frame whose launches failed part way
+    CU(ctx, cudaMemsetAsync(r->ctr, 0, sizeof(ReyesCounters), st));
+    r->ctr_clean = ran;
+  }
   ReyesArgs a;
   memset(&a, 0, sizeof(a));
   a.W = s->W; a.H = s->H; a.nBx = s->W / 64; a.nBy = s->H / 64;
@@ -1636,6 +1833,7 @@ piko_status piko_reyes_run(piko_scene* s, cudaStream_t st, bool timed)
   a.id_color = b->id_color; a.id_key = b->id_key; a.id_cap = b->id_cap;
   a.ties = b->ties; a.tie_cap = b->tie_cap;
   a.ctr = r->ctr;
+  a.host_ctr = r->h_ctr;
   a.fb = s->fb; a.depth = s->depth;
   a.samp = b->samp; a.first0 = b->first0;
   a.spp = p->samples_per_pixel;
@@ -1645,10 +1843,10 @@ piko_status piko_reyes_run(piko_scene* s, cudaStream_t st, bool timed)
     // fresh sample buffers, or a frame whose launches failed part way
     CU(ctx, cudaMemsetAsync(b->samp, 0xff, sizeof(unsigned long long) * b->npx_cap, st));
     CU(ctx, cudaMemsetAsync(b->first0, 0xff, sizeof(uint32_t) * b->npx_cap, st));
-    b->clean = true;
+    b->clean = ran;
   }
-  const cudaError_t le = launch_reyes_frame(a, (uint32_t)npx, ctx->sms, st, timed ? r->ev : nullptr);
-  if (le != cudaSuccess) b->clean = false;
+  const cudaError_t le = launch_reyes_frame(a, (uint32_t)npx, ctx->sms, r->sparse, st, timed ? r->ev : nullptr);
+  if (le != cudaSuccess) b->clean = r->ctr_clean = false;
   CU(ctx, le);
   return PIKO_OK;
 }
@@ -1659,7 +1857,6 @@ piko_status piko_reyes_finish(piko_scene* s)
   ReyesState* r = s->reyes;
   if (!r) { s->pending = false; return PIKO_OK; }
   for (int attempt = 0; attempt < 6; ++attempt) {
-    CU(ctx, cudaMemcpyAsync(r->h_ctr, r->ctr, sizeof(ReyesCounters), cudaMemcpyDeviceToHost, s->last_stream));
     CU(ctx, cudaStreamSynchronize(s->last_stream));
     const ReyesCounters& c = *r->h_ctr;
     const uint32_t st = c.fc.status;
@@ -1678,7 +1875,13 @@ piko_status piko_reyes_finish(piko_scene* s)
     const auto more = [](uint32_t n) {   // (an id of kNoId means none)
       return (uint32_t)std::min<unsigned long long>(n + n / 4ull + 4096, 0xfffffffeull);
     };
-    if (c.id_count > ids) ids = more(c.id_count);
+    // ids for all micropolygons while their tables stay below 3 GB
+    // (the first frame without them then tells how many it needs)
+    const bool was_sparse = r->sparse;
+    if (c.upolys > kMaxSparse) r->sparse = false;
+    const uint32_t need_ids = r->sparse ? (uint32_t)c.upolys + std::min(c.big_count, kMaxSparse)
+                                        : was_sparse ? ids : c.id_count;
+    if (need_ids > ids) ids = more(need_ids);
     if (c.tie_count > ties) ties = more(c.tie_count);
     CU(ctx, reyes_alloc(r, lvl, lf, up, ids, ties, b->npx_cap));
     piko_status rr = piko_reyes_run(s, s->last_stream, s->timed);
@@ -1721,8 +1924,6 @@ piko_status piko_reyes_stats(piko_scene* s, piko_frame_stats* o)
 {
   ReyesState* r = s->reyes;
   if (!r || !r->h_ctr) return PIKO_OK;
-  piko_ctx* ctx = s->pipe->ctx;
-  CU(ctx, cudaMemcpy(r->h_ctr, r->ctr, sizeof(ReyesCounters), cudaMemcpyDeviceToHost));
   const ReyesCounters& c = *r->h_ctr;
   o->prims_in = (uint64_t)s->N;
   o->prims_kept = c.leaf_meta >> 40;
