@@ -1736,7 +1736,7 @@ void reyes_borrow_buffers(piko_scene* s, ReyesState* b)
   s->reyes->buffers = b;
 }
 
-constexpr uint32_t kMaxSparse = 1u << 28;
+constexpr uint32_t kMaxSparse = 1u << 24;
 
 static cudaError_t reyes_alloc(ReyesState* r, uint32_t lvl_cap, uint32_t leaf_cap, uint32_t up_cap, uint32_t id_cap,
                                uint32_t tie_cap, size_t npx)
@@ -1875,7 +1875,7 @@ piko_status piko_reyes_finish(piko_scene* s)
     const auto more = [](uint32_t n) {   // (an id of kNoId means none)
       return (uint32_t)std::min<unsigned long long>(n + n / 4ull + 4096, 0xfffffffeull);
     };
-    // ids for all micropolygons while their tables stay below 3 GB
+    // ids for all micropolygons while their tables stay below 200 MB
     // (the first frame without them then tells how many it needs)
     const bool was_sparse = r->sparse;
     if (c.upolys > kMaxSparse) r->sparse = false;
