@@ -46,11 +46,9 @@ constexpr size_t kOffSetup = align256(kOffCtr + sizeof(FrameCounters));
 constexpr size_t kOffLargeSeg = align256(kOffSetup + sizeof(TriSetup) * kNaMaxTris);
 constexpr size_t kOffLargeWalk = align256(kOffLargeSeg + sizeof(uint2) * kNaMaxSegs);
 constexpr size_t kOffCnt = align256(kOffLargeWalk + sizeof(WalkTri) * kNaMaxBig);
-constexpr size_t kOffOff = align256(kOffCnt + sizeof(uint32_t) * kNaMaxTiles);
-constexpr size_t kOffHeavy = align256(kOffOff + sizeof(uint32_t) * (kNaMaxTiles + 1));
-constexpr size_t kOffFlags = align256(kOffHeavy + sizeof(uint32_t) * kNaMaxTiles);
-constexpr uint32_t kNaScanBlocks = (kNaMaxTiles + kScanTile - 1) / kScanTile;
-constexpr size_t kOffList = align256(kOffFlags + sizeof(unsigned long long) * kNaScanBlocks);
+constexpr size_t kOffSpan = align256(kOffCnt + sizeof(uint32_t) * kNaMaxTiles);
+constexpr size_t kOffHeavy = align256(kOffSpan + sizeof(uint2) * kNaMaxTiles);
+constexpr size_t kOffList = align256(kOffHeavy + sizeof(uint32_t) * kNaMaxTiles);
 constexpr size_t kOffPairTl = align256(kOffList + sizeof(uint32_t) * kNaMaxList);
 constexpr size_t kOffPairG = align256(kOffPairTl + sizeof(unsigned long long) * kNaMaxList);
 constexpr size_t kArenaBytes = align256(kOffPairG + sizeof(uint32_t) * kNaMaxList);
@@ -108,8 +106,7 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
 
   // the arena keeps the previous call's contents: zero what must start at zero
   if (cudaMemsetAsync(base + kOffWork, 0, sizeof(BinWork), st) != cudaSuccess ||
-      cudaMemsetAsync(base + kOffCnt, 0, sizeof(uint32_t) * n_tiles, st) != cudaSuccess ||
-      cudaMemsetAsync(base + kOffFlags, 0, sizeof(unsigned long long) * kNaScanBlocks, st) != cudaSuccess)
+      cudaMemsetAsync(base + kOffCnt, 0, sizeof(uint32_t) * n_tiles, st) != cudaSuccess)
     return PIKO_ERR_CUDA;
 
   RasterFrameArgs a;
@@ -124,7 +121,7 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
   a.n_tiles_total = n_tiles;
   a.setup = reinterpret_cast<TriSetup*>(base + kOffSetup);
   a.tile_cnt = reinterpret_cast<uint32_t*>(base + kOffCnt);
-  a.tile_off = reinterpret_cast<uint32_t*>(base + kOffOff);
+  a.tile_span = reinterpret_cast<uint2*>(base + kOffSpan);
   a.tile_list = reinterpret_cast<uint32_t*>(base + kOffList);
   a.pair_tl = reinterpret_cast<unsigned long long*>(base + kOffPairTl);
   a.pair_g = reinterpret_cast<uint32_t*>(base + kOffPairG);
@@ -137,7 +134,6 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
   a.seg_cap = kNaMaxSegs;
   a.large_walk = reinterpret_cast<WalkTri*>(base + kOffLargeWalk);
   a.big_cap = kNaMaxBig;
-  a.scan_flags = reinterpret_cast<unsigned long long*>(base + kOffFlags);
   a.work = reinterpret_cast<BinWork*>(base + kOffWork);
   a.ctr = reinterpret_cast<FrameCounters*>(base + kOffCtr);
   if (launch_raster_frame(a, ctas, st, nullptr) != cudaSuccess) return PIKO_ERR_CUDA;
@@ -148,7 +144,6 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
   if (cudaMemcpyAsync(&c, base + kOffCtr, sizeof(c), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return PIKO_ERR_CUDA;
-  if (c.bin.status & kStatusScanTimeout) return PIKO_ERR_TIMEOUT;
   // (the documented limit counts every queue entry, listed here or not)
   if ((c.bin.status & kStatusListOverflow) || c.bin.list_total + c.bin.skipped > kNaMaxList) return PIKO_ERR_QUEUE_OVERFLOW;
   return PIKO_OK;

@@ -54,7 +54,6 @@ __host__ __device__ __forceinline__ uint32_t tile_chunks(uint32_t cnt, uint32_t 
 
 // frame status bits (the C ABI maps them to piko_status)
 constexpr uint32_t kStatusListOverflow = 1u << 0;
-constexpr uint32_t kStatusScanTimeout = 1u << 1;
 constexpr uint32_t kStatusUpolyOverflow = 1u << 2;
 constexpr uint32_t kStatusPatchOverflow = 1u << 3;
 constexpr uint32_t kStatusDepthNeverSettles = 1u << 4;
@@ -203,13 +202,11 @@ struct FrameCounters {
 // scene-record copy and three memsets that used to precede the setup kernel
 // took 15 us of a frame, a fifth of the 1080p forest's): they are zero between
 // frames because a later kernel of the frame sets back what an earlier one
-// used -- raster_scatter the counts and the scan's flags, the fragment kernels
-// the pair partitions, scan_tiles the tile counters it has read.  The host
+// used -- raster_scatter the counts, the fragment kernels the pair partitions,
+// scan_tiles the tile counters it has read.  The host
 // clears them when they are allocated and after a launch that failed.
 struct BinWork {
   BinCounts bin;
-  uint32_t scan_ticket;
-  uint32_t pad[3];
   // The count passes record their (triangle, tile) pairs in kPairParts
   // partitions of list_cap / kPairParts slots each (chosen by block and warp),
   // so that slot reservations spread over kPairParts counters instead of
@@ -261,7 +258,7 @@ struct RasterFrameArgs {
   uint32_t batch;           // triangles a raster_setup CTA takes at a time (set by the launch)
   TriSetup* setup;          // [n_tris_total]; written only for triangles that reach a bin (rank1 != 0)
   uint32_t* tile_cnt;       // [n_tiles_total]
-  uint32_t* tile_off;       // [n_tiles_total + 1]
+  uint2* tile_span;         // [n_tiles_total] first list entry, entries
   uint32_t* tile_list;      // [list_cap]
   uint32_t list_cap;
   uint32_t* heavy;          // [heavy_cap] heavy tiles, when there are no chunk buffers
@@ -291,7 +288,6 @@ struct RasterFrameArgs {
   uint32_t* hdone;          // [key_cap][bins per tile] finished chunks, at a tile's first key slot
   unsigned long long* chunk_keys;  // [key_cap][tile * tile]
   uint32_t key_cap;
-  unsigned long long* scan_flags;  // per scan block
   BinWork* work;
   FrameCounters* ctr;
   BinCounts* host_bin;      // pinned host memory (or null): the fragment kernel leaves ctr->bin there, so that

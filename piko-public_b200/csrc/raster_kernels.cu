@@ -12,8 +12,7 @@
 //                   record.  Triangles with more than 256 box tiles are queued
 //                   as 128-tile segments for
 //   raster_large_count, which walks them the same way over the whole grid.
-//   scan_tiles      exclusive prefix sum of the tile counts (single pass,
-//                   decoupled look-back) -> per-tile list offsets.  Tiles with
+//   scan_tiles      tile counts -> each tile's place in the lists.  Tiles with
 //                   long lists are queued as chunks of list entries.
 //   raster_scatter  a streaming pass over the pair records: each becomes its
 //                   list entry at its tile's offset plus its index (no walk, no
@@ -803,23 +802,19 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(const __grid_const
 }
 
 // ------------------------------------------------------------------ kernel 2
-// Exclusive scan of tile_cnt (decoupled look-back); the counters are set back
-// to 0 as they are read.  Flags per block hold (state << 32) | value, state
-// 1 = aggregate, 2 = inclusive.
-
+// Gives every tile its place in the tile lists: a scan within the block, and one
+// atomic for the block's share of the lists.  The lists' order means nothing, so
+// the blocks need not wait for one another (a decoupled look-back took 1 to 2 us
+// of the frame).  The tile counters are set back to 0 as they are read.
 __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_wait();
   pdl_trigger();
-  __shared__ uint32_t s_bid;
   __shared__ uint32_t s_warp[kScanThreads / 32];
-  __shared__ uint32_t s_prefix;
+  __shared__ uint32_t s_first;
   __shared__ unsigned long long s_heavy[kScanThreads / 32];   // per warp: (key slots << 32) | items
-  if (threadIdx.x == 0) s_bid = atomicAdd(&a.work->scan_ticket, 1u);
-  __syncthreads();
-  const uint32_t bid = s_bid;
   const uint32_t n = a.n_tiles_total;
-  const uint32_t base = bid * kScanTile + threadIdx.x * kScanItems;
+  const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
   uint32_t sum = 0;
 #pragma unroll
@@ -838,7 +833,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
   // Heavy tiles (lists longer than queue_min) become items of the fragment
   // kernel's queue -- their chunks, or without chunk buffers the tiles -- and
   // the chunks of lists in several chunks need key slots: counted now, reserved
-  // below with one atomic per block while warp 0 looks back
+  // below with one atomic per block
   const bool t8 = a.tile == kRefBin;
   const bool chunked = a.chunk_desc != nullptr;
   const uint32_t thr = a.queue_min, bins = (uint32_t)(a.tile / kRefBin) * (uint32_t)(a.tile / kRefBin);
@@ -881,54 +876,21 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
     if (w < warp) warp_excl += s_warp[w];
     agg += s_warp[w];
   }
-  if (warp == 0) {
-    // Look-back by the whole warp: lane j reads the flag of block
-    // (end - j), so 32 predecessors are examined per step.  The window is
-    // summed once every lane up to the nearest inclusive prefix is published.
-    uint32_t prefix = 0;
-    if (bid == 0) {
-      if (lane == 0) atomicExch(&a.scan_flags[0], (2ull << 32) | agg);
-    } else {
-      if (lane == 0) atomicExch(&a.scan_flags[bid], (1ull << 32) | agg);
-      int end = (int)bid - 1;
-      uint32_t spins = 0;
-      for (;;) {
-        const int idx = end - lane;
-        uint32_t state = 2, val = 0;  // lanes before block 0 read as an inclusive 0
-        if (idx >= 0) {
-          const unsigned long long f = __ldcv(&a.scan_flags[idx]);
-          state = (uint32_t)(f >> 32) & 3u;
-          val = (uint32_t)f;
-        }
-        const unsigned pending = __ballot_sync(kFull, state == 0);
-        const unsigned inclusive = __ballot_sync(kFull, state == 2);
-        const int first = inclusive ? __ffs(inclusive) - 1 : 31;
-        const unsigned need = first == 31 ? kFull : ((2u << first) - 1u);
-        if (pending & need) {
-          if (++spins > (1u << 22)) {
-            if (lane == 0) atomicOr(&a.work->bin.status, kStatusScanTimeout);
-            break;
-          }
-          __nanosleep(32);
-          continue;
-        }
-        prefix += __reduce_add_sync(kFull, lane <= first ? val : 0u);
-        if (inclusive) break;
-        end -= 32;
-      }
-      if (lane == 0) atomicExch(&a.scan_flags[bid], (2ull << 32) | (uint32_t)(prefix + agg));
-    }
-    if (lane == 0) s_prefix = prefix;
+  if (threadIdx.x == 0) {
+    const uint32_t first = agg ? atomicAdd(&a.work->bin.list_total, agg) : 0u;
+    // (a total past 32 bits is past the capacity before it wraps)
+    if (first + agg > a.list_cap || first + agg < first) atomicOr(&a.work->bin.status, kStatusListOverflow);
+    s_first = first;
   }
   __syncthreads();
-  uint32_t run = s_prefix + warp_excl + (incl - sum);
+  uint32_t run = s_first + warp_excl + (incl - sum);
   const unsigned long long old = s_heavy[warp];
   uint32_t ks = (uint32_t)(old >> 32) + ki - nk;
   uint32_t c = (uint32_t)old + ci - nc;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     if (base + i < n) {
-      a.tile_off[base + i] = run;
+      a.tile_span[base + i] = make_uint2(run, v[i]);
       if (v[i] > thr) {
         if (chunked) {
           const uint32_t ce = tile_chunk_entries(v[i], a.chunk, t8), nch = (v[i] + ce - 1) / ce;
@@ -951,12 +913,6 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const __grid_constant
       }
     }
     run += v[i];
-  }
-  if (base < n && base + kScanItems >= n) {
-    // the thread holding the last element publishes the total
-    a.tile_off[n] = run;
-    a.work->bin.list_total = run;
-    if (run > a.list_cap) atomicOr(&a.work->bin.status, kStatusListOverflow);
   }
 }
 
@@ -1013,25 +969,21 @@ __global__ void __launch_bounds__(256, 4) raster_large_count(const __grid_consta
 }
 
 // The scatter pass (the compaction): every recorded pair becomes its list
-// entry at tile_off[tile] + its index in the tile, a streaming pass with no
+// entry at its tile's first entry + its index in the tile, a streaming pass with no
 // atomics; four pairs per thread per trip, loads first.
 __global__ void __launch_bounds__(256) raster_scatter(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_wait();
   pdl_trigger();
   // the counts are final: they become the frame's result, and the next frame
-  // finds the working counters and the scan's flags at 0
+  // finds the working counters at 0
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.ctr->bin = a.work->bin;
     a.ctr->covered = 0ull;
     a.ctr->work_next = 0u;
     a.ctr->cov_count = 0u;
     a.work->bin = BinCounts{};
-    a.work->scan_ticket = 0u;
   }
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (a.n_tiles_total + kScanTile - 1) / kScanTile;
-       i += gridDim.x * blockDim.x)
-    a.scan_flags[i] = 0ull;
   // gridDim.x is a multiple of kPairParts: every partition gets
   // gridDim.x / kPairParts CTAs
   const uint32_t p = blockIdx.x % kPairParts, sub = blockIdx.x / kPairParts;
@@ -1051,7 +1003,7 @@ __global__ void __launch_bounds__(256) raster_scatter(const __grid_constant__ Ra
     }
     uint32_t off[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) off[q] = tl[q] != ~0ull ? a.tile_off[(uint32_t)tl[q]] : 0u;
+    for (int q = 0; q < 4; ++q) off[q] = tl[q] != ~0ull ? a.tile_span[(uint32_t)tl[q]].x : 0u;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (tl[q] == ~0ull) continue;
@@ -1555,7 +1507,7 @@ __global__ void __launch_bounds__(256, 4) raster_frag8(const __grid_constant__ R
   const uint32_t n_groups = (a.n_tiles_total + a.group - 1) / a.group;
   const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
   uint32_t g = blockIdx.x * (blockDim.x >> 5) + (uint32_t)wid;   // the next group
-  // The group being drawn: tiles t0 + ja .. t0 + nt remain; lane j <= nt holds
+  // The group being drawn: tiles t0 + ja .. t0 + nt remain; lane j < nt holds
   // the offset, the entries (0 when it is served as chunks) and the inclusive
   // prefix of tile t0 + j.
   uint32_t t0 = 0, off_j = 0, cnt_j = 0, incl_j = 0;
@@ -1577,8 +1529,9 @@ __global__ void __launch_bounds__(256, 4) raster_frag8(const __grid_constant__ R
         nt = (int)min(a.group, a.n_tiles_total - t0);
         g += nwarps;
         ja = 0;
-        off_j = lane <= nt ? a.tile_off[t0 + lane] : 0u;
-        cnt_j = __shfl_down_sync(kFull, off_j, 1) - off_j;
+        const uint2 span = lane < nt ? a.tile_span[t0 + lane] : make_uint2(0u, 0u);
+        off_j = span.x;
+        cnt_j = span.y;
         const bool fits = lane < nt && cnt_j <= a.queue_min;
         if (!fits) cnt_j = 0;
         served = __ballot_sync(kFull, fits);
@@ -1742,8 +1695,9 @@ __global__ void __launch_bounds__(256, 4) raster_bins(const __grid_constant__ Ra
       tile = g / parts;
       quad = g % parts;
       g += nwarps;
-      off = a.tile_off[tile];
-      len = a.tile_off[tile + 1] - off;
+      const uint2 span = a.tile_span[tile];
+      off = span.x;
+      len = span.y;
       if (len > a.queue_min) continue;   // drawn from the queue
     } else {
       uint32_t it = 0;
@@ -1758,8 +1712,9 @@ __global__ void __launch_bounds__(256, 4) raster_bins(const __grid_constant__ Ra
         j = d1.x; nch = d1.y;
       } else {
         tile = a.heavy[it / parts];
-        off = a.tile_off[tile];
-        len = a.tile_off[tile + 1] - off;
+        const uint2 span = a.tile_span[tile];
+        off = span.x;
+        len = span.y;
       }
     }
     // entries past the list capacity are never read (the frame reports the overflow)
@@ -1882,7 +1837,7 @@ __global__ void __launch_bounds__(256, 4) raster_bins(const __grid_constant__ Ra
 }
 
 // ------------------------------------------------------------------ launch
-int raster_scan_blocks(uint32_t n_tiles) { return (int)((n_tiles + kScanTile - 1) / kScanTile); }
+static int raster_scan_blocks(uint32_t n_tiles) { return (int)((n_tiles + kScanTile - 1) / kScanTile); }
 
 // CTAs of one full wave of a kernel on the current device (cached; every
 // launch of this library targets B200s of one kind).  Host threads may launch

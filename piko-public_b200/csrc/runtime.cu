@@ -112,7 +112,6 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
     // capture records have not run yet)
     CU(ctx, cudaMemsetAsync(scr.work, 0, sizeof(BinWork), st));
     CU(ctx, cudaMemsetAsync(scr.tile_cnt, 0, sizeof(uint32_t) * scr.tiles_cap, st));
-    CU(ctx, cudaMemsetAsync(scr.scan_flags, 0, sizeof(unsigned long long) * scr.scan_cap, st));
     scr.clean = !capturing;
   }
   a.scenes = scr.d_scenes;
@@ -122,7 +121,7 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   a.n_tiles_total = tiles;
   a.setup = scr.setup;
   a.tile_cnt = scr.tile_cnt;
-  a.tile_off = scr.tile_off;
+  a.tile_span = scr.tile_span;
   a.tile_list = scr.tile_list;
   a.pair_tl = scr.pair_tl;
   a.pair_g = scr.pair_g;
@@ -139,7 +138,6 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   a.chunk_keys = scr.chunk_keys;
   a.chunk_cap = scr.chunk_cap;
   a.key_cap = scr.key_cap;
-  a.scan_flags = scr.scan_flags;
   a.work = scr.work;
   a.ctr = scr.ctr;
   a.host_bin = &scr.h_ctr->bin;
@@ -172,7 +170,6 @@ namespace {
 piko_status check_counters(piko_ctx* ctx, RasterScratch& scr)
 {
   const BinCounts& c = scr.h_ctr->bin;
-  if (c.status & kStatusScanTimeout) return set_err(ctx, PIKO_ERR_TIMEOUT, "%s", "tile scan look-back timed out");
   if (c.status & kStatusListOverflow) {
     CU(ctx, scr.regrow(c));
     return PIKO_ERR_QUEUE_OVERFLOW;

@@ -9,9 +9,6 @@
 #include "piko_device.cuh"
 #include "../../include/piko_b200.h"
 
-namespace piko {
-int raster_scan_blocks(uint32_t n_tiles);
-}
 using namespace piko;
 
 struct ReyesState;
@@ -99,7 +96,7 @@ inline void dfree(T*& p)
 struct RasterScratch {
   TriSetup* setup = nullptr;
   uint32_t* tile_cnt = nullptr;
-  uint32_t* tile_off = nullptr;
+  uint2* tile_span = nullptr;
   uint32_t* tile_list = nullptr;
   unsigned long long* pair_tl = nullptr;  // count-pass pair records, [list_cap] each
   uint32_t* pair_g = nullptr;
@@ -111,15 +108,14 @@ struct RasterScratch {
   ChunkDesc* chunk_desc = nullptr;
   uint32_t chunk_cap = 0, key_cap = 0;
   uint32_t key_stride = 0;                  // keys per key slot (tile * tile)
-  unsigned long long* scan_flags = nullptr;
   BinWork* work = nullptr;
   FrameCounters* ctr = nullptr;
   FrameCounters* h_ctr = nullptr;  // pinned; the fragment kernel writes its bin part
-  bool clean = false;              // tile_cnt, scan_flags and work are all zero (every frame leaves them so)
+  bool clean = false;              // tile_cnt and work are all zero (every frame leaves them so)
   RasterSceneDev* d_scenes = nullptr;      // scene table of launch sequences over several scenes
   std::vector<RasterSceneDev> h_scenes;    // pageable: a copy from it has read it when the call returns
   RasterSceneDev* cap_scenes = nullptr;    // pinned: the source of a copy that a stream capture records
-  uint32_t tris_cap = 0, tiles_cap = 0, list_cap = 0, scan_cap = 0;
+  uint32_t tris_cap = 0, tiles_cap = 0, list_cap = 0;
   int scenes_cap = 0;
   uint32_t cov_cap = 0;
   uint32_t* cov_tri = nullptr;
@@ -129,17 +125,17 @@ struct RasterScratch {
 
   void release()
   {
-    dfree(setup); dfree(tile_cnt); dfree(tile_off); dfree(tile_list); dfree(pair_tl); dfree(pair_g);
+    dfree(setup); dfree(tile_cnt); dfree(tile_span); dfree(tile_list); dfree(pair_tl); dfree(pair_g);
     dfree(large_seg); dfree(large_walk); dfree(hdone); dfree(chunk_keys);
     dfree(chunk_desc);
-    dfree(scan_flags); dfree(work); dfree(ctr); dfree(d_scenes); dfree(cov_tri); dfree(cov_pix);
+    dfree(work); dfree(ctr); dfree(d_scenes); dfree(cov_tri); dfree(cov_pix);
     if (h_ctr) cudaFreeHost(h_ctr);
     if (cap_scenes) cudaFreeHost(cap_scenes);
     h_ctr = nullptr; cap_scenes = nullptr;
     clean = false;
     if (ev_made) for (auto& e : ev) cudaEventDestroy(e);
     ev_made = false;
-    tris_cap = tiles_cap = list_cap = scan_cap = chunk_cap = key_cap = seg_cap = key_stride = 0;
+    tris_cap = tiles_cap = list_cap = chunk_cap = key_cap = seg_cap = key_stride = 0;
     scenes_cap = 0;
     cov_cap = 0;
   }
@@ -237,17 +233,10 @@ struct RasterScratch {
     }
     if (n_tiles > tiles_cap) {
       clean = false;
-      dfree(tile_cnt); dfree(tile_off);
+      dfree(tile_cnt); dfree(tile_span);
       if ((e = dalloc(&tile_cnt, n_tiles))) return e;
-      if ((e = dalloc(&tile_off, (size_t)n_tiles + 1))) return e;
+      if ((e = dalloc(&tile_span, n_tiles))) return e;
       tiles_cap = n_tiles;
-    }
-    uint32_t sb = (uint32_t)raster_scan_blocks(n_tiles);
-    if (sb > scan_cap) {
-      clean = false;
-      dfree(scan_flags);
-      if ((e = dalloc(&scan_flags, sb))) return e;
-      scan_cap = sb;
     }
     if (list_need > list_cap) {
       if ((e = grow_list(list_need))) return e;

@@ -106,7 +106,7 @@ size_t scratch_bytes(const RasterScratch& r)
 {
   // setup records, per-tile counters and offsets, tile lists and the count
   // passes' pair records (12 bytes per list entry)
-  return (size_t)r.tris_cap * sizeof(TriSetup) + (size_t)r.tiles_cap * 8 + (size_t)r.list_cap * 16;
+  return (size_t)r.tris_cap * sizeof(TriSetup) + (size_t)r.tiles_cap * 12 + (size_t)r.list_cap * 16;
 }
 
 // slot with room for `pixels`, allocating one within the budget; -1 if none
@@ -222,7 +222,7 @@ bool dispatch(piko_server* sv, SrvLane& lane, std::unique_lock<std::mutex>& lk)
 
 // Checks a completed lane's frames, re-rendering after a queue overflow (and
 // waiting for the re-render), and returns the lane's status: a CUDA error, a
-// scan timeout, queues that kept overflowing, or a Reyes frame's error.
+// queues that kept overflowing, or a Reyes frame's error.
 // Called without the lock.
 piko_status finish_lane(piko_server* sv, SrvLane& lane)
 {
@@ -234,7 +234,6 @@ piko_status finish_lane(piko_server* sv, SrvLane& lane)
       const cudaError_t e = cudaStreamSynchronize(lane.st);
       if (e) { st = PIKO_ERR_CUDA; break; }
       const uint32_t status = scr.h_ctr->bin.status;
-      if (status & kStatusScanTimeout) { st = PIKO_ERR_TIMEOUT; break; }
       if (!(status & kStatusListOverflow)) { st = PIKO_OK; break; }
       if (attempt == 4) break;   // still overflowing: reported
       if (scr.regrow(scr.h_ctr->bin) != cudaSuccess) { st = PIKO_ERR_OOM; break; }
