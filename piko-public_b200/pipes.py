@@ -77,10 +77,18 @@ class PikoScreen:
 
     def getData(self):
         """RGBA8 words, R in the low byte, row 0 = bottom (pixel (x, y) at y*W + x)."""
-        fb, depth = self._pipe._scene.read()
+        scene, ms = self._pipe._scene, self._pipe.mutableState_
+        n = scene.W * scene.H
+        z = None if ms is None else ms.zBuffer
+        if isinstance(z, np.ndarray) and z.dtype == np.float32 and z.ndim == 1 and z.size >= n and \
+                z.flags.c_contiguous and z.flags.writeable and z.flags.aligned:
+            # the depth buffer is read in place
+            fb, depth = scene.read(out_depth=z[:n].reshape(scene.H, scene.W))
+        else:
+            fb, depth = scene.read()
+            if ms is not None:
+                z[: depth.size] = depth.reshape(-1)
         self._pipe._last_depth = depth
-        if self._pipe.mutableState_ is not None:
-            self._pipe.mutableState_.zBuffer[: depth.size] = depth.reshape(-1)
         return fb.reshape(-1)
 
 

@@ -6,6 +6,7 @@ without a CUDA device raises :class:`PikoError`.
 """
 import ctypes
 import os
+import sys
 
 import numpy as np
 
@@ -306,6 +307,7 @@ class Scene:
         desc, keep = scene_desc(scene, packed=packed)
         self.packed = packed
         self.W, self.H, self.N = desc.width, desc.height, desc.count
+        self._images = {np.uint32: [], np.float32: []}   # result arrays of read(), reused once the caller lets go
         self.h = ctypes.c_void_p()
         self.ctx.check(lib.piko_scene_create(pipe.h, ctypes.byref(desc), ctypes.byref(self.h)), "piko_scene_create")
         if not isinstance(scene, dict):
@@ -330,9 +332,24 @@ class Scene:
     def finish(self):
         self.ctx.check(self.ctx.lib.piko_frame_finish(self.h), "piko_frame_finish")
 
+    def _image(self, dtype):
+        """An array for one image that nobody else holds.  The pages of a fresh
+        one cost more than the copy into it (1 MB: 110 us against 27), so up to
+        two per image are kept, and one is handed out again when the caller has
+        let go of it and of every view of it."""
+        kept = self._images[dtype]
+        for a in kept:
+            if sys.getrefcount(a) == 3:   # the list's, the loop's and the call's reference
+                return a
+        a = np.empty((self.H, self.W), dtype)
+        if len(kept) == 2:
+            kept.pop(0)
+        kept.append(a)
+        return a
+
     def read(self, out_fb=None, out_depth=None):
-        fb = np.empty((self.H, self.W), np.uint32) if out_fb is None else out_fb
-        depth = np.empty((self.H, self.W), np.float32) if out_depth is None else out_depth
+        fb = self._image(np.uint32) if out_fb is None else out_fb
+        depth = self._image(np.float32) if out_depth is None else out_depth
         self.ctx.check(self.ctx.lib.piko_frame_read(self.h, _p(fb), _p(depth)), "piko_frame_read")
         return fb, depth
 
