@@ -843,7 +843,7 @@ __device__ __forceinline__ uint32_t sample_index(const ReyesArgs& a, int x, int 
 
 // Tie records of a CTA not yet in the list (a global append each, a tenth to a
 // quarter of the fragments, took 16 us of the default-constants sphere's dice).
-constexpr uint32_t kTieStage = 384;
+constexpr uint32_t kTieStage = 192;
 struct TieStage {
   uint4 rec[kTieStage];
   uint32_t n, base;
@@ -1030,12 +1030,13 @@ __device__ __forceinline__ void make_upoly(const ReyesArgs& a, unsigned long lon
 // shared list and every thread tests one cell at a time, so lanes stay busy
 // whatever the micropolygons' sizes.  A covered cell sets bit (its index in
 // the rectangle) of its micropolygon's mask; the owner then emits.
-constexpr int kMaxGridPts = 34 * 34;
+// (shared memory for four CTAs per SM: three 18 x 18 grids of points, 30 rows of the widest)
+constexpr int kMaxGridPts = 30 * 34;
 constexpr int kLeafBatch = 32;     // leaf segments per group
 constexpr int kDiceThreads = 256;
 constexpr int kUpBudget = 1024;    // micropolygons per group
 constexpr int kMaxPtRows = 128;    // grid point rows per group
-constexpr int kCellCap = 4096;     // cells per pass of the shared list
+constexpr int kCellCap = 2048;     // cells per pass of the shared list
 
 constexpr uint32_t kNoDepth = 0xffffffffu;
 constexpr uint32_t kBothWindings = 1u << 31;   // (else the corners' order makes the first winding the one to test)
@@ -1220,8 +1221,15 @@ __device__ __forceinline__ void dice_group(const ReyesArgs& a, DiceSmem& S, uint
   }
 }
 
-// Three CTAs per SM (at most 80 registers): the extra warps hide more of the
-// fixed-latency stalls than the few spilled values cost.
+// Four CTAs per SM (64 registers, 55 KB): bound by issue and latency together (at
+// three CTAs the schedulers issued 53% of the time, a fifth of the stalls on
+// memory and a sixth at barriers), so the extra warps hide more than a fourth
+// more spilled values cost: 95 -> 89 us on the 4-sample 1280x720 sphere's 817,003
+// micropolygons, 65 -> 60 us on the default constants' 451,467 of 50,163 leaves.
+// (8 CTAs of 128 threads: 91 and 58 us; 5 of 192: 98 and 61; a warp per 32
+// micropolygons with its own cell list instead of block-wide lists: 98 and 61,
+// its lists end in half-empty trips.  Of the 89 us the cells take 46: the
+// sample positions' hashes 13, the atomics 12, the edge tests the rest.)
 //
 // SPARSE: a group takes the ids of all of its micropolygons when it starts (the
 // tables hold every micropolygon of the frame), and a covered cell is an atomic
@@ -1230,7 +1238,7 @@ __device__ __forceinline__ void dice_group(const ReyesArgs& a, DiceSmem& S, uint
 // afterwards: for frames of so many micropolygons that ids or tables for all of
 // them would not fit.
 template <bool SPARSE>
-__global__ void __launch_bounds__(kDiceThreads, 3) reyes_dice(ReyesArgs a)
+__global__ void __launch_bounds__(kDiceThreads, 4) reyes_dice(ReyesArgs a)
 {
   pdl_wait();
   pdl_trigger();
