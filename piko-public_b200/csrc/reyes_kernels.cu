@@ -199,32 +199,6 @@ __device__ __forceinline__ int pow2roundup(int x)
   return x + 1;
 }
 
-__device__ __forceinline__ int cvt_i32_x86_d(double d)
-{
-  return (d >= -2147483648.0 && d < 2147483648.0) ? __double2int_rz(d) : INT32_MIN;
-}
-
-// One row (or column) of splitU / splitV (split.pikostage:95-224): de Casteljau
-// at t = 1/2 of the four points p0..p3; a0..a3 is the first half, b0..b3 the
-// second.  Returns the j-th point of half `second`.
-__device__ __forceinline__ float4 casteljau_half(float4 p0, float4 p1, float4 p2, float4 p3, int j, bool second)
-{
-  const float4 a1 = f4mul(f4add(p0, p1), 0.5f);
-  const float4 b2 = f4mul(f4add(p2, p3), 0.5f);
-  const float4 t = f4mul(f4add(p1, p2), 0.5f);
-  const float4 a2 = f4mul(f4add(a1, t), 0.5f);
-  const float4 b1 = f4mul(f4add(b2, t), 0.5f);
-  const float4 a3 = f4mul(f4add(a2, b1), 0.5f);
-  if (!second) return j == 0 ? p0 : (j == 1 ? a1 : (j == 2 ? a2 : a3));
-  return j == 0 ? a3 : (j == 1 ? b1 : (j == 2 ? b2 : p3));
-}
-
-__device__ __forceinline__ float4 shfl4(unsigned mask, float4 v, int src)
-{
-  return make_float4(__shfl_sync(mask, v.x, src, 16), __shfl_sync(mask, v.y, src, 16), __shfl_sync(mask, v.z, src, 16),
-                     __shfl_sync(mask, v.w, src, 16));
-}
-
 // Grid-wide barrier between split levels that also carries the next level's
 // patch count: every CTA arrives with the children it reserved; the last
 // arrival sums them and releases barrier k with (k + 1) << 32 | count, so no
@@ -317,21 +291,19 @@ __device__ __forceinline__ SplitDecision split_measure(const ReyesArgs& a, int L
   const float vx = __shfl_sync(hmask, cx, c + 4, 16), vy = __shfl_sync(hmask, cy, c + 4, 16);
   const float du = dist2(cx, cy, ux, uy);
   const float dv = dist2(cx, cy, vx, vy);
+  // a row's (column's) length is ((d0 + d1) + d2), on its first lane; the largest
+  // of 0 and the four lengths, which a NaN never is
+  float su = du + __shfl_sync(hmask, du, c + 1, 16);
+  float sv = dv + __shfl_sync(hmask, dv, c + 4, 16);
+  su = fmaxf(0.0f, su + __shfl_sync(hmask, du, c + 2, 16));
+  sv = fmaxf(0.0f, sv + __shfl_sync(hmask, dv, c + 8, 16));
+  su = fmaxf(su, __shfl_xor_sync(hmask, su, 4, 16));
+  sv = fmaxf(sv, __shfl_xor_sync(hmask, sv, 1, 16));
+  su = fmaxf(su, __shfl_xor_sync(hmask, su, 8, 16));
+  sv = fmaxf(sv, __shfl_xor_sync(hmask, sv, 2, 16));
   SplitDecision d;
-  d.ue = 0.0f;
-  d.ve = 0.0f;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    float su = __shfl_sync(hmask, du, 4 * r, 16) + __shfl_sync(hmask, du, 4 * r + 1, 16);
-    su = su + __shfl_sync(hmask, du, 4 * r + 2, 16);
-    d.ue = std_maxf(d.ue, su);
-  }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    float sv = __shfl_sync(hmask, dv, k, 16) + __shfl_sync(hmask, dv, k + 4, 16);
-    sv = sv + __shfl_sync(hmask, dv, k + 8, 16);
-    d.ve = std_maxf(d.ve, sv);
-  }
+  d.ue = __shfl_sync(hmask, su, 0, 16);
+  d.ve = __shfl_sync(hmask, sv, 0, 16);
   d.split = (d.ue >= a.thr) || (d.ve >= a.thr);
   if (L >= a.max_splits) d.split = false;
   d.nu = d.nv = 0;
@@ -339,8 +311,9 @@ __device__ __forceinline__ SplitDecision split_measure(const ReyesArgs& a, int L
     if (a.grid > 0) {   // a fixed dice grid replaces the extent-derived one
       d.nu = d.nv = a.grid;
     } else {
-      int nu = pow2roundup(cvt_i32_x86_d(ceil((double)(d.ue / a.thr))) + 1);
-      int nv = pow2roundup(cvt_i32_x86_d(ceil((double)(d.ve / a.thr))) + 1);
+      // (the reference rounds up in double: a float widened and rounded up is the float rounded up)
+      int nu = pow2roundup(cvt_i32_x86(ceilf(d.ue / a.thr)) + 1);
+      int nv = pow2roundup(cvt_i32_x86(ceilf(d.ve / a.thr)) + 1);
       d.nu = nu < 2 ? 2 : (nu > 32 ? 32 : nu);
       d.nv = nv < 2 ? 2 : (nv > 32 ? 32 : nv);
     }
@@ -360,11 +333,16 @@ __device__ __forceinline__ SplitDecision split_measure(const ReyesArgs& a, int L
 // least kSplitShare of them on the frontier: with few input patches the CTAs'
 // subtrees differ in size, and dealt out at that width they even out (a split
 // that put every patch past 64 per level on the frontier took 89 us of the
-// default-constants sphere's 14 levels, in four steps; this takes SPLIT us).  Nothing
+// default-constants sphere's 14 levels, in four steps; this takes 51 us).  The
+// levels' passes are bound by issue (about 700 patches per CTA in the last step)
+// and by their own chain of latencies where they are narrow, so a patch takes as
+// few instructions as its arithmetic needs, and 64 of them are in flight (the
+// sphere's frame 131.6 -> 127.0 us by the former, 124.3 by the latter; 32 in
+// flight are 0.3 us faster where the split ends after a few narrow levels).  Nothing
 // depends on which CTA or pass handles a patch: every leaf carries its input
 // index, level and in-level position (children of s are 2s and 2s + 1), which
 // give the order key.
-constexpr int kSplitThreads = 512;
+constexpr int kSplitThreads = 1024;
 constexpr int kSplitKeep = 128;         // patches a CTA takes per level
 constexpr int kSplitStage = 192;
 constexpr uint32_t kSplitStack = 1024;  // patches of a CTA's own stack
@@ -462,7 +440,7 @@ __device__ __forceinline__ void flush_leaves(const ReyesArgs& a, SplitSmem& S)
 }
 
 // One level of the CTA's current patches (at most kSplitKeep; 16-lane group
-// q takes patches q, q + 32): split ones put their children in nxt, leaves
+// q takes patches q, q + 64): split ones put their children in nxt, leaves
 // go to the stage.
 __device__ __forceinline__ void split_one(const ReyesArgs& a, SplitSmem& S, const PatchRec* cur, PatchRec* nxt,
                                           uint32_t p)
@@ -478,12 +456,21 @@ __device__ __forceinline__ void split_one(const ReyesArgs& a, SplitSmem& S, cons
   slot = __shfl_sync(hmask, slot, 0, 16);
   if (d.split) {
     const bool along_u = d.ue >= a.thr;
-    // the four points of this lane's row (split along u) or column (along v)
-    const int base = along_u ? (c & ~3) : (c & 3), st = along_u ? 1 : 4, j = along_u ? (c & 3) : (c >> 2);
-    const float4 p0 = shfl4(hmask, cp, base), p1 = shfl4(hmask, cp, base + st);
-    const float4 p2 = shfl4(hmask, cp, base + 2 * st), p3 = shfl4(hmask, cp, base + 3 * st);
-    nxt[slot].cp[c] = casteljau_half(p0, p1, p2, p3, j, false);
-    nxt[slot + 1].cp[c] = casteljau_half(p0, p1, p2, p3, j, true);
+    // The lane's row (split along u) or column (along v), halved at t = 1/2 by de
+    // Casteljau (splitU / splitV, split.pikostage:95-224): with points p0 .. p3 the
+    // halves are p0, a1, a2, a3 and a3, b1, b2, p3.  Lane j writes point j of both;
+    // lanes 2 and 3 take the points in reverse order (the sums commute), which
+    // makes their points lane 1's and 0's with the halves exchanged.
+    const int j = along_u ? (c & 3) : (c >> 2), st = along_u ? 1 : 4, at = c - j * st;
+    const bool rev = j >= 2;
+    const float4* q = cur[p].cp + (rev ? at + 3 * st : at);
+    const int qs = rev ? -st : st;
+    const float4 p0 = q[0], p1 = q[qs], p2 = q[2 * qs], p3 = q[3 * qs];
+    const float4 a1 = f4mul(f4add(p0, p1), 0.5f), t = f4mul(f4add(p1, p2), 0.5f), b2 = f4mul(f4add(p2, p3), 0.5f);
+    const float4 a2 = f4mul(f4add(a1, t), 0.5f), b1 = f4mul(f4add(b2, t), 0.5f);
+    const bool end = j == 0 || j == 3;
+    nxt[slot + (rev ? 1 : 0)].cp[c] = end ? p0 : a1;
+    nxt[slot + (rev ? 0 : 1)].cp[c] = end ? f4mul(f4add(a2, b1), 0.5f) : b1;
     if (c < 2) {
       PatchRec& o = nxt[slot + c];
       o.i0 = i0;
