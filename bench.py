@@ -437,7 +437,7 @@ def main():
     kscene = pk.Scene(kpipe, sc)
     # event spans of a frame: setup + large-triangle count, scan, scatter (list
     # and large-triangle walks), tile raster (raster_frag8 for 8x8 tiles)
-    tile_kernel = "raster_frag8" if args.tile == 8 else "raster_tiles"
+    tile_kernel = "raster_frag8" if args.tile == 8 else "raster_bins"
     names = ["raster_setup", "scan_tiles", "raster_scatter", tile_kernel]
     kms = np.zeros(4)
     reps = max(5, min(args.steps, 20))

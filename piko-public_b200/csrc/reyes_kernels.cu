@@ -334,11 +334,12 @@ __device__ __forceinline__ SplitDecision split_measure(const ReyesArgs& a, int L
 // subtrees differ in size, and dealt out at that width they even out (a split
 // that put every patch past 64 per level on the frontier took 89 us of the
 // default-constants sphere's 14 levels, in four steps; this takes 51 us).  The
-// levels' passes are bound by issue (about 700 patches per CTA in the last step)
-// and by their own chain of latencies where they are narrow, so a patch takes as
-// few instructions as its arithmetic needs, and 64 of them are in flight (the
-// sphere's frame 131.6 -> 127.0 us by the former, 124.3 by the latter; 32 in
-// flight are 0.3 us faster where the split ends after a few narrow levels).  Nothing
+// levels' passes are chains of latencies: 0.9 us a narrow level, and 37% issue
+// active over the default-constants sphere's 50 us, whose last step takes some 700
+// patches per CTA.  So a patch takes as few instructions as its arithmetic needs,
+// and 64 of them are in flight (that sphere's frame 131.6 -> 127.0 us by the former,
+// 124.3 by the latter; 32 in flight are 0.3 us faster where the split ends after a
+// few narrow levels).  Nothing
 // depends on which CTA or pass handles a patch: every leaf carries its input
 // index, level and in-level position (children of s are 2s and 2s + 1), which
 // give the order key.
@@ -1015,8 +1016,7 @@ __device__ __forceinline__ void make_upoly(const ReyesArgs& a, unsigned long lon
 // rectangle of cells (one per sample: a pixel quadrant with four samples, the
 // pixel with one), cut to the cells exact_box allows; the CTA's cells go to a
 // shared list and every thread tests one cell at a time, so lanes stay busy
-// whatever the micropolygons' sizes.  A covered cell sets bit (its index in
-// the rectangle) of its micropolygon's mask; the owner then emits.
+// whatever the micropolygons' sizes.
 // (shared memory for four CTAs per SM: three 18 x 18 grids of points, 30 rows of the widest)
 constexpr int kMaxGridPts = 30 * 34;
 constexpr int kLeafBatch = 32;     // leaf segments per group
