@@ -41,11 +41,16 @@
 namespace piko {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kSetupThreads = 256;
+// Threads of a raster_setup CTA, for one scene and for several.  Smaller CTAs wait
+// less at the barriers between their steps (24-scene batch 378 -> 371 us with 128
+// instead of 256), but leave fewer kept triangles to fill each step where most
+// are culled (the packed 1277x715 forest alone: 57 -> 59 us).
+template <bool ONE>
+constexpr int kSetupThreads = ONE ? 256 : 128;
 constexpr uint32_t kLargeTiles = 256; // box tiles above which a triangle's walk is spread over the grid
 constexpr uint32_t kWalkQueue = 256;  // tiles a warp of the walk can have queued
 constexpr uint32_t kItemMap = 4096;   // row items of a block's walk whose triangle is looked up
-static_assert(kLargeTiles <= 256 && kSetupThreads <= 256, "the walk's queue holds 8-bit tiles and triangles");
+static_assert(kLargeTiles <= 256 && kSetupThreads<true> <= 256, "the walk's queue holds 8-bit tiles and triangles");
 constexpr uint32_t kLargeSeg = 128;   // box tiles per work item of the large-triangle walk
 
 // ------------------------------------------------------------------ helpers
@@ -407,7 +412,7 @@ __device__ __forceinline__ uint32_t walk_tiles(const RasterFrameArgs& a, const W
     return tile_key(w, e & 255u);
   };
   uint32_t skipped = 0, qn = 0;
-  for (uint32_t base = threadIdx.x & ~31u; base < total; base += kSetupThreads) {
+  for (uint32_t base = threadIdx.x & ~31u; base < total; base += blockDim.x) {
     const uint32_t i = base + (uint32_t)lane;
     uint32_t m = 0, tri = 0, at = 0;
     if (i < total) {
@@ -511,29 +516,29 @@ __device__ __forceinline__ float4 load_attr3(const float4* a4, const float* a3, 
 // pair that passes the reject, as the reference's queues do, but lists only
 // tiles that can hold a covered pixel centre: a third fewer list entries, which
 // the later kernels do not touch (200K triangles: fragment pass 100 -> 92 us).
-constexpr int kSetupWarps = kSetupThreads / 32;
-
+template <int T>   // threads of the CTA
 struct SetupSmem {
-  WalkTri walk[kSetupThreads];
+  WalkTri walk[T];
   union {
     struct {   // the kept triangles, in order (steps 1 to 3)
-      int32_t x[3][kSetupThreads], y[3][kSetupThreads];
-      float z[3][kSetupThreads];
-      uint32_t c[3][kSetupThreads];
-      uint32_t g[kSetupThreads];
+      int32_t x[3][T], y[3][T];
+      float z[3][T];
+      uint32_t c[3][T];
+      uint32_t g[T];
     };
     struct {   // step 4
-      uint32_t pre[kSetupThreads];
+      uint32_t pre[T];
       uint8_t item_tri[kItemMap];
-      uint16_t queue[kSetupWarps][kWalkQueue];
+      uint16_t queue[T / 32][kWalkQueue];
     };
   };
-  uint32_t warp[kSetupWarps];
+  uint32_t warp[T / 32];
   unsigned nk, nr;
   unsigned skipped;   // pairs that pass the reject and are not listed (of one CTA: below 2^32)
 };
 
-// Inclusive scan of v over the block.
+// Inclusive scan of v over the block of T threads.
+template <int T>
 __device__ __forceinline__ uint32_t block_scan_incl(uint32_t v, uint32_t* s_warp)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -545,17 +550,18 @@ __device__ __forceinline__ uint32_t block_scan_incl(uint32_t v, uint32_t* s_warp
   if (lane == 31) s_warp[warp] = v;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < kSetupWarps; ++w)
+  for (int w = 0; w < T / 32; ++w)
     if (w < warp) v += s_warp[w];
   return v;
 }
 
 template <bool ONE>
-__global__ void __launch_bounds__(kSetupThreads) raster_setup(const __grid_constant__ RasterFrameArgs a)
+__global__ void __launch_bounds__(kSetupThreads<ONE>) raster_setup(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_trigger();
   extern __shared__ __align__(16) unsigned char setup_smem[];
-  SetupSmem& B = *reinterpret_cast<SetupSmem*>(setup_smem);
+  constexpr int T = kSetupThreads<ONE>;
+  SetupSmem<T>& B = *reinterpret_cast<SetupSmem<T>*>(setup_smem);
   uint32_t* s_tb = reinterpret_cast<uint32_t*>(&B + 1);   // the scene table, several scenes only
   load_scene_table<ONE, kSceneTable>(a, s_tb, false);
   if (threadIdx.x == 0) B.nk = B.nr = B.skipped = 0u;
@@ -629,7 +635,7 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(const __grid_const
       __syncthreads();
       uint32_t at = (uint32_t)__popc(m & ((1u << lane) - 1u));
 #pragma unroll
-      for (int w = 0; w < kSetupWarps; ++w)
+      for (int w = 0; w < T / 32; ++w)
         if (w < (int)(threadIdx.x >> 5)) at += B.warp[w];
       if (keep) {
 #pragma unroll
@@ -643,12 +649,12 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(const __grid_const
     }
     uint32_t n = 0;
 #pragma unroll
-    for (int w = 0; w < kSetupWarps; ++w) n += B.warp[w];
+    for (int w = 0; w < T / 32; ++w) n += B.warp[w];
     __syncthreads();
     // 2.  R1, main.cpp:310-400: per-vertex Gouraud lighting with the normal
     // normalised by HOST::normalize; no colour array: the reference's fixed
     // material colour (main.cpp:380)
-    for (uint32_t v = threadIdx.x; v < 3 * n; v += kSetupThreads) {
+    for (uint32_t v = threadIdx.x; v < 3 * n; v += T) {
       const uint32_t t = v / 3u, k = v - 3u * t, vg = B.g[t];
       const int s = scene_of<ONE, kSceneTable>(a, s_tb, vg, false);
       const RasterSceneDev& S = scene_at<ONE>(a, s);
@@ -784,7 +790,7 @@ __global__ void __launch_bounds__(kSetupThreads) raster_setup(const __grid_const
       items = (ntiles / tw) * ((tw + 31u) >> 5);
     }
     // (the scan's barrier lies between the last read of x .. g and this write)
-    const uint32_t incl = block_scan_incl(items, B.warp);
+    const uint32_t incl = block_scan_incl<T>(items, B.warp);
     B.pre[threadIdx.x] = incl;
     for (uint32_t i = incl - items; i < min(incl, kItemMap); ++i) B.item_tri[i] = (uint8_t)threadIdx.x;
     __syncthreads();
@@ -1903,11 +1909,13 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& args, int raster_ctas, cu
   const bool one = a.n_scenes == 1;
   const bool tri_blocks = a.n_tris_total > 0;
   const auto setup = one ? raster_setup<true> : raster_setup<false>;
-  const size_t setup_smem = sizeof(SetupSmem) + (one ? 0 : kSceneTable * sizeof(uint32_t));
+  const int threads = one ? kSetupThreads<true> : kSetupThreads<false>;
+  const size_t setup_smem = one ? sizeof(SetupSmem<kSetupThreads<true>>)
+                                : sizeof(SetupSmem<kSetupThreads<false>>) + kSceneTable * sizeof(uint32_t);
   // One wave of CTAs; every CTA takes the same number of equal batches, and a
   // small scene is spread over the whole device, at least 8 triangles a batch.
-  const uint32_t wave = (uint32_t)wave_ctas(setup, &setup_wave[one], kSetupThreads, setup_smem);
-  const uint32_t rounds = (a.n_tris_total + wave * kSetupThreads - 1) / (wave * kSetupThreads);
+  const uint32_t wave = (uint32_t)wave_ctas(setup, &setup_wave[one], threads, setup_smem);
+  const uint32_t rounds = (a.n_tris_total + wave * threads - 1) / (wave * threads);
   a.batch = (a.n_tris_total + wave * rounds - 1) / std::max(wave * rounds, 1u);
   a.batch = a.batch > 32 ? (a.batch + 31) & ~31u : std::max(a.batch, 8u);
   const int setup_blocks = (int)std::min(wave, (a.n_tris_total + a.batch - 1) / a.batch);
@@ -1919,7 +1927,7 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& args, int raster_ctas, cu
   // every launch after the first may start while its predecessor drains
   // (programmatic dependent launch); each waits for it before touching memory
   cudaError_t e = cudaSuccess;
-  if (tri_blocks) setup<<<setup_blocks, kSetupThreads, setup_smem, st>>>(a);
+  if (tri_blocks) setup<<<setup_blocks, threads, setup_smem, st>>>(a);
   if (tri_blocks && !e) e = launch_pdl(raster_large_count, large_blocks, 256, st, a);
   if (ev) cudaEventRecord(ev[1], st);
   if (!e) e = launch_pdl(scan_tiles, raster_scan_blocks(a.n_tiles_total), kScanThreads, st, a);
