@@ -248,6 +248,25 @@ struct __align__(16) ChunkDesc {
 };
 static_assert(sizeof(ChunkDesc) == 32, "ChunkDesc layout");
 
+// raster_setup's launch for n triangles, given a full wave of CTAs: one wave at
+// most; every CTA takes the same number of equal batches, and a small scene is
+// spread over the whole device, at least 8 triangles a batch.  No triangles: no
+// CTAs.
+struct SetupShape {
+  uint32_t batch;    // triangles a CTA takes at a time
+  uint32_t blocks;
+};
+inline SetupShape setup_shape(uint32_t n, uint32_t wave, uint32_t threads)
+{
+  if (n == 0) return {8u, 0u};
+  const uint64_t n64 = n, full = (uint64_t)wave * threads;
+  const uint64_t slots = (n64 + full - 1) / full * wave;
+  uint64_t batch = (n64 + slots - 1) / slots;
+  batch = batch > 32 ? (batch + 31) & ~31ull : batch < 8 ? 8 : batch;
+  const uint64_t blocks = (n64 + batch - 1) / batch;
+  return {(uint32_t)batch, (uint32_t)(blocks < wave ? blocks : wave)};
+}
+
 struct RasterFrameArgs {
   RasterSceneDev one;       // the scene of a one-scene frame: it travels with the launch, no copy precedes the frame
   const RasterSceneDev* scenes;  // [n_scenes] when there are several

@@ -1907,18 +1907,13 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& args, int raster_ctas, cu
   RasterFrameArgs a = args;
   static std::atomic<int> setup_wave[2] = {{0}, {0}}, scatter_wave{0}, large_wave{0};
   const bool one = a.n_scenes == 1;
-  const bool tri_blocks = a.n_tris_total > 0;
   const auto setup = one ? raster_setup<true> : raster_setup<false>;
   const int threads = one ? kSetupThreads<true> : kSetupThreads<false>;
   const size_t setup_smem = one ? sizeof(SetupSmem<kSetupThreads<true>>)
                                 : sizeof(SetupSmem<kSetupThreads<false>>) + kSceneTable * sizeof(uint32_t);
-  // One wave of CTAs; every CTA takes the same number of equal batches, and a
-  // small scene is spread over the whole device, at least 8 triangles a batch.
-  const uint32_t wave = (uint32_t)wave_ctas(setup, &setup_wave[one], threads, setup_smem);
-  const uint32_t rounds = (a.n_tris_total + wave * threads - 1) / (wave * threads);
-  a.batch = (a.n_tris_total + wave * rounds - 1) / std::max(wave * rounds, 1u);
-  a.batch = a.batch > 32 ? (a.batch + 31) & ~31u : std::max(a.batch, 8u);
-  const int setup_blocks = (int)std::min(wave, (a.n_tris_total + a.batch - 1) / a.batch);
+  const SetupShape shape =
+      setup_shape(a.n_tris_total, (uint32_t)wave_ctas(setup, &setup_wave[one], threads, setup_smem), (uint32_t)threads);
+  a.batch = shape.batch;
   // the scatter grid covers the list groups of every triangle plus the large
   // triangles' segments (a grid-stride loop takes any excess)
   const int scatter_blocks = std::max(1, wave_ctas(raster_scatter, &scatter_wave) / (int)kPairParts) * (int)kPairParts;
@@ -1927,8 +1922,8 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& args, int raster_ctas, cu
   // every launch after the first may start while its predecessor drains
   // (programmatic dependent launch); each waits for it before touching memory
   cudaError_t e = cudaSuccess;
-  if (tri_blocks) setup<<<setup_blocks, threads, setup_smem, st>>>(a);
-  if (tri_blocks && !e) e = launch_pdl(raster_large_count, large_blocks, 256, st, a);
+  if (shape.blocks) setup<<<(int)shape.blocks, threads, setup_smem, st>>>(a);
+  if (shape.blocks && !e) e = launch_pdl(raster_large_count, large_blocks, 256, st, a);
   if (ev) cudaEventRecord(ev[1], st);
   if (!e) e = launch_pdl(scan_tiles, raster_scan_blocks(a.n_tiles_total), kScanThreads, st, a);
   if (ev) cudaEventRecord(ev[2], st);

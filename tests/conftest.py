@@ -32,3 +32,13 @@ def ctx(pk):
     c = pk.Context()
     yield c
     c.close()
+
+
+@pytest.fixture(scope="session")
+def host(tmp_path_factory):
+    """run(code): Python code in a child process, with the library's host code on a
+    stub of the CUDA runtime."""
+    import functools
+
+    import hostlib
+    return functools.partial(hostlib.run, hostlib.build(str(tmp_path_factory.mktemp("host"))))

@@ -1,0 +1,16 @@
+// What the stub of the CUDA runtime knows of the library's kernels (decode.cu).
+#pragma once
+#include <functional>
+#include <string>
+#include <vector>
+
+struct StubLaunch {
+  std::vector<const void*> objects;                // working counters that the launch changes
+  bool null_argument = false;                      // a buffer that the kernel uses is null
+  std::function<std::vector<float>()> cameras = [] { return std::vector<float>(); };   // view_proj[12] of the scenes drawn
+};
+
+// "raster_setup", ... from the mangled name
+std::string stub_kernel_name(const char* mangled);
+// A launch's arguments, copied
+StubLaunch stub_decode(const char* name, void** args);
