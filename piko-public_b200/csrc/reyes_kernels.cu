@@ -1742,18 +1742,22 @@ static cudaError_t reyes_alloc(ReyesState* r, uint32_t lvl_cap, uint32_t leaf_ca
     lvl_cap = leaf_cap = up_cap = id_cap = tie_cap = 0;
     npx = 0;
   }
+  // (a capacity stands only while all of its buffers do)
   if (lvl_cap > r->lvl_cap) {
     dfree(r->lvl[0]); dfree(r->lvl[1]);
+    r->lvl_cap = 0;
     if ((e = dalloc(&r->lvl[0], lvl_cap)) || (e = dalloc(&r->lvl[1], lvl_cap))) return e;
     r->lvl_cap = lvl_cap;
   }
   if (leaf_cap > r->leaf_cap) {
     dfree(r->leaves);
+    r->leaf_cap = 0;
     if ((e = dalloc(&r->leaves, leaf_cap))) return e;
     r->leaf_cap = leaf_cap;
   }
   if (up_cap > r->up_cap) {
     dfree(r->up);
+    r->up_cap = 0;
     if ((e = dalloc(&r->up, up_cap))) return e;
     r->up_cap = up_cap;
   }
@@ -1777,10 +1781,10 @@ static cudaError_t reyes_alloc(ReyesState* r, uint32_t lvl_cap, uint32_t leaf_ca
     r->npx_cap = npx;
   }
   if (!r->ctr) {
+    r->ctr_clean = false;
     if ((e = dalloc(&r->ctr, 1))) return e;
-    if ((e = cudaMallocHost((void**)&r->h_ctr, sizeof(ReyesCounters)))) return e;
-    memset(r->h_ctr, 0, sizeof(ReyesCounters));
   }
+  if (!r->h_ctr && (e = halloc(&r->h_ctr, 1))) return e;
   if (!r->ev_made) {
     for (auto& ev : r->ev)
       if ((e = cudaEventCreate(&ev))) return e;
@@ -1850,7 +1854,7 @@ piko_status piko_reyes_finish(piko_scene* s)
 {
   piko_ctx* ctx = s->pipe->ctx;
   ReyesState* r = s->reyes;
-  if (!r) { s->pending = false; return PIKO_OK; }
+  if (!r || !r->h_ctr) { s->pending = false; return PIKO_OK; }   // no frame was enqueued
   for (int attempt = 0; attempt < 6; ++attempt) {
     CU(ctx, cudaStreamSynchronize(s->last_stream));
     const ReyesCounters& c = *r->h_ctr;

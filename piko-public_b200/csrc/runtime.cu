@@ -594,6 +594,7 @@ piko_status piko_frame_coverage(piko_scene* s, uint32_t* tri, uint32_t* pix, uin
   for (int attempt = 0; attempt < 4; ++attempt) {
     if (want > s->scr.cov_cap) {
       dfree(s->scr.cov_tri); dfree(s->scr.cov_pix);
+      s->scr.cov_cap = 0;
       CU(ctx, dalloc(&s->scr.cov_tri, want));
       CU(ctx, dalloc(&s->scr.cov_pix, want));
       s->scr.cov_cap = want;

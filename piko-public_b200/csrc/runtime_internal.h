@@ -78,12 +78,25 @@ inline piko_status set_err(piko_ctx* ctx, piko_status st, const char* fmt, const
     }                                                                                 \
   } while (0)
 
+// Allocations of device and of pinned memory.  A failed one leaves null and no
+// error behind: cudaGetLastError after a later launch is to tell of that launch.
 template <class T>
 inline cudaError_t dalloc(T** p, size_t count)
 {
   *p = nullptr;
   if (count == 0) count = 1;
-  return cudaMalloc((void**)p, count * sizeof(T));
+  const cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+  if (e) { *p = nullptr; cudaGetLastError(); }
+  return e;
+}
+template <class T>
+inline cudaError_t halloc(T** p, size_t count)
+{
+  *p = nullptr;
+  const cudaError_t e = cudaMallocHost((void**)p, count * sizeof(T));
+  if (e) { *p = nullptr; cudaGetLastError(); return e; }
+  memset((void*)*p, 0, count * sizeof(T));
+  return cudaSuccess;
 }
 template <class T>
 inline void dfree(T*& p)
@@ -221,19 +234,23 @@ struct RasterScratch {
     return cudaSuccess;
   }
 
+  // Buffers for a frame.  A capacity stands only while all of its buffers do: one
+  // whose allocation failed part way is 0 until the next frame allocates again.
   cudaError_t ensure(uint32_t n_tris, uint32_t n_tiles, uint32_t list_need, int n_scenes)
   {
     cudaError_t e = cudaSuccess;
-    if (n_tris > tris_cap) {
+    if (n_tris > tris_cap || !setup) {
       dfree(setup);
+      tris_cap = 0;
       if ((e = dalloc(&setup, n_tris))) return e;
-      // segment items of large triangles: an estimate, grown after an overflow
-      if (n_tris / 8 + 1024 > seg_cap && (e = grow_segs(n_tris / 8 + 1024))) return e;
       tris_cap = n_tris;
     }
+    // segment items of large triangles: an estimate, grown after an overflow
+    if (tris_cap / 8 + 1024 > seg_cap && (e = grow_segs(tris_cap / 8 + 1024))) return e;
     if (n_tiles > tiles_cap) {
       clean = false;
       dfree(tile_cnt); dfree(tile_span);
+      tiles_cap = 0;
       if ((e = dalloc(&tile_cnt, n_tiles))) return e;
       if ((e = dalloc(&tile_span, n_tiles))) return e;
       tiles_cap = n_tiles;
@@ -241,19 +258,19 @@ struct RasterScratch {
     if (list_need > list_cap) {
       if ((e = grow_list(list_need))) return e;
     }
-    if (!ctr) {
+    if (!work) {
       clean = false;
       if ((e = dalloc(&work, 1))) return e;
-      if ((e = dalloc(&ctr, 1))) return e;
-      if ((e = cudaMallocHost((void**)&h_ctr, sizeof(FrameCounters)))) return e;
-      memset(h_ctr, 0, sizeof(FrameCounters));
     }
+    if (!ctr && (e = dalloc(&ctr, 1))) return e;
+    if (!h_ctr && (e = halloc(&h_ctr, 1))) return e;
     if (n_scenes > 1 && n_scenes > scenes_cap) {
       dfree(d_scenes);
       if (cap_scenes) cudaFreeHost(cap_scenes);
       cap_scenes = nullptr;
+      scenes_cap = 0;
       if ((e = dalloc(&d_scenes, n_scenes))) return e;
-      if ((e = cudaMallocHost((void**)&cap_scenes, sizeof(RasterSceneDev) * n_scenes))) return e;
+      if ((e = halloc(&cap_scenes, n_scenes))) return e;
       scenes_cap = n_scenes;
     }
     if (!ev_made) {

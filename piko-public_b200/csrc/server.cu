@@ -198,21 +198,29 @@ bool dispatch(piko_server* sv, SrvLane& lane, std::unique_lock<std::mutex>& lk)
   sv->batches++;
   sv->batched_reqs += taken.size();
   lk.unlock();
+  // what could not be enqueued is not finished either: the lane keeps only the
+  // draws and slots whose frames are on their way
   piko_status st = PIKO_OK;
-  for (auto& kv : lane.draws) {
-    const int T = kv.first;
-    const int cps = kv.second.front().mesh->pipe->ctas_per_sm;
-    piko_status r = enqueue_raster_draws(sv->ctx, kv.second.data(), (int)kv.second.size(), lane.scr[T], T,
-                                         raster_ctas(sv->ctx, T, cps), lane.st, false, false,
-                                         kv.second.front().mesh->pipe->chunk);
+  for (auto it = lane.draws.begin(); it != lane.draws.end();) {
+    const int T = it->first;
+    const std::vector<RasterDraw>& d = it->second;
+    const int cps = d.front().mesh->pipe->ctas_per_sm;
+    const piko_status r = enqueue_raster_draws(sv->ctx, d.data(), (int)d.size(), lane.scr[T], T,
+                                               raster_ctas(sv->ctx, T, cps), lane.st, false, false,
+                                               d.front().mesh->pipe->chunk);
     if (r != PIKO_OK) st = r;
+    it = r == PIKO_OK ? std::next(it) : lane.draws.erase(it);
   }
+  std::vector<int> enqueued;
   for (int si : lane.reyes_slots) {
-    piko_status r = piko_reyes_run(sv->slots[si].shadow, lane.st, false);
-    sv->slots[si].shadow->last_stream = lane.st;
-    sv->slots[si].shadow->pending = true;
-    if (r != PIKO_OK) st = r;
+    piko_scene* v = sv->slots[si].shadow;
+    const piko_status r = piko_reyes_run(v, lane.st, false);
+    v->last_stream = lane.st;
+    v->pending = r == PIKO_OK;
+    if (r == PIKO_OK) enqueued.push_back(si);
+    else st = r;
   }
+  lane.reyes_slots = enqueued;
   cudaEventRecord(lane.ev, lane.st);
   lk.lock();
   if (st != PIKO_OK)
@@ -221,7 +229,7 @@ bool dispatch(piko_server* sv, SrvLane& lane, std::unique_lock<std::mutex>& lk)
 }
 
 // Checks a completed lane's frames, re-rendering after a queue overflow (and
-// waiting for the re-render), and returns the lane's status: a CUDA error, a
+// waiting for the re-render), and returns the lane's status: a CUDA error,
 // queues that kept overflowing, or a Reyes frame's error.
 // Called without the lock.
 piko_status finish_lane(piko_server* sv, SrvLane& lane)
