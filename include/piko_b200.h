@@ -194,7 +194,11 @@ typedef struct piko_const_state {
  * 0xff663313 at the start of every frame. */
 piko_status piko_frame_prepare(piko_scene* scene, const piko_const_state* state);
 /* Replaces run_single() (CPUBackend.cpp:381-398): enqueues one frame on
- * `stream` and returns without waiting. */
+ * `stream` (NULL: the scene's own) and returns without waiting.  The frames of
+ * one scene follow one another whichever streams they are given.  Frames that the
+ * caller captures into a graph are outside that order: a replay must not overlap
+ * another frame of the same scene (both images, and the frame after them, would be
+ * undefined). */
 piko_status piko_frame_run(piko_scene* scene, void* stream);
 /* Waits for the scene's last frame and checks its status; a bin-queue
  * overflow grows the queues and re-renders the frame before returning OK. */
@@ -234,8 +238,10 @@ piko_status piko_frame_coverage(piko_scene* scene, uint32_t* tri, uint32_t* pix,
  * Many raster scenes drawn by one set of launches over a global tile queue;
  * no reference counterpart (the reference renders one scene per run_single). */
 piko_status piko_batch_create(piko_ctx* ctx, piko_scene* const* scenes, int n, piko_batch** out);
-/* Enqueues one frame of every scene of the batch; capture=1 records the launch
- * sequence as a CUDA graph on first use and replays it afterwards. */
+/* Enqueues one frame of every scene of the batch; use_graph=1 records the launch
+ * sequence as a CUDA graph on first use and replays it afterwards.  The frames of
+ * one batch follow one another whichever streams they are given (NULL: the
+ * context's own). */
 piko_status piko_batch_run(piko_batch* batch, void* stream, int use_graph);
 /* Waits for the batch, checks the status (growing queues and re-rendering on
  * overflow) and returns the summed counters. */

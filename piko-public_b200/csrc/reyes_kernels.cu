@@ -1700,6 +1700,7 @@ struct ReyesState {
   ReyesCounters* ctr = nullptr;
   ReyesCounters* h_ctr = nullptr;   // pinned, written by reyes_pixels
   bool ctr_clean = false;
+  bool captured = false;            // a caller's capture holds a frame: the counters are cleared before every frame
   cudaEvent_t ev[5] = {};
   bool ev_made = false;
 };
@@ -1808,10 +1809,11 @@ piko_status piko_reyes_run(piko_scene* s, cudaStream_t st, bool timed)
                       b->id_cap ? b->id_cap : (uint32_t)std::max<size_t>(1u << 20, npx),
                       b->tie_cap ? b->tie_cap : (uint32_t)std::max<size_t>(1u << 18, nsamp / 8), nsamp));
   if (!b->stack) CU(ctx, dalloc(&b->stack, (size_t)ctx->sms * kSplitStack));
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  CU(ctx, cudaStreamIsCapturing(st, &capture));
-  const bool ran = capture == cudaStreamCaptureStatusNone;   // (what a capture records has not run yet)
-  if (!r->ctr_clean) {   // fresh, or a frame whose launches failed part way
+  bool capturing = false;
+  CU(ctx, stream_capturing(st, &capturing));
+  if (capturing) r->captured = true;
+  const bool ran = !capturing;   // (what a capture records has not run yet)
+  if (!r->ctr_clean || r->captured) {   // fresh, a frame whose launches failed part way, replays that nothing orders
     CU(ctx, cudaMemsetAsync(r->ctr, 0, sizeof(ReyesCounters), st));
     r->ctr_clean = ran;
   }
@@ -1886,6 +1888,7 @@ piko_status piko_reyes_finish(piko_scene* s)
     piko_status rr = piko_reyes_run(s, s->last_stream, s->timed);
     if (rr != PIKO_OK) return rr;
   }
+  cudaStreamSynchronize(s->last_stream);   // (FrameOrder's mark lies before the last run)
   return set_err(ctx, PIKO_ERR_QUEUE_OVERFLOW, "%s", "Reyes queues kept overflowing");
 }
 

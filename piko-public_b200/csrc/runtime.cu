@@ -84,9 +84,10 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   if (T != kRefBin) group = tiles * (uint32_t)(T / kRefBin) * (uint32_t)(T / kRefBin) < 4u * warps ? 1u : 4u;
   const uint32_t queue_min = std::min(T == kRefBin && tiles / warps >= 4u * kLightGroup ? 2u * kQueueMin : kQueueMin, chunk);
   CU(ctx, scr.ensure_heavy(tiles, T, chunk, queue_min));
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  CU(ctx, cudaStreamIsCapturing(st, &capture));
-  const bool capturing = capture != cudaStreamCaptureStatusNone;
+  bool capturing = false;
+  CU(ctx, stream_capturing(st, &capturing));
+  // (a capture of the library's own finds the table ready: FrameOrder covers its replays)
+  if (capturing && !table_ready) scr.captured = true;
   RasterFrameArgs a;
   memset(&a, 0, sizeof(a));
   if (n == 1) {
@@ -107,9 +108,9 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
     }
     CU(ctx, cudaMemcpyAsync(scr.d_scenes, src, sizeof(RasterSceneDev) * n, cudaMemcpyHostToDevice, st));
   }
-  if (!scr.clean) {
-    // fresh counters, or a frame whose launches failed part way (memsets that a
-    // capture records have not run yet)
+  if (!scr.clean || scr.captured) {
+    // fresh counters, a frame whose launches failed part way (memsets that a
+    // capture records have not run yet), or replays that nothing orders
     CU(ctx, cudaMemsetAsync(scr.work, 0, sizeof(BinWork), st));
     CU(ctx, cudaMemsetAsync(scr.tile_cnt, 0, sizeof(uint32_t) * scr.tiles_cap, st));
     scr.clean = !capturing;
@@ -321,6 +322,7 @@ static void scene_free(piko_scene* s)
   dfree(s->pos); dfree(s->nrm); dfree(s->pos3); dfree(s->nrm3); dfree(s->col); dfree(s->uv); dfree(s->tex);
   dfree(s->wtri_xyz); dfree(s->wtri_icol); dfree(s->patches); dfree(s->fb); dfree(s->depth);
   s->scr.release();
+  s->order.release();
   piko_reyes_release(s);
   if (s->own_stream) cudaStreamDestroy(s->own_stream);
   s->own_stream = nullptr;
@@ -477,6 +479,7 @@ piko_status piko_frame_run(piko_scene* s, void* stream)
   piko_ctx* ctx = s->pipe->ctx;
   cudaStream_t st = pick_stream(s, stream);
   s->timed = ctx->time_kernels;
+  CU(ctx, s->order.before(st));
   piko_status r;
   if (s->pipe->kind == kPipeReyes) {
     r = piko_reyes_run(s, st, s->timed);
@@ -484,6 +487,7 @@ piko_status piko_frame_run(piko_scene* s, void* stream)
     piko_scene* one[1] = {s};
     r = enqueue_raster(ctx, one, 1, s->scr, pipe_cfg(s->pipe), st, s->timed, false);
   }
+  CU(ctx, s->order.after(st, s->own_stream));   // (after a failure too: part of the frame may be on its way)
   if (r == PIKO_OK) { s->last_stream = st; s->pending = true; }
   return r;
 }
@@ -502,6 +506,7 @@ piko_status piko_frame_finish(piko_scene* s)
     r = enqueue_raster(ctx, one, 1, s->scr, pipe_cfg(s->pipe), s->last_stream, s->timed, false);
     if (r != PIKO_OK) return r;
   }
+  cudaStreamSynchronize(s->last_stream);   // (FrameOrder's mark lies before the last redraw)
   return set_err(ctx, PIKO_ERR_QUEUE_OVERFLOW, "%s", "bin queues kept overflowing");
 }
 
@@ -600,7 +605,9 @@ piko_status piko_frame_coverage(piko_scene* s, uint32_t* tri, uint32_t* pix, uin
       s->scr.cov_cap = want;
     }
     piko_scene* one[1] = {s};
+    CU(ctx, s->order.before(st));
     r = enqueue_raster(ctx, one, 1, s->scr, pipe_cfg(s->pipe), st, false, true);
+    CU(ctx, s->order.after(st, st));
     if (r != PIKO_OK) return r;
     r = check_frame(ctx, s->scr, st, true);
     if (r == PIKO_OK) break;
@@ -650,24 +657,25 @@ piko_status batch_make(piko_ctx* ctx, piko_scene* const* scenes, int n, const Tu
 }
 
 // Enqueues every group: group 0 on st, the others on their own streams forked
-// from st and joined back into it (parallel branches when captured).
+// from st and joined back into it (parallel branches when captured; joined after a
+// failure too: what was enqueued is then in st's order).
 // table_ready: the groups' scene tables already hold the scenes as they are now.
 static piko_status batch_enqueue(piko_batch* b, cudaStream_t st, bool timed, bool table_ready = false)
 {
   piko_ctx* ctx = b->ctx;
   const bool fork = b->groups.size() > 1;
   if (fork) CU(ctx, cudaEventRecord(b->fork, st));
-  for (size_t k = 0; k < b->groups.size(); ++k) {
-    BatchGroup* g = b->groups[k];
-    cudaStream_t gs = k == 0 ? st : g->stream;
-    if (k > 0) CU(ctx, cudaStreamWaitEvent(gs, b->fork, 0));
-    piko_status r = enqueue_raster(ctx, g->scenes.data(), (int)g->scenes.size(), g->scr, g->cfg, gs, timed, false,
-                                   table_ready);
-    if (r != PIKO_OK) return r;
-    if (k > 0) CU(ctx, cudaEventRecord(g->done, gs));
+  piko_status r = PIKO_OK;
+  size_t n = 0;
+  for (; n < b->groups.size() && r == PIKO_OK; ++n) {
+    BatchGroup* g = b->groups[n];
+    cudaStream_t gs = n == 0 ? st : g->stream;
+    if (n > 0) CU(ctx, cudaStreamWaitEvent(gs, b->fork, 0));
+    r = enqueue_raster(ctx, g->scenes.data(), (int)g->scenes.size(), g->scr, g->cfg, gs, timed, false, table_ready);
+    if (n > 0) CU(ctx, cudaEventRecord(g->done, gs));
   }
-  for (size_t k = 1; k < b->groups.size(); ++k) CU(ctx, cudaStreamWaitEvent(st, b->groups[k]->done, 0));
-  return PIKO_OK;
+  for (size_t k = 1; k < n; ++k) CU(ctx, cudaStreamWaitEvent(st, b->groups[k]->done, 0));
+  return r;
 }
 
 extern "C" {
@@ -693,7 +701,30 @@ static void drop_graph(piko_batch* b)
   if (b->graph) cudaGraphDestroy(b->graph);
   b->graph_exec = nullptr;
   b->graph = nullptr;
-  b->graph_stream = nullptr;
+}
+
+static piko_status batch_frame(piko_batch* b, cudaStream_t st, bool use_graph)
+{
+  piko_ctx* ctx = b->ctx;
+  const bool timed = ctx->time_kernels;
+  if (!use_graph || timed) return batch_enqueue(b, st, timed);
+  if (!b->graph_exec) {
+    // size the scratch outside the capture (allocation is not capturable)
+    piko_status r = batch_enqueue(b, st, false);
+    if (r != PIKO_OK) return r;
+    CU(ctx, cudaStreamSynchronize(st));
+    // the frame just drawn filled the scene tables: the graph is its kernels alone
+    CU(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    r = batch_enqueue(b, st, false, true);
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamEndCapture(st, &g);
+    if (r != PIKO_OK) { if (g) cudaGraphDestroy(g); return r; }
+    CU(ctx, e);
+    b->graph = g;
+    CU(ctx, cudaGraphInstantiate(&b->graph_exec, g, 0));
+  }
+  CU(ctx, cudaGraphLaunch(b->graph_exec, st));
+  return PIKO_OK;
 }
 
 piko_status piko_batch_run(piko_batch* b, void* stream, int use_graph)
@@ -701,28 +732,10 @@ piko_status piko_batch_run(piko_batch* b, void* stream, int use_graph)
   if (!b) return PIKO_ERR_INVALID;
   piko_ctx* ctx = b->ctx;
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-  const bool timed = ctx->time_kernels;
-  if (use_graph && !timed) {
-    if (!b->graph_exec) {
-      // size the scratch outside the capture (allocation is not capturable)
-      piko_status r = batch_enqueue(b, st, false);
-      if (r != PIKO_OK) return r;
-      CU(ctx, cudaStreamSynchronize(st));
-      // the frame just drawn filled the scene tables: the graph is its kernels alone
-      CU(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      r = batch_enqueue(b, st, false, true);
-      cudaGraph_t g = nullptr;
-      cudaError_t e = cudaStreamEndCapture(st, &g);
-      if (r != PIKO_OK) { if (g) cudaGraphDestroy(g); return r; }
-      CU(ctx, e);
-      b->graph = g;
-      CU(ctx, cudaGraphInstantiate(&b->graph_exec, g, 0));
-    }
-    CU(ctx, cudaGraphLaunch(b->graph_exec, st));
-  } else {
-    piko_status r = batch_enqueue(b, st, timed);
-    if (r != PIKO_OK) return r;
-  }
+  CU(ctx, b->order.before(st));
+  const piko_status r = batch_frame(b, st, use_graph != 0);
+  CU(ctx, b->order.after(st, ctx->stream));
+  if (r != PIKO_OK) return r;
   b->last_stream = st;
   b->pending = true;
   return PIKO_OK;
@@ -759,6 +772,7 @@ piko_status piko_batch_destroy(piko_batch* b)
   if (!b) return PIKO_ERR_INVALID;
   if (b->last_stream) cudaStreamSynchronize(b->last_stream);
   drop_graph(b);
+  b->order.release();
   for (auto* g : b->groups) {
     if (g->stream) cudaStreamSynchronize(g->stream);
     g->scr.release();

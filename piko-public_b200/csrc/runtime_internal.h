@@ -105,6 +105,67 @@ inline void dfree(T*& p)
   p = nullptr;
 }
 
+// Is st recording a graph?  (What it is given then runs later, or never.)
+inline cudaError_t stream_capturing(cudaStream_t st, bool* capturing)
+{
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(st, &c);
+  *capturing = c != cudaStreamCaptureStatusNone;
+  return e;
+}
+
+// The frames of one scene or batch follow one another whichever streams they are
+// given: a frame leaves the working counters as the next one needs them, so two at
+// once would spoil them for every later frame too.  before() makes a frame's stream
+// wait for the frame before, after() marks where the frame ends.  The object's own
+// stream is marked only once another one is used (it lives as long as the object);
+// a caller's stream may be destroyed behind the frame, and its handle given to
+// another, so it is marked at once and told by its id.  Frames that a stream capture
+// records are left out: their order is the caller's.
+struct FrameOrder {
+  cudaEvent_t ev = nullptr;
+  unsigned long long id = 0;         // the last frame's stream
+  bool any = false;
+  cudaStream_t unmarked = nullptr;   // the object's own stream, if the last frame ran there
+
+  cudaError_t mark(cudaStream_t st)
+  {
+    cudaError_t e = ev ? cudaSuccess : cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (!e) e = cudaEventRecord(ev, st);
+    return e;
+  }
+  cudaError_t before(cudaStream_t st)
+  {
+    if (!any || st == unmarked) return cudaSuccess;
+    bool capturing = false;
+    unsigned long long now = 0;
+    cudaError_t e = stream_capturing(st, &capturing);
+    if (e || capturing) return e;
+    if ((e = cudaStreamGetId(st, &now)) || now == id) return e;
+    if (unmarked) {
+      if ((e = mark(unmarked))) return e;
+      unmarked = nullptr;
+    }
+    return cudaStreamWaitEvent(st, ev, 0);
+  }
+  cudaError_t after(cudaStream_t st, cudaStream_t own)
+  {
+    if (any && st == unmarked) return cudaSuccess;
+    bool capturing = false;
+    cudaError_t e = stream_capturing(st, &capturing);
+    if (e || capturing) return e;
+    if ((e = cudaStreamGetId(st, &id))) return e;
+    any = true;
+    unmarked = st == own ? st : nullptr;
+    return unmarked ? cudaSuccess : mark(st);
+  }
+  void release()
+  {
+    if (ev) cudaEventDestroy(ev);
+    *this = FrameOrder();
+  }
+};
+
 // Frame scratch shared by every scene drawn in one launch sequence.
 struct RasterScratch {
   TriSetup* setup = nullptr;
@@ -125,6 +186,7 @@ struct RasterScratch {
   FrameCounters* ctr = nullptr;
   FrameCounters* h_ctr = nullptr;  // pinned; the fragment kernel writes its bin part
   bool clean = false;              // tile_cnt and work are all zero (every frame leaves them so)
+  bool captured = false;           // a caller's capture holds a frame on them: cleared before every frame
   RasterSceneDev* d_scenes = nullptr;      // scene table of launch sequences over several scenes
   std::vector<RasterSceneDev> h_scenes;    // pageable: a copy from it has read it when the call returns
   RasterSceneDev* cap_scenes = nullptr;    // pinned: the source of a copy that a stream capture records
@@ -305,7 +367,7 @@ struct piko_scene {
   cudaStream_t last_stream = nullptr;
   bool pending = false;
   bool timed = false;
-  uint64_t list_total_seen = 0;
+  FrameOrder order;
   ReyesState* reyes = nullptr;
 };
 
@@ -348,8 +410,8 @@ struct piko_batch {
   cudaStream_t last_stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
-  cudaStream_t graph_stream = nullptr;
   bool pending = false;
+  FrameOrder order;
 };
 piko_status batch_make(piko_ctx* ctx, piko_scene* const* scenes, int n, const TuneCfg* cfgs, piko_batch** out);
 

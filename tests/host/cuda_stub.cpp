@@ -34,7 +34,7 @@ struct Stream {
   Clock clock;
   long seq = 0;
   Graph* capture = nullptr;
-  bool origin = false;
+  bool gone = false;
 };
 struct Event { Clock clock; Graph* capture = nullptr; };
 
@@ -53,9 +53,14 @@ thread_local struct { dim3 grid, block; size_t smem; cudaStream_t st; } pushed;
 int next_stream = 1;
 Stream legacy{0};
 
-Stream& at(cudaStream_t st) { return st ? *reinterpret_cast<Stream*>(st) : legacy; }
-
 void say(const std::string& s) { log_text += s + "\n"; }
+
+Stream& at(cudaStream_t st)
+{
+  Stream& s = st ? *reinterpret_cast<Stream*>(st) : legacy;
+  if (s.gone) say("GONE stream " + std::to_string(s.id));
+  return s;
+}
 
 cudaError_t fail(cudaError_t e)
 {
@@ -133,6 +138,19 @@ int stub_log(char* out, int size)
   log_text.clear();
   return n;
 }
+void stub_destroy_stream(void* s) { cudaStreamDestroy(reinterpret_cast<cudaStream_t>(s)); }
+// A capture of what the caller enqueues on the stream; stub_end_capture gives a graph to launch.
+void stub_begin_capture(void* s) { cudaStreamBeginCapture(reinterpret_cast<cudaStream_t>(s), cudaStreamCaptureModeGlobal); }
+void* stub_end_capture(void* s)
+{
+  cudaGraph_t g;
+  cudaStreamEndCapture(reinterpret_cast<cudaStream_t>(s), &g);
+  return g;
+}
+void stub_replay(void* g, void* s)
+{
+  cudaGraphLaunch(reinterpret_cast<cudaGraphExec_t>(g), reinterpret_cast<cudaStream_t>(s));
+}
 void* stub_stream()
 {
   cudaStream_t s;
@@ -190,7 +208,18 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned)
   *s = reinterpret_cast<cudaStream_t>(n);
   return cudaSuccess;
 }
-cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }   // (kept: clocks refer to it)
+cudaError_t cudaStreamDestroy(cudaStream_t st)
+{
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  at(st).gone = true;   // (kept: clocks refer to it; what it was given goes on)
+  return cudaSuccess;
+}
+cudaError_t cudaStreamGetId(cudaStream_t st, unsigned long long* id)
+{
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  *id = (unsigned long long)at(st).id;
+  return cudaSuccess;
+}
 cudaError_t cudaStreamSynchronize(cudaStream_t st)
 {
   std::lock_guard<std::recursive_mutex> lk(mu);

@@ -42,7 +42,10 @@ sys.path.insert(0, {root!r})
 import piko_loader
 pk = piko_loader.load()
 lib = pk.load_library({lib!r})
-lib.stub_stream.restype = ctypes.c_void_p
+lib.stub_stream.restype = lib.stub_end_capture.restype = ctypes.c_void_p
+for f in ["stub_destroy_stream", "stub_begin_capture", "stub_end_capture"]:
+    getattr(lib, f).argtypes = [ctypes.c_void_p]
+lib.stub_replay.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
 
 def log():
     b = ctypes.create_string_buffer(1 << 20)
