@@ -198,7 +198,8 @@ piko_status piko_frame_prepare(piko_scene* scene, const piko_const_state* state)
  * one scene follow one another whichever streams they are given.  Frames that the
  * caller captures into a graph are outside that order: a replay must not overlap
  * another frame of the same scene (both images, and the frame after them, would be
- * undefined). */
+ * undefined).  A replay of a raster frame draws with the camera and light that the
+ * scene's last run or capture had; a Reyes frame keeps those of its capture. */
 piko_status piko_frame_run(piko_scene* scene, void* stream);
 /* Waits for the scene's last frame and checks its status; a bin-queue
  * overflow grows the queues and re-renders the frame before returning OK. */
@@ -239,7 +240,10 @@ piko_status piko_frame_coverage(piko_scene* scene, uint32_t* tri, uint32_t* pix,
  * no reference counterpart (the reference renders one scene per run_single). */
 piko_status piko_batch_create(piko_ctx* ctx, piko_scene* const* scenes, int n, piko_batch** out);
 /* Enqueues one frame of every scene of the batch; use_graph=1 records the launch
- * sequence as a CUDA graph on first use and replays it afterwards.  The frames of
+ * sequence as a CUDA graph on first use and replays it afterwards.  A replay draws
+ * every scene with the camera and light of the batch's last run without the graph
+ * (or of its first use, or of a re-render after an overflow, if that was later):
+ * after piko_frame_prepare, run once with use_graph=0.  The frames of
  * one batch follow one another whichever streams they are given (NULL: the
  * context's own). */
 piko_status piko_batch_run(piko_batch* batch, void* stream, int use_graph);

@@ -269,7 +269,7 @@ inline SetupShape setup_shape(uint32_t n, uint32_t wave, uint32_t threads)
 
 struct RasterFrameArgs {
   RasterSceneDev one;       // the scene of a one-scene frame: it travels with the launch, no copy precedes the frame
-  const RasterSceneDev* scenes;  // [n_scenes] when there are several
+  const RasterSceneDev* scenes;  // [n_scenes] when there are several (or a capture holds one); else null
   int n_scenes;
   int tile;                 // tile edge in pixels: 8, 16 or 32
   uint32_t n_tris_total;    // sum of N

@@ -1906,7 +1906,7 @@ cudaError_t launch_raster_frame(const RasterFrameArgs& args, int raster_ctas, cu
 {
   RasterFrameArgs a = args;
   static std::atomic<int> setup_wave[2] = {{0}, {0}}, scatter_wave{0}, large_wave{0};
-  const bool one = a.n_scenes == 1;
+  const bool one = !a.scenes;
   const auto setup = one ? raster_setup<true> : raster_setup<false>;
   const int threads = one ? kSetupThreads<true> : kSetupThreads<false>;
   const size_t setup_smem = one ? sizeof(SetupSmem<kSetupThreads<true>>)

@@ -90,24 +90,32 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   if (capturing && !table_ready) scr.captured = true;
   RasterFrameArgs a;
   memset(&a, 0, sizeof(a));
-  if (n == 1) {
-    fill_scene_dev(draws[0], T, 0u, 0u, a.one);
-  } else if (!table_ready) {
+  // The kernels of one scene take its record as an argument, those of several read
+  // a table.  In a capture of the caller's one scene is read from a table too: a
+  // replay draws with the records of the last frame enqueued, whatever their number
+  // (an argument would stay as it was captured).
+  RasterSceneDev* const table = n > 1 ? scr.d_scenes : scr.one_scene;
+  if (!table_ready) {
+    scr.h_scenes.resize((size_t)n);
+    uint32_t tb = 0, rb = 0;
+    for (int i = 0; i < n; ++i) {
+      int tx, ty;
+      fill_scene_dev(draws[i], T, tb, rb, scr.h_scenes[i]);
+      tb += (uint32_t)tiles_for(draws[i].mesh->W, draws[i].mesh->H, T, &tx, &ty);
+      rb += (uint32_t)draws[i].mesh->N;
+    }
     // Frames may be queued faster than the device takes them: the source of a
     // copy is pageable memory, which the call has read when it returns, and
     // not a pinned buffer that the next frame would overwrite under the copy.
     // (A captured copy reads its source at every replay: memory of its own.)
-    scr.h_scenes.resize((size_t)n);
-    RasterSceneDev* src = capturing ? scr.cap_scenes : scr.h_scenes.data();
-    uint32_t tb = 0, rb = 0;
-    for (int i = 0; i < n; ++i) {
-      int tx, ty;
-      fill_scene_dev(draws[i], T, tb, rb, src[i]);
-      tb += (uint32_t)tiles_for(draws[i].mesh->W, draws[i].mesh->H, T, &tx, &ty);
-      rb += (uint32_t)draws[i].mesh->N;
-    }
-    CU(ctx, cudaMemcpyAsync(scr.d_scenes, src, sizeof(RasterSceneDev) * n, cudaMemcpyHostToDevice, st));
+    RasterSceneDev* const cap = n > 1 ? scr.cap_scenes : scr.cap_one;
+    if (scr.captured) memcpy((void*)cap, scr.h_scenes.data(), sizeof(RasterSceneDev) * n);
+    if (n > 1 || capturing)
+      CU(ctx, cudaMemcpyAsync(table, capturing ? cap : scr.h_scenes.data(), sizeof(RasterSceneDev) * n,
+                              cudaMemcpyHostToDevice, st));
   }
+  if (n > 1 || (capturing && !table_ready)) a.scenes = table;
+  else a.one = scr.h_scenes[0];
   if (!scr.clean || scr.captured) {
     // fresh counters, a frame whose launches failed part way (memsets that a
     // capture records have not run yet), or replays that nothing orders
@@ -115,7 +123,6 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
     CU(ctx, cudaMemsetAsync(scr.tile_cnt, 0, sizeof(uint32_t) * scr.tiles_cap, st));
     scr.clean = !capturing;
   }
-  a.scenes = scr.d_scenes;
   a.n_scenes = n;
   a.tile = T;
   a.n_tris_total = tris;
@@ -659,7 +666,7 @@ piko_status batch_make(piko_ctx* ctx, piko_scene* const* scenes, int n, const Tu
 // Enqueues every group: group 0 on st, the others on their own streams forked
 // from st and joined back into it (parallel branches when captured; joined after a
 // failure too: what was enqueued is then in st's order).
-// table_ready: the groups' scene tables already hold the scenes as they are now.
+// table_ready: the groups' scene records are those of the last run.
 static piko_status batch_enqueue(piko_batch* b, cudaStream_t st, bool timed, bool table_ready = false)
 {
   piko_ctx* ctx = b->ctx;
@@ -703,6 +710,34 @@ static void drop_graph(piko_batch* b)
   b->graph = nullptr;
 }
 
+// Records the batch's launches, kernels alone: the frame before it filled the scene
+// tables.  A group of one scene has its record in the graph.
+static piko_status record_graph(piko_batch* b, cudaStream_t st)
+{
+  piko_ctx* ctx = b->ctx;
+  drop_graph(b);
+  CU(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+  const piko_status r = batch_enqueue(b, st, false, true);
+  cudaGraph_t g = nullptr;
+  const cudaError_t e = cudaStreamEndCapture(st, &g);
+  if (r != PIKO_OK) { if (g) cudaGraphDestroy(g); return r; }
+  CU(ctx, e);
+  b->graph = g;
+  CU(ctx, cudaGraphInstantiate(&b->graph_exec, g, 0));
+  for (auto* x : b->groups)
+    if (x->scenes.size() == 1) memcpy((void*)&x->recorded, x->scr.h_scenes.data(), sizeof(RasterSceneDev));
+  return PIKO_OK;
+}
+
+// Did a run without the graph draw a one-scene group with another record (camera)
+// than the graph has?  (The tables of larger groups hold the last run's.)
+static bool graph_behind(const piko_batch* b)
+{
+  for (auto* g : b->groups)
+    if (g->scenes.size() == 1 && memcmp(&g->recorded, g->scr.h_scenes.data(), sizeof(RasterSceneDev)) != 0) return true;
+  return false;
+}
+
 static piko_status batch_frame(piko_batch* b, cudaStream_t st, bool use_graph)
 {
   piko_ctx* ctx = b->ctx;
@@ -713,15 +748,11 @@ static piko_status batch_frame(piko_batch* b, cudaStream_t st, bool use_graph)
     piko_status r = batch_enqueue(b, st, false);
     if (r != PIKO_OK) return r;
     CU(ctx, cudaStreamSynchronize(st));
-    // the frame just drawn filled the scene tables: the graph is its kernels alone
-    CU(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    r = batch_enqueue(b, st, false, true);
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(st, &g);
-    if (r != PIKO_OK) { if (g) cudaGraphDestroy(g); return r; }
-    CU(ctx, e);
-    b->graph = g;
-    CU(ctx, cudaGraphInstantiate(&b->graph_exec, g, 0));
+    r = record_graph(b, st);
+    if (r != PIKO_OK) return r;
+  } else if (graph_behind(b)) {
+    const piko_status r = record_graph(b, st);
+    if (r != PIKO_OK) return r;
   }
   CU(ctx, cudaGraphLaunch(b->graph_exec, st));
   return PIKO_OK;

@@ -166,6 +166,13 @@ struct FrameOrder {
   }
 };
 
+// A launch sequence's counters, and a scene record: the table of a captured frame of
+// one scene.
+struct CounterBlock {
+  FrameCounters ctr;
+  RasterSceneDev one;
+};
+
 // Frame scratch shared by every scene drawn in one launch sequence.
 struct RasterScratch {
   TriSetup* setup = nullptr;
@@ -188,8 +195,10 @@ struct RasterScratch {
   bool clean = false;              // tile_cnt and work are all zero (every frame leaves them so)
   bool captured = false;           // a caller's capture holds a frame on them: cleared before every frame
   RasterSceneDev* d_scenes = nullptr;      // scene table of launch sequences over several scenes
-  std::vector<RasterSceneDev> h_scenes;    // pageable: a copy from it has read it when the call returns
+  RasterSceneDev* one_scene = nullptr;     // that of a caller's captured frame of one scene (beside ctr)
+  std::vector<RasterSceneDev> h_scenes;    // the last frame's records; pageable: a copy from it has read it when the call returns
   RasterSceneDev* cap_scenes = nullptr;    // pinned: the source of a copy that a stream capture records
+  RasterSceneDev* cap_one = nullptr;       // the same for one scene (beside h_ctr)
   uint32_t tris_cap = 0, tiles_cap = 0, list_cap = 0;
   int scenes_cap = 0;
   uint32_t cov_cap = 0;
@@ -203,10 +212,10 @@ struct RasterScratch {
     dfree(setup); dfree(tile_cnt); dfree(tile_span); dfree(tile_list); dfree(pair_tl); dfree(pair_g);
     dfree(large_seg); dfree(large_walk); dfree(hdone); dfree(chunk_keys);
     dfree(chunk_desc);
-    dfree(work); dfree(ctr); dfree(d_scenes); dfree(cov_tri); dfree(cov_pix);
+    dfree(work); dfree(ctr); dfree(d_scenes); dfree(cov_tri); dfree(cov_pix);   // (ctr begins its CounterBlock)
     if (h_ctr) cudaFreeHost(h_ctr);
     if (cap_scenes) cudaFreeHost(cap_scenes);
-    h_ctr = nullptr; cap_scenes = nullptr;
+    h_ctr = nullptr; cap_scenes = nullptr; one_scene = nullptr; cap_one = nullptr;
     clean = false;
     if (ev_made) for (auto& e : ev) cudaEventDestroy(e);
     ev_made = false;
@@ -324,8 +333,18 @@ struct RasterScratch {
       clean = false;
       if ((e = dalloc(&work, 1))) return e;
     }
-    if (!ctr && (e = dalloc(&ctr, 1))) return e;
-    if (!h_ctr && (e = halloc(&h_ctr, 1))) return e;
+    if (!ctr) {
+      CounterBlock* p;
+      if ((e = dalloc(&p, 1))) return e;
+      ctr = &p->ctr;
+      one_scene = &p->one;
+    }
+    if (!h_ctr) {
+      CounterBlock* p;
+      if ((e = halloc(&p, 1))) return e;
+      h_ctr = &p->ctr;
+      cap_one = &p->one;
+    }
     if (n_scenes > 1 && n_scenes > scenes_cap) {
       dfree(d_scenes);
       if (cap_scenes) cudaFreeHost(cap_scenes);
@@ -398,6 +417,7 @@ struct BatchGroup {
   TuneCfg cfg;
   std::vector<piko_scene*> scenes;
   RasterScratch scr;
+  RasterSceneDev recorded;        // a single scene's record in the batch's graph
   cudaStream_t stream = nullptr;  // the branch (group 0 runs on the caller's stream)
   cudaEvent_t done = nullptr;
 };

@@ -33,7 +33,7 @@ StubLaunch stub_decode(const char* name, void** args)
   if (!strcmp(name, "raster_frag8") || !strcmp(name, "raster_bins"))
     l.cameras = [a] {
       std::vector<float> c;
-      for (int i = 0; i < a.n_scenes; ++i) c.push_back((a.n_scenes == 1 ? a.one : a.scenes[i]).vp[12]);
+      for (int i = 0; i < a.n_scenes; ++i) c.push_back((a.scenes ? a.scenes[i] : a.one).vp[12]);
       return c;
     };
   return l;
