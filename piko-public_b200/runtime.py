@@ -6,7 +6,7 @@ without a CUDA device raises :class:`PikoError`.
 """
 import ctypes
 import os
-import sys
+import weakref
 
 import numpy as np
 
@@ -297,6 +297,16 @@ def const_state(scene=None, view_proj=None, light_mode=0, light=(0.5773, 0.5773,
     return cs
 
 
+class _ImageHolder:
+    """What the array over one image of read(), and every view of it, keeps alive."""
+    __slots__ = ("__array_interface__", "__weakref__")
+
+
+def _give_back(free, memory):
+    if len(free) < 2:
+        free.append(memory)
+
+
 class Scene:
     """One scene: device-resident inputs, framebuffer and depth buffer."""
 
@@ -307,7 +317,7 @@ class Scene:
         desc, keep = scene_desc(scene, packed=packed)
         self.packed = packed
         self.W, self.H, self.N = desc.width, desc.height, desc.count
-        self._images = {np.uint32: [], np.float32: []}   # result arrays of read(), reused once the caller lets go
+        self._free = {np.uint32: [], np.float32: []}   # memory of read()'s images that nobody holds
         self.h = ctypes.c_void_p()
         self.ctx.check(lib.piko_scene_create(pipe.h, ctypes.byref(desc), ctypes.byref(self.h)), "piko_scene_create")
         if not isinstance(scene, dict):
@@ -333,19 +343,20 @@ class Scene:
         self.ctx.check(self.ctx.lib.piko_frame_finish(self.h), "piko_frame_finish")
 
     def _image(self, dtype):
-        """An array for one image that nobody else holds.  The pages of a fresh
-        one cost more than the copy into it (1 MB: 110 us against 27), so up to
-        two per image are kept, and one is handed out again when the caller has
-        let go of it and of every view of it."""
-        kept = self._images[dtype]
-        for a in kept:
-            if sys.getrefcount(a) == 3:   # the list's, the loop's and the call's reference
-                return a
-        a = np.empty((self.H, self.W), dtype)
-        if len(kept) == 2:
-            kept.pop(0)
-        kept.append(a)
-        return a
+        """An array for one image that nobody else holds.  The pages of fresh
+        memory cost more than the copy into it (1 MB: 110 us against 27), so up to
+        two images' memory is kept: it comes back when the caller has let go of
+        the array and of every view of it."""
+        free = self._free[dtype]
+        try:
+            memory = free.pop()
+        except IndexError:
+            a = np.empty((self.H, self.W), dtype)
+            memory = a, a.__array_interface__
+        holder = _ImageHolder()
+        holder.__array_interface__ = memory[1]
+        weakref.finalize(holder, _give_back, free, memory).atexit = False
+        return np.asarray(holder)
 
     def read(self, out_fb=None, out_depth=None):
         fb = self._image(np.uint32) if out_fb is None else out_fb
