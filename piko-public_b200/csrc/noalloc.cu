@@ -35,7 +35,7 @@ constexpr uint32_t kNaTile = 16;
 constexpr uint32_t kNaMaxTiles = 5120;          // 16x16 tiles of any W x H <= 2^20 pixels, sides <= 16384
 constexpr uint32_t kNaMaxList = 1u << 20;       // (triangle, tile) queue entries
 constexpr uint32_t kNaMaxSegs = 1u << 16;       // 128-tile segments of large triangles
-constexpr uint32_t kNaMaxBig = 1u << 13;        // large triangles (more than 32 tiles in their box)
+constexpr uint32_t kNaMaxBig = 1u << 13;        // large triangles (more than 256 tiles in their box)
 
 constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
@@ -126,6 +126,7 @@ extern "C" piko_status piko_raster_frame_noalloc(const float* d_xyz, const uint3
   a.pair_tl = reinterpret_cast<unsigned long long*>(base + kOffPairTl);
   a.pair_g = reinterpret_cast<uint32_t*>(base + kOffPairG);
   a.list_cap = kNaMaxList;
+  a.spill = 1;
   a.heavy = reinterpret_cast<uint32_t*>(base + kOffHeavy);
   a.heavy_cap = kNaMaxTiles;
   a.queue_min = kQueueMin;

@@ -280,6 +280,7 @@ struct RasterFrameArgs {
   uint2* tile_span;         // [n_tiles_total] first list entry, entries
   uint32_t* tile_list;      // [list_cap]
   uint32_t list_cap;
+  uint32_t spill;           // a full pair partition spills into the next ones (lists of a fixed size)
   uint32_t* heavy;          // [heavy_cap] heavy tiles, when there are no chunk buffers
   uint32_t heavy_cap;
   // one record per (triangle, tile) pair, written by the count passes: the

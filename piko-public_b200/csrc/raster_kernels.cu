@@ -213,6 +213,26 @@ __device__ __forceinline__ bool tile_may_cover(const WalkTri& w, int tx, int ty,
   return true;
 }
 
+// Writes the records of the warp's pairs (bits m) to slots from `slot` on of a
+// partition, those that lie in [base, part_cap) of it.
+template <int R>
+__device__ __forceinline__ void put_pairs(const RasterFrameArgs& a, const uint32_t (&key)[R], const uint32_t (&gidx)[R],
+                                          const uint32_t (&local)[R], const unsigned (&m)[R], uint32_t part,
+                                          uint32_t part_cap, uint32_t base, uint32_t slot, int lane)
+{
+  const unsigned lt = (1u << lane) - 1u;
+  const size_t at = (size_t)part * part_cap;
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const uint32_t mine = slot + (uint32_t)__popc(m[q] & lt);
+    if (key[q] != 0xffffffffu && mine >= base && mine < part_cap) {
+      a.pair_tl[at + mine] = (unsigned long long)key[q] | ((unsigned long long)local[q] << 32);
+      a.pair_g[at + mine] = gidx[q];
+    }
+    slot += (uint32_t)__popc(m[q]);
+  }
+}
+
 // Counts the pairs of R rounds held by the warp's lanes (key = global tile, or
 // ~0 for none): one atomicAdd per pair on its tile's counter (per group of
 // lanes with the same tile at 16/32-px tiles), whose old value gives the
@@ -259,27 +279,27 @@ __device__ __forceinline__ void count_pairs(const RasterFrameArgs& a, const uint
   const uint32_t part = (blockIdx.x + (threadIdx.x >> 5) * (kPairParts / 8)) & (kPairParts - 1u);
   const uint32_t part_cap = a.list_cap / kPairParts;
   uint32_t base = 0;
-  if (lane == 0) {
-    base = atomicAdd(&a.work->pair_part[part], n);
-    if (base + n > part_cap) {
-      // the host grows the lists so that every partition fits, and draws again
-      atomicMax(&a.work->bin.pair_part_max, base + n);
-      atomicOr(&a.work->bin.status, kStatusListOverflow);
+  if (lane == 0) base = atomicAdd(&a.work->pair_part[part], n);
+  base = __shfl_sync(kFull, base, 0);
+  put_pairs<R>(a, key, gidx, local, m, part, part_cap, base, base, lane);
+  if (base + n <= part_cap) return;
+  // The partition is full.  Lists that grow: the host grows them so that every
+  // partition fits, and draws again.  Fixed ones: the rest goes to the next
+  // partitions, which fills all of them before a pair is dropped.
+  uint32_t done = part_cap - min(base, part_cap), p = part;   // pairs that have their records
+  if (a.spill) {
+#pragma unroll 1
+    for (uint32_t k = 1; k < kPairParts && done < n; ++k) {
+      p = (p + 1u) & (kPairParts - 1u);
+      if (lane == 0) base = atomicAdd(&a.work->pair_part[p], n - done);
+      base = __shfl_sync(kFull, base, 0);
+      put_pairs<R>(a, key, gidx, local, m, p, part_cap, base, base - done, lane);
+      done += min(part_cap - min(base, part_cap), n - done);
     }
   }
-  base = __shfl_sync(kFull, base, 0);
-  const unsigned lt = (1u << lane) - 1u;
-  const size_t at = (size_t)part * part_cap;
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    if (key[q] != 0xffffffffu) {
-      const uint32_t slot = base + (uint32_t)__popc(m[q] & lt);
-      if (slot < part_cap) {
-        a.pair_tl[at + slot] = (unsigned long long)key[q] | ((unsigned long long)local[q] << 32);
-        a.pair_g[at + slot] = gidx[q];
-      }
-    }
-    base += (uint32_t)__popc(m[q]);
+  if (lane == 0 && done < n) {
+    atomicMax(&a.work->bin.pair_part_max, base + n);
+    atomicOr(&a.work->bin.status, kStatusListOverflow);
   }
 }
 
@@ -555,8 +575,10 @@ __device__ __forceinline__ uint32_t block_scan_incl(uint32_t v, uint32_t* s_warp
   return v;
 }
 
+// (1024 threads an SM: 64 registers)
 template <bool ONE>
-__global__ void __launch_bounds__(kSetupThreads<ONE>) raster_setup(const __grid_constant__ RasterFrameArgs a)
+__global__ void __launch_bounds__(kSetupThreads<ONE>, 1024 / kSetupThreads<ONE>)
+raster_setup(const __grid_constant__ RasterFrameArgs a)
 {
   pdl_trigger();
   extern __shared__ __align__(16) unsigned char setup_smem[];

@@ -35,4 +35,3 @@ def test_held_images(host):
     print("done")
     """)
     assert out == "done\n"
-
