@@ -41,6 +41,7 @@
 // order -- (Dice bin, split level, position in the level, grid index) -- so
 // the kernels may visit fragments in any order.
 #include <mutex>
+#include <type_traits>
 
 #include "runtime_internal.h"
 
@@ -1684,6 +1685,8 @@ using namespace piko;
 // while every scene keeps its own counters for its overflow checks.
 struct ReyesState {
   ReyesState* buffers = nullptr;  // borrowed work buffers (not owned), or null
+  unsigned char* block = nullptr; // the buffers as first allocated; one that grew has memory of its own
+  size_t block_bytes = 0;
   PatchRec* lvl[2] = {nullptr, nullptr};
   PatchRec* stack = nullptr;
   PatchRec* leaves = nullptr;
@@ -1703,12 +1706,21 @@ struct ReyesState {
   bool captured = false;            // a caller's capture holds a frame: the counters are cleared before every frame
   cudaEvent_t ev[5] = {};
   bool ev_made = false;
+
+  template <class T>
+  void drop(T*& p)
+  {
+    const unsigned char* q = reinterpret_cast<const unsigned char*>(p);
+    if (q >= block && q < block + block_bytes) p = nullptr;
+    else dfree(p);
+  }
 };
 
 static void reyes_state_free(ReyesState* r)
 {
-  dfree(r->lvl[0]); dfree(r->lvl[1]); dfree(r->stack); dfree(r->leaves); dfree(r->up);
-  dfree(r->id_color); dfree(r->id_key); dfree(r->ties); dfree(r->samp); dfree(r->first0); dfree(r->ctr);
+  r->drop(r->lvl[0]); r->drop(r->lvl[1]); r->drop(r->stack); r->drop(r->leaves); r->drop(r->up);
+  r->drop(r->id_color); r->drop(r->id_key); r->drop(r->ties); r->drop(r->samp); r->drop(r->first0); r->drop(r->ctr);
+  dfree(r->block);
   if (r->h_ctr) cudaFreeHost(r->h_ctr);
   if (r->ev_made) for (auto& e : r->ev) cudaEventDestroy(e);
   delete r;
@@ -1734,48 +1746,88 @@ void reyes_borrow_buffers(piko_scene* s, ReyesState* b)
 
 constexpr uint32_t kMaxSparse = 1u << 24;
 
-static cudaError_t reyes_alloc(ReyesState* r, uint32_t lvl_cap, uint32_t leaf_cap, uint32_t up_cap, uint32_t id_cap,
-                               uint32_t tie_cap, size_t npx)
+// A state's first buffers, by one allocation: one takes 0.2 to 0.35 ms, whatever its
+// size, a frame a tenth of a millisecond (fresh 320x240 sphere: first frame with
+// fourteen allocations 5.1 ms, with one 3.0).  The split's stacks share their memory
+// with the tables that only later kernels of a frame use (device memory of that
+// sphere 122 -> 103 MB).
+static cudaError_t reyes_block(ReyesState* r, int sms, uint32_t lvl_cap, uint32_t leaf_cap, uint32_t up_cap,
+                               uint32_t id_cap, uint32_t tie_cap, size_t npx)
+{
+  size_t end = 0;
+  const auto place = [&end](size_t bytes) {
+    const size_t at = end;
+    end += (bytes + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t lvl0 = place(sizeof(PatchRec) * lvl_cap), lvl1 = place(sizeof(PatchRec) * lvl_cap);
+  const size_t leaves = place(sizeof(PatchRec) * leaf_cap);
+  const size_t samp = place(sizeof(*r->samp) * npx), first0 = place(sizeof(*r->first0) * npx);
+  const size_t ctr = place(sizeof(ReyesCounters));
+  const size_t shared = place(sizeof(PatchRec) * (size_t)sms * kSplitStack), stack_end = end;
+  end = shared;
+  const size_t up = place(sizeof(UpolyRec) * up_cap);
+  const size_t id_color = place(sizeof(*r->id_color) * id_cap), id_key = place(sizeof(*r->id_key) * id_cap);
+  const size_t ties = place(sizeof(uint4) * tie_cap);
+  end = std::max(end, stack_end);
+  unsigned char* p;
+  if (const cudaError_t e = dalloc(&p, end)) return e;
+  r->block = p;
+  r->block_bytes = end;
+  const auto cut = [p](auto*& q, size_t at) { q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(p + at); };
+  cut(r->lvl[0], lvl0); cut(r->lvl[1], lvl1); cut(r->leaves, leaves);
+  cut(r->samp, samp); cut(r->first0, first0); cut(r->stack, shared);
+  cut(r->up, up); cut(r->id_color, id_color); cut(r->id_key, id_key); cut(r->ties, ties);
+  if (!r->ctr) cut(r->ctr, ctr);
+  r->lvl_cap = lvl_cap; r->leaf_cap = leaf_cap; r->up_cap = up_cap;
+  r->id_cap = id_cap; r->tie_cap = tie_cap; r->npx_cap = npx;
+  r->clean = r->ctr_clean = false;
+  return cudaSuccess;
+}
+
+static cudaError_t reyes_alloc(ReyesState* r, int sms, uint32_t lvl_cap, uint32_t leaf_cap, uint32_t up_cap,
+                               uint32_t id_cap, uint32_t tie_cap, size_t npx)
 {
   cudaError_t e = cudaSuccess;
   if (r->buffers) {
-    if ((e = reyes_alloc(r->buffers, lvl_cap, leaf_cap, up_cap, id_cap, tie_cap, npx))) return e;
+    if ((e = reyes_alloc(r->buffers, sms, lvl_cap, leaf_cap, up_cap, id_cap, tie_cap, npx))) return e;
     lvl_cap = leaf_cap = up_cap = id_cap = tie_cap = 0;
     npx = 0;
   }
+  if (!r->block && lvl_cap && (e = reyes_block(r, sms, lvl_cap, leaf_cap, up_cap, id_cap, tie_cap, npx))) return e;
   // (a capacity stands only while all of its buffers do)
   if (lvl_cap > r->lvl_cap) {
-    dfree(r->lvl[0]); dfree(r->lvl[1]);
+    r->drop(r->lvl[0]); r->drop(r->lvl[1]);
     r->lvl_cap = 0;
     if ((e = dalloc(&r->lvl[0], lvl_cap)) || (e = dalloc(&r->lvl[1], lvl_cap))) return e;
     r->lvl_cap = lvl_cap;
   }
   if (leaf_cap > r->leaf_cap) {
-    dfree(r->leaves);
+    r->drop(r->leaves);
     r->leaf_cap = 0;
     if ((e = dalloc(&r->leaves, leaf_cap))) return e;
     r->leaf_cap = leaf_cap;
   }
   if (up_cap > r->up_cap) {
-    dfree(r->up);
+    r->drop(r->up);
     r->up_cap = 0;
     if ((e = dalloc(&r->up, up_cap))) return e;
     r->up_cap = up_cap;
   }
   if (id_cap > r->id_cap) {
-    dfree(r->id_color); dfree(r->id_key);
+    r->drop(r->id_color); r->drop(r->id_key);
     r->id_cap = 0;
     if ((e = dalloc(&r->id_color, id_cap)) || (e = dalloc(&r->id_key, id_cap))) return e;
     r->id_cap = id_cap;
   }
   if (tie_cap > r->tie_cap) {
-    dfree(r->ties);
+    r->drop(r->ties);
     r->tie_cap = 0;
     if ((e = dalloc(&r->ties, tie_cap))) return e;
     r->tie_cap = tie_cap;
   }
   if (npx > r->npx_cap) {
-    dfree(r->samp); dfree(r->first0);
+    r->drop(r->samp); r->drop(r->first0);
     r->npx_cap = 0;
     r->clean = false;
     if ((e = dalloc(&r->samp, npx)) || (e = dalloc(&r->first0, npx))) return e;
@@ -1804,11 +1856,10 @@ piko_status piko_reyes_run(piko_scene* s, cudaStream_t st, bool timed)
   const uint32_t P = (uint32_t)s->N;
   const size_t npx = (size_t)s->W * (size_t)s->H;
   const size_t nsamp = npx * (size_t)p->samples_per_pixel;
-  CU(ctx, reyes_alloc(r, std::max<uint32_t>(1u << 16, 64u * P), std::max<uint32_t>(1u << 16, 64u * P),
+  CU(ctx, reyes_alloc(r, ctx->sms, std::max<uint32_t>(1u << 16, 64u * P), std::max<uint32_t>(1u << 16, 64u * P),
                       b->up_cap ? b->up_cap : (1u << 16),
                       b->id_cap ? b->id_cap : (uint32_t)std::max<size_t>(1u << 20, npx),
                       b->tie_cap ? b->tie_cap : (uint32_t)std::max<size_t>(1u << 18, nsamp / 8), nsamp));
-  if (!b->stack) CU(ctx, dalloc(&b->stack, (size_t)ctx->sms * kSplitStack));
   bool capturing = false;
   CU(ctx, stream_capturing(st, &capturing));
   if (capturing) r->captured = true;
@@ -1884,7 +1935,7 @@ piko_status piko_reyes_finish(piko_scene* s)
                                         : was_sparse ? ids : c.id_count;
     if (need_ids > ids) ids = more(need_ids);
     if (c.tie_count > ties) ties = more(c.tie_count);
-    CU(ctx, reyes_alloc(r, lvl, lf, up, ids, ties, b->npx_cap));
+    CU(ctx, reyes_alloc(r, ctx->sms, lvl, lf, up, ids, ties, b->npx_cap));
     piko_status rr = piko_reyes_run(s, s->last_stream, s->timed);
     if (rr != PIKO_OK) return rr;
   }

@@ -36,7 +36,7 @@ def test_frames(host):
             assert not [x for x in lines if "NULL" in x], (kind, k, [x for x in lines if "NULL" in x])
             if ok:
                 break
-        assert ok and failed >= 8, (kind, failed)
+        assert ok and failed >= (2 if kind == "reyes" else 8), (kind, failed)
     print("done")
     """)
     assert out == "done\n"
