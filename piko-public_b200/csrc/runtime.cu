@@ -522,19 +522,33 @@ piko_status piko_frame_read(piko_scene* s, uint32_t* rgba, float* depth)
   if (!s) return PIKO_ERR_INVALID;
   piko_ctx* ctx = s->pipe->ctx;
   const size_t n = (size_t)s->W * s->H;
-  auto copy_image = [&](cudaStream_t st) -> cudaError_t {
-    cudaError_t e = cudaSuccess;
-    if (rgba) e = cudaMemcpyAsync(rgba, s->fb, n * 4, cudaMemcpyDeviceToHost, st);
-    if (!e && depth) e = cudaMemcpyAsync(depth, s->depth, n * 4, cudaMemcpyDeviceToHost, st);
-    return e;
+  const auto copy_rgba = [&](cudaStream_t st) {
+    return rgba ? cudaMemcpyAsync(rgba, s->fb, n * 4, cudaMemcpyDeviceToHost, st) : cudaSuccess;
+  };
+  const auto copy_depth = [&](cudaStream_t st) {
+    return depth ? cudaMemcpyAsync(depth, s->depth, n * 4, cudaMemcpyDeviceToHost, st) : cudaSuccess;
   };
   if (s->pending && s->pipe->kind == kPipeRaster) {
     // one wait for the frame's counts and image together; a frame that
     // overflowed its queues is drawn again (finish) and copied again
     cudaStream_t st = s->last_stream;
-    CU(ctx, copy_image(st));
-    CU(ctx, cudaStreamSynchronize(st));
+    CU(ctx, copy_rgba(st));
+    // A copy to pageable memory has waited for the frame: the depth buffer, which may
+    // be memory that the caller goes on using after an error, is then copied only if
+    // the frame is good.
+    const cudaError_t over = cudaStreamQuery(st);
+    if (over == cudaErrorNotReady) {
+      cudaGetLastError();
+      CU(ctx, copy_depth(st));
+      CU(ctx, cudaStreamSynchronize(st));
+    } else {
+      CU(ctx, over);
+    }
     const piko_status r = check_counters(ctx, s->scr);
+    if (r == PIKO_OK && over == cudaSuccess) {
+      CU(ctx, copy_depth(st));
+      CU(ctx, cudaStreamSynchronize(st));
+    }
     if (r == PIKO_OK) {
       s->pending = false;
       return PIKO_OK;
@@ -547,7 +561,8 @@ piko_status piko_frame_read(piko_scene* s, uint32_t* rgba, float* depth)
   piko_status r = piko_frame_finish(s);
   if (r != PIKO_OK) return r;
   cudaStream_t st = s->last_stream ? s->last_stream : s->own_stream;
-  CU(ctx, copy_image(st));
+  CU(ctx, copy_rgba(st));
+  CU(ctx, copy_depth(st));
   CU(ctx, cudaStreamSynchronize(st));
   return PIKO_OK;
 }

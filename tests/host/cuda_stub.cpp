@@ -47,7 +47,7 @@ Clock host_clock;
 std::string log_text;
 std::map<const void*, std::pair<int, long>> last_use;  // working counters -> last launch on them
 std::map<const void*, void*> var_mem;
-int fail_skip = -1, fail_count = 0;
+int fail_skip = -1, fail_count = 0, overflows = 0;
 thread_local cudaError_t last_error = cudaSuccess;
 thread_local struct { dim3 grid, block; size_t smem; cudaStream_t st; } pushed;
 int next_stream = 1;
@@ -94,6 +94,7 @@ void run_launch(const std::string& name, const StubLaunch& l, int stream)
   for (float c : l.cameras()) { char b[32]; snprintf(b, sizeof(b), " %g", c); line += b; }
   say(line);
   if (l.null_argument) say("NULL argument of " + name);
+  if (name == "raster_frag8" || name == "raster_bins") l.counts(overflows > 0 && overflows-- > 0);
   for (const void* o : l.objects) {
     auto& u = last_use[o];
     if (u.second && s->clock[u.first] < u.second) say("RACE " + name + " stream " + std::to_string(stream));
@@ -129,6 +130,12 @@ void stub_fail_alloc(int skip, int count)
   std::lock_guard<std::recursive_mutex> lk(mu);
   fail_skip = skip;
   fail_count = count;
+}
+// The next n raster frames report that their lists overflowed.
+void stub_overflow(int n)
+{
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  overflows = n;
 }
 int stub_log(char* out, int size)
 {
@@ -227,6 +234,7 @@ cudaError_t cudaStreamSynchronize(cudaStream_t st)
   merge(host_clock, at(st).clock);
   return cudaSuccess;
 }
+cudaError_t cudaStreamQuery(cudaStream_t st) { return cudaStreamSynchronize(st); }
 cudaError_t cudaStreamWaitEvent(cudaStream_t st, cudaEvent_t ev, unsigned)
 {
   std::lock_guard<std::recursive_mutex> lk(mu);

@@ -7,6 +7,7 @@
 struct StubLaunch {
   std::vector<const void*> objects;                // working counters that the launch changes
   bool null_argument = false;                      // a buffer that the kernel uses is null
+  std::function<void(bool)> counts = [](bool) {};  // leaves the frame's counts on the host: an overflow, or none
   std::function<std::vector<float>()> cameras = [] { return std::vector<float>(); };   // view_proj[12] of the scenes drawn
 };
 

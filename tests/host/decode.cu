@@ -30,12 +30,18 @@ StubLaunch stub_decode(const char* name, void** args)
   l.null_argument = !a.setup || !a.tile_cnt || !a.tile_span || !a.tile_list || !a.pair_tl || !a.pair_g || !a.large_seg ||
                     !a.large_walk || !a.work || !a.ctr ||
                     (noalloc ? !a.heavy : !a.hdone || !a.chunk_keys || !a.host_bin) || (a.n_scenes > 1 && !a.scenes);
-  if (!strcmp(name, "raster_frag8") || !strcmp(name, "raster_bins"))
+  if (!strcmp(name, "raster_frag8") || !strcmp(name, "raster_bins")) {
+    if (a.host_bin)
+      l.counts = [a](bool overflow) {
+        a.host_bin->status = overflow ? kStatusListOverflow : 0u;
+        a.host_bin->list_total = overflow ? a.list_cap + 1u : 0u;
+      };
     l.cameras = [a] {
       std::vector<float> c;
       for (int i = 0; i < a.n_scenes; ++i) c.push_back((a.scenes ? a.scenes[i] : a.one).vp[12]);
       return c;
     };
+  }
   return l;
 }
 
