@@ -6,7 +6,6 @@ without a CUDA device raises :class:`PikoError`.
 """
 import ctypes
 import os
-import weakref
 
 import numpy as np
 
@@ -298,13 +297,14 @@ def const_state(scene=None, view_proj=None, light_mode=0, light=(0.5773, 0.5773,
 
 
 class _ImageHolder:
-    """What the array over one image of read(), and every view of it, keeps alive."""
-    __slots__ = ("__array_interface__", "__weakref__")
+    """What the array over one image of read(), and every view of it, keeps alive;
+    it gives the memory back to those that nobody holds.  (By weakref.finalize: 3.4 us
+    an image instead of 1.6.)"""
+    __slots__ = ("__array_interface__", "_memory", "_free")
 
-
-def _give_back(free, memory):
-    if len(free) < 2:
-        free.append(memory)
+    def __del__(self):
+        if len(self._free) < 2:
+            self._free.append(self._memory)
 
 
 class Scene:
@@ -354,8 +354,8 @@ class Scene:
             a = np.empty((self.H, self.W), dtype)
             memory = a, a.__array_interface__
         holder = _ImageHolder()
+        holder._free, holder._memory = free, memory
         holder.__array_interface__ = memory[1]
-        weakref.finalize(holder, _give_back, free, memory).atexit = False
         return np.asarray(holder)
 
     def read(self, out_fb=None, out_depth=None):
