@@ -804,8 +804,14 @@ piko_status piko_batch_finish(piko_batch* b, piko_frame_stats* out)
       }
     }
     b->pending = false;
+    b->counted = out != nullptr;
   }
   if (out) {
+    // (a finish that was not asked for them left the fragment kernel's counts where they are)
+    for (auto* g : b->groups)
+      if (!b->counted && g->scr.h_ctr)
+        CU(ctx, cudaMemcpy(g->scr.h_ctr, g->scr.ctr, sizeof(FrameCounters), cudaMemcpyDeviceToHost));
+    b->counted = true;
     for (auto* s : b->scenes) out->prims_in += (uint64_t)s->N;
     for (auto* g : b->groups)
       if (g->scr.h_ctr) fill_stats(g->scr, ctx->time_kernels, out);

@@ -431,6 +431,7 @@ struct piko_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   bool pending = false;
+  bool counted = true;   // the groups' h_ctr hold all counts of the last finished frame
   FrameOrder order;
 };
 piko_status batch_make(piko_ctx* ctx, piko_scene* const* scenes, int n, const TuneCfg* cfgs, piko_batch** out);

@@ -35,6 +35,8 @@ StubLaunch stub_decode(const char* name, void** args)
       l.counts = [a](bool overflow) {
         a.host_bin->status = overflow ? kStatusListOverflow : 0u;
         a.host_bin->list_total = overflow ? a.list_cap + 1u : 0u;
+        static unsigned frames = 0;
+        a.ctr->covered = ++frames;
       };
     l.cameras = [a] {
       std::vector<float> c;
