@@ -259,6 +259,15 @@ __device__ __forceinline__ uint32_t barrier_wait(ReyesCounters* c, uint32_t k, u
   return *s_count;
 }
 
+// The patches of the split's next step, of `count` put on a frontier of `cap`.  A
+// frontier that overflowed has slots that no patch was written to: what lies there is
+// no patch, and splitting it might never end.  The split ends instead (every CTA has
+// the same count), and the host grows the buffers and runs the frame again.
+__host__ __device__ __forceinline__ uint32_t next_patches(uint32_t count, uint32_t cap)
+{
+  return count <= cap ? count : 0u;
+}
+
 // The per-sample state starts every frame empty: the buffers are set so when
 // allocated, and reyes_pixels, which visits every sample last, sets a reached
 // sample back.  The split clears nothing.
@@ -642,7 +651,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) reyes_split(ReyesArgs a)
     // read them, so the arrival need not wait for their stores.
     barrier_arrive(a.ctr, (uint32_t)step, &S.children);
     flush_leaves(a, S);
-    n_in = min(barrier_wait(a.ctr, (uint32_t)step, &S.word[1]), a.lvl_cap);
+    n_in = next_patches(barrier_wait(a.ctr, (uint32_t)step, &S.word[1]), a.lvl_cap);
   }
   if (threadIdx.x == 0 && a.P > 0) atomicMax(&a.ctr->levels_run, S.maxlevel + 1u);
 }
@@ -1922,7 +1931,12 @@ piko_status piko_reyes_finish(piko_scene* s)
     const uint32_t leaves = (uint32_t)(c.leaf_meta >> 40);
     const ReyesState* b = r->buffers ? r->buffers : r;
     uint32_t lvl = b->lvl_cap, lf = b->leaf_cap, up = b->up_cap, ids = b->id_cap, ties = b->tie_cap;
-    if (st & kStatusPatchOverflow) { lvl = std::max(lvl, maxlvl + maxlvl / 2 + 1024); lf = std::max(lf, 2 * leaves + 1024); }
+    if (st & kStatusPatchOverflow) {
+      // (the patches of a frontier that overflowed were not split: each has a leaf at least)
+      const uint32_t unsplit = maxlvl > lvl ? maxlvl : 0u;
+      lvl = std::max(lvl, maxlvl + maxlvl / 2 + 1024);
+      lf = std::max(lf, 2 * (leaves + unsplit) + 1024);
+    }
     if (st & kStatusUpolyOverflow) up = (uint32_t)std::min<unsigned long long>(c.big_count + c.big_count / 4ull + 4096, 0xffffffffull);
     const auto more = [](uint32_t n) {   // (an id of kNoId means none)
       return (uint32_t)std::min<unsigned long long>(n + n / 4ull + 4096, 0xfffffffeull);

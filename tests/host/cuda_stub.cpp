@@ -95,6 +95,7 @@ void run_launch(const std::string& name, const StubLaunch& l, int stream)
   say(line);
   if (l.null_argument) say("NULL argument of " + name);
   if (name == "raster_frag8" || name == "raster_bins") l.counts(overflows > 0 && overflows-- > 0);
+  if (name == "reyes_pixels") l.counts(false);
   for (const void* o : l.objects) {
     auto& u = last_use[o];
     if (u.second && s->clock[u.first] < u.second) say("RACE " + name + " stream " + std::to_string(stream));
@@ -136,6 +137,13 @@ void stub_overflow(int n)
 {
   std::lock_guard<std::recursive_mutex> lk(mu);
   overflows = n;
+}
+// The next Reyes frame reports so many patches on a frontier, leaves, and that one did not fit.
+void stub_patches(unsigned frontier, unsigned leaves)
+{
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  stub_frontier = frontier;
+  stub_leaves = leaves;
 }
 int stub_log(char* out, int size)
 {

@@ -4,6 +4,8 @@
 
 #include "cuda_stub.h"
 
+unsigned stub_frontier = 0, stub_leaves = 0;
+
 std::string stub_kernel_name(const char* mangled)
 {
   for (const char* n : {"raster_setup", "raster_large_count", "scan_tiles", "raster_scatter", "raster_frag8", "raster_bins",
@@ -21,6 +23,16 @@ StubLaunch stub_decode(const char* name, void** args)
     l.objects = {a.ctr, a.samp};
     l.null_argument = !a.in_patches || !a.lvl[0] || !a.lvl[1] || !a.stack || !a.leaves || !a.up || !a.id_color || !a.id_key ||
                       !a.ties || !a.ctr || !a.host_ctr || !a.fb || !a.depth || !a.samp || !a.first0;
+    if (!strcmp(name, "reyes_pixels"))
+      l.counts = [a](bool) {
+        ReyesCounters c = {};
+        if (stub_frontier || stub_leaves) c.fc.status = kStatusPatchOverflow;
+        c.level_count[1] = stub_frontier;
+        c.leaf_meta = (unsigned long long)stub_leaves << 40;
+        stub_frontier = stub_leaves = 0;
+        *a.host_ctr = c;
+      };
+    if (!strcmp(name, "reyes_split")) l.cameras = [a] { return std::vector<float>{(float)a.lvl_cap, (float)a.leaf_cap}; };
     if (!strcmp(name, "reyes_pixels")) l.cameras = [a] { return std::vector<float>{a.vp[12]}; };
     return l;
   }
@@ -46,6 +58,8 @@ StubLaunch stub_decode(const char* name, void** args)
   }
   return l;
 }
+
+extern "C" uint32_t stub_next_patches(uint32_t count, uint32_t cap) { return next_patches(count, cap); }
 
 extern "C" void stub_setup_shape(uint32_t n, uint32_t wave, uint32_t threads, uint32_t* batch, uint32_t* blocks)
 {
