@@ -42,9 +42,12 @@ namespace piko {
 
 constexpr unsigned kFull = 0xffffffffu;
 // Threads of a raster_setup CTA, for one scene and for several.  Smaller CTAs wait
-// less at the barriers between their steps (24-scene batch 378 -> 371 us with 128
-// instead of 256), but leave fewer kept triangles to fill each step where most
-// are culled (the packed 1277x715 forest alone: 57 -> 59 us).
+// less at the barriers between their steps, but leave fewer kept triangles to fill
+// each step.  Several scenes, 256 -> 128 threads: faster whatever share is kept (six
+// of 200,000 triangles, 10% kept 217 -> 215 us, half 745 -> 741, all 648 -> 637; six
+// forests, 23% kept, 181.1 -> 180.6).  One scene: 200,000 triangles, half kept, at
+// 1080p 134.0 -> 132.4 and the others within 0.5%, but the packed 1277x715 forest
+// with a wait for every frame 60.7 -> 61.5, which keeps it at 256.
 template <bool ONE>
 constexpr int kSetupThreads = ONE ? 256 : 128;
 constexpr uint32_t kLargeTiles = 256; // box tiles above which a triangle's walk is spread over the grid
@@ -109,22 +112,6 @@ template <bool ONE>
 __device__ __forceinline__ int scene_of_tile(const RasterFrameArgs& a, const uint32_t* tb, uint32_t tile)
 {
   return scene_of<ONE, kSceneTable>(a, tb, tile, true);
-}
-
-// The last index i in [0, n) with base[i] <= x, for an ascending base with
-// base[0] <= x; the whole warp searches, 32 probes per step.
-__device__ __forceinline__ uint32_t warp_search(const uint32_t* base, uint32_t n, uint32_t x, int lane)
-{
-  uint32_t lo = 0, hi = n;  // answer in [lo, hi)
-  while (hi - lo > 1) {
-    const uint32_t step = (hi - lo + 31) / 32;
-    const uint32_t probe = lo + (uint32_t)lane * step;
-    const bool ok = probe < hi && __ldg(&base[probe]) <= x;
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    lo += (uint32_t)(31 - __clz(m)) * step;
-    hi = min(hi, lo + step);
-  }
-  return lo;
 }
 
 // Rank of triangle `id` in the order the one-thread CPU backend submits
