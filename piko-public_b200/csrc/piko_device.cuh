@@ -300,7 +300,7 @@ struct RasterFrameArgs {
   // tile's chunks and resolves the tile.  Without chunk buffers (chunk_desc
   // null) heavy tiles are rasterized whole.
   uint32_t chunk;
-  uint32_t queue_min;       // 8x8 tiles with more entries than this are queued as chunks
+  uint32_t queue_min;       // tiles with more entries than this are queued as chunks
   uint32_t group;           // 8x8 tiles per short-list group (at most kLightGroup); 16/32-px tiles: 8x8 bins
                             // of a quad that a work item draws (1 or 4)
   ChunkDesc* chunk_desc;    // [chunk_cap]; the chunks of a tile are consecutive
