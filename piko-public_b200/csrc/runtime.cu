@@ -57,7 +57,7 @@ int raster_ctas(piko_ctx* ctx, int tile, int ctas_per_sm)
 
 // Enqueues one frame of draws [0, n) sharing one scratch.
 piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, RasterScratch& scr, int T, int ctas,
-                                 cudaStream_t st, bool timed, bool coverage, uint32_t chunk, bool table_ready)
+                                 cudaStream_t st, bool timed, bool coverage, uint32_t chunk, Records records)
 {
   if (chunk == 0) chunk = default_chunk(T);
   uint32_t tris = 0, tiles = 0;
@@ -86,8 +86,9 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   CU(ctx, scr.ensure_heavy(tiles, T, chunk, queue_min));
   bool capturing = false;
   CU(ctx, stream_capturing(st, &capturing));
-  // (a capture of the library's own finds the table ready: FrameOrder covers its replays)
-  if (capturing && !table_ready) scr.captured = true;
+  // (FrameOrder covers the replays of the library's own captures)
+  const bool callers = capturing && records != Records::graph;
+  if (callers) scr.captured = true;
   RasterFrameArgs a;
   memset(&a, 0, sizeof(a));
   // The kernels of one scene take its record as an argument, those of several read
@@ -95,7 +96,7 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
   // replay draws with the records of the last frame enqueued, whatever their number
   // (an argument would stay as it was captured).
   RasterSceneDev* const table = n > 1 ? scr.d_scenes : scr.one_scene;
-  if (!table_ready) {
+  if (records == Records::now) {
     scr.h_scenes.resize((size_t)n);
     uint32_t tb = 0, rb = 0;
     for (int i = 0; i < n; ++i) {
@@ -104,6 +105,8 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
       tb += (uint32_t)tiles_for(draws[i].mesh->W, draws[i].mesh->H, T, &tx, &ty);
       rb += (uint32_t)draws[i].mesh->N;
     }
+  }
+  if (records == Records::now || callers) {
     // Frames may be queued faster than the device takes them: the source of a
     // copy is pageable memory, which the call has read when it returns, and
     // not a pinned buffer that the next frame would overwrite under the copy.
@@ -114,7 +117,7 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
       CU(ctx, cudaMemcpyAsync(table, capturing ? cap : scr.h_scenes.data(), sizeof(RasterSceneDev) * n,
                               cudaMemcpyHostToDevice, st));
   }
-  if (n > 1 || (capturing && !table_ready)) a.scenes = table;
+  if (n > 1 || callers) a.scenes = table;
   else a.one = scr.h_scenes[0];
   if (!scr.clean || scr.captured) {
     // fresh counters, a frame whose launches failed part way (memsets that a
@@ -161,12 +164,12 @@ piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, 
 }
 
 piko_status enqueue_raster(piko_ctx* ctx, piko_scene* const* scenes, int n, RasterScratch& scr, const TuneCfg& cfg,
-                           cudaStream_t st, bool timed, bool coverage, bool table_ready)
+                           cudaStream_t st, bool timed, bool coverage, Records records)
 {
   std::vector<RasterDraw> draws((size_t)n);
   for (int i = 0; i < n; ++i) draws[i] = RasterDraw{scenes[i], &scenes[i]->state, scenes[i]->fb, scenes[i]->depth};
   return enqueue_raster_draws(ctx, draws.data(), n, scr, cfg.tile, raster_ctas(ctx, cfg.tile, cfg.ctas_per_sm), st, timed,
-                              coverage, cfg.chunk, table_ready);
+                              coverage, cfg.chunk, records);
 }
 
 namespace {
@@ -681,8 +684,7 @@ piko_status batch_make(piko_ctx* ctx, piko_scene* const* scenes, int n, const Tu
 // Enqueues every group: group 0 on st, the others on their own streams forked
 // from st and joined back into it (parallel branches when captured; joined after a
 // failure too: what was enqueued is then in st's order).
-// table_ready: the groups' scene records are those of the last run.
-static piko_status batch_enqueue(piko_batch* b, cudaStream_t st, bool timed, bool table_ready = false)
+static piko_status batch_enqueue(piko_batch* b, cudaStream_t st, bool timed, Records records = Records::now)
 {
   piko_ctx* ctx = b->ctx;
   const bool fork = b->groups.size() > 1;
@@ -693,7 +695,7 @@ static piko_status batch_enqueue(piko_batch* b, cudaStream_t st, bool timed, boo
     BatchGroup* g = b->groups[n];
     cudaStream_t gs = n == 0 ? st : g->stream;
     if (n > 0) CU(ctx, cudaStreamWaitEvent(gs, b->fork, 0));
-    r = enqueue_raster(ctx, g->scenes.data(), (int)g->scenes.size(), g->scr, g->cfg, gs, timed, false, table_ready);
+    r = enqueue_raster(ctx, g->scenes.data(), (int)g->scenes.size(), g->scr, g->cfg, gs, timed, false, records);
     if (n > 0) CU(ctx, cudaEventRecord(g->done, gs));
   }
   for (size_t k = 1; k < n; ++k) CU(ctx, cudaStreamWaitEvent(st, b->groups[k]->done, 0));
@@ -732,22 +734,27 @@ static piko_status record_graph(piko_batch* b, cudaStream_t st)
   piko_ctx* ctx = b->ctx;
   drop_graph(b);
   CU(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  const piko_status r = batch_enqueue(b, st, false, true);
+  const piko_status r = batch_enqueue(b, st, false, Records::graph);
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(st, &g);
   if (r != PIKO_OK) { if (g) cudaGraphDestroy(g); return r; }
   CU(ctx, e);
   b->graph = g;
   CU(ctx, cudaGraphInstantiate(&b->graph_exec, g, 0));
-  for (auto* x : b->groups)
+  for (auto* x : b->groups) {
+    x->recorded_clears = x->scr.captured;
     if (x->scenes.size() == 1) memcpy((void*)&x->recorded, x->scr.h_scenes.data(), sizeof(RasterSceneDev));
+  }
   return PIKO_OK;
 }
 
 // Did a run without the graph draw a one-scene group with another record (camera)
-// than the graph has?  (The tables of larger groups hold the last run's.)
+// than the graph has (the tables of larger groups hold the last run's), or was one
+// captured since, whose replays nothing orders?
 static bool graph_behind(const piko_batch* b)
 {
+  for (auto* g : b->groups)
+    if (g->scr.captured != g->recorded_clears) return true;
   for (auto* g : b->groups)
     if (g->scenes.size() == 1 && memcmp(&g->recorded, g->scr.h_scenes.data(), sizeof(RasterSceneDev)) != 0) return true;
   return false;
@@ -758,6 +765,10 @@ static piko_status batch_frame(piko_batch* b, cudaStream_t st, bool use_graph)
   piko_ctx* ctx = b->ctx;
   const bool timed = ctx->time_kernels;
   if (!use_graph || timed) return batch_enqueue(b, st, timed);
+  bool capturing = false;
+  CU(ctx, stream_capturing(st, &capturing));
+  // (in a capture of the caller's the launches, not the graph: they clear the counters and read the tables)
+  if (capturing && b->graph_exec) return batch_enqueue(b, st, false, Records::kept);
   if (!b->graph_exec) {
     // size the scratch outside the capture (allocation is not capturable)
     piko_status r = batch_enqueue(b, st, false);

@@ -418,6 +418,7 @@ struct BatchGroup {
   std::vector<piko_scene*> scenes;
   RasterScratch scr;
   RasterSceneDev recorded;        // a single scene's record in the batch's graph
+  bool recorded_clears = false;   // that graph clears the counters (scr.captured)
   cudaStream_t stream = nullptr;  // the branch (group 0 runs on the caller's stream)
   cudaEvent_t done = nullptr;
 };
@@ -460,11 +461,13 @@ struct RasterDraw {
 // chunks: 200K triangles at 1080p 206 -> 186 us, 24-scene batch 494 -> 457)
 inline uint32_t default_chunk(int tile) { return tile == 32 ? 128u : 64u; }
 constexpr uint32_t kQueueMin = 8;
-// table_ready: the scene table in scr already holds these draws
+// The scene records that a launch sequence draws with: the scenes' present state; the
+// last frame's (scr.h_scenes); or those in the batch's own graph.
+enum class Records { now, kept, graph };
 piko_status enqueue_raster_draws(piko_ctx* ctx, const RasterDraw* draws, int n, RasterScratch& scr, int T, int ctas,
                                  cudaStream_t st, bool timed, bool coverage, uint32_t chunk = 0,
-                                 bool table_ready = false);
+                                 Records records = Records::now);
 // One launch sequence over resident scenes drawn with their own camera states.
 piko_status enqueue_raster(piko_ctx* ctx, piko_scene* const* scenes, int n, RasterScratch& scr, const TuneCfg& cfg,
-                           cudaStream_t st, bool timed, bool coverage, bool table_ready = false);
+                           cudaStream_t st, bool timed, bool coverage, Records records = Records::now);
 int raster_ctas(piko_ctx* ctx, int tile, int ctas_per_sm);

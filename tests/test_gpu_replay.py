@@ -18,11 +18,11 @@ def moved(pk, sc, x):
 
 
 @pytest.mark.parametrize("tile", [8, 16])
-@pytest.mark.parametrize("form", ["scene", "batch1", "batch2", "batch1_capture"])
+@pytest.mark.parametrize("form", ["scene", "batch1", "batch2", "batch1_capture", "batch2_graph_capture"])
 def test_moved_camera(pk, ctx, tile, form):
     import torch
     scs = [pk.scenes.plain_scene(n=3000, W=333, H=250, seed=3), pk.scenes.plain_scene(n=500, W=200, H=200, seed=5)]
-    scs = scs[: 2 if form == "batch2" else 1]
+    scs = scs[: 2 if form.startswith("batch2") else 1]
     pipe = pk.Pipe(ctx, "raster", tile_px=tile)
     plain, scenes = [pk.Scene(pipe, sc) for sc in scs], [pk.Scene(pipe, sc) for sc in scs]
     batch = None if form == "scene" else pk.Batch(ctx, scenes)
@@ -53,11 +53,15 @@ def test_moved_camera(pk, ctx, tile, form):
 
         aim(0.0)
         run()
-        if form in ("scene", "batch1_capture"):
+        if form == "scene" or "capture" in form:
             st, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+            own = "graph" in form       # the batch has a graph of its own by then
+            if own:
+                batch.run(graph=True)
+                batch.finish()
             with torch.cuda.graph(g, stream=st):
                 if batch:
-                    batch.run(st.cuda_stream, graph=False)
+                    batch.run(st.cuda_stream, graph=own)
                 else:
                     scenes[0].run(st.cuda_stream)
 
@@ -78,7 +82,7 @@ def test_moved_camera(pk, ctx, tile, form):
             for _ in range(2):
                 replay()
                 check(x)
-        if form in ("scene", "batch1_capture"):
+        if form == "scene" or "capture" in form:
             del g
     finally:
         if batch:

@@ -50,25 +50,34 @@ print("done")
     assert out == "done\n"
 
 
-@pytest.mark.parametrize("n", [0, 1, 2])
-def test_callers_capture(host, n):
-    """n = 0: a scene's own frame; else a batch of n scenes, its launches captured."""
+@pytest.mark.parametrize("n,graph", [(0, False), (1, False), (2, False), (1, True), (2, True)])
+def test_callers_capture(host, n, graph):
+    """n = 0: a scene's own frame; else a batch of n scenes, its launches captured (graph:
+    the batch has a graph of its own, whose run is captured)."""
     out = host(MAKE + f"""
 scenes = [small(k) for k in range(max({n}, 1))]
 f = pk.Batch(ctx, scenes) if {n} else scenes[0]
-go = (lambda s=None: f.run(s, graph=False)) if {n} else f.run
+go = (lambda s=None, graph=False: f.run(s, graph=graph)) if {n} else f.run
 want = lambda x: [[x + i for i in range(len(scenes))]]
 aim(scenes, 10.0)
 go()
 f.finish()
 a = lib.stub_stream()
+if {graph}:
+    go(graph=True)
 aim(scenes, 20.0)
 lib.stub_begin_capture(a)
-go(a)
+if {graph}:
+    go(a, graph=True)
+else:
+    go(a)
 g = lib.stub_end_capture(a)
 log()
 lib.stub_replay(g, a)
-assert shown() == want(20.0)
+lines = log()
+assert "memset" in lines[0], lines                  # (a replay starts from cleared counters)
+got = [[float(c) for c in x.split()[4:]] for x in lines if x.startswith(("launch raster_frag8", "launch raster_bins"))]
+assert got == want(10.0 if {graph} else 20.0), got  # (a run of the graph takes no notice of prepare())
 for x in (30.0, 40.0):
     aim(scenes, x)
     go()
@@ -79,6 +88,12 @@ for x in (30.0, 40.0):
         lib.stub_replay(g, a)
         got = shown()
         assert got == want(x), (x, got)
+    if {graph}:
+        for _ in range(2):
+            go(graph=True)
+            lines = log()
+            assert "memset" in [y for y in lines if y.startswith(("memset", "launch"))][0], lines
+        f.finish()
 print("done")
 """)
     assert out == "done\n"
